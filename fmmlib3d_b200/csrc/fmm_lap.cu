@@ -21,6 +21,7 @@
 #include "hess.cuh"
 #include "tri.cuh"
 #include "m2l_dense.cuh"
+#include "m2l_fold.cuh"
 #include "tree.cuh"
 #include "driver_common.cuh"
 #include "tuning.cuh"
@@ -99,11 +100,13 @@ struct LapPlan {
     std::vector<Slot> hslots;
     int kt = 8;       // targets per tile of M2M / L2L
     int kt_m2l = 8;   // targets per tile of the rotate-shift-rotate M2L
-    // dense M2L operators (p <= kDenseMaxP): one per list-2 offset, and the
-    // operator offset of every M2L slot
+    // FP64 M2L operators folded over the reflections of the offsets (p <= kFoldMaxP)
+    bool folded = false;
+    FoldPlan fold;
+    // mixed form: dense M2L operators rounded to FP32 (p <= kDenseMaxP), one per
+    // list-2 offset, and the operator offset of every M2L slot
     bool dense = false;
-    DBuf<double2> T;
-    DBuf<float2> T32;        // the same operators rounded to FP32 (mixed form)
+    DBuf<float2> T32;
     DBuf<long long> slot_toff;
 };
 // Switches of the Laplace calls: a process-wide value (fmm3d_set_m2l_mode,
@@ -113,8 +116,8 @@ struct LapPlan {
 // thread (a serving worker) can set its own without touching other threads'
 // calls.
 enum Switch {
-    kSwM2LMode = 0,    // 0 automatic, 1 rotate-shift-rotate, 2 dense operators, 3 rotate-shift-rotate
-                       // on the CUDA cores (1 and 0 use the FP64 tensor cores up to order 28)
+    kSwM2LMode = 0,    // 0 automatic, 1 rotate-shift-rotate (on the FP64 tensor cores up to order 28),
+                       // 2 folded dense operators (up to order 26, as 0), 3 rotate-shift-rotate on the CUDA cores
     kSwPrecision = 1,  // 0 FP64 throughout, 1 mixed (FP32 P2P and M2L) for iprec <= 1
     kSwTensorM2L = 2,  // mixed-form M2L: 0 FP32 CUDA cores, 1/2 tensor cores (stage variants 0/1)
     kSwTcGroup = 3,    // tensor-core M2L: slots per TMEM sum (0: one sum per tile)
@@ -244,6 +247,20 @@ static std::shared_ptr<LapPlan> get_plan(int p, double eps, cudaStream_t s, Stat
     const int m2l_nbuf = NC <= 3 * 256 ? 2 : 3;
     P->kt_m2l = 8;
     while (P->kt_m2l > 1 && (size_t)m2l_nbuf * P->kt_m2l * NC * 16 > 200 * 1024) P->kt_m2l /= 2;
+    if (p <= kFoldMaxP) {
+        // the 56 offsets with no negative component: those of the octant-0 targets
+        FoldOffset off[kFoldClasses];
+        int n = 0;
+        for (int si = 0; si < 189; si++) {
+            const Slot &sl = P->hslots[si];
+            const int a = 2 * (sl.coll / 9 - 1) + (sl.oct & 1), b = 2 * ((sl.coll / 3) % 3 - 1) + (sl.oct >> 1 & 1);
+            const int c = 2 * (sl.coll % 3 - 1) + (sl.oct >> 2 & 1);
+            if (a < 0 || b < 0 || c < 0) continue;
+            off[n++] = {a, b, c, sl.pt, sl.cls, sl.ex, sl.ey, sl.rt};
+        }
+        P->folded = fold_build(P->fold, p, off, P->rot.p, P->dc.p, P->lddc, s, st);
+        if (!st.ok()) return nullptr;
+    }
     if (p <= kDenseMaxP) {
         // unique list-2 offsets and their operators
         std::map<int, int> uidx;
@@ -271,17 +288,17 @@ static std::shared_ptr<LapPlan> get_plan(int p, double eps, cudaStream_t s, Stat
             }
         }
         DBuf<M2LOp> dops;
-        if (dops.alloc(uops.size(), s, st) && P->T.alloc(tot, s, st) && P->slot_toff.alloc(stoff.size(), s, st)) {
+        DBuf<double2> T;
+        if (dops.alloc(uops.size(), s, st) && T.alloc(tot, s, st) && P->slot_toff.alloc(stoff.size(), s, st)) {
             FMM_TRY(st, cudaMemcpyAsync(dops.p, uops.data(), sizeof(M2LOp) * uops.size(), cudaMemcpyHostToDevice, s));
             FMM_TRY(st, cudaMemcpyAsync(P->slot_toff.p, stoff.data(), sizeof(long long) * stoff.size(),
                                         cudaMemcpyHostToDevice, s));
-            build_m2l_ops(p, (int)uops.size(), dops.p, P->rot.p, P->dc.p, P->lddc, P->T.p, s, st);
-            if (P->T32.alloc(tot, s, st)) convert_f32(tot, P->T.p, P->T32.p, s, st);
+            build_m2l_ops(p, (int)uops.size(), dops.p, P->rot.p, P->dc.p, P->lddc, T.p, s, st);
+            if (P->T32.alloc(tot, s, st)) convert_f32(tot, T.p, P->T32.p, s, st);
             FMM_TRY(st, cudaStreamSynchronize(s));
         }
         if (!st.ok()) return nullptr;
         P->dense = true;
-        P->T.s = nullptr;
         P->T32.s = nullptr;
         P->slot_toff.s = nullptr;
     }
@@ -351,6 +368,8 @@ struct LapSetup {
     int ifcharge = 0, ifdipole = 0, ifpot = 0, iffld = 0, ifpottarg = 0, iffldtarg = 0;
     int do_src = 0, do_trg = 0, prune = 0;
     bool mixed = false, dense = false, tcm2l = false;
+    bool fold = false;   // FP64 M2L by folded operators
+    FoldWork fw;
     std::shared_ptr<LapPlan> plan;
     Tree T;
     TreeView tv;
@@ -488,7 +507,7 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
     int m2l_kt = S.tcm2l ? kTcTileTargets : S.dense ? kDenseTileTargets : plan->kt_m2l;
     if (k.m2l_kt) {
         m2l_kt = k.m2l_kt;
-    } else if (S.dense && !(S.mixed && !S.tcm2l)) {
+    } else if (S.tcm2l) {
         const int rows = div_up(S.K, 64), want = 2 * device_sms();
         auto ntiles = [&](int kt) {
             long t = 0;
@@ -499,10 +518,10 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
         // (256-target tensor-core tiles run one CTA per SM and measured slower on every
         // workload tried; they are reached through the tuning knob only)
         while (m2l_kt > 16 && ntiles(m2l_kt) * rows < want) m2l_kt /= 2;
-        if (!S.tcm2l && m2l_kt < kDenseTileTargets) m2l_kt = 16;   // FP64 dense kernel: 64 or 16
     }
     const int m2l_a = ntile;
-    for (int l = 2; l <= T.nlev; l++) make_tiles(l, m2l_kt, 0, 189, 189);
+    // (the folded M2L takes runs of box ids; its tile is its own)
+    for (int l = 2; l <= T.nlev && !S.fold; l++) make_tiles(l, m2l_kt, 0, 189, 189);
     const int m2l_n = ntile - m2l_a;
     for (int l = 2; l <= T.nlev - 1; l++) {
         int a = ntile;
@@ -718,6 +737,12 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
     // triangles in the mixed form: the M2L runs on the tensor cores (split TF32), the exact
     // near field and every other pass stay FP64
     if (S.tri && form == 1 && iprec <= 1 && plan->dense && sw(kSwTensorM2L) > 0) S.dense = S.tcm2l = true;
+    const int m2l_mode = sw(kSwM2LMode);
+    S.fold = plan->folded && !S.mixed && !S.tcm2l && m2l_mode != 1 && m2l_mode != 3;
+    if (S.fold && T.nlev >= 2 && !fold_prepare(plan->fold, S.fw, T.nboxes, T.nboxes - T.lev_start[2], s, st)) {
+        g_ti.err = cudaGetErrorString(st.err);
+        return 16;
+    }
     // launch shapes: the autotuner's cached setting for this problem, else automatic
     S.signature = lap_signature(S);
     TuneKnobs kn;
@@ -855,9 +880,11 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     } else if (S.mixed)
         launch_m2l_dense32(S.dtiles.p + S.m2l_a, S.m2l_n, T.grouped.p, plan->slots.p, plan->slot_toff.p,
                            plan->T32.p, tv, p, S.mpole.p, S.local.p, prune, f, st);
-    else if (S.dense)
-        launch_m2l_dense(S.dtiles.p + S.m2l_a, S.m2l_n, T.grouped.p, plan->slots.p, plan->slot_toff.p, plan->T.p,
-                         tv, p, S.mpole.p, S.local.p, prune, S.m2l_kt, f, st);
+    else if (S.fold) {
+        if (T.nlev >= 2)
+            launch_m2l_fold(plan->fold, S.fw, tv, T.nboxes, T.lev_start[2], T.nboxes - T.lev_start[2], S.mpole.p,
+                            S.local.p, prune, f, st);
+    }
     else if (sw(kSwM2LMode) != 3 && S.m2l_kt <= 8 && m2l_rot_dmma_supported(p))
         launch_m2l_rot_dmma(S.dtiles.p + S.m2l_a, S.m2l_n, T.grouped.p, plan->slots.p, tv, p, plan->rot.p,
                             plan->dc.p, plan->lddc, S.mpole.p, S.local.p, prune, f, st);

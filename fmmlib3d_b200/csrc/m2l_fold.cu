@@ -1,0 +1,506 @@
+// M2L by dense operators folded over the reflections of the list-2 offsets.
+//
+// The translation of a list-2 offset D (l3dmplocquad2_trunc0,
+// src/l3dtrans.f:1260-1387, truncated to nterms_trunc = pt) is a linear map
+// T_D of the source coefficients.  Two symmetries make it cheap:
+//   - in the real basis A = (M_n^m + M_n^{-m}) / 2 (cosine part) and
+//     B = (M_n^m - M_n^{-m}) / 2i (sine part) T_D is a real matrix, and the
+//     real and imaginary parts of the strengths are two right-hand sides;
+//   - every real harmonic is even or odd under x -> -x, y -> -y and z -> -z.
+//     With the coefficients in 8 parity classes, a reflection g of D only
+//     changes signs, T_{gD}[a][b] = chi_a(g) chi_b(g) T_D[a][b], so the sources
+//     of a target at all reflections of D are added first,
+//       X[c][b] = sum_g chi_c(g) M_{gD}[b],
+//     and L[a] += sum_b T_D[a][b] X[a ^ b][b] once for all of them.
+// The 189 offsets of a target fall into 56 classes |D|; a zero component of D
+// leaves only the blocks with equal parity on that axis.  At order 14
+// that is 0.57 M multiply-adds per target against 7.95 M for one complex
+// operator per offset; at order 26 6.8 M against 7.6 M of rotate-shift-
+// rotate, all of them in matrix products.
+//
+// k_m2l_fold: a CTA owns 16 consecutive target boxes (32 columns: 16 targets x
+// 2 right-hand sides) and all their coefficients; warp w owns the rows of
+// parity class w (of half of it for high orders) in DMMA accumulators.  Per
+// batch all warps stage X (one 36-row slot per parity class: 83 KB; two CTAs
+// per SM fill each other's staging gaps up to order 14), then
+// each warp multiplies its operator fragments, read from L2 in the lane order
+// of the MMA and each used for all 32 columns, with its slot.  Offset classes
+// that no target of the tile has a source in are skipped.
+// The sums of a target are formed in 8 fixed groups of batches, added in
+// order; a small problem runs one CTA per (tile, group) and adds the groups
+// afterwards, with the same result bit for bit.
+#include <algorithm>
+
+#include "dmma.cuh"
+#include "m2l_fold.cuh"
+
+namespace fmm {
+
+constexpr int kFoldCap = 36;                    // operand rows per parity class and batch
+// Row stride of the operands of NT targets: = 4 mod 16 doubles, so that the 4 x 4
+// lanes of a half warp reading a fragment meet different banks.
+template <int NT>
+constexpr int kFoldLd = 2 * NT + 4;
+constexpr int kFoldSplitTiles = 296;            // fewer tiles than this: one CTA per group
+
+// ---------------------------------------------------------------- operators
+struct FoldBlock {
+    long long off;
+    int k4, rb, off_id, alpha, beta, na, nb, work0;
+};
+
+// T_D[(j, m)][(n, mc)] = e^{i (mc - m) phi} sum_k D^j[m][k] Z(j, k, n) D^n[mc][k],
+// Z(j, k, n) = (-1)^(j+k) sqrt(C(n+j, n-k) C(n+j, n+k)) / rt^(n+j+1).
+__device__ double2 fold_entry(const FoldOffset &o, const double *Rm, const double *dc, int lddc, int j, int m, int n,
+                              int mc)
+{
+    const double *Dn = Rm + (size_t)n * (4 * n * n - 1) / 3 + (size_t)(mc + n) * (2 * n + 1);
+    const double *Dj = Rm + (size_t)j * (4 * j * j - 1) / 3 + (size_t)(m + j) * (2 * j + 1);
+    const double ir = 1.0 / o.rt;
+    double pw = 1;
+    for (int i = 0; i < n + j + 1; i++) pw *= ir;
+    const int kmax = j < n ? j : n;
+    double s = 0;
+    for (int k = -kmax; k <= kmax; k++) {
+        const double z = (((j + k) & 1) ? -1.0 : 1.0) * pw * dc[(n + j) * lddc + (n - k)] * dc[(n + j) * lddc + (n + k)];
+        s += Dj[k + j] * z * Dn[k + n];
+    }
+    const int d = mc - m;
+    double2 e = cmk(1, 0);
+    for (int i = 0; i < (d < 0 ? -d : d); i++) e = cmul(e, cmk(o.ex, o.ey));
+    if (d < 0) e = cconj(e);
+    return cscal(s, e);
+}
+
+// One thread per fragment entry: blocks (offset class, row class, column
+// class) as K steps x row blocks x 32 lanes.
+__global__ void k_fold_ops(const FoldBlock *blocks, const FoldOffset *offs, const int4 *kmap, const int *base, int p,
+                           const double *rot, const double *dc, int lddc, double *A)
+{
+    const FoldBlock B = blocks[blockIdx.x];
+    const FoldOffset o = offs[B.off_id];
+    const double *Rm = rot + rot_class_size(p) * o.cls;
+    for (int e = threadIdx.x; e < B.k4 * B.rb * 32; e += blockDim.x) {
+        const int lane = e & 31, rb = (e >> 5) % B.rb, ks = (e >> 5) / B.rb;
+        const int row = rb * 8 + (lane >> 2), col = ks * 4 + (lane & 3);
+        double v = 0;
+        if (row < B.na && col < B.nb) {
+            const int4 r = kmap[base[B.alpha] + row], c = kmap[base[B.beta] + col];
+            int j = 0, n = 0;
+            while ((j + 1) * (j + 1) <= r.x) j++;
+            while ((n + 1) * (n + 1) <= c.x) n++;
+            const int m = r.x - j * j - j, mc = c.x - n * n - n;
+            const double2 t1 = fold_entry(o, Rm, dc, lddc, j, m, n, mc);
+            const double2 t2 = mc > 0 ? fold_entry(o, Rm, dc, lddc, j, m, n, -mc) : cmk(0, 0);
+            // the reality of the map, T[-m][-mc] = conj T[m][mc], gives the four parts
+            if (!r.z) v = c.z ? t2.y - t1.y : t1.x + t2.x;
+            else v = c.z ? t1.x - t2.x : t1.y + t2.y;
+        }
+        A[B.off + e] = v;
+    }
+}
+
+bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, const double *dc, int lddc,
+                cudaStream_t s, Status &st)
+{
+    F.p = p;
+    F.K = (p + 1) * (p + 1);
+    // parity classes: bit 0 odd in x, bit 1 odd in y (sine parts), bit 2 odd in z; by degree inside a class
+    std::vector<int4> kmap, rmap;
+    std::vector<int> base(16);
+    std::vector<std::vector<int>> cnt(8, std::vector<int>(p + 1, 0));   // coefficients of degree <= n
+    std::vector<int> kc((size_t)(p + 1) * (p + 1), -1), ksn((size_t)(p + 1) * (p + 1), -1);
+    for (int c = 0; c < 8; c++) {
+        base[c] = (int)kmap.size();
+        for (int n = 0; n <= p; n++) {
+            const int sine = (c >> 1) & 1;
+            for (int m = sine; m <= n; m++) {
+                if (((m + sine) & 1) != (c & 1) || ((n + m) & 1) != (c >> 2)) continue;
+                (sine ? ksn : kc)[n * (p + 1) + m] = (int)kmap.size();
+                kmap.push_back(make_int4(eidx(n, m), eidx(n, -m), sine, m));
+            }
+            cnt[c][n] = (int)kmap.size() - base[c];
+        }
+        base[8 + c] = cnt[c][p];
+        F.rows = std::max(F.rows, div_up(cnt[c][p], 8));
+    }
+    for (int n = 0; n <= p; n++)
+        for (int m = 0; m <= n; m++)
+            rmap.push_back(make_int4(eidx(n, m), eidx(n, -m), kc[n * (p + 1) + m], m ? ksn[n * (p + 1) + m] : -1));
+
+    // operator blocks and their fragments
+    std::vector<FoldBlock> blocks;
+    std::vector<long long> aoff((size_t)kFoldClasses * 64, -1);
+    std::vector<int4> cls;
+    long long tot = 0;
+    for (int q = 0; q < kFoldClasses; q++) {
+        const FoldOffset &o = off[q];
+        const int z = (o.a == 0) | (o.b == 0) << 1 | (o.c == 0) << 2;
+        cls.push_back(make_int4(o.a, o.b, o.c, 7 ^ z));
+        for (int al = 0; al < 8; al++)
+            for (int be = 0; be < 8; be++) {
+                const int na = cnt[al][o.pt], nb = cnt[be][o.pt];
+                if (((al ^ be) & z) || na == 0 || nb == 0) continue;
+                FoldBlock b;
+                b.off = tot; b.k4 = div_up(nb, 4); b.rb = div_up(na, 8); b.off_id = q;
+                b.alpha = al; b.beta = be; b.na = na; b.nb = nb; b.work0 = 0;
+                aoff[(size_t)q * 64 + al * 8 + be] = tot;
+                tot += (long long)b.k4 * b.rb * 32;
+                blocks.push_back(b);
+            }
+    }
+    // segments (offset class, round of column classes, K range) packed into batches
+    std::vector<FoldTask> tasks;
+    std::vector<FoldBatch> batches;
+    std::vector<int> seg_cls;
+    std::vector<int4> wseg;
+    std::vector<double> cost;
+    int fill[8] = {};
+    for (int q = 0; q < kFoldClasses; q++) {
+        const FoldOffset &o = off[q];
+        const int free_ = cls[q].w, z = 7 ^ free_;
+        int axis[3], bits = 0;
+        for (int i = 0; i < 3; i++)
+            if (free_ >> i & 1) axis[bits++] = i;
+        auto spread = [&](int j) {
+            int g = 0;
+            for (int i = 0; i < bits; i++) g |= (j >> i & 1) << axis[i];
+            return g;
+        };
+        int most = 0;
+        for (int c = 0; c < 8; c++) most = std::max(most, cnt[c][o.pt]);
+        for (int r = 0; r < 1 << bits; r++)
+            for (int k0 = 0; k0 < most; k0 += kFoldCap) {
+                const int rb = spread(r);
+                int depth[8];   // operand rows of row class al: column class (al & z) | rb
+                bool fits = true, any = false;
+                for (int al = 0; al < 8; al++) {
+                    const int nb = cnt[(al & z) | rb][o.pt] - k0, na = cnt[al][o.pt];
+                    depth[al] = nb > 0 && na > 0 ? 4 * div_up(std::min(nb, kFoldCap), 4) : 0;
+                    any |= depth[al] > 0;
+                    fits &= fill[al] + depth[al] <= kFoldCap;
+                }
+                if (!any) continue;
+                if (batches.empty() || !fits) {
+                    batches.push_back({(int)tasks.size(), 0, (int)seg_cls.size(), 0});
+                    cost.push_back(8.0);   // staging latency of a batch, in K steps of one row block
+                    std::fill(fill, fill + 8, 0);
+                }
+                double most_steps = 0;
+                for (int al = 0; al < 8; al++) {
+                    const int be = (al & z) | rb, nrb = div_up(cnt[al][o.pt], 8);
+                    wseg.push_back(depth[al] ? make_int4((int)(aoff[(size_t)q * 64 + al * 8 + be] / 32) + k0 / 4 * nrb,
+                                                         depth[al] / 4, nrb, fill[al])
+                                             : make_int4(0, 0, 0, 0));
+                    most_steps = std::max(most_steps, depth[al] / 4.0 * nrb);
+                }
+                // staging tasks: the round's column classes, 4 coefficients each
+                for (int be = 0; be < 8; be++) {
+                    if ((be & free_) != rb) continue;
+                    const int nb = std::min(cnt[be][o.pt] - k0, kFoldCap);
+                    for (int k = 0; k < nb; k += 4) {
+                        FoldTask t = {};
+                        t.src0 = base[be] + k0 + k;
+                        t.cls = (unsigned char)q; t.n = (unsigned char)std::min(4, nb - k);
+                        t.bits = (unsigned char)bits; t.beta = (unsigned char)be;
+                        for (int i = 0; i < bits; i++) t.axis[i] = (unsigned char)axis[i];
+                        bool used = false;
+                        for (int j = 0; j < 1 << bits; j++) {
+                            const int al = be ^ spread(j);
+                            t.row[j] = depth[al] ? (unsigned char)(fill[al] + k) : 255;
+                            used |= depth[al] > 0;
+                        }
+                        if (used) tasks.push_back(t);
+                    }
+                }
+                for (int al = 0; al < 8; al++) fill[al] += depth[al];
+                seg_cls.push_back(q);
+                batches.back().nseg++;
+                batches.back().ntask = (int)tasks.size() - batches.back().task0;
+                cost.back() += most_steps;
+            }
+    }
+    F.nbatch = (int)batches.size();
+    double all = 0, run = 0;
+    for (double c : cost) all += c;
+    std::vector<int> group;
+    for (int b = 0; b < F.nbatch; b++) {
+        while (group.size() < kFoldGroups && run >= all * group.size() / kFoldGroups) group.push_back(b);
+        run += cost[b];
+    }
+    group.resize(kFoldGroups + 1, F.nbatch);
+
+    DBuf<FoldBlock> dblocks;
+    DBuf<FoldOffset> doffs;
+    auto put = [&](auto &d, const auto &h) {
+        if (d.alloc(std::max<size_t>(h.size(), 1), s, st) && !h.empty())
+            FMM_TRY(st, cudaMemcpyAsync(d.p, h.data(), sizeof(h[0]) * h.size(), cudaMemcpyHostToDevice, s));
+    };
+    std::vector<FoldOffset> offs(off, off + kFoldClasses);
+    put(F.kmap, kmap); put(F.rmap, rmap); put(F.base, base); put(F.group, group); put(F.cls, cls); put(F.tasks, tasks);
+    put(F.batches, batches); put(F.seg_cls, seg_cls); put(F.wseg, wseg); put(dblocks, blocks); put(doffs, offs);
+    F.A.alloc(tot, s, st);
+    if (!st.ok()) return false;
+    k_fold_ops<<<(unsigned)blocks.size(), 128, 0, s>>>(dblocks.p, doffs.p, F.kmap.p, F.base.p, p, rot, dc, lddc,
+                                                       F.A.p); FMM_COUNT_LAUNCH();
+    FMM_LAUNCH_CHECK(st);
+    FMM_TRY(st, cudaStreamSynchronize(s));
+    F.kmap.s = F.rmap.s = F.base.s = F.group.s = F.cls.s = F.tasks.s = F.batches.s = F.seg_cls.s = F.wseg.s = F.A.s = nullptr;
+    return st.ok();
+}
+
+// ---------------------------------------------------------------- complex <-> real basis
+__global__ void k_fold_real(long long n, int K, const int4 *kmap, const double2 *in, double2 *mr)
+{
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const long long b = i / K;
+    const int4 k = kmap[i - b * K];
+    const double2 u = in[b * K + k.x], v = in[b * K + k.y];
+    // A = (u + v) / 2, B = (u - v) / 2i
+    mr[i] = k.z ? cmk(0.5 * (u.y - v.y), 0.5 * (v.x - u.x)) : cmk(0.5 * (u.x + v.x), 0.5 * (u.y + v.y));
+}
+
+// Adds the slots' sums in order and, as complex coefficients, to the local expansions.
+__global__ void k_fold_add(long long n, int nr, int K, int slots, const int4 *rmap, const double2 *lr, double2 *out)
+{
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n * nr) return;
+    const long long b = i / nr;
+    const int4 r = rmap[i - b * nr];
+    double2 a = lr[b * K + r.z], c = r.w >= 0 ? lr[b * K + r.w] : cmk(0, 0);
+    for (int s = 1; s < slots; s++) {
+        const double2 *l = lr + ((long long)s * n + b) * K;
+        a = cadd(a, l[r.z]);
+        if (r.w >= 0) c = cadd(c, l[r.w]);
+    }
+    double2 *o = out + b * K;
+    if (r.w < 0) {
+        o[r.x] = cadd(o[r.x], a);
+        return;
+    }
+    o[r.x] = cadd(o[r.x], cmk(a.x - c.y, a.y + c.x));
+    o[r.y] = cadd(o[r.y], cmk(a.x + c.y, a.y - c.x));
+}
+
+// ---------------------------------------------------------------- the products
+struct FoldView {
+    const int *base;
+    const int4 *cls;
+    const FoldTask *tasks;
+    const FoldBatch *batches;
+    const int *seg_cls;
+    const int4 *wseg;
+    const double *A;
+    const int *group;
+    int K;
+};
+
+// Stage one task for the 8 targets of this lane group: BITS reflections.
+template <int BITS, int NT>
+__device__ __forceinline__ void fold_stage(const FoldTask &t, const int *idx, int tl, int kk, int K,
+                                           const double2 *mr, double *X)
+{
+    constexpr int NS = 1 << BITS;
+    double2 v[NS];
+#pragma unroll
+    for (int g = 0; g < NS; g++) {
+        const int b = idx[(t.cls * 8 + g) * NT + tl];
+        v[g] = b >= 0 && kk < t.n ? __ldg(mr + (size_t)b * K + t.src0 + kk) : cmk(0, 0);
+    }
+    // sums over the reflections with the signs of every character
+#pragma unroll
+    for (int h = 1; h < NS; h <<= 1)
+#pragma unroll
+        for (int g = 0; g < NS; g++)
+            if (!(g & h)) {
+                const double2 a = v[g], b = v[g | h];
+                v[g] = cadd(a, b);
+                v[g | h] = csub(a, b);
+            }
+#pragma unroll
+    for (int c = 0; c < NS; c++) {
+        int sp = 0;
+#pragma unroll
+        for (int i = 0; i < BITS; i++) sp |= (c >> i & 1) << t.axis[i];
+        if (t.row[c] != 255)
+            *reinterpret_cast<double2 *>(X + ((t.beta ^ sp) * kFoldCap + t.row[c] + kk) * kFoldLd<NT> + 2 * tl) = v[c];
+    }
+}
+
+template <int R, int RT, int NT>
+__device__ __forceinline__ void fold_mma(double (&acc)[RT][NT / 4][2], const double *A, int astep, int k4,
+                                         const double *X)
+{
+    for (int ks = 0; ks < k4; ks++) {
+        double a[R], b[NT / 4];
+#pragma unroll
+        for (int r = 0; r < R; r++) a[r] = __ldg(A + 32 * r);
+#pragma unroll
+        for (int c = 0; c < NT / 4; c++) b[c] = X[8 * c];
+        A += astep;
+        X += 4 * kFoldLd<NT>;
+#pragma unroll
+        for (int r = 0; r < R; r++)
+#pragma unroll
+            for (int c = 0; c < NT / 4; c++) dmma(acc[r][c][0], acc[r][c][1], a[r], b[c]);
+    }
+}
+
+template <int R, int RT, int NT>
+__device__ __forceinline__ void fold_mma_n(int n, double (&acc)[RT][NT / 4][2], const double *A, int astep,
+                                           int k4, const double *X)
+{
+    if constexpr (R > 0) {
+        if (n == R) fold_mma<R, RT, NT>(acc, A, astep, k4, X);
+        else fold_mma_n<R - 1, RT, NT>(n, acc, A, astep, k4, X);
+    }
+}
+
+// RS warps per parity class, each with up to RT 8-row blocks of it.
+template <int RS, int RT, int NT, int CTAS>
+__global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeView tv, int first, int count,
+                                                          const double2 *mr, double2 *lr, int slots, int prune)
+{
+    extern __shared__ double fold_sm[];
+    double *X = fold_sm;                                               // [8][kFoldCap][kFoldLd]
+    int *idx = reinterpret_cast<int *>(X + 8 * kFoldCap * kFoldLd<NT>);    // source boxes [class][reflection][target]
+    __shared__ unsigned present[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int al = warp & 7, rs = warp >> 3;
+    const int t0 = blockIdx.x * NT;
+    if (tid < 2) present[tid] = 0;
+    __syncthreads();
+    {
+        // tid % NT is the target throughout
+        const int t = tid & (NT - 1);
+        const int b = t0 + t < count ? first + t0 + t : -1;
+        const bool use = b >= 0 && !(prune && tv.ntrg[b] == 0);
+        const int o = use ? tv.octant[b] : 0, P = use ? tv.parent[b] : -1;
+        for (int e = tid / NT; e < kFoldClasses * 8; e += 256 * RS / NT) {
+            const int q = e >> 3, j = e & 7;
+            const int4 c = f.cls[q];
+            int src = -1;
+            if (P >= 0 && j < 1 << __popc(c.w)) {
+                // reflection bits of the nonzero axes, then the source's position
+                // in the parent's grid of children
+                int d[3] = {c.x, c.y, c.z}, k = 0, cp = 0, oct = 0;
+                bool in = true;
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    if (c.w >> i & 1) {
+                        if (j >> k & 1) d[i] = -d[i];
+                        k++;
+                    }
+                    const int pos = (o >> i & 1) + d[i], pp = pos >> 1;
+                    in &= pp >= -1 && pp <= 1;
+                    cp = cp * 3 + pp + 1;
+                    oct |= (pos & 1) << i;
+                }
+                const int C = in ? tv.coll[27L * P + cp] : -1;
+                src = C >= 0 ? tv.child[8L * C + oct] : -1;
+                if (src >= 0 && tv.nsrc[src] == 0) src = -1;
+            }
+            idx[e * NT + t] = src;
+            if (src >= 0) atomicOr(&present[q >> 5], 1u << (q & 31));
+        }
+    }
+    __syncthreads();
+    const unsigned long long have = present[0] | (unsigned long long)present[1] << 32;
+    double acc[RT][NT / 4][2];
+    const int g0 = slots > 1 ? blockIdx.y : 0, g1 = slots > 1 ? g0 + 1 : kFoldGroups;
+    for (int g = g0; g < g1; g++) {
+#pragma unroll
+        for (int r = 0; r < RT; r++)
+#pragma unroll
+            for (int c = 0; c < NT / 4; c++) acc[r][c][0] = acc[r][c][1] = 0;
+        bool any = false;
+        for (int bi = f.group[g]; bi < f.group[g + 1]; bi++) {
+            const FoldBatch B = f.batches[bi];
+            bool need = false;
+            for (int sg = 0; sg < B.nseg; sg++) need |= have >> f.seg_cls[B.seg0 + sg] & 1;
+            if (!need) continue;
+            any = true;
+            __syncthreads();
+            for (int ti = warp; ti < NT / 8 * B.ntask; ti += 8 * RS) {
+                const FoldTask t = f.tasks[B.task0 + ti / (NT / 8)];
+                if (!(have >> t.cls & 1)) continue;
+                const int tl = ti % (NT / 8) * 8 + (lane & 7), kk = lane >> 3;
+                if (t.bits == 3) fold_stage<3, NT>(t, idx, tl, kk, f.K, mr, X);
+                else if (t.bits == 2) fold_stage<2, NT>(t, idx, tl, kk, f.K, mr, X);
+                else fold_stage<1, NT>(t, idx, tl, kk, f.K, mr, X);
+            }
+            __syncthreads();
+            for (int sg = 0; sg < B.nseg; sg++) {
+                if (!(have >> f.seg_cls[B.seg0 + sg] & 1)) continue;
+                const int4 w = f.wseg[(B.seg0 + sg) * 8 + al];
+                // this warp's row blocks of the class
+                const int r0 = rs * RT, nr = min(w.z - r0, RT);
+                if (w.y == 0 || nr <= 0) continue;
+                fold_mma_n<RT, RT, NT>(nr, acc, f.A + (size_t)w.x * 32 + r0 * 32 + lane, w.z * 32, w.y,
+                                   X + (al * kFoldCap + w.w + (lane & 3)) * kFoldLd<NT> + (lane >> 2));
+            }
+        }
+        // the group's sums: lane l holds both right-hand sides of target 4 c + l % 4, row 8 r + l / 4
+        if (!any && slots == 1 && g > 0) continue;
+        const int na = f.base[8 + al];
+#pragma unroll
+        for (int r = 0; r < RT; r++) {
+            const int row = (rs * RT + r) * 8 + (lane >> 2);
+#pragma unroll
+            for (int c = 0; c < NT / 4; c++) {
+                const int t = t0 + 4 * c + (lane & 3);
+                if (row >= na || t >= count) continue;
+                double2 *o = lr + ((size_t)(slots > 1 ? g : 0) * count + t) * f.K + f.base[al] + row;
+                const double2 v = cmk(acc[r][c][0], acc[r][c][1]);
+                *o = slots > 1 || g == 0 ? v : cadd(*o, v);
+            }
+        }
+    }
+}
+
+bool fold_prepare(const FoldPlan &F, FoldWork &W, int nboxes, int count, cudaStream_t s, Status &st)
+{
+    if (count <= 0) return true;
+    W.tile = F.rows <= 5 ? 16 : 8;
+    W.slots = div_up(count, W.tile) < kFoldSplitTiles ? kFoldGroups : 1;
+    // at most 1 GB of sums at a time
+    const long long most = std::max<long long>((1LL << 30) / (16LL * F.K * W.slots) / W.tile, 1) * W.tile;
+    W.chunk = (int)std::min<long long>(count, W.slots > 1 ? count : most);
+    return W.mr.alloc((size_t)nboxes * F.K, s, st) && W.lr.alloc((size_t)W.chunk * F.K * W.slots, s, st);
+}
+
+template <int RS, int RT, int NT, int CTAS>
+static void launch_fold_t(const FoldPlan &F, const FoldView &f, const FoldWork &W, const TreeView &tv, int first,
+                          int count, double2 *out, int prune, cudaStream_t s, Status &st)
+{
+    constexpr size_t sm = sizeof(double) * 8 * kFoldCap * kFoldLd<NT> + sizeof(int) * kFoldClasses * 8 * NT;
+    FMM_TRY(st, smem_allow(k_m2l_fold<RS, RT, NT, CTAS>, sm));
+    const int nr = (F.p + 1) * (F.p + 2) / 2;
+    for (int c0 = 0; c0 < count && st.ok(); c0 += W.chunk) {
+        const int n = std::min(W.chunk, count - c0);
+        k_m2l_fold<RS, RT, NT, CTAS><<<dim3(div_up(n, NT), W.slots), 256 * RS, sm, s>>>(
+            f, tv, first + c0, n, W.mr.p, W.lr.p, W.slots, prune); FMM_COUNT_LAUNCH();
+        k_fold_add<<<div_up((long)n * nr, 256), 256, 0, s>>>(n, nr, F.K, W.slots, F.rmap.p, W.lr.p,
+                                                             out + (size_t)(first + c0) * F.K); FMM_COUNT_LAUNCH();
+        FMM_LAUNCH_CHECK(st);
+    }
+}
+
+void launch_m2l_fold(const FoldPlan &F, const FoldWork &W, const TreeView &tv, int nboxes, int first, int count,
+                     const double2 *in, double2 *out, int prune, cudaStream_t s, Status &st)
+{
+    if (!st.ok() || count <= 0) return;
+    const long long n = (long long)nboxes * F.K;
+    k_fold_real<<<div_up(n, 256), 256, 0, s>>>(n, F.K, F.kmap.p, in, W.mr.p); FMM_COUNT_LAUNCH();
+    FoldView f;
+    f.base = F.base.p; f.cls = F.cls.p; f.tasks = F.tasks.p; f.batches = F.batches.p; f.seg_cls = F.seg_cls.p;
+    f.wseg = F.wseg.p; f.A = F.A.p; f.group = F.group.p; f.K = F.K;
+    // row blocks of the largest parity class: orders <= 6, <= 9, <= 14, above
+    if (F.rows <= 1) launch_fold_t<1, 1, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);
+    else if (F.rows <= 2) launch_fold_t<1, 2, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);
+    else if (F.rows <= 5) launch_fold_t<1, 5, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);
+    else launch_fold_t<2, 7, 8, 1>(F, f, W, tv, first, count, out, prune, s, st);
+}
+
+}  // namespace fmm

@@ -22,6 +22,7 @@
 // MMAs; z-shift B fragments are formed from the binomial table (L1) and the
 // powers of rt.  Orders up to kRdMaxP (28): two 16-row expansion buffers in
 // shared memory, one CTA of 16 warps per SM.
+#include "dmma.cuh"
 #include "lap_kernels.cuh"
 
 namespace fmm {
@@ -30,13 +31,6 @@ constexpr int kRdWarps = 16;
 constexpr int kRdMaxP = 28;
 constexpr int kRdMaxTasks = 8;      // back-rotation tasks per warp (orders <= 28: at most 120 tasks)
 constexpr int kRdMaxKs = 15;        // K steps of one degree (2 * 28 + 1 = 57 columns: 15 steps of 4)
-
-__device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
 
 // Row stride of the expansion buffers: at least (p+1)^2 + 4 (the A fragments
 // of a degree's last K step read up to 3 entries past the degree; those meet
