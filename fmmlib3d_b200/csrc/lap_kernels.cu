@@ -139,113 +139,252 @@ __device__ __forceinline__ double box_side(const TreeView &tv, int b)
 }
 
 // ================================================================ P2P
-// Near field for one childless box per CTA: evaluation points of the box
-// (its sources, then its targets) against the sources of the box itself and
-// of its list 1.  Source chunks are staged in shared memory; every thread
-// owns one evaluation point and writes it without atomics.
+// Near field of the childless boxes: evaluation points of a box (its sources,
+// then its targets) against the sources of the box itself and of its list 1.
 // Follows lfmm3dpart_direct_self/_targ (src/lfmm3dpart.f:1175-1385) with the
 // pair formulas of lpotfld3d / lpotfld3d_dp (src/laprouts3d.f:1308, 1962).
+//
+// One warp per (leaf, run of 32 EMAX points), each lane with up to EMAX points;
+// 32 sources at a time staged as records in the warp's shared memory.  Bound by
+// the FP64 pipe: 35 operations a pair with charges and dipoles, 23 with charges
+// (the products -d v are made once per source, the field is summed as
+// r^-3 [(q + 3 d t) dx - d v], and 1/r takes five operations), against 49 and 29
+// with a thread per point, the library's rsqrt and charge and dipole terms apart:
+// 25.2 -> 19.5 ms at the 2M + 2M cube (6.25e9 pairs; 72% of the 17e12 FP64
+// operations/s that a loop of independent multiply-adds reaches), 44.1 -> 34.6 ms
+// at the 1M + 1M cube at order 26 (1.17e10 pairs).  Loading the next batch into
+// registers during the current one, or four points per lane, cost more in
+// resident warps than they saved (20.5, 23.9 ms).  All multiply-adds are written
+// out, so that every instantiation rounds alike.
+constexpr int kP2PThreads = 128;      // direct sums
+constexpr int kNearWarps = 2;
 
-constexpr int kP2PThreads = 128, kP2PChunkCTAs = 4;
-
-template <bool CHG, bool DIP>
-__global__ void __launch_bounds__(kP2PThreads) k_p2p(const int *leaves, TreeView tv, PointsSoA src,
-                                                      const double *tx, const double *ty, const double *tz,
-                                                      OutSoA outs, OutSoA outt, int do_src, int do_trg,
-                                                      int want_fs, int want_ft, int want_ps, int want_pt)
+// 1/sqrt(x) for ordinary x: the hardware's approximation (relative error below
+// 2^-19) and one step of Halley's iteration, y (1 + e/2 + 3 e^2/8) with
+// e = 1 - x y^2, which cubes the error.  Zeros, infinities, NaN and numbers near
+// the ends of the range need the library function: `odd` collects the largest
+// position of the exponent above the ordinary range's start, so that a warp tests
+// it once for all its pairs; with LIB every such number takes the library function.
+constexpr unsigned kRsqrtLow = 0x03000000u, kRsqrtSpan = 0x79000000u;   // 2^-975 .. 2^961
+template <bool LIB>
+__device__ __forceinline__ double rsqrt_near(double x, unsigned &odd)
 {
-    __shared__ double sx[kP2PThreads], sy[kP2PThreads], sz[kP2PThreads];
-    __shared__ double2 sq[kP2PThreads], sd[kP2PThreads];
-    __shared__ double svx[kP2PThreads], svy[kP2PThreads], svz[kP2PThreads];
-    const int b = leaves[blockIdx.x];
-    const int s0 = tv.src0[b], ns = do_src ? tv.nsrc[b] : 0;
-    const int t0 = tv.trg0[b], nt = do_trg ? tv.ntrg[b] : 0;
-    const int ne = ns + nt;
-    const int l1a = tv.l1_start[b], nl = 1 + tv.l1_start[b + 1] - l1a;
-    // CTA (leaf, y) serves the leaf's point chunks y, y + gridDim.y, ... (large leaves on
-    // adaptive trees would otherwise hold the pass's tail alone)
-    for (int e0 = blockIdx.y * kP2PThreads; e0 < ne; e0 += gridDim.y * kP2PThreads) {
-        const int e = e0 + threadIdx.x;
-        const bool act = e < ne;
-        const bool is_src = e < ns;
-        double ex = 0, ey = 0, ez = 0;
-        int self = -1;
-        if (act) {
-            if (is_src) { int i = s0 + e; ex = src.x[i]; ey = src.y[i]; ez = src.z[i]; self = i; }
-            else { int i = t0 + e - ns; ex = tx[i]; ey = ty[i]; ez = tz[i]; }
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    y = fma(y * e, fma(e, 0.375, 0.5), y);
+    const unsigned at = (unsigned)__double2hiint(x) - kRsqrtLow;
+    if (LIB) {
+        if (at > kRsqrtSpan) y = rsqrt(x);
+    } else {
+        odd = max(odd, at);
+    }
+    return y;
+}
+
+// Source record: x, y, z, [q], [d, v, -d v (re), -d v (im)], padded to a stride
+// whose 16-byte parts fall into different banks for consecutive sources.
+template <bool CHG, bool DIP>
+struct NearRec {
+    static constexpr int kStride = DIP ? (CHG ? 18 : 14) : 6;
+    static constexpr int kQ = 3, kD = CHG ? 5 : 3, kV = kD + 2, kN = kV + 3;
+};
+
+template <bool CHG, bool DIP, bool LIB>
+__device__ __forceinline__ void near_pair(double dx, double dy, double dz, double qx, double qy, double ddx,
+                                          double ddy, double vx, double vy, double vz, const double *nv, double *a,
+                                          unsigned &odd)
+{
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const double ri = rsqrt_near<LIB>(r2, odd);
+    const double ri2 = ri * ri, ri3 = ri * ri2;
+    if (!DIP) {
+        a[0] = fma(qx, ri, a[0]);
+        a[1] = fma(qy, ri, a[1]);
+        const double bx = qx * ri3, by = qy * ri3;
+        a[2] = fma(bx, dx, a[2]); a[3] = fma(by, dx, a[3]);
+        a[4] = fma(bx, dy, a[4]); a[5] = fma(by, dy, a[5]);
+        a[6] = fma(bx, dz, a[6]); a[7] = fma(by, dz, a[7]);
+    } else {
+        // pot = (q + d t) / r with t = (v.dx) / r^2;  fld = [(q + 3 d t) dx - d v] / r^3
+        const double t = fma(dx, vx, fma(dy, vy, dz * vz)) * ri2;
+        const double ax = CHG ? fma(ddx, t, qx) : ddx * t, ay = CHG ? fma(ddy, t, qy) : ddy * t;
+        a[0] = fma(ax, ri, a[0]);
+        a[1] = fma(ay, ri, a[1]);
+        const double t2 = t + t;
+        const double bx = fma(ddx, t2, ax), by = fma(ddy, t2, ay);
+        a[2] = fma(ri3, fma(bx, dx, nv[0]), a[2]); a[3] = fma(ri3, fma(by, dx, nv[3]), a[3]);
+        a[4] = fma(ri3, fma(bx, dy, nv[1]), a[4]); a[5] = fma(ri3, fma(by, dy, nv[4]), a[5]);
+        a[6] = fma(ri3, fma(bx, dz, nv[2]), a[6]); a[7] = fma(ri3, fma(by, dz, nv[5]), a[7]);
+    }
+}
+
+// cn staged sources at E points of a lane.  OWN: the sources are the points' own
+// box; a point's own source (selfk) adds exact zeros (no strength, unit offset).
+template <bool CHG, bool DIP, bool LIB, int E, bool OWN, int U>
+__device__ __forceinline__ void near_batch(const double *rec, int cn, const double (&px)[E], const double (&py)[E],
+                                           const double (&pz)[E], const int (&selfk)[E], double (&acc)[E][8],
+                                           unsigned &odd)
+{
+    using R = NearRec<CHG, DIP>;
+    constexpr int W = R::kStride;
+#pragma unroll U
+    for (int k = 0; k < cn; k++) {
+        double r[W];
+#pragma unroll
+        for (int i = 0; i < W / 2; i++) {
+            const double2 v = reinterpret_cast<const double2 *>(rec + k * W)[i];
+            r[2 * i] = v.x;
+            r[2 * i + 1] = v.y;
         }
-        double pr = 0, pi = 0, fxr = 0, fxi = 0, fyr = 0, fyi = 0, fzr = 0, fzi = 0;
-        for (int j = 0; j < nl; j++) {
-            const int jb = j == 0 ? b : tv.l1_idx[l1a + j - 1];
-            const int js0 = tv.src0[jb], jn = tv.nsrc[jb];
-            for (int c0 = 0; c0 < jn; c0 += kP2PThreads) {
-                const int cn = min(kP2PThreads, jn - c0);
-                __syncthreads();
-                if (threadIdx.x < cn) {
-                    int i = js0 + c0 + threadIdx.x;
-                    sx[threadIdx.x] = src.x[i]; sy[threadIdx.x] = src.y[i]; sz[threadIdx.x] = src.z[i];
-                    if (CHG) sq[threadIdx.x] = src.q[i];
-                    if (DIP) {
-                        sd[threadIdx.x] = src.dq[i];
-                        svx[threadIdx.x] = src.vx[i]; svy[threadIdx.x] = src.vy[i]; svz[threadIdx.x] = src.vz[i];
-                    }
-                }
-                __syncthreads();
-                if (!act) continue;
-                const int selfk = self - (js0 + c0);
-                // the self pair adds exact zeros (no strength, unit offset) instead of a branch
-#pragma unroll 4
-                for (int k = 0; k < cn; k++) {
-                    const bool me = k == selfk;
-                    double dx = me ? 1.0 : ex - sx[k], dy = me ? 0.0 : ey - sy[k], dz = me ? 0.0 : ez - sz[k];
-                    double r2 = dx * dx + dy * dy + dz * dz;
-                    double ri = rsqrt(r2);
-                    double ri2 = ri * ri, ri3 = ri * ri2;
-                    if (CHG) {
-                        double2 q = me ? make_double2(0.0, 0.0) : sq[k];
-                        pr = fma(q.x, ri, pr);
-                        pi = fma(q.y, ri, pi);
-                        double qx = q.x * ri3, qy = q.y * ri3;
-                        fxr = fma(qx, dx, fxr); fxi = fma(qy, dx, fxi);
-                        fyr = fma(qx, dy, fyr); fyi = fma(qy, dy, fyi);
-                        fzr = fma(qx, dz, fzr); fzi = fma(qy, dz, fzi);
-                    }
-                    if (DIP) {
-                        double2 d = me ? make_double2(0.0, 0.0) : sd[k];
-                        double vx = me ? 0.0 : svx[k], vy = me ? 0.0 : svy[k], vz = me ? 0.0 : svz[k];
-                        double dot = dx * vx + dy * vy + dz * vz;
-                        double a = dot * ri3;
-                        pr = fma(d.x, a, pr);
-                        pi = fma(d.y, a, pi);
-                        double rt = 3.0 * dot * ri3 * ri2;
-                        double gx = rt * dx - ri3 * vx, gy = rt * dy - ri3 * vy, gz = rt * dz - ri3 * vz;
-                        fxr = fma(d.x, gx, fxr); fxi = fma(d.y, gx, fxi);
-                        fyr = fma(d.x, gy, fyr); fyi = fma(d.y, gy, fyi);
-                        fzr = fma(d.x, gz, fzr); fzi = fma(d.y, gz, fzi);
-                    }
-                }
-            }
-        }
-        if (act) {
-            if (is_src) {
-                int i = s0 + e;
-                if (want_ps) outs.pot[i] = cadd(outs.pot[i], cmk(pr, pi));
-                if (want_fs) {
-                    outs.fx[i] = cadd(outs.fx[i], cmk(fxr, fxi));
-                    outs.fy[i] = cadd(outs.fy[i], cmk(fyr, fyi));
-                    outs.fz[i] = cadd(outs.fz[i], cmk(fzr, fzi));
-                }
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            double dx = px[e] - r[0], dy = py[e] - r[1], dz = pz[e] - r[2];
+            double qx = CHG ? r[R::kQ] : 0, qy = CHG ? r[R::kQ + 1] : 0;
+            double ddx = DIP ? r[R::kD] : 0, ddy = DIP ? r[R::kD + 1] : 0;
+            if (OWN) {
+                const bool me = k == selfk[e];
+                dx = me ? 1.0 : dx; dy = me ? 0.0 : dy; dz = me ? 0.0 : dz;
+                qx = me ? 0.0 : qx; qy = me ? 0.0 : qy;
+                ddx = me ? 0.0 : ddx; ddy = me ? 0.0 : ddy;
+                double nv[6], v[3];
+#pragma unroll
+                for (int i = 0; i < 6; i++) nv[i] = DIP ? (me ? 0.0 : r[R::kN + i]) : 0;
+#pragma unroll
+                for (int i = 0; i < 3; i++) v[i] = DIP ? (me ? 0.0 : r[R::kV + i]) : 0;
+                near_pair<CHG, DIP, LIB>(dx, dy, dz, qx, qy, ddx, ddy, v[0], v[1], v[2], nv, acc[e], odd);
             } else {
-                int i = t0 + e - ns;
-                if (want_pt) outt.pot[i] = cadd(outt.pot[i], cmk(pr, pi));
-                if (want_ft) {
-                    outt.fx[i] = cadd(outt.fx[i], cmk(fxr, fxi));
-                    outt.fy[i] = cadd(outt.fy[i], cmk(fyr, fyi));
-                    outt.fz[i] = cadd(outt.fz[i], cmk(fzr, fzi));
-                }
+                near_pair<CHG, DIP, LIB>(dx, dy, dz, qx, qy, ddx, ddy, DIP ? r[R::kV] : 0, DIP ? r[R::kV + 1] : 0,
+                                    DIP ? r[R::kV + 2] : 0, r + (DIP ? R::kN : 0), acc[e], odd);
             }
         }
     }
+}
+
+struct NearArgs {
+    const int *leaves;
+    int nleaves;
+    TreeView tv;
+    PointsSoA src;
+    const double *tx, *ty, *tz;
+    OutSoA outs, outt;
+    int do_src, do_trg, want_fs, want_ft, want_ps, want_pt;
+};
+
+// Points e0 + lane, + 32, ... of leaf b (E per lane).  Returns whether a pair of
+// this warp needs the library's rsqrt; nothing is written then (LIB: never).
+template <bool CHG, bool DIP, bool LIB, int E, int U>
+__device__ __forceinline__ bool near_points(const NearArgs &A, int b, int e0, int ne, int ns, double *rec)
+{
+    using R = NearRec<CHG, DIP>;
+    constexpr int W = R::kStride;
+    const int lane = threadIdx.x & 31;
+    const int s0 = A.tv.src0[b], t0 = A.tv.trg0[b];
+    double px[E], py[E], pz[E], acc[E][8];
+    int self[E];
+    unsigned odd = 0;
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        // (lanes past the end repeat the last point; nothing of theirs is written)
+        self[k] = -1;
+        const int ee = min(e0 + lane + 32 * k, ne - 1);
+        if (ee < ns) { const int i = s0 + ee; px[k] = A.src.x[i]; py[k] = A.src.y[i]; pz[k] = A.src.z[i]; self[k] = ee; }
+        else { const int i = t0 + ee - ns; px[k] = A.tx[i]; py[k] = A.ty[i]; pz[k] = A.tz[i]; }
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[k][i] = 0;
+    }
+    const int l1a = A.tv.l1_start[b], nl = 1 + A.tv.l1_start[b + 1] - l1a;
+    for (int j = 0; j < nl; j++) {
+        const int jb = j == 0 ? b : A.tv.l1_idx[l1a + j - 1];
+        const int js0 = A.tv.src0[jb], jn = A.tv.nsrc[jb];
+        for (int c0 = 0; c0 < jn; c0 += 32) {
+            const int cn = min(32, jn - c0);
+            __syncwarp();
+            if (lane < cn) {
+                const int i = js0 + c0 + lane;
+                double r[W] = {};
+                r[0] = A.src.x[i]; r[1] = A.src.y[i]; r[2] = A.src.z[i];
+                if (CHG) { const double2 q = A.src.q[i]; r[R::kQ] = q.x; r[R::kQ + 1] = q.y; }
+                if (DIP) {
+                    const double2 d = A.src.dq[i];
+                    const double v[3] = {A.src.vx[i], A.src.vy[i], A.src.vz[i]};
+                    r[R::kD] = d.x; r[R::kD + 1] = d.y;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        r[R::kV + c] = v[c];
+                        r[R::kN + c] = -d.x * v[c];
+                        r[R::kN + 3 + c] = -d.y * v[c];
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < W / 2; c++)
+                    reinterpret_cast<double2 *>(rec + lane * W)[c] = make_double2(r[2 * c], r[2 * c + 1]);
+            }
+            __syncwarp();
+            int selfk[E];
+            if (j == 0 && e0 < ns) {
+#pragma unroll
+                for (int k = 0; k < E; k++) selfk[k] = self[k] < 0 ? -1 : self[k] - c0;
+                near_batch<CHG, DIP, LIB, E, true, 1>(rec, cn, px, py, pz, selfk, acc, odd);
+            } else {
+                near_batch<CHG, DIP, LIB, E, false, U>(rec, cn, px, py, pz, selfk, acc, odd);
+            }
+        }
+    }
+    if (!LIB && __any_sync(0xffffffffu, odd > kRsqrtSpan)) return true;
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        const int e = e0 + lane + 32 * k;
+        if (e >= ne) continue;
+        const bool is_src = e < ns;
+        const int i = is_src ? s0 + e : t0 + e - ns;
+        const OutSoA o = is_src ? A.outs : A.outt;
+        if (is_src ? A.want_ps : A.want_pt) o.pot[i] = cadd(o.pot[i], cmk(acc[k][0], acc[k][1]));
+        if (is_src ? A.want_fs : A.want_ft) {
+            o.fx[i] = cadd(o.fx[i], cmk(acc[k][2], acc[k][3]));
+            o.fy[i] = cadd(o.fy[i], cmk(acc[k][4], acc[k][5]));
+            o.fz[i] = cadd(o.fz[i], cmk(acc[k][6], acc[k][7]));
+        }
+    }
+    return false;
+}
+
+template <bool CHG, bool DIP, int E, int U>
+__device__ __forceinline__ void near_run(const NearArgs &A, int b, int e0, int ne, int ns, double *rec)
+{
+    if (near_points<CHG, DIP, false, E, U>(A, b, e0, ne, ns, rec))
+        near_points<CHG, DIP, true, E, 1>(A, b, e0, ne, ns, rec);
+}
+
+template <bool CHG, bool DIP, int EMAX, int U, int CT>
+__global__ void __launch_bounds__(32 * kNearWarps, CT) k_p2p(NearArgs A)
+{
+    __shared__ __align__(16) double rec[kNearWarps][32 * NearRec<CHG, DIP>::kStride];
+    const int warp = threadIdx.x >> 5, li = blockIdx.x * kNearWarps + warp;
+    if (li >= A.nleaves) return;
+    const int b = A.leaves[li];
+    const int ns = A.do_src ? A.tv.nsrc[b] : 0, ne = ns + (A.do_trg ? A.tv.ntrg[b] : 0);
+    // runs blockIdx.y, + gridDim.y, ... of the leaf's points (a large leaf of an
+    // adaptive tree would otherwise hold the pass's tail alone)
+    for (int e0 = blockIdx.y * 32 * EMAX; e0 < ne; e0 += gridDim.y * 32 * EMAX) {
+        if (EMAX == 2 && ne - e0 > 32) near_run<CHG, DIP, EMAX, U>(A, b, e0, ne, ns, rec[warp]);
+        else near_run<CHG, DIP, 1, U>(A, b, e0, ne, ns, rec[warp]);
+    }
+}
+
+template <bool CHG, bool DIP>
+static void launch_p2p_t(const NearArgs &A, cudaStream_t s, Status &st)
+{
+    const int ctas = div_up(A.nleaves, kNearWarps);
+    // Two points per lane share the staging and the record reads, one gives twice the
+    // warps: 2M + 2M cube (32,768 leaves) 19.5 against 20.1 ms, 1M + 1M cube (4,096)
+    // 34.6 / 34.9; 100k sphere (1,489) 0.41 / 0.38, 64 leaves 0.13 / 0.08 ms.  The
+    // line is the 16 warps a multiprocessor holds, on all of them.
+    if (A.nleaves >= 16 * 148)
+        k_p2p<CHG, DIP, 2, 1, 8><<<dim3(ctas, 4), 32 * kNearWarps, 0, s>>>(A);
+    else
+        k_p2p<CHG, DIP, 1, 2, 1><<<dim3(ctas, 8), 32 * kNearWarps, 0, s>>>(A);
+    FMM_COUNT_LAUNCH();
 }
 
 void launch_p2p(const int *leaves, int nleaves, const TreeView &tv, const PointsSoA &src, const double *tx,
@@ -253,19 +392,16 @@ void launch_p2p(const int *leaves, int nleaves, const TreeView &tv, const Points
                 int ifpot, int iffld, int ifpottarg, int iffldtarg, cudaStream_t s, Status &st)
 {
     if (nleaves == 0 || !st.ok()) return;
-    int do_src = (ifpot == 1 || iffld == 1), do_trg = (ifpottarg == 1 || iffldtarg == 1);
-    bool c = ifcharge == 1, d = ifdipole == 1;
+    const bool c = ifcharge == 1, d = ifdipole == 1;
     if (!c && !d) return;
-    if (c && d) {
-        k_p2p<true, true><<<dim3(nleaves, kP2PChunkCTAs), kP2PThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, outs, outt, do_src, do_trg,
-                                                         iffld == 1, iffldtarg == 1, ifpot == 1, ifpottarg == 1); FMM_COUNT_LAUNCH();
-    } else if (c) {
-        k_p2p<true, false><<<dim3(nleaves, kP2PChunkCTAs), kP2PThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, outs, outt, do_src, do_trg,
-                                                          iffld == 1, iffldtarg == 1, ifpot == 1, ifpottarg == 1); FMM_COUNT_LAUNCH();
-    } else {
-        k_p2p<false, true><<<dim3(nleaves, kP2PChunkCTAs), kP2PThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, outs, outt, do_src, do_trg,
-                                                          iffld == 1, iffldtarg == 1, ifpot == 1, ifpottarg == 1); FMM_COUNT_LAUNCH();
-    }
+    NearArgs A;
+    A.leaves = leaves; A.nleaves = nleaves; A.tv = tv; A.src = src; A.tx = tx; A.ty = ty; A.tz = tz;
+    A.outs = outs; A.outt = outt;
+    A.do_src = ifpot == 1 || iffld == 1; A.do_trg = ifpottarg == 1 || iffldtarg == 1;
+    A.want_fs = iffld == 1; A.want_ft = iffldtarg == 1; A.want_ps = ifpot == 1; A.want_pt = ifpottarg == 1;
+    if (c && d) launch_p2p_t<true, true>(A, s, st);
+    else if (c) launch_p2p_t<true, false>(A, s, st);
+    else launch_p2p_t<false, true>(A, s, st);
     FMM_LAUNCH_CHECK(st);
 }
 
