@@ -22,6 +22,7 @@
 #include <map>
 #include <mutex>
 
+#include "dmma.cuh"
 #include "lap_kernels.cuh"
 
 namespace fmm {
@@ -673,25 +674,20 @@ __global__ void __launch_bounds__(kFormThreads) k_form(const int *boxes, const i
                 if (n > p) continue;
                 double2 a1 = ap[k], a2 = am[k];
                 if (ifcharge == 1) {
-                    // two independent partial sums per coefficient (even / odd sources)
-                    // so consecutive FMAs do not wait on each other
+                    // four real sums give both coefficients: q h = (c0 - c1, c2 + c3),
+                    // q conj(h) = (c0 + c1, c3 - c2)
                     const double2 *tp = tab + (size_t)S * tidx(n, mm);
-                    double2 b1 = cmk(0, 0), b2 = cmk(0, 0);
-                    int jj = 0;
-                    for (; jj + 1 < cn; jj += 2) {
-                        const double2 t0 = tp[jj], q0 = qs[jj], t1 = tp[jj + 1], q1 = qs[jj + 1];
-                        cfma(a1, q0, t0);
-                        a2 = cadd(a2, cmulc(q0, t0));
-                        cfma(b1, q1, t1);
-                        b2 = cadd(b2, cmulc(q1, t1));
+                    double c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+#pragma unroll 4
+                    for (int jj = 0; jj < cn; jj++) {
+                        const double2 t = tp[jj], q = qs[jj];
+                        c0 = fma(q.x, t.x, c0);
+                        c1 = fma(q.y, t.y, c1);
+                        c2 = fma(q.x, t.y, c2);
+                        c3 = fma(q.y, t.x, c3);
                     }
-                    if (jj < cn) {
-                        const double2 t0 = tp[jj], q0 = qs[jj];
-                        cfma(a1, q0, t0);
-                        a2 = cadd(a2, cmulc(q0, t0));
-                    }
-                    a1 = cadd(a1, b1);
-                    a2 = cadd(a2, b2);
+                    a1 = cadd(a1, cmk(c0 - c1, c2 + c3));
+                    a2 = cadd(a2, cmk(c0 + c1, c3 - c2));
                 }
                 if (ifdipole == 1) {
                     const int nn = IRREG ? n + 1 : n - 1;
@@ -778,11 +774,233 @@ static void launch_form_t(const int *boxes, int nboxes, const TreeView &tv, cons
     FMM_LAUNCH_CHECK(st);
 }
 
+// ---------------------------------------------------------------- dipoles: in matrix products
+// With dipoles every harmonic h = C + iS meets four complex weights of a source:
+// q, d vz, d vx and d vy (the ladder identities turn the derivative along v into
+// harmonics of degree n +- 1 with weights of the degree and order alone, applied
+// once to the sums).  The sums of all real harmonics with the 8 real weights are
+// one (harmonics x sources) (sources x 8) product, an exact fit for the 8 columns
+// of the FP64 MMA.  Per chunk of C sources the CTA writes the table of real
+// harmonics in shared memory (row n^2, then n^2 + 2m - 1 and n^2 + 2m for the
+// cosine and sine parts of (n, m); row stride = 4 mod 16 doubles, so the 4 x 4
+// lanes of a half warp reading a fragment meet different banks), then each warp
+// multiplies its 8-row blocks, whose sums stay in its accumulators.  Bound by the
+// FP64 pipe: about 0.9 k operations for the table and 2 k in MMAs a source at order
+// 14, against 4.6 k with one thread per (n, m).
+template <int C>
+constexpr int kFmmLd = C + 4;
+constexpr int kFmmLdw = 12;   // row stride of the weights, = 12 mod 16
+
+template <bool IRREG, int NW, int C, int TPW>
+__global__ void __launch_bounds__(32 * NW) k_form_mm(const int *boxes, const int *l4s, const int *l4i, TreeView tv,
+                                                     PointsSoA src, int ifcharge, int p, double2 *coef)
+{
+    constexpr int S = kFmmLd<C>, NT = 32 * NW, G = NT / C;
+    extern __shared__ double fsm[];
+    const int pt = IRREG ? p + 1 : p;                 // table degree
+    const int rows = (pt + 1) * (pt + 1), ntile = (rows + 7) / 8;
+    double *tab = fsm;                                // [8 ntile][S]
+    double *wt = tab + (size_t)8 * ntile * S;         // [C][kFmmLdw]
+    int *pre = (int *)(wt + C * kFmmLdw);             // [kFormWin + 1]
+    const int b = boxes[blockIdx.x];
+    const int nsb = IRREG ? l4s[b + 1] - l4s[b] : 1;
+    if (IRREG && nsb == 0) return;
+    if (!IRREG && tv.nsrc[b] == 0) return;            // the coefficients are zero already
+    const double s = box_side(tv, b), is = 1.0 / s;
+    const double cx = tv.center[3L * b], cy = tv.center[3L * b + 1], cz = tv.center[3L * b + 2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int j = tid % C, g = tid / C;
+    double acc[TPW][2];
+#pragma unroll
+    for (int i = 0; i < TPW; i++) acc[i][0] = acc[i][1] = 0;
+    for (int i = rows * S + tid; i < 8 * ntile * S; i += NT) tab[i] = 0;
+    for (int w0 = 0; w0 < nsb; w0 += kFormWin) {
+        const int nw = min(kFormWin, nsb - w0);
+        __syncthreads();
+        if (tid < 32) {
+            int run = 0;
+            if (tid == 0) pre[0] = 0;
+            for (int g0 = 0; g0 < nw; g0 += 32) {
+                const int k = g0 + tid;
+                int v = k < nw ? tv.nsrc[IRREG ? l4i[l4s[b] + w0 + k] : b] : 0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, v, o);
+                    if (tid >= o) v += t;
+                }
+                if (k < nw) pre[k + 1] = run + v;
+                run += __shfl_sync(0xffffffffu, v, 31);
+            }
+        }
+        __syncthreads();
+        const int total = pre[nw];
+        for (int c0 = 0; c0 < total; c0 += C) {
+            const int cn = min(C, total - c0);
+            __syncthreads();
+            if (j < ((cn + 3) & ~3)) {
+                // the source of concatenated position c0 + j: last window box with pre[k] <= pos
+                // (positions that fill the last K step repeat the last source, without weight)
+                const int pos = c0 + min(j, cn - 1);
+                int lo = 0, hi = nw - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (pre[mid] <= pos) lo = mid;
+                    else hi = mid - 1;
+                }
+                const int jb = IRREG ? l4i[l4s[b] + w0 + lo] : b;
+                const int i = tv.src0[jb] + pos - pre[lo];
+                const double ux = (src.x[i] - cx) * is, uy = (src.y[i] - cy) * is, uz = (src.z[i] - cz) * is;
+                if (g == 0) {
+                    const double2 q = ifcharge == 1 ? src.q[i] : cmk(0, 0), d = cscal(is, src.dq[i]);
+                    const double v[3] = {src.vz[i], src.vx[i], src.vy[i]};
+                    double *w = wt + j * kFmmLdw;
+                    const bool in = j < cn;
+                    w[0] = in ? q.x : 0; w[1] = in ? q.y : 0;
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        w[2 + 2 * k] = in ? d.x * v[k] : 0;
+                        w[3 + 2 * k] = in ? d.y * v[k] : 0;
+                    }
+                }
+                const double r2 = ux * ux + uy * uy + uz * uz;
+                const double ir2 = IRREG ? 1.0 / r2 : 1.0;
+                const double zz = IRREG ? uz * ir2 : uz, rr = IRREG ? ir2 : r2;
+                double2 diag = cmk(IRREG ? sqrt(ir2) : 1.0, 0.0);
+                for (int m = 0; m <= pt; m++) {
+                    if (m > 0) {
+                        const double cc = -c_cm[m] * ir2;
+                        diag = cmk(cc * (ux * diag.x + uy * diag.y), cc * (ux * diag.y - uy * diag.x));
+                    }
+                    if (m % G != g) continue;
+                    double2 h0 = diag, h1 = cmk(0, 0);
+                    for (int n = m; n <= pt; n++) {
+                        if (n > m) {
+                            const double a = (n == m + 1 ? c_sq[m] : c_ra[tidx(n, m)]) * zz, bb = c_rb[tidx(n, m)] * rr;
+                            const double2 h = cmk(a * h0.x - bb * h1.x, a * h0.y - bb * h1.y);
+                            h1 = h0;
+                            h0 = h;
+                        }
+                        double *t = tab + (size_t)(m ? n * n + 2 * m - 1 : n * n) * S + j;
+                        t[0] = h0.x;
+                        if (m) t[S] = h0.y;
+                    }
+                }
+            }
+            __syncthreads();
+            double bf[C / 4];
+#pragma unroll
+            for (int ks = 0; ks < C / 4; ks++) bf[ks] = 4 * ks < cn ? wt[(4 * ks + (lane & 3)) * kFmmLdw + (lane >> 2)] : 0;
+#pragma unroll
+            for (int i = 0; i < TPW; i++) {
+                const int t = warp + NW * i;
+                if (t >= ntile) continue;
+                const double *ta = tab + (size_t)(8 * t + (lane >> 2)) * S + (lane & 3);
+#pragma unroll
+                for (int ks = 0; ks < C / 4; ks++)
+                    if (4 * ks < cn) dmma(acc[i][0], acc[i][1], ta[4 * ks], bf[ks]);
+            }
+        }
+    }
+    // sums of row r with weight k (0: q, 1: d vz, 2: d vx, 3: d vy)
+    __syncthreads();
+    double2 *sum = reinterpret_cast<double2 *>(fsm);
+#pragma unroll
+    for (int i = 0; i < TPW; i++) {
+        const int t = warp + NW * i;
+        if (t < ntile) sum[(8 * t + (lane >> 2)) * 4 + (lane & 3)] = cmk(acc[i][0], acc[i][1]);
+    }
+    __syncthreads();
+    // cosine and sine sums of (n, m) with weight k; the sums of M = d (vx - i vy) / 2 and
+    // P = d (vx + i vy) / 2 follow from those of d vx and d vy
+    auto cs = [&](int n, int m, int k, double2 &c, double2 &sn) {
+        c = cmk(0, 0);
+        sn = cmk(0, 0);
+        if (n < 0 || m > n || m < 0) return;
+        c = sum[(m ? n * n + 2 * m - 1 : n * n) * 4 + k];
+        if (m) sn = sum[(n * n + 2 * m) * 4 + k];
+    };
+    auto weighted = [&](int n, int m, int k, bool conj) {   // k: 1 A, 2 M, 3 P; sum of the weight times h or conj(h)
+        double2 c, sn;
+        if (k == 1) cs(n, m, 1, c, sn);
+        else {
+            double2 xc, xs, yc, ys;
+            cs(n, m, 2, xc, xs);
+            cs(n, m, 3, yc, ys);
+            const double f = k == 2 ? 0.5 : -0.5;   // M: (x - i y) / 2, P: (x + i y) / 2
+            c = cmk(0.5 * xc.x + f * yc.y, 0.5 * xc.y - f * yc.x);
+            sn = cmk(0.5 * xs.x + f * ys.y, 0.5 * xs.y - f * ys.x);
+        }
+        return conj ? cmk(c.x + sn.y, c.y - sn.x) : cmk(c.x - sn.y, c.y + sn.x);
+    };
+    const int npair = (p + 1) * (p + 2) / 2;
+    double2 *out = coef + (size_t)b * (p + 1) * (p + 1);
+    for (int u = tid; u < npair; u += NT) {
+        int n = (int)((sqrtf(8.0f * u + 1.0f) - 1.0f) * 0.5f);
+        while (n * (n + 1) / 2 > u) n--;
+        while ((n + 1) * (n + 2) / 2 <= u) n++;
+        const int mm = u - n * (n + 1) / 2;
+        double2 a1, a2;
+        {
+            double2 c, sn;
+            cs(n, mm, 0, c, sn);
+            a1 = cmk(c.x - sn.y, c.y + sn.x);
+            a2 = cmk(c.x + sn.y, c.y - sn.x);
+        }
+        const int nn = IRREG ? n + 1 : n - 1;
+        double z, pp, mp;
+        dip_weights<IRREG>(n, mm, z, pp, mp);
+        a1 = cadd(a1, cadd(cadd(cscal(z, weighted(nn, mm, 1, false)),
+                                cscal(pp, mm >= 1 ? weighted(nn, mm - 1, 2, false) : weighted(nn, 1, 2, true))),
+                           cscal(mp, weighted(nn, mm + 1, 3, false))));
+        if (mm > 0) {
+            dip_weights<IRREG>(n, -mm, z, pp, mp);
+            a2 = cadd(a2, cadd(cadd(cscal(z, weighted(nn, mm, 1, true)), cscal(pp, weighted(nn, mm + 1, 2, true))),
+                               cscal(mp, weighted(nn, mm - 1, 3, mm >= 2))));
+        }
+        const int ep = eidx(n, mm), em = eidx(n, -mm);
+        if (IRREG) {
+            out[ep] = cadd(out[ep], a1);
+            if (mm > 0) out[em] = cadd(out[em], a2);
+        } else {
+            out[ep] = a1;
+            if (mm > 0) out[em] = a2;
+        }
+    }
+}
+
+template <bool IRREG, int NW, int C, int TPW>
+static void launch_form_mm(const int *boxes, int nboxes, const TreeView &tv, const PointsSoA &src, int ifcharge, int p,
+                           double2 *coef, cudaStream_t s, Status &st)
+{
+    const int pt = IRREG ? p + 1 : p, ntile = ((pt + 1) * (pt + 1) + 7) / 8;
+    const size_t sm = sizeof(double) * ((size_t)8 * ntile * kFmmLd<C> + C * kFmmLdw) + sizeof(int) * (kFormWin + 1);
+    FMM_TRY(st, smem_allow(k_form_mm<IRREG, NW, C, TPW>, sm));
+    k_form_mm<IRREG, NW, C, TPW><<<nboxes, 32 * NW, sm, s>>>(boxes, IRREG ? tv.l4_start : nullptr,
+                                                             IRREG ? tv.l4_idx : nullptr, tv, src, ifcharge, p,
+                                                             coef); FMM_COUNT_LAUNCH();
+    FMM_LAUNCH_CHECK(st);
+}
+
+// Dipoles up to order 28 (table degree 29: 113 blocks of 8 harmonics).  32 sources a
+// chunk while three CTAs fit an SM, then 16 with twice the warps.
+template <bool IRREG>
+static bool form_mm(const int *boxes, int nboxes, const TreeView &tv, const PointsSoA &src, int ifcharge, int p,
+                    double2 *coef, cudaStream_t s, Status &st)
+{
+    const int pt = IRREG ? p + 1 : p, ntile = ((pt + 1) * (pt + 1) + 7) / 8;
+    if (pt > 29) return false;
+    if (ntile <= 16) launch_form_mm<IRREG, 4, 32, 4>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
+    else if (ntile <= 32) launch_form_mm<IRREG, 4, 32, 8>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
+    else launch_form_mm<IRREG, 8, 16, 15>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
+    return true;
+}
+
 template <bool IRREG>
 static void launch_form(const int *boxes, int nboxes, const TreeView &tv, const PointsSoA &src, int ifcharge,
                         int ifdipole, int p, double2 *coef, cudaStream_t s, Status &st)
 {
     if (nboxes == 0 || !st.ok()) return;
+    if (ifdipole == 1 && form_mm<IRREG>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st)) return;
     const int npair = (p + 1) * (p + 2) / 2;
     if (npair <= kFormThreads) launch_form_t<IRREG, 1>(boxes, nboxes, tv, src, ifcharge, ifdipole, p, coef, s, st);
     else if (npair <= 2 * kFormThreads) launch_form_t<IRREG, 2>(boxes, nboxes, tv, src, ifcharge, ifdipole, p, coef, s, st);
