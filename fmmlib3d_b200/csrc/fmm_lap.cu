@@ -756,7 +756,8 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
     // mixed form: small list-3 / list-4 interactions join the near field (FP64 keeps the reference's lists)
     lap_widen_near(S, S.mixed ? (p + 2) * (p + 2) / 2 : 0, s, st);
     if (!st.ok()) { g_ti.err = cudaGetErrorString(st.err); return 16; }
-    eval_items_prepare(T.leaves.p, T.nleaves, S.tv_far, S.do_src, S.do_trg, S.ev, s, st);
+    eval_items_prepare(T.leaves.p, T.nleaves, S.tv_far, S.do_src, S.do_trg, S.ifhess == 1 || S.ifhesstarg == 1, S.ev, s,
+                       st);
     if (!st.ok()) { g_ti.err = cudaGetErrorString(st.err); return 16; }
     if (S.tri) {
         // triangle data in tree order and the quadrature nodes (filled per call)
@@ -907,8 +908,8 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     // STEPS 6, 7: M2P from list 3 and L2P (add the far field to the outputs)
     launch_eval(T.leaves.p, T.nleaves, S.ev, S.tv_far, S.sx.p, S.sy.p, S.sz.p, S.tx.p, S.ty.p, S.tz.p, p,
                 S.mpole.p, S.local.p, S.os, S.ot, S.do_src, S.do_trg, s, st);
-    launch_eval_hess(T.leaves.p, T.nleaves, S.tv_far, S.sx.p, S.sy.p, S.sz.p, S.tx.p, S.ty.p, S.tz.p, p, S.mpole.p,
-                     S.local.p, S.hs, S.ht, hsrc, htrg, s, st);
+    launch_eval_hess(T.leaves.p, T.nleaves, S.ev, S.tv_far, S.sx.p, S.sy.p, S.sz.p, S.tx.p, S.ty.p, S.tz.p, p,
+                     S.mpole.p, S.local.p, S.hs, S.ht, S.do_src, S.do_trg, hsrc, htrg, s, st);
     tm.mark();
     if (tm.on) {
         // intervals: ..., l2l, [wait for the near field], eval, scatter, total ->

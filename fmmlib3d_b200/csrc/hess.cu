@@ -20,6 +20,7 @@
 // built in shared memory per source box, in as many phases as shared memory
 // requires, and every point's harmonics are generated on the fly.
 #include "hess.cuh"
+#include "eval_mm.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -302,14 +303,8 @@ __device__ __forceinline__ void stage_phase(bool loc, int p, int first, int n, c
 }
 
 // ---------------------------------------------------------------- far field of the FMM
+// (orders above 34, whose two column blocks exceed shared memory: a CTA per leaf, one point per thread)
 constexpr int kEvalHThreads = 128;
-
-// Side of box b: its instance's root side (forests) or the tree's, halved per level.
-__device__ __forceinline__ double hbox_side(const TreeView &tv, int b)
-{
-    const double size = tv.binst ? tv.inst_geom[4 * tv.binst[b] + 3] : tv.size;
-    return size / (double)(1L << tv.level[b]);
-}
 
 __global__ void __launch_bounds__(kEvalHThreads) k_eval_hess(const int *leaves, TreeView tv, const double *sx,
                                                               const double *sy, const double *sz, const double *tx,
@@ -342,7 +337,7 @@ __global__ void __launch_bounds__(kEvalHThreads) k_eval_hess(const int *leaves, 
         for (int ib = 0; ib < nsrcbox; ib++) {
             const bool loc = has_local && ib == 0;
             const int c = loc ? b : tv.l3_idx[l3a + ib - (has_local ? 1 : 0)];
-            const double s = hbox_side(tv, c), is = 1.0 / s;
+            const double s = box_side(tv, c), is = 1.0 / s;
             const double2 *coef = loc ? local + (size_t)c * K : mpole + (size_t)c * K;
             const double ux = (px - tv.center[3L * c]) * is, uy = (py - tv.center[3L * c + 1]) * is,
                          uz = (pz - tv.center[3L * c + 2]) * is;
@@ -371,22 +366,113 @@ __global__ void __launch_bounds__(kEvalHThreads) k_eval_hess(const int *leaves, 
     }
 }
 
+// Hessians of one work item in matrix products (eval_mm.cuh): six complex
+// quantities in two column blocks.  Balanced like the potentials' pass: on a
+// Plummer ball of 40k + 25k points, where one leaf has dozens of list-3 boxes,
+// a CTA per leaf with one point per thread took 19.4 ms.
+__global__ void __launch_bounds__(kEvalThreads) k_eval_hess_mm(const int *leaves, int nleaves, const int *off,
+                                                               const int *soff, TreeView tv, const double *sx,
+                                                               const double *sy, const double *sz, const double *tx,
+                                                               const double *ty, const double *tz, int p,
+                                                               const double2 *mpole, const double2 *local,
+                                                               HessSoA hs, HessSoA ht, int do_src, int do_trg,
+                                                               int hsrc, int htrg, double *part)
+{
+    extern __shared__ double hmm_sm[];
+    const int l = emm_leaf(off, nleaves, blockIdx.x), b = leaves[l];
+    const int ns = do_src ? tv.nsrc[b] : 0, ne = ns + (do_trg ? tv.ntrg[b] : 0);
+    const int ngr = (eval_nbx(tv, b) + kEvalGroup - 1) / kEvalGroup;
+    const int local_item = blockIdx.x - off[l], ck = local_item / ngr, grp = local_item - ck * ngr;
+    const int e0 = ck * kEvalThreads, s0 = tv.src0[b], t0 = tv.trg0[b];
+    // chunks of points that want no Hessians
+    if ((!hsrc && e0 + kEvalThreads <= ns) || (!htrg && e0 >= ns)) return;
+    emm_item<2>(
+        hmm_sm, p + 2, tv, b, grp, e0, ne, ns, sx, sy, sz, tx, ty, tz, (p + 1) * (p + 1), mpole, local,
+        [&](bool loc) { return loc ? p - 2 : p + 2; },
+        [](double is, int) { return is * is * is; },
+        [&](bool loc, const double2 *C, int n, int mu, double2 *v) {
+            int lo, hi;
+            kind_range(loc, p, 4, lo, hi);
+            if (n < lo || n > hi) return;
+            double2 a[kNumKinds], h[6];
+#pragma unroll
+            for (int q = 4; q < kNumKinds; q++)
+                a[q] = deriv_coef(loc, p, q, n, mu, [&](int k, int m) { return C[eidx(k, m)]; });
+#pragma unroll
+            for (int c = 0; c < 6; c++) h[c] = cmk(0, 0);
+            hess_from_ladders(a, 1.0, h);
+#pragma unroll
+            for (int c = 0; c < 6; c++) v[c] = h[c];
+        },
+        [&](int e, int k, double2 v) {
+            if (k >= 6 || !(e < ns ? hsrc : htrg)) return;
+            if (ngr > 1) {
+                double *o = part + ((size_t)(soff[l] + local_item) * 12 + 2 * k) * kEvalThreads + e - e0;
+                o[0] = v.x;
+                o[kEvalThreads] = v.y;
+                return;
+            }
+            double2 *o = (e < ns ? hs : ht).h[k] + (e < ns ? s0 + e : t0 + e - ns);
+            *o = cadd(*o, v);
+        });
+}
+
+// Adds the groups' sums of the leaves with more than one group, group by group.
+__global__ void __launch_bounds__(kEvalThreads) k_eval_hess_add(const int *leaves, const int *soff, TreeView tv,
+                                                                HessSoA hs, HessSoA ht, int do_src, int do_trg,
+                                                                int hsrc, int htrg, const double *part)
+{
+    const int l = blockIdx.x, b = leaves[l], nbx = eval_nbx(tv, b);
+    if (nbx <= kEvalGroup) return;
+    const int ns = do_src ? tv.nsrc[b] : 0, ne = ns + (do_trg ? tv.ntrg[b] : 0);
+    const int ngr = (nbx + kEvalGroup - 1) / kEvalGroup, nch = (ne + kEvalThreads - 1) / kEvalThreads;
+    for (int ck = blockIdx.y; ck < nch; ck += gridDim.y) {
+        const int e = ck * kEvalThreads + threadIdx.x;
+        if (e >= ne || !(e < ns ? hsrc : htrg)) continue;
+        const int i = e < ns ? tv.src0[b] + e : tv.trg0[b] + e - ns;
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            double2 *o = (e < ns ? hs : ht).h[c] + i, v = *o;
+            for (int g = 0; g < ngr; g++) {
+                const double *q = part + ((size_t)(soff[l] + ck * ngr + g) * 12 + 2 * c) * kEvalThreads + threadIdx.x;
+                v = cadd(v, cmk(q[0], q[kEvalThreads]));
+            }
+            *o = v;
+        }
+    }
+}
+
 static constexpr size_t kHessSmemMax = 200 * 1024;
 
-void launch_eval_hess(const int *leaves, int nleaves, const TreeView &tv, const double *sx, const double *sy,
-                      const double *sz, const double *tx, const double *ty, const double *tz, int p,
+void launch_eval_hess(const int *leaves, int nleaves, const EvalItems &E, const TreeView &tv, const double *sx,
+                      const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, int p,
                       const double2 *mpole, const double2 *local, HessSoA hs, HessSoA ht, int do_src, int do_trg,
-                      cudaStream_t s, Status &st)
+                      int hsrc, int htrg, cudaStream_t s, Status &st)
 {
-    if (nleaves == 0 || !st.ok() || !(do_src || do_trg)) return;
+    if (nleaves == 0 || !st.ok() || !(hsrc || htrg)) return;
     if (p > kHessMaxP) { st.err = cudaErrorInvalidValue; st.where = "Hessian: expansion order above the table"; return; }
+    const size_t mm = sizeof(double) * emm_smem(p + 2, 2);
+    if (mm <= kEmmSmemMax) {
+        if (E.nitems == 0) return;
+        FMM_TRY(st, smem_allow(k_eval_hess_mm, mm));
+        if (!st.ok()) return;
+        k_eval_hess_mm<<<E.nitems, kEvalThreads, mm, s>>>(leaves, nleaves, E.off.p, E.soff.p, tv, sx, sy, sz, tx, ty,
+                                                          tz, p, mpole, local, hs, ht, do_src, do_trg, hsrc, htrg,
+                                                          E.hpart.p); FMM_COUNT_LAUNCH();
+        if (E.nscratch > 0) {
+            k_eval_hess_add<<<dim3(nleaves, 2), kEvalThreads, 0, s>>>(leaves, E.soff.p, tv, hs, ht, do_src, do_trg,
+                                                                      hsrc, htrg, E.hpart.p); FMM_COUNT_LAUNCH();
+        }
+        FMM_LAUNCH_CHECK(st);
+        return;
+    }
     const size_t arr = (size_t)(p + 3) * (p + 3) * sizeof(double2);
     const int per_phase = (int)std::min<size_t>(5, kHessSmemMax / arr);
     const size_t smem = per_phase * arr;
     FMM_TRY(st, smem_allow(k_eval_hess, (int)smem));
     if (!st.ok()) return;
     k_eval_hess<<<nleaves, kEvalHThreads, smem, s>>>(leaves, tv, sx, sy, sz, tx, ty, tz, p, mpole, local, hs, ht,
-                                                     do_src, do_trg, per_phase);
+                                                     hsrc, htrg, per_phase);
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
 }

@@ -22,8 +22,7 @@
 #include <map>
 #include <mutex>
 
-#include "dmma.cuh"
-#include "lap_kernels.cuh"
+#include "eval_mm.cuh"
 
 namespace fmm {
 
@@ -130,13 +129,6 @@ __device__ __forceinline__ double2 tab_get(const double2 *tab, int stride, int n
     if (n < 0 || m > n || -m > n) return cmk(0, 0);
     double2 v = tab[stride * tidx(n, m < 0 ? -m : m)];
     return m < 0 ? cconj(v) : v;
-}
-
-// Side of box b: the root side of its instance (forests) or of the tree, halved per level.
-__device__ __forceinline__ double box_side(const TreeView &tv, int b)
-{
-    const double size = tv.binst ? tv.inst_geom[4 * tv.binst[b] + 3] : tv.size;
-    return size / (double)(1L << tv.level[b]);
 }
 
 // ================================================================ P2P
@@ -1030,8 +1022,6 @@ void launch_p2l(const int *boxes, int nboxes, const TreeView &tv, const PointsSo
 // are four dot products of coefficient arrays (in shared memory) with the
 // harmonics of the point, generated on the fly.  Adds to the outputs (the
 // near field is summed into them first, concurrently with the far field).
-constexpr int kEvalThreads = 128;
-
 // MASK selects the sums that a call feeds: bit 0 the potential (A), bit 1 the
 // z-gradient (Gz), bit 2 the two transverse gradients (Gp, Gm).
 template <int MASK>
@@ -1168,19 +1158,9 @@ __device__ __forceinline__ void eval_point(bool loc, int p, double ux, double uy
 // the scratch offsets (soff) come from k_eval_count and two scans, made with
 // the tree.
 //
-// NPH = 1: the coefficients and the three gradient arrays are staged together
-// (4 (p+2)^2 complex values of shared memory).  NPH = 2, for orders whose four
-// arrays exceed shared memory (p > 58): the potential and z-gradient first,
-// then the transverse gradients, in half the space; each point's harmonics
-// are generated once per phase, and every sum gets the same terms in the same
-// order as with one phase.
-constexpr int kEvalGroup = 8;
-
-__device__ __forceinline__ int eval_nbx(const TreeView &tv, int b)
-{
-    return (tv.level[b] >= 2 ? 1 : 0) + tv.l3_start[b + 1] - tv.l3_start[b];
-}
-
+// k_eval_mm serves the orders whose columns fit shared memory (p <= 51).  k_eval, above
+// them: the potential and z-gradient first, then the transverse gradients, each
+// point's harmonics generated once per phase, one point per thread.
 __global__ void k_eval_count(const int *leaves, int nleaves, TreeView tv, int do_src, int do_trg, int *cnt,
                              int *scnt)
 {
@@ -1195,7 +1175,70 @@ __global__ void k_eval_count(const int *leaves, int nleaves, TreeView tv, int do
     scnt[l] = nbx > kEvalGroup ? items : 0;
 }
 
-template <int NPH>
+// Gradient coefficients of (k, mu) of an order-p expansion C: d/dz, D+ and D-.
+__device__ __forceinline__ void grad_coefs(bool loc, int p, const double2 *C, int k, int mu, double2 &z, double2 &dp,
+                                           double2 &dm)
+{
+    z = dp = dm = cmk(0, 0);
+    if (loc) {
+        if (k >= p) return;
+        z = cscal(sqrt((double)(k + 1 + mu) * (k + 1 - mu)), C[eidx(k + 1, mu)]);
+        dp = cscal((mu <= 0 ? -1.0 : 1.0) * sqrt((double)(k + 2 - mu) * (k + 1 - mu)), C[eidx(k + 1, mu - 1)]);
+        dm = cscal((mu >= 0 ? -1.0 : 1.0) * sqrt((double)(k + 2 + mu) * (k + 1 + mu)), C[eidx(k + 1, mu + 1)]);
+    } else {
+        if (k < 1) return;
+        if (abs(mu) <= k - 1) z = cscal(-sqrt((double)(k + mu) * (k - mu)), C[eidx(k - 1, mu)]);
+        if (abs(mu - 1) <= k - 1)
+            dp = cscal((mu <= 0 ? -1.0 : 1.0) * sqrt((double)(k + mu - 1) * (k + mu)), C[eidx(k - 1, mu - 1)]);
+        if (abs(mu + 1) <= k - 1)
+            dm = cscal((mu >= 0 ? -1.0 : 1.0) * sqrt((double)(k - mu - 1) * (k - mu)), C[eidx(k - 1, mu + 1)]);
+    }
+}
+
+// Potential and field of a work item in matrix products (eval_mm.cuh): the 8
+// columns are the potential and the three gradient components, real and
+// imaginary.
+__global__ void __launch_bounds__(kEvalThreads) k_eval_mm(const int *leaves, int nleaves, const int *off,
+                                                          const int *soff, TreeView tv, const double *sx,
+                                                          const double *sy, const double *sz, const double *tx,
+                                                          const double *ty, const double *tz, int p,
+                                                          const double2 *mpole, const double2 *local, OutSoA outs,
+                                                          OutSoA outt, int do_src, int do_trg, double *part)
+{
+    extern __shared__ double emm_sm[];
+    const int l = emm_leaf(off, nleaves, blockIdx.x), b = leaves[l];
+    const int ns = do_src ? tv.nsrc[b] : 0, ne = ns + (do_trg ? tv.ntrg[b] : 0);
+    const int ngr = (eval_nbx(tv, b) + kEvalGroup - 1) / kEvalGroup;
+    const int local_item = blockIdx.x - off[l], ck = local_item / ngr, grp = local_item - ck * ngr;
+    const int s0 = tv.src0[b], t0 = tv.trg0[b];
+    emm_item<1>(
+        emm_sm, p + 1, tv, b, grp, ck * kEvalThreads, ne, ns, sx, sy, sz, tx, ty, tz, (p + 1) * (p + 1), mpole, local,
+        [&](bool loc) { return loc ? p : p + 1; },
+        [](double is, int k) { return k ? is * is : is; },
+        [&](bool loc, const double2 *C, int n, int mu, double2 *v) {
+            if (n <= p) v[0] = C[eidx(n, mu)];
+            double2 z, dp, dm;
+            grad_coefs(loc, p, C, n, mu, z, dp, dm);
+            const double2 d = csub(dp, dm);
+            v[1] = cscal(0.5, cadd(dp, dm));             // d/dx = (D+ + D-) / 2
+            v[2] = cmk(0.5 * d.y, -0.5 * d.x);           // d/dy = (D+ - D-) / 2i
+            v[3] = z;
+        },
+        [&](int e, int k, double2 v) {
+            if (k) v = cmk(-v.x, -v.y);                  // the field is minus the gradient
+            if (ngr > 1) {
+                double *o = part + ((size_t)(soff[l] + local_item) * 8 + 2 * k) * kEvalThreads + e - ck * kEvalThreads;
+                o[0] = v.x;
+                o[kEvalThreads] = v.y;
+                return;
+            }
+            const OutSoA &o = e < ns ? outs : outt;
+            double2 *a = k == 0 ? o.pot : k == 1 ? o.fx : k == 2 ? o.fy : o.fz;
+            const int i = e < ns ? s0 + e : t0 + e - ns;
+            if (a) a[i] = cadd(a[i], v);
+        });
+}
+
 __global__ void __launch_bounds__(kEvalThreads) k_eval(const int *leaves, int nleaves, const int *off,
                                                        const int *soff, TreeView tv, const double *sx,
                                                        const double *sy, const double *sz, const double *tx,
@@ -1206,18 +1249,7 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval(const int *leaves, int nl
     extern __shared__ double2 sm[];
     const int K = (p + 1) * (p + 1), K1 = (p + 2) * (p + 2);
     double2 *b0 = sm, *b1 = sm + K1;
-    double2 *b2 = NPH == 1 ? b1 + K1 : b0, *b3 = NPH == 1 ? b2 + K1 : b1;
-    const int item = blockIdx.x;
-    int l;
-    {
-        int lo = 0, hi = nleaves - 1;   // the last leaf with off[l] <= item
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (off[mid] <= item) lo = mid;
-            else hi = mid - 1;
-        }
-        l = lo;
-    }
+    const int item = blockIdx.x, l = emm_leaf(off, nleaves, item);
     const int b = leaves[l];
     const int lev = tv.level[b];
     const int s0 = tv.src0[b], ns = do_src ? tv.nsrc[b] : 0;
@@ -1245,22 +1277,17 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval(const int *leaves, int nl
         const double ux = (px - tv.center[3L * c]) * is, uy = (py - tv.center[3L * c + 1]) * is,
                      uz = (pz - tv.center[3L * c + 2]) * is;
         double2 phi = cmk(0, 0), dz = cmk(0, 0), dp = cmk(0, 0), dm = cmk(0, 0);
-        for (int ph = 0; ph < NPH; ph++) {
+        for (int ph = 0; ph < 2; ph++) {
             __syncthreads();
-            if (NPH == 1 || ph == 0)
+            if (ph == 0) {
                 for (int i = threadIdx.x; i < K; i += kEvalThreads) b0[i] = coef[i];
-            if (NPH == 1) {
-                __syncthreads();
-                stage_grad<6>(loc, p, b0, b1, b2, b3);
-            } else if (ph == 0) {
                 stage_grad<2>(loc, p, coef, b1, nullptr, nullptr);
             } else {
                 stage_grad<4>(loc, p, coef, nullptr, b0, b1);
             }
             __syncthreads();
             if (!act) continue;
-            if (NPH == 1) eval_point<7>(loc, p, ux, uy, uz, b0, b1, b2, b3, phi, dz, dp, dm);
-            else if (ph == 0) eval_point<3>(loc, p, ux, uy, uz, b0, b1, nullptr, nullptr, phi, dz, dp, dm);
+            if (ph == 0) eval_point<3>(loc, p, ux, uy, uz, b0, b1, nullptr, nullptr, phi, dz, dp, dm);
             else eval_point<4>(loc, p, ux, uy, uz, nullptr, nullptr, b0, b1, phi, dz, dp, dm);
         }
         if (!act) continue;
@@ -1338,8 +1365,8 @@ __global__ void k_eval_totals(int n, const int *cnt, const int *scnt, const int 
     tot[1] = soff[n - 1] + scnt[n - 1];
 }
 
-int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, EvalItems &E,
-                       cudaStream_t s, Status &st)
+int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, int hess,
+                       EvalItems &E, cudaStream_t s, Status &st)
 {
     E.nitems = E.nscratch = 0;
     if (nleaves == 0 || !st.ok()) return 0;
@@ -1364,6 +1391,7 @@ int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int d
     E.nitems = h[0];
     E.nscratch = h[1];
     if (E.nscratch > 0) E.part.alloc((size_t)E.nscratch * 8 * kEvalThreads, s, st);
+    if (E.nscratch > 0 && hess) E.hpart.alloc((size_t)E.nscratch * 12 * kEvalThreads, s, st);
     return E.nitems;
 }
 
@@ -1373,18 +1401,18 @@ void launch_eval(const int *leaves, int nleaves, const EvalItems &E, const TreeV
                  cudaStream_t s, Status &st)
 {
     if (nleaves == 0 || E.nitems == 0 || !st.ok()) return;
-    const size_t arr = (size_t)(p + 2) * (p + 2) * sizeof(double2);
-    if (4 * arr <= 226 * 1024) {
-        FMM_TRY(st, smem_allow(k_eval<1>, (int)(4 * arr)));
-        k_eval<1><<<E.nitems, kEvalThreads, 4 * arr, s>>>(leaves, nleaves, E.off.p, E.soff.p, tv, sx, sy, sz, tx, ty,
-                                                          tz, p, mpole, local, outs, outt, do_src, do_trg, E.part.p);
-        FMM_COUNT_LAUNCH();
+    const size_t mm = sizeof(double) * emm_smem(p + 1, 1);
+    if (mm <= kEmmSmemMax) {
+        FMM_TRY(st, smem_allow(k_eval_mm, mm));
+        k_eval_mm<<<E.nitems, kEvalThreads, mm, s>>>(leaves, nleaves, E.off.p, E.soff.p, tv, sx, sy, sz, tx, ty, tz, p,
+                                                     mpole, local, outs, outt, do_src, do_trg, E.part.p);
     } else {
-        FMM_TRY(st, smem_allow(k_eval<2>, (int)(2 * arr)));
-        k_eval<2><<<E.nitems, kEvalThreads, 2 * arr, s>>>(leaves, nleaves, E.off.p, E.soff.p, tv, sx, sy, sz, tx, ty,
-                                                          tz, p, mpole, local, outs, outt, do_src, do_trg, E.part.p);
-        FMM_COUNT_LAUNCH();
+        const size_t arr = (size_t)(p + 2) * (p + 2) * sizeof(double2);
+        FMM_TRY(st, smem_allow(k_eval, 2 * arr));
+        k_eval<<<E.nitems, kEvalThreads, 2 * arr, s>>>(leaves, nleaves, E.off.p, E.soff.p, tv, sx, sy, sz, tx, ty, tz,
+                                                       p, mpole, local, outs, outt, do_src, do_trg, E.part.p);
     }
+    FMM_COUNT_LAUNCH();
     if (E.nscratch > 0) {
         k_eval_add<<<dim3(nleaves, 2), kEvalThreads, 0, s>>>(leaves, E.soff.p, tv, outs, outt, do_src, do_trg,
                                                              E.part.p);

@@ -70,11 +70,11 @@ void launch_p2l(const int *boxes, int nboxes, const TreeView &tv, const PointsSo
 // enqueues kernels (graph-capturable).
 struct EvalItems {
     DBuf<int> off, soff;
-    DBuf<double> part;
+    DBuf<double> part, hpart;   // hpart: the Hessians' sums
     int nitems = 0, nscratch = 0;
 };
-int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, EvalItems &E,
-                       cudaStream_t s, Status &st);
+int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, int hess,
+                       EvalItems &E, cudaStream_t s, Status &st);
 void launch_eval(const int *leaves, int nleaves, const EvalItems &E, const TreeView &tv, const double *sx,
                  const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, int p,
                  const double2 *mpole, const double2 *local, OutSoA outs, OutSoA outt, int do_src, int do_trg,
