@@ -147,8 +147,22 @@ inline int div_up(long a, long b) { return (int)((a + b - 1) / b); }
 // Exclusive prefix sum of n ints; out may alias in. Returns total (host) when
 // want_total is set (one device->host read).
 void scan_exclusive_int(const int *d_in, int *d_out, int n, cudaStream_t s, Status &st, int *h_total);
-// Stable LSD radix sort of 64-bit keys with 32-bit payload over the low
-// `bits` bits of the key.
-void radix_sort_u64(uint64_t *d_keys, int *d_vals, int n, int bits, cudaStream_t s, Status &st);
+// Several scans at once, their totals on the device.  n_dev (if set) holds the
+// length on the device; n is then unused.
+struct ScanJob {
+    const int *in;
+    int *out;
+    int n;
+    const int *n_dev;
+};
+constexpr int kScanJobs = 4;
+struct ScanJobs {
+    ScanJob job[kScanJobs];
+};
+void scan_exclusive_multi(const ScanJob *jobs, int njobs, int *d_totals, cudaStream_t s, Status &st);
+// Stable LSD radix sort of 64-bit keys with 32-bit payload over the bits low ..
+// bits - 1 of the key, of one array or of two in the same launches (k2 may be null).
+void radix_sort_pair(DBuf<uint64_t> &k1, DBuf<int> &v1, int n1, DBuf<uint64_t> *k2, DBuf<int> *v2, int n2, int low,
+                     int bits, cudaStream_t s, Status &st);
 
 }  // namespace fmm

@@ -624,12 +624,17 @@ static void lap_widen_near(LapSetup &S, int thr, cudaStream_t s, Status &st)
     c4.zero(st);
     k_near_count<<<div_up(nb, 256), 256, 0, s>>>(nb, S.tv, thr, S.do_src, S.do_trg, cn.p, c3.p, c4.p); FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
-    int tn = 0, t3 = 0, t4 = 0;
-    scan_exclusive_int(cn.p, S.nl_start.p, nb + 1, s, st, &tn);
-    scan_exclusive_int(c3.p, S.fl_start.p, nb + 1, s, st, &t3);
-    scan_exclusive_int(c4.p, S.f4_start.p, nb + 1, s, st, &t4);
-    if (!st.ok() || !S.nl_idx.alloc(std::max(tn, 1), s, st) || !S.fl_idx.alloc(std::max(t3, 1), s, st) ||
-        !S.f4_idx.alloc(std::max(t4, 1), s, st))
+    DBuf<int> tot;
+    int h[3] = {0, 0, 0};   // entries of the near and the two far lists
+    if (!tot.alloc(3, s, st)) return;
+    const ScanJob jobs[3] = {{cn.p, S.nl_start.p, nb + 1, nullptr},
+                             {c3.p, S.fl_start.p, nb + 1, nullptr},
+                             {c4.p, S.f4_start.p, nb + 1, nullptr}};
+    scan_exclusive_multi(jobs, 3, tot.p, s, st);
+    FMM_TRY(st, cudaMemcpyAsync(h, tot.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FMM_TRY(st, cudaStreamSynchronize(s));
+    if (!st.ok() || !S.nl_idx.alloc(std::max(h[0], 1), s, st) || !S.fl_idx.alloc(std::max(h[1], 1), s, st) ||
+        !S.f4_idx.alloc(std::max(h[2], 1), s, st))
         return;
     k_near_fill<<<div_up(nb, 256), 256, 0, s>>>(nb, S.tv, thr, S.do_src, S.do_trg, S.nl_start.p, S.fl_start.p,
                                                S.f4_start.p, S.nl_idx.p, S.fl_idx.p, S.f4_idx.p); FMM_COUNT_LAUNCH();

@@ -1359,12 +1359,6 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_add(const int *leaves, co
     }
 }
 
-__global__ void k_eval_totals(int n, const int *cnt, const int *scnt, const int *off, const int *soff, int *tot)
-{
-    tot[0] = off[n - 1] + cnt[n - 1];
-    tot[1] = soff[n - 1] + scnt[n - 1];
-}
-
 int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, int hess,
                        EvalItems &E, cudaStream_t s, Status &st)
 {
@@ -1377,14 +1371,11 @@ int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int d
     k_eval_count<<<div_up(nleaves, 256), 256, 0, s>>>(leaves, nleaves, tv, do_src, do_trg, cnt.p, scnt.p);
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
-    scan_exclusive_int(cnt.p, E.off.p, nleaves, s, st, nullptr);
-    scan_exclusive_int(scnt.p, E.soff.p, nleaves, s, st, nullptr);
-    // both totals in one copy: the last offsets plus the last counts
     DBuf<int> tot;
     int h[2] = {0, 0};
     if (!tot.alloc(2, s, st)) return 0;
-    k_eval_totals<<<1, 1, 0, s>>>(nleaves, cnt.p, scnt.p, E.off.p, E.soff.p, tot.p);
-    FMM_COUNT_LAUNCH();
+    const ScanJob jobs[2] = {{cnt.p, E.off.p, nleaves, nullptr}, {scnt.p, E.soff.p, nleaves, nullptr}};
+    scan_exclusive_multi(jobs, 2, tot.p, s, st);
     FMM_TRY(st, cudaMemcpyAsync(h, tot.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     FMM_TRY(st, cudaStreamSynchronize(s));
     if (!st.ok()) return 0;
@@ -1494,8 +1485,9 @@ __device__ void regular_table_rot(double x, double y, double z, int p, double2 *
     }
 }
 
-__global__ void k_rot_nodes(int p, int nq, const double *gl_x, const double *cs, int cls, double2 *Sr, double2 *S0)
+__global__ void k_rot_nodes(int p, int nq, const double *gl_x, const double *cs, int cls0, double2 *Sr, double2 *S0)
 {
+    const int cls = cls0 + blockIdx.y;
     // one thread per quadrature node: harmonics at the node and at the rotated node
     int nphi = 2 * p + 1;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1509,8 +1501,8 @@ __global__ void k_rot_nodes(int p, int nq, const double *gl_x, const double *cs,
     double ct = cs[2 * cls], stt = cs[2 * cls + 1];
     double rx = wx * ct + wz * stt, ry = wy, rz = -wx * stt + wz * ct;
     int ntab = (p + 1) * (p + 2) / 2;
-    regular_table_rot(rx, ry, rz, p, Sr + (size_t)i * ntab);
-    if (S0) regular_table_rot(wx, wy, wz, p, S0 + (size_t)i * ntab);
+    regular_table_rot(rx, ry, rz, p, Sr + ((size_t)blockIdx.y * nq * nphi + i) * ntab);
+    if (S0 && blockIdx.y == 0) regular_table_rot(wx, wy, wz, p, S0 + (size_t)i * ntab);
 }
 
 __global__ void k_rot_reduce(int p, int nq, const double *gl_w, const double2 *Sr, const double2 *S0, double *rot)
@@ -1526,6 +1518,8 @@ __global__ void k_rot_reduce(int p, int nq, const double *gl_w, const double2 *S
     int r = (int)((e - off) / w), c = (int)((e - off) % w);
     int m = r - n, mp = c - n;
     int nphi = 2 * p + 1, ntab = (p + 1) * (p + 2) / 2;
+    Sr += (size_t)blockIdx.y * nq * nphi * ntab;
+    rot += tot * blockIdx.y;
     double acc = 0;
     int tm = tidx(n, m < 0 ? -m : m), tmp = tidx(n, mp < 0 ? -mp : mp);
     for (int i = 0; i < nq * nphi; i++) {
@@ -1595,15 +1589,20 @@ void build_rotations(int p, int ncls, const double *d_cs, double *d_rot, cudaStr
     DBuf<double2> Sr, S0;
     dx.alloc(nq, s, st);
     dw.alloc(nq, s, st);
-    Sr.alloc((size_t)nodes * ntab, s, st);
+    // as many classes per launch as 256 MB of node tables hold
+    const int per = (int)std::max<size_t>(1, std::min<size_t>(ncls, (256u << 20) / ((size_t)nodes * ntab * 16)));
+    Sr.alloc((size_t)nodes * ntab * per, s, st);
     S0.alloc((size_t)nodes * ntab, s, st);
     if (!st.ok()) return;
     FMM_TRY(st, cudaMemcpyAsync(dx.p, gx.data(), sizeof(double) * nq, cudaMemcpyHostToDevice, s));
     FMM_TRY(st, cudaMemcpyAsync(dw.p, gw.data(), sizeof(double) * nq, cudaMemcpyHostToDevice, s));
     size_t csz = rot_class_size(p);
-    for (int c = 0; c < ncls; c++) {
-        k_rot_nodes<<<div_up(nodes, 128), 128, 0, s>>>(p, nq, dx.p, d_cs, c, Sr.p, c == 0 ? S0.p : nullptr); FMM_COUNT_LAUNCH();
-        k_rot_reduce<<<div_up((long)csz, 128), 128, 0, s>>>(p, nq, dw.p, Sr.p, S0.p, d_rot + csz * c); FMM_COUNT_LAUNCH();
+    for (int c = 0; c < ncls; c += per) {
+        const int k = std::min(per, ncls - c);
+        k_rot_nodes<<<dim3(div_up(nodes, 128), k), 128, 0, s>>>(p, nq, dx.p, d_cs, c, Sr.p, c == 0 ? S0.p : nullptr);
+        FMM_COUNT_LAUNCH();
+        k_rot_reduce<<<dim3(div_up((long)csz, 128), k), 128, 0, s>>>(p, nq, dw.p, Sr.p, S0.p, d_rot + csz * c);
+        FMM_COUNT_LAUNCH();
     }
     FMM_LAUNCH_CHECK(st);
     FMM_TRY(st, cudaStreamSynchronize(s));  // the host vectors above must outlive the copies

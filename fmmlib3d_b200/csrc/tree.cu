@@ -171,17 +171,28 @@ __device__ int lower_digit(const uint64_t *keys, int lo, int hi, int child_level
     return lo;
 }
 
+// Boxes of every level on the device: first box and count, so that several
+// levels can be built before the host reads the counts back.
+struct LevelTable {
+    int start[kMaxLevel + 2], count[kMaxLevel + 2];
+    int total;   // children of the current level
+    int over;    // level whose boxes did not fit the arrays (0: none)
+    int want;    // and their number
+    double geom[4];   // bounding cube of the (first) tree
+};
+
 // Split decision and child ranges for the boxes of one level
 // (d3tallbem, src/d3tstrcr.f:1458-1578).  Sixteen threads per box: the
 // fourteen digit boundaries (7 source, 7 target) are independent binary
 // searches over the box's sorted range, done in parallel.
 constexpr int kSplitLanes = 16;
 
-__global__ void k_split(int b0, int nb, int level, int nbox, TreeOptions opt, const int *src0, const int *nsrc,
+__global__ void k_split(const LevelTable *L, int level, int nbox, TreeOptions opt, const int *src0, const int *nsrc,
                         const int *trg0, const int *ntrg, const uint64_t *ksrc, const uint64_t *ktrg, int *nkids,
                         int *cs0, int *cns, int *ct0, int *cnt)
 {
     __shared__ int bound[128 / kSplitLanes][16];
+    const int b0 = L->start[level], nb = L->count[level];
     const int g = threadIdx.x / kSplitLanes, j = threadIdx.x % kSplitLanes;
     const int t = blockIdx.x * (blockDim.x / kSplitLanes) + g;
     const bool live = t < nb;
@@ -217,13 +228,24 @@ __global__ void k_split(int b0, int nb, int level, int nbox, TreeOptions opt, co
     nkids[t] = k;
 }
 
-__global__ void k_make_children(int b0, int nb, int level, int next0, int keep_empty, const int *kbase,
+__global__ void k_make_children(LevelTable *L, int level, int cap, int keep_empty, const int *kbase,
                                 const int *nkids, const int *cs0, const int *cns, const int *ct0, const int *cnt,
                                 const double *geom_all, int *ijk, int *lev, int *par, int *oct, int *nch,
                                 int *child, int *src0, int *nsrc, int *trg0, int *ntrg, double *center, int *binst)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nb) return;
+    const int b0 = L->start[level], nb = L->count[level], next0 = b0 + nb;
+    const int total = nb > 0 ? L->total : 0;
+    const bool fits = total <= cap - next0;
+    if (t == 0) {
+        L->start[level + 1] = next0;
+        L->count[level + 1] = fits ? total : 0;
+        if (!fits) {
+            L->over = level + 1;
+            L->want = total;
+        }
+    }
+    if (t >= nb || !fits) return;
     int b = b0 + t;
     int id = next0 + kbase[t];
     nch[b] = nkids[t];
@@ -258,43 +280,49 @@ __global__ void k_make_children(int b0, int nb, int level, int next0, int keep_e
 }
 
 // Root box of every instance (box id = instance id).
-__global__ void k_root(int ninst, const int *so, const int *to, const double *geom, int *ijk, int *lev, int *par,
+__global__ void k_root(int ninst, const int *so, const int *to, int n, int m, LevelTable *L, const double *geom, int *ijk, int *lev, int *par,
                        int *oct, int *nch, int *child, int *src0, int *nsrc, int *trg0, int *ntrg, double *center,
                        int *binst)
 {
     int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r == 0) {
+        L->start[0] = 0;
+        L->count[0] = ninst;
+        L->over = L->want = 0;
+        for (int e = 0; e < 4; e++) L->geom[e] = geom[e];
+    }
     if (r >= ninst) return;
     for (int e = 0; e < 3; e++) { ijk[3 * r + e] = 0; center[3 * r + e] = geom[4 * r + e]; }
     lev[r] = 0; par[r] = -1; oct[r] = 0; nch[r] = 0; binst[r] = r;
     for (int e = 0; e < 8; e++) child[8 * r + e] = -1;
-    src0[r] = so[r]; nsrc[r] = so[r + 1] - so[r]; trg0[r] = to[r]; ntrg[r] = to[r + 1] - to[r];
+    // (one tree: the whole arrays)
+    src0[r] = so ? so[r] : 0; nsrc[r] = so ? so[r + 1] - so[r] : n;
+    trg0[r] = to ? to[r] : 0; ntrg[r] = to ? to[r + 1] - to[r] : m;
 }
 
 // ---------------------------------------------------------------- colleagues (list 5 plus self)
-__global__ void k_colleagues(int b0, int nb, const int *ijk, const int *par, const int *child, int *coll)
+// One thread per (box, slot): the neighbour at offset d of a box with octant bits
+// o lies in the parent's colleague at floor((o + d) / 2), child (o + d) mod 2.
+__global__ void k_colleagues(int b0, int nb, const int *oct, const int *par, const int *child, int *coll)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nb) return;
-    int b = b0 + t;
-    int out[27];
-    for (int s = 0; s < 27; s++) out[s] = -1;
-    int P = par[b];
+    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (t >= 27L * nb) return;
+    const int b = b0 + (int)(t / 27), s = (int)(t % 27), P = par[b];
+    int out = -1;
     if (P < 0) {
-        out[13] = b;
+        out = s == 13 ? b : -1;
     } else {
-        for (int s = 0; s < 27; s++) {
-            int C = coll[27L * P + s];
-            if (C < 0) continue;
-            for (int d = 0; d < 8; d++) {
-                int ch = child[8L * C + d];
-                if (ch < 0) continue;
-                int dx = ijk[3L * ch] - ijk[3L * b], dy = ijk[3L * ch + 1] - ijk[3L * b + 1],
-                    dz = ijk[3L * ch + 2] - ijk[3L * b + 2];
-                if (abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1) out[coll_slot(dx, dy, dz)] = ch;
-            }
+        const int o = oct[b], d[3] = {s / 9 - 1, (s / 3) % 3 - 1, s % 3 - 1};
+        int slot = 0, ch = 0;
+        for (int e = 0; e < 3; e++) {
+            const int pos = (o >> e & 1) + d[e];
+            slot = slot * 3 + (pos >> 1) + 1;
+            ch |= (pos & 1) << e;
         }
+        const int C = coll[27L * P + slot];
+        if (C >= 0) out = child[8L * C + ch];
     }
-    for (int s = 0; s < 27; s++) coll[27L * b + s] = out[s];
+    coll[27L * b + s] = out;
 }
 
 // Closed boxes on (possibly different) levels intersect or touch: the
@@ -314,68 +342,81 @@ __device__ __forceinline__ bool touch(const int *ijk, const int *lev, int a, int
 // Lists 1 and 3 of a childless non-root box b (d3tlsts/d3tlst31,
 // src/d3tstrcr.f:827-851 and :912-1069).  List 1 = childless boxes that
 // touch b (any level); list 3 = boxes on finer levels that do not touch b
-// but whose parents do.  mode 0 counts, mode 1 writes.
-__global__ void k_lists13(const int *leaves, int nleaves, const int *ijk, const int *lev, const int *par,
-                          const int *nch, const int *child, const int *coll, int mode, int *n1, int *n3,
-                          const int *s1, int *i1, const int *s3, int *i3)
+// but whose parents do.  One warp per box: lane s walks the boxes below
+// colleague s, then the lanes take the ancestors' colleagues (childless boxes on
+// coarser levels are colleagues of an ancestor); entries in the order of the
+// slots.  FILL 0 counts (n1, n3 and the leaf flag of every box, zeros in the
+// entry past the end), 1 writes and counts the dual of list 3, list 4.
+template <int FILL>
+__device__ __forceinline__ void walk_below(int b, int C, const int *ijk, const int *lev, const int *nch,
+                                           const int *child, int &c1, int &c3, int *i1, int *i3, int *n4)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nleaves) return;
-    int b = leaves[t];
-    if (lev[b] == 0) {
-        if (mode == 0) { n1[b] = 0; n3[b] = 0; }
+    if (nch[C] == 0) {
+        if (FILL) i1[c1] = C;
+        c1++;
         return;
     }
-    int c1 = 0, c3 = 0;
-    int o1 = mode ? s1[b] : 0, o3 = mode ? s3[b] : 0;
-    int stk[8 * kMaxLevel + 8];
-    for (int s = 0; s < 27; s++) {
-        if (s == 13) continue;
-        int C = coll[27L * b + s];
-        if (C < 0) continue;
-        if (nch[C] == 0) {
-            if (mode) i1[o1 + c1] = C;
+    int stk[8 * kMaxLevel + 8], top = 0;
+    for (int d = 7; d >= 0; d--)
+        if (child[8L * C + d] >= 0) stk[top++] = child[8L * C + d];
+    while (top) {
+        const int x = stk[--top];
+        if (!touch(ijk, lev, b, x)) {
+            if (FILL) {
+                i3[c3] = x;
+                atomicAdd(&n4[x], 1);
+            }
+            c3++;
+        } else if (nch[x] == 0) {
+            if (FILL) i1[c1] = x;
             c1++;
-            continue;
-        }
-        int top = 0;
-        for (int d = 7; d >= 0; d--)
-            if (child[8L * C + d] >= 0) stk[top++] = child[8L * C + d];
-        while (top) {
-            int x = stk[--top];
-            if (!touch(ijk, lev, b, x)) {
-                if (mode) i3[o3 + c3] = x;
-                c3++;
-            } else if (nch[x] == 0) {
-                if (mode) i1[o1 + c1] = x;
-                c1++;
-            } else {
-                for (int d = 7; d >= 0; d--)
-                    if (child[8L * x + d] >= 0) stk[top++] = child[8L * x + d];
-            }
+        } else {
+            for (int d = 7; d >= 0; d--)
+                if (child[8L * x + d] >= 0) stk[top++] = child[8L * x + d];
         }
     }
-    // childless boxes on coarser levels are colleagues of an ancestor of b
-    for (int A = par[b]; A >= 0 && lev[A] >= 1; A = par[A]) {
-        for (int s = 0; s < 27; s++) {
-            if (s == 13) continue;
-            int C = coll[27L * A + s];
-            if (C < 0 || nch[C] != 0) continue;
-            if (touch(ijk, lev, b, C)) {
-                if (mode) i1[o1 + c1] = C;
-                c1++;
-            }
-        }
-    }
-    if (mode == 0) { n1[b] = c1; n3[b] = c3; }
 }
 
-__global__ void k_list4_count(const int *leaves, int nleaves, const int *s3, const int *i3, int *n4)
+template <int FILL>
+__global__ void __launch_bounds__(128) k_lists13(int nboxes, const int *ijk, const int *lev, const int *par,
+                                                 const int *nch, const int *child, const int *coll, int *n1, int *n3,
+                                                 int *flag, const int *s1, int *i1, const int *s3, int *i3, int *n4)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nleaves) return;
-    int b = leaves[t];
-    for (int k = s3[b]; k < s3[b + 1]; k++) atomicAdd(&n4[i3[k]], 1);
+    const int b = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b > nboxes) return;
+    if (b == nboxes || nch[b] != 0) {
+        if (!FILL && lane == 0) {
+            n1[b] = n3[b] = 0;
+            if (b < nboxes) flag[b] = 0;
+        }
+        return;
+    }
+    const int C = lane < 27 && lane != 13 ? coll[27L * b + lane] : -1;
+    int c1 = 0, c3 = 0;
+    if (C >= 0) walk_below<0>(b, C, ijk, lev, nch, child, c1, c3, nullptr, nullptr, nullptr);
+    int p1 = c1, p3 = c3;   // inclusive sums over the lanes
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, p1, o), v = __shfl_up_sync(0xffffffffu, p3, o);
+        if (lane >= o) { p1 += u; p3 += v; }
+    }
+    int t1 = __shfl_sync(0xffffffffu, p1, 31);
+    const int t3 = __shfl_sync(0xffffffffu, p3, 31);
+    if (FILL && C >= 0) {
+        int k1 = 0, k3 = 0;
+        walk_below<1>(b, C, ijk, lev, nch, child, k1, k3, i1 + s1[b] + p1 - c1, i3 + s3[b] + p3 - c3, n4);
+    }
+    for (int A = par[b]; A >= 0 && lev[A] >= 1; A = par[A]) {
+        const int D = lane < 27 && lane != 13 ? coll[27L * A + lane] : -1;
+        const bool in = D >= 0 && nch[D] == 0 && touch(ijk, lev, b, D);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (FILL && in) i1[s1[b] + t1 + __popc(m & ((1u << lane) - 1))] = D;
+        t1 += __popc(m);
+    }
+    if (!FILL && lane == 0) {
+        n1[b] = t1;
+        n3[b] = t3;
+        flag[b] = 1;
+    }
 }
 
 __global__ void k_list4_fill(const int *leaves, int nleaves, const int *s3, const int *i3, int *cursor, int *i4)
@@ -397,12 +438,6 @@ __global__ void k_sort_rows(int nb, const int *st, int *idx)
         while (j >= lo && idx[j] > v) { idx[j + 1] = idx[j]; j--; }
         idx[j + 1] = v;
     }
-}
-
-__global__ void k_flag_leaves(int nb, const int *nch, int *flag)
-{
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < nb) flag[b] = nch[b] == 0;
 }
 
 __global__ void k_compact(int nb, const int *flag, const int *pos, int *out)
@@ -441,6 +476,9 @@ bool grow(DBuf<T> &b, size_t need, size_t copy, cudaStream_t s, Status &st)
     return st.ok();
 }
 
+// Levels whose key bits the first sort covers (3 (21 - 13) = 24 bits left out).
+constexpr int kSortedLevel = 13;
+
 // Stable reorder of (key, perm) into instance-major order: sort by the
 // instance of each point (gathered through perm), carrying the position,
 // then gather keys and perm by the resulting order.
@@ -468,7 +506,7 @@ void instance_major(DBuf<uint64_t> &keys, DBuf<int> &perm, const DBuf<int> &pins
     DBuf<int> pos, p2;
     if (!ik.alloc(n, s, st) || !pos.alloc(n, s, st) || !k2.alloc(n, s, st) || !p2.alloc(n, s, st)) return;
     k_gather_inst<<<div_up(n, 256), 256, 0, s>>>(n, perm.p, pinst.p, ik.p, pos.p); FMM_COUNT_LAUNCH();
-    radix_sort_u64(ik.p, pos.p, n, ibits, s, st);
+    radix_sort_pair(ik, pos, n, nullptr, nullptr, 0, 0, ibits, s, st);
     k_apply_pos<<<div_up(n, 256), 256, 0, s>>>(n, pos.p, keys.p, perm.p, k2.p, p2.p); FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
     std::swap(keys.p, k2.p);
@@ -530,16 +568,18 @@ void build_forest(Tree &T, const double *d_src, const std::vector<int> &so, cons
     if (n) { k_keys<<<div_up(n, 256), 256, 0, s>>>(d_src, n, geom.p, ninst > 1 ? pis.p : nullptr, ks.p, T.perm_src.p); FMM_COUNT_LAUNCH(); }
     if (m) { k_keys<<<div_up(m, 256), 256, 0, s>>>(d_trg, m, geom.p, ninst > 1 ? pit.p : nullptr, kt.p, T.perm_trg.p); FMM_COUNT_LAUNCH(); }
     FMM_LAUNCH_CHECK(st);
-    radix_sort_u64(ks.p, T.perm_src.p, n, 3 * kMaxLevel, s, st);
-    radix_sort_u64(kt.p, T.perm_trg.p, m, 3 * kMaxLevel, s, st);
-    if (ninst > 1) {
-        int ibits = 8;
-        while ((1L << ibits) < ninst) ibits += 8;
-        instance_major(ks, T.perm_src, pis, n, ibits, s, st);
-        instance_major(kt, T.perm_trg, pit, m, ibits, s, st);
-    }
-    double hgeom[4];
-    FMM_TRY(st, cudaMemcpyAsync(hgeom, geom.p, sizeof(hgeom), cudaMemcpyDeviceToHost, s));
+    // The bits of the first kSortedLevel levels only: five passes instead of eight (a
+    // deeper tree sorts again by all bits before it splits below that level).
+    auto sort_keys = [&](int low) {
+        radix_sort_pair(ks, T.perm_src, n, &kt, &T.perm_trg, m, low, 3 * kMaxLevel, s, st);
+        if (ninst > 1) {
+            int ibits = 8;
+            while ((1L << ibits) < ninst) ibits += 8;
+            instance_major(ks, T.perm_src, pis, n, ibits, s, st);
+            instance_major(kt, T.perm_trg, pit, m, ibits, s, st);
+        }
+    };
+    sort_keys(3 * (kMaxLevel - kSortedLevel));
     // boxes
     int cap = std::max(1024, 2 * (int)(((long)n + m) / std::max(nbox, 1)) + 64 + 2 * ninst);
     auto ensure = [&](int need, int used) {
@@ -562,43 +602,87 @@ void build_forest(Tree &T, const double *d_src, const std::vector<int> &so, cons
     };
     T.cap = 0;
     if (!ensure(cap, 0)) return;
-    {
-        DBuf<int> rso, rto;
+    DBuf<LevelTable> dlev;
+    DBuf<int> rso, rto;
+    if (!dlev.alloc(1, s, st)) return;
+    if (ninst > 1) {
         if (!rso.alloc(ninst + 1, s, st) || !rto.alloc(ninst + 1, s, st)) return;
         // root ranges in sorted order: instances are contiguous and in order
         FMM_TRY(st, cudaMemcpyAsync(rso.p, so.data(), sizeof(int) * (ninst + 1), cudaMemcpyHostToDevice, s));
         FMM_TRY(st, cudaMemcpyAsync(rto.p, to.data(), sizeof(int) * (ninst + 1), cudaMemcpyHostToDevice, s));
-        k_root<<<div_up(ninst, 128), 128, 0, s>>>(ninst, rso.p, rto.p, geom.p, T.ijk.p, T.level.p, T.parent.p,
-                                                  T.octant.p, T.nchild.p, T.child.p, T.src0.p, T.nsrc.p, T.trg0.p,
-                                                  T.ntrg.p, T.center.p, T.binst.p); FMM_COUNT_LAUNCH();
-        FMM_TRY(st, cudaStreamSynchronize(s));  // the host range vectors are read by the copies above
     }
+    k_root<<<div_up(ninst, 128), 128, 0, s>>>(ninst, rso.p, rto.p, n, m, dlev.p, geom.p, T.ijk.p, T.level.p, T.parent.p,
+                                              T.octant.p, T.nchild.p, T.child.p, T.src0.p, T.nsrc.p, T.trg0.p,
+                                              T.ntrg.p, T.center.p, T.binst.p); FMM_COUNT_LAUNCH();
+    if (ninst > 1) FMM_TRY(st, cudaStreamSynchronize(s));  // the host range vectors are read by the copies above
     T.lev_start.assign(1, 0);
     T.lev_count.assign(1, ninst);
     int nboxes = ninst;
     DBuf<int> nk, kb, cs0, cns, ct0, cnt;
-    for (int level = 0; level < kMaxLevel; level++) {
-        int b0 = T.lev_start[level], nb = T.lev_count[level];
-        if (!nk.alloc(nb, s, st) || !kb.alloc(nb, s, st) || !cs0.alloc(8L * nb, s, st) ||
-            !cns.alloc(8L * nb, s, st) || !ct0.alloc(8L * nb, s, st) || !cnt.alloc(8L * nb, s, st))
-            return;
-        k_split<<<div_up(nb, 128 / kSplitLanes), 128, 0, s>>>(b0, nb, level, nbox, opt, T.src0.p, T.nsrc.p,
-                                                               T.trg0.p, T.ntrg.p, ks.p, kt.p, nk.p, cs0.p, cns.p,
-                                                               ct0.p, cnt.p); FMM_COUNT_LAUNCH();
-        FMM_LAUNCH_CHECK(st);
-        int total = 0;
-        scan_exclusive_int(nk.p, kb.p, nb, s, st, &total);
+    size_t ncap = 0;
+    auto scratch = [&](size_t need) {
+        if (need <= ncap) return true;
+        ncap = need;
+        return nk.alloc(need, s, st) && kb.alloc(need, s, st) && cs0.alloc(8 * need, s, st) && cns.alloc(8 * need, s, st) &&
+               ct0.alloc(8 * need, s, st) && cnt.alloc(8 * need, s, st);
+    };
+    // Several levels are built between two reads of their counts: as many as a uniform
+    // volume of points needs and one more, then two at a time (a read costs about
+    // as much as the kernels of two small levels).  With arrays too long for the one-CTA scan the
+    // exact count of each level is read.
+    int ahead = 2;
+    for (double c = (double)std::max(n, m) / std::max(nbox, 1) / ninst; c > 1; c /= 8) ahead++;
+    bool sorted_all = false;
+    LevelTable hl;
+    for (int level = 0; level < kMaxLevel;) {
+        const bool blind = T.cap <= 65536;
+        int last = std::min(level + (blind ? ahead : 1), kMaxLevel);
+        if (!sorted_all && last > kSortedLevel) {
+            if (level >= kSortedLevel) {
+                sort_keys(0);
+                sorted_all = true;
+            } else {
+                last = kSortedLevel;
+            }
+        }
+        for (int q = level; q < last; q++) {
+            long bound = T.lev_count[level];
+            for (int k = level; k < q && bound < T.cap; k++) bound *= 8;
+            bound = std::min(bound, (long)T.cap);
+            if (!scratch(blind ? T.cap : bound)) return;
+            k_split<<<div_up(bound, 128 / kSplitLanes), 128, 0, s>>>(dlev.p, q, nbox, opt, T.src0.p, T.nsrc.p, T.trg0.p,
+                                                                   T.ntrg.p, ks.p, kt.p, nk.p, cs0.p, cns.p, ct0.p,
+                                                                   cnt.p); FMM_COUNT_LAUNCH();
+            FMM_LAUNCH_CHECK(st);
+            const ScanJob job = {nk.p, kb.p, (int)bound, blind ? &dlev.p->count[q] : nullptr};
+            scan_exclusive_multi(&job, 1, &dlev.p->total, s, st);
+            k_make_children<<<div_up(bound, 128), 128, 0, s>>>(dlev.p, q, T.cap, opt.ifempty, kb.p, nk.p, cs0.p, cns.p,
+                                                              ct0.p, cnt.p, geom.p, T.ijk.p, T.level.p, T.parent.p,
+                                                              T.octant.p, T.nchild.p, T.child.p, T.src0.p, T.nsrc.p,
+                                                              T.trg0.p, T.ntrg.p, T.center.p, T.binst.p);
+            FMM_COUNT_LAUNCH();
+            FMM_LAUNCH_CHECK(st);
+        }
+        FMM_TRY(st, cudaMemcpyAsync(&hl, dlev.p, sizeof(hl), cudaMemcpyDeviceToHost, s));
+        FMM_TRY(st, cudaStreamSynchronize(s));
         if (!st.ok()) return;
-        if (total > 0 && !ensure(nboxes + total, nboxes)) return;
-        k_make_children<<<div_up(nb, 128), 128, 0, s>>>(b0, nb, level, nboxes, opt.ifempty, kb.p, nk.p, cs0.p, cns.p, ct0.p,
-                                                         cnt.p, geom.p, T.ijk.p, T.level.p, T.parent.p,
-                                                         T.octant.p, T.nchild.p, T.child.p, T.src0.p, T.nsrc.p,
-                                                         T.trg0.p, T.ntrg.p, T.center.p, T.binst.p); FMM_COUNT_LAUNCH();
-        FMM_LAUNCH_CHECK(st);
-        if (total == 0) break;
-        T.lev_start.push_back(nboxes);
-        T.lev_count.push_back(total);
-        nboxes += total;
+        bool done = false;
+        for (int q = level; q < last; q++) {
+            if (hl.over == q + 1) {
+                // the arrays were too short: grow them and build this level again
+                if (!ensure(nboxes + hl.want, nboxes)) return;
+                FMM_TRY(st, cudaMemsetAsync(&dlev.p->over, 0, sizeof(int), s));
+                last = q;
+                break;
+            }
+            if (hl.count[q + 1] == 0) { done = true; break; }
+            T.lev_start.push_back(nboxes);
+            T.lev_count.push_back(hl.count[q + 1]);
+            nboxes += hl.count[q + 1];
+        }
+        if (done) break;
+        level = last;
+        ahead = 2;
     }
     T.nboxes = nboxes;
     T.nlev = (int)T.lev_start.size() - 1;
@@ -611,68 +695,60 @@ void build_forest(Tree &T, const double *d_src, const std::vector<int> &so, cons
         FMM_TRY(st, cudaStreamSynchronize(s));
         for (int i = 0; i < nb && st.ok(); i++) T.capped += (hs[i] > nbox || ht[i] > nbox) ? 1 : 0;
     }
-    for (int d = 0; d < 3; d++) T.center0[d] = hgeom[d];
-    T.size = hgeom[3];
+    for (int d = 0; d < 3; d++) T.center0[d] = hl.geom[d];
+    T.size = hl.geom[3];
 
     // colleagues, level by level
     T.coll.alloc(27L * nboxes, s, st);
     if (!st.ok()) return;
     for (int l = 0; l <= T.nlev; l++) {
-        k_colleagues<<<div_up(T.lev_count[l], 128), 128, 0, s>>>(T.lev_start[l], T.lev_count[l], T.ijk.p,
-                                                                  T.parent.p, T.child.p, T.coll.p); FMM_COUNT_LAUNCH();
+        k_colleagues<<<div_up(27L * T.lev_count[l], 256), 256, 0, s>>>(T.lev_start[l], T.lev_count[l], T.octant.p,
+                                                                      T.parent.p, T.child.p, T.coll.p);
+        FMM_COUNT_LAUNCH();
     }
     FMM_LAUNCH_CHECK(st);
 
-    // leaves
-    DBuf<int> flag, pos;
+    // leaves and lists 1 and 3 (count, scan, fill), list 4 as the dual of list 3
+    DBuf<int> flag, pos, n1, n3, n4, cur, tot;
     flag.alloc(nboxes, s, st);
     pos.alloc(nboxes, s, st);
-    if (!st.ok()) return;
-    k_flag_leaves<<<div_up(nboxes, 256), 256, 0, s>>>(nboxes, T.nchild.p, flag.p); FMM_COUNT_LAUNCH();
-    int nleaves = 0;
-    scan_exclusive_int(flag.p, pos.p, nboxes, s, st, &nleaves);
-    T.nleaves = nleaves;
-    T.leaves.alloc(std::max(nleaves, 1), s, st);
-    if (!st.ok()) return;
-    k_compact<<<div_up(nboxes, 256), 256, 0, s>>>(nboxes, flag.p, pos.p, T.leaves.p); FMM_COUNT_LAUNCH();
-
-    // lists 1 and 3 (count, scan, fill), list 4 as the dual of list 3
-    DBuf<int> n1, n3;
     n1.alloc(nboxes + 1, s, st);
     n3.alloc(nboxes + 1, s, st);
+    n4.alloc(nboxes + 1, s, st);
+    cur.alloc(nboxes + 1, s, st);
+    tot.alloc(3, s, st);
     T.l1_start.alloc(nboxes + 1, s, st);
     T.l3_start.alloc(nboxes + 1, s, st);
     T.l4_start.alloc(nboxes + 1, s, st);
     if (!st.ok()) return;
-    n1.zero(st);
-    n3.zero(st);
-    int lb = std::max(nleaves, 1);
-    k_lists13<<<div_up(lb, 128), 128, 0, s>>>(T.leaves.p, nleaves, T.ijk.p, T.level.p, T.parent.p, T.nchild.p,
-                                              T.child.p, T.coll.p, 0, n1.p, n3.p, nullptr, nullptr, nullptr,
-                                              nullptr); FMM_COUNT_LAUNCH();
-    int tot1 = 0, tot3 = 0;
-    scan_exclusive_int(n1.p, T.l1_start.p, nboxes + 1, s, st, &tot1);
-    scan_exclusive_int(n3.p, T.l3_start.p, nboxes + 1, s, st, &tot3);
-    T.l1_idx.alloc(std::max(tot1, 1), s, st);
-    T.l3_idx.alloc(std::max(tot3, 1), s, st);
-    if (!st.ok()) return;
-    k_lists13<<<div_up(lb, 128), 128, 0, s>>>(T.leaves.p, nleaves, T.ijk.p, T.level.p, T.parent.p, T.nchild.p,
-                                              T.child.p, T.coll.p, 1, nullptr, nullptr, T.l1_start.p,
-                                              T.l1_idx.p, T.l3_start.p, T.l3_idx.p); FMM_COUNT_LAUNCH();
-    DBuf<int> n4, cur;
-    n4.alloc(nboxes + 1, s, st);
-    cur.alloc(nboxes + 1, s, st);
-    if (!st.ok()) return;
     n4.zero(st);
-    k_list4_count<<<div_up(lb, 128), 128, 0, s>>>(T.leaves.p, nleaves, T.l3_start.p, T.l3_idx.p, n4.p); FMM_COUNT_LAUNCH();
-    int tot4 = 0;
-    scan_exclusive_int(n4.p, T.l4_start.p, nboxes + 1, s, st, &tot4);
-    T.l4_idx.alloc(std::max(tot4, 1), s, st);
+    k_lists13<0><<<div_up(nboxes + 1, 4), 128, 0, s>>>(nboxes, T.ijk.p, T.level.p, T.parent.p, T.nchild.p, T.child.p,
+                                                      T.coll.p, n1.p, n3.p, flag.p, nullptr, nullptr, nullptr, nullptr,
+                                                      nullptr); FMM_COUNT_LAUNCH();
+    const ScanJob jobs[3] = {{flag.p, pos.p, nboxes, nullptr},
+                             {n1.p, T.l1_start.p, nboxes + 1, nullptr},
+                             {n3.p, T.l3_start.p, nboxes + 1, nullptr}};
+    scan_exclusive_multi(jobs, 3, tot.p, s, st);
+    int h[3] = {0, 0, 0};   // leaves, entries of lists 1 and 3
+    FMM_TRY(st, cudaMemcpyAsync(h, tot.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FMM_TRY(st, cudaStreamSynchronize(s));
+    const int nleaves = T.nleaves = h[0];
+    T.leaves.alloc(std::max(nleaves, 1), s, st);
+    T.l1_idx.alloc(std::max(h[1], 1), s, st);
+    T.l3_idx.alloc(std::max(h[2], 1), s, st);
+    T.l4_idx.alloc(std::max(h[2], 1), s, st);
     if (!st.ok()) return;
-    FMM_TRY(st, cudaMemcpyAsync(cur.p, T.l4_start.p, sizeof(int) * (nboxes + 1), cudaMemcpyDeviceToDevice, s));
-    k_list4_fill<<<div_up(lb, 128), 128, 0, s>>>(T.leaves.p, nleaves, T.l3_start.p, T.l3_idx.p, cur.p,
-                                                 T.l4_idx.p); FMM_COUNT_LAUNCH();
-    k_sort_rows<<<div_up(nboxes, 128), 128, 0, s>>>(nboxes, T.l4_start.p, T.l4_idx.p); FMM_COUNT_LAUNCH();
+    k_compact<<<div_up(nboxes, 256), 256, 0, s>>>(nboxes, flag.p, pos.p, T.leaves.p); FMM_COUNT_LAUNCH();
+    k_lists13<1><<<div_up(nboxes + 1, 4), 128, 0, s>>>(nboxes, T.ijk.p, T.level.p, T.parent.p, T.nchild.p, T.child.p,
+                                                      T.coll.p, nullptr, nullptr, nullptr, T.l1_start.p, T.l1_idx.p,
+                                                      T.l3_start.p, T.l3_idx.p, n4.p); FMM_COUNT_LAUNCH();
+    const ScanJob jobs4[2] = {{n4.p, T.l4_start.p, nboxes + 1, nullptr}, {n4.p, cur.p, nboxes + 1, nullptr}};
+    scan_exclusive_multi(jobs4, 2, nullptr, s, st);
+    if (h[2] > 0) {
+        k_list4_fill<<<div_up(nleaves, 128), 128, 0, s>>>(T.leaves.p, nleaves, T.l3_start.p, T.l3_idx.p, cur.p,
+                                                          T.l4_idx.p); FMM_COUNT_LAUNCH();
+        k_sort_rows<<<div_up(nboxes, 128), 128, 0, s>>>(nboxes, T.l4_start.p, T.l4_idx.p); FMM_COUNT_LAUNCH();
+    }
     FMM_LAUNCH_CHECK(st);
 
     // boxes grouped by (level, octant)
@@ -686,7 +762,7 @@ void build_forest(Tree &T, const double *d_src, const std::vector<int> &so, cons
     k_group_keys<<<div_up(nboxes, 256), 256, 0, s>>>(nboxes, T.level.p, T.octant.p, gk.p, T.grouped.p); FMM_COUNT_LAUNCH();
     int gbits = 8;
     while ((1 << gbits) < ngroups + 1) gbits += 8;
-    radix_sort_u64(gk.p, T.grouped.p, nboxes, gbits, s, st);
+    radix_sort_pair(gk, T.grouped, nboxes, nullptr, nullptr, 0, 0, gbits, s, st);
     if (!st.ok()) return;
     k_group_bounds<<<div_up(nboxes + 1, 256), 256, 0, s>>>(nboxes, gk.p, ngroups, gs.p); FMM_COUNT_LAUNCH();
     T.group_start.assign(ngroups + 1, 0);
