@@ -3,6 +3,7 @@
 #include <mutex>
 
 #include "helm_kernels.cuh"
+#include "near.cuh"
 
 namespace fmm {
 
@@ -1449,79 +1450,170 @@ __device__ __forceinline__ void hpair(double dx, double dy, double dz, double2 z
     }
 }
 
-constexpr int kHP2PThreads = 128;
+// P2P: hfmm3dpart_direct_self / _targ (src/hfmm3dpart.f:1092-1262), the pair
+// formulas above.  One warp per (leaf, run of 32 points), a point per lane, sources of the
+// box itself and of list 1 staged 32 at a time as records in the warp's shared
+// memory.  Bound by the FP64 pipe: 53 operations a pair with charges and real k
+// (1/r in five, sine and cosine in 21: near.cuh), against about 105 with the
+// library's functions.  CPX: k has an imaginary part (exp from the library).
+// Products and sums are written as fused multiply-adds, so that both forms of
+// the functions and every instantiation round alike.
+constexpr int kHNearWarps = 2;
 
-// P2P: hfmm3dpart_direct_self / _targ (src/hfmm3dpart.f:1092-1262).  CTA per
-// leaf, one evaluation point (sources, then targets) per thread, source boxes
-// self and list 1 staged through shared memory, the self pair skipped by index.
 template <bool CHG, bool DIP>
-__global__ void __launch_bounds__(kHP2PThreads) k_hp2p(const int *leaves, TreeView tv, PointsSoA src,
-                                                      const double *tx, const double *ty, const double *tz,
-                                                      double2 zk, OutSoA outs, OutSoA outt, int do_src, int do_trg)
+struct HNearRec {
+    static constexpr int kStride = DIP ? 10 : 6;   // (16-byte parts of consecutive records in different banks)
+    static constexpr int kQ = 3, kD = CHG ? 5 : 3, kV = kD + 2;
+};
+
+template <bool CHG, bool DIP, bool CPX, bool LIB>
+__device__ __forceinline__ void hnear_pair(double dx, double dy, double dz, double2 zk, double2 k2, double2 q,
+                                           double2 ds, double vx, double vy, double vz, double2 (&a)[4],
+                                           unsigned &odd_r, unsigned &odd_s)
 {
-    __shared__ double sx[kHP2PThreads], sy[kHP2PThreads], sz[kHP2PThreads];
-    __shared__ double2 sq[kHP2PThreads], sd[kHP2PThreads];
-    __shared__ double svx[kHP2PThreads], svy[kHP2PThreads], svz[kHP2PThreads];
-    const int b = leaves[blockIdx.x];
-    const int s0 = tv.src0[b], ns = do_src ? tv.nsrc[b] : 0;
-    const int t0 = tv.trg0[b], nt = do_trg ? tv.ntrg[b] : 0;
-    const int ne = ns + nt;
-    const int l1a = tv.l1_start[b], nl = 1 + tv.l1_start[b + 1] - l1a;
-    const double2 k2 = cmul(zk, zk);
-    // CTA (leaf, y) serves the leaf's point chunks y, y + gridDim.y, ...
-    for (int e0 = blockIdx.y * kHP2PThreads; e0 < ne; e0 += gridDim.y * kHP2PThreads) {
-        const int e = e0 + threadIdx.x;
-        const bool act = e < ne;
-        const bool is_src = e < ns;
-        double ex = 0, ey = 0, ez = 0;
-        int self = -1;
-        if (act) {
-            if (is_src) { int i = s0 + e; ex = src.x[i]; ey = src.y[i]; ez = src.z[i]; self = i; }
-            else { int i = t0 + e - ns; ex = tx[i]; ey = ty[i]; ez = tz[i]; }
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const double ri = rsqrt_near<LIB>(r2, odd_r), r = r2 * ri, ri2 = ri * ri, x = zk.x * r;
+    double s, c;
+    sincos_near<LIB>(x, s, c, odd_s);
+    const double ee = CPX ? exp(-zk.y * r) * ri : ri;
+    const double2 g = cmk(c * ee, s * ee);
+    const double m = CPX ? fma(zk.y, r, 1.0) : 1.0;   // 1 - ikr = m - i x
+    if (CHG) {
+        const double2 u = cmul(q, g);
+        a[0] = cadd(a[0], u);
+        const double2 w = cscal(ri2, cmk(fma(x, u.y, CPX ? m * u.x : u.x), fma(-x, u.x, CPX ? m * u.y : u.y)));
+        crfma(a[1], dx, w);
+        crfma(a[2], dy, w);
+        crfma(a[3], dz, w);
+    }
+    if (DIP) {
+        const double dot = fma(dx, vx, fma(dy, vy, dz * vz));
+        const double2 u = cmul(ds, g);
+        const double2 w = cscal(ri2, cmk(fma(x, u.y, CPX ? m * u.x : u.x), fma(-x, u.x, CPX ? m * u.y : u.y)));
+        crfma(a[0], dot, w);
+        // 3ik/r^2 + k^2/r - 3/r^3
+        const double t3 = 3.0 * ri2;
+        const double2 t = cmk(fma(ri, k2.x, CPX ? fma(-t3, ri, -(t3 * zk.y)) : -(t3 * ri)),
+                              CPX ? fma(ri, k2.y, t3 * zk.x) : t3 * zk.x);
+        const double2 f = cscal(-(ri * dot), cmul(u, t));
+        crfma(a[1], dx, f); crfma(a[1], -vx, w);
+        crfma(a[2], dy, f); crfma(a[2], -vy, w);
+        crfma(a[3], dz, f); crfma(a[3], -vz, w);
+    }
+}
+
+struct HNearArgs {
+    const int *leaves;
+    int nleaves;
+    TreeView tv;
+    PointsSoA src;
+    const double *tx, *ty, *tz;
+    double2 zk, k2;
+    OutSoA outs, outt;
+    int do_src, do_trg;
+};
+
+// cn staged sources at the lane's point; OWN: a point's own source (selfk) adds exact zeros
+// (no strength, unit offset).
+template <bool CHG, bool DIP, bool CPX, bool LIB, bool OWN>
+__device__ __forceinline__ void hnear_batch(const HNearArgs &A, const double *rec, int cn, double px, double py, double pz,
+                                            int selfk, double2 (&a)[4], unsigned &odd_r, unsigned &odd_s)
+{
+    using R = HNearRec<CHG, DIP>;
+    constexpr int W = R::kStride;
+#pragma unroll(LIB ? 1 : 2)
+    for (int k = 0; k < cn; k++) {
+        double r[W];
+#pragma unroll
+        for (int i = 0; i < W / 2; i++) {
+            const double2 v = reinterpret_cast<const double2 *>(rec + k * W)[i];
+            r[2 * i] = v.x;
+            r[2 * i + 1] = v.y;
         }
-        double2 pot = cmk(0, 0), fx = cmk(0, 0), fy = cmk(0, 0), fz = cmk(0, 0);
-        for (int j = 0; j < nl; j++) {
-            const int jb = j == 0 ? b : tv.l1_idx[l1a + j - 1];
-            const int js0 = tv.src0[jb], jn = tv.nsrc[jb];
-            for (int c0 = 0; c0 < jn; c0 += kHP2PThreads) {
-                const int cn = min(kHP2PThreads, jn - c0);
-                __syncthreads();
-                if (threadIdx.x < cn) {
-                    int i = js0 + c0 + threadIdx.x;
-                    sx[threadIdx.x] = src.x[i]; sy[threadIdx.x] = src.y[i]; sz[threadIdx.x] = src.z[i];
-                    if (CHG) sq[threadIdx.x] = src.q[i];
-                    if (DIP) {
-                        sd[threadIdx.x] = src.dq[i];
-                        svx[threadIdx.x] = src.vx[i]; svy[threadIdx.x] = src.vy[i]; svz[threadIdx.x] = src.vz[i];
-                    }
+        const bool me = OWN && k == selfk;
+        const double2 q = CHG && !me ? cmk(r[R::kQ], r[R::kQ + 1]) : cmk(0, 0);
+        const double2 d = DIP && !me ? cmk(r[R::kD], r[R::kD + 1]) : cmk(0, 0);
+        hnear_pair<CHG, DIP, CPX, LIB>(me ? 1.0 : px - r[0], me ? 0.0 : py - r[1], me ? 0.0 : pz - r[2], A.zk, A.k2, q, d,
+                                       DIP && !me ? r[DIP ? R::kV : 0] : 0.0, DIP && !me ? r[DIP ? R::kV + 1 : 0] : 0.0,
+                                       DIP && !me ? r[DIP ? R::kV + 2 : 0] : 0.0, a, odd_r, odd_s);
+    }
+}
+
+// Points e0 .. e0 + 31 of leaf b.  Returns whether a pair of this warp needs the library
+// functions; nothing is written then (LIB: never).
+template <bool CHG, bool DIP, bool CPX, bool LIB>
+__device__ __forceinline__ bool hnear_points(const HNearArgs &A, int b, int e0, int ne, int ns, double *rec)
+{
+    using R = HNearRec<CHG, DIP>;
+    constexpr int W = R::kStride;
+    const int lane = threadIdx.x & 31, s0 = A.tv.src0[b], t0 = A.tv.trg0[b];
+    const int e = min(e0 + lane, ne - 1);   // (lanes past the end repeat the last point; nothing of theirs is written)
+    const bool is_src = e < ns;
+    const int i = is_src ? s0 + e : t0 + e - ns;
+    const double px = is_src ? A.src.x[i] : A.tx[i], py = is_src ? A.src.y[i] : A.ty[i],
+                 pz = is_src ? A.src.z[i] : A.tz[i];
+    double2 a[4] = {cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)};
+    unsigned odd_r = 0, odd_s = 0;
+    const int l1a = A.tv.l1_start[b], nl = 1 + A.tv.l1_start[b + 1] - l1a;
+    for (int j = 0; j < nl; j++) {
+        const int jb = j == 0 ? b : A.tv.l1_idx[l1a + j - 1];
+        const int js0 = A.tv.src0[jb], jn = A.tv.nsrc[jb];
+        for (int c0 = 0; c0 < jn; c0 += 32) {
+            const int cn = min(32, jn - c0);
+            __syncwarp();
+            if (lane < cn) {
+                const int k = js0 + c0 + lane;
+                double r[W] = {};
+                r[0] = A.src.x[k]; r[1] = A.src.y[k]; r[2] = A.src.z[k];
+                if (CHG) { const double2 q = A.src.q[k]; r[R::kQ] = q.x; r[R::kQ + 1] = q.y; }
+                if (DIP) {
+                    const double2 d = A.src.dq[k];
+                    r[R::kD] = d.x; r[R::kD + 1] = d.y;
+                    r[R::kV] = A.src.vx[k]; r[R::kV + 1] = A.src.vy[k]; r[R::kV + 2] = A.src.vz[k];
                 }
-                __syncthreads();
-                if (!act) continue;
-                const int selfk = self - (js0 + c0);
-                // the self pair adds exact zeros (no strength, unit offset) instead of a branch,
-                // so consecutive pairs interleave
-#pragma unroll 2
-                for (int k = 0; k < cn; k++) {
-                    const bool me = k == selfk;
-                    hpair<CHG, DIP>(me ? 1.0 : ex - sx[k], me ? 0.0 : ey - sy[k], me ? 0.0 : ez - sz[k], zk, k2,
-                                    CHG && !me ? sq[k] : cmk(0, 0), DIP && !me ? sd[k] : cmk(0, 0),
-                                    DIP && !me ? svx[k] : 0.0, DIP && !me ? svy[k] : 0.0, DIP && !me ? svz[k] : 0.0,
-                                    pot, fx, fy, fz);
-                }
+#pragma unroll
+                for (int c = 0; c < W / 2; c++)
+                    reinterpret_cast<double2 *>(rec + lane * W)[c] = make_double2(r[2 * c], r[2 * c + 1]);
             }
-        }
-        if (act) {
-            double2 *po = is_src ? outs.pot : outt.pot;
-            double2 *ox = is_src ? outs.fx : outt.fx, *oy = is_src ? outs.fy : outt.fy, *oz = is_src ? outs.fz : outt.fz;
-            int i = is_src ? s0 + e : t0 + e - ns;
-            if (po) po[i] = cadd(po[i], pot);
-            if (ox) {
-                ox[i] = cadd(ox[i], fx);
-                oy[i] = cadd(oy[i], fy);
-                oz[i] = cadd(oz[i], fz);
-            }
+            __syncwarp();
+            if (j == 0 && e0 < ns)
+                hnear_batch<CHG, DIP, CPX, LIB, true>(A, rec, cn, px, py, pz, is_src ? e - c0 : -1, a, odd_r, odd_s);
+            else
+                hnear_batch<CHG, DIP, CPX, LIB, false>(A, rec, cn, px, py, pz, -1, a, odd_r, odd_s);
         }
     }
+    if (!LIB && __any_sync(0xffffffffu, odd_r > kRsqrtSpan || odd_s >= kSinCosMax)) return true;
+    if (e0 + lane < ne) {
+        const OutSoA &o = is_src ? A.outs : A.outt;
+        if (o.pot) o.pot[i] = cadd(o.pot[i], a[0]);
+        if (o.fx) {
+            o.fx[i] = cadd(o.fx[i], a[1]);
+            o.fy[i] = cadd(o.fy[i], a[2]);
+            o.fz[i] = cadd(o.fz[i], a[3]);
+        }
+    }
+    return false;
+}
+
+template <bool CHG, bool DIP, bool CPX>
+__global__ void __launch_bounds__(32 * kHNearWarps) k_hp2p(HNearArgs A)
+{
+    __shared__ __align__(16) double rec[kHNearWarps][32 * HNearRec<CHG, DIP>::kStride];
+    const int warp = threadIdx.x >> 5, li = blockIdx.x * kHNearWarps + warp;
+    if (li >= A.nleaves) return;
+    const int b = A.leaves[li];
+    const int ns = A.do_src ? A.tv.nsrc[b] : 0, ne = ns + (A.do_trg ? A.tv.ntrg[b] : 0);
+    for (int e0 = blockIdx.y * 32; e0 < ne; e0 += gridDim.y * 32)
+        if (hnear_points<CHG, DIP, CPX, false>(A, b, e0, ne, ns, rec[warp]))
+            hnear_points<CHG, DIP, CPX, true>(A, b, e0, ne, ns, rec[warp]);
+}
+
+template <bool CHG, bool DIP>
+static void launch_hp2p_t(const HNearArgs &A, cudaStream_t s)
+{
+    const dim3 g(div_up(A.nleaves, kHNearWarps), 8);
+    if (A.zk.y == 0.0) k_hp2p<CHG, DIP, false><<<g, 32 * kHNearWarps, 0, s>>>(A);
+    else k_hp2p<CHG, DIP, true><<<g, 32 * kHNearWarps, 0, s>>>(A);
 }
 
 void launch_hp2p(const int *leaves, int nleaves, const TreeView &tv, const PointsSoA &src, const double *tx,
@@ -1529,12 +1621,15 @@ void launch_hp2p(const int *leaves, int nleaves, const TreeView &tv, const Point
                  int ifdipole, int ifpot, int iffld, int ifpottarg, int iffldtarg, cudaStream_t s, Status &st)
 {
     if (nleaves == 0 || !st.ok()) return;
-    int do_src = (ifpot == 1 || iffld == 1), do_trg = (ifpottarg == 1 || iffldtarg == 1);
     bool c = ifcharge == 1, d = ifdipole == 1;
     if (!c && !d) return;
-    if (c && d) k_hp2p<true, true><<<dim3(nleaves, 4), kHP2PThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, zk, outs, outt, do_src, do_trg);
-    else if (c) k_hp2p<true, false><<<dim3(nleaves, 4), kHP2PThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, zk, outs, outt, do_src, do_trg);
-    else k_hp2p<false, true><<<dim3(nleaves, 4), kHP2PThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, zk, outs, outt, do_src, do_trg);
+    HNearArgs A;
+    A.leaves = leaves; A.nleaves = nleaves; A.tv = tv; A.src = src; A.tx = tx; A.ty = ty; A.tz = tz;
+    A.zk = zk; A.k2 = cmul(zk, zk); A.outs = outs; A.outt = outt;
+    A.do_src = ifpot == 1 || iffld == 1; A.do_trg = ifpottarg == 1 || iffldtarg == 1;
+    if (c && d) launch_hp2p_t<true, true>(A, s);
+    else if (c) launch_hp2p_t<true, false>(A, s);
+    else launch_hp2p_t<false, true>(A, s);
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
 }

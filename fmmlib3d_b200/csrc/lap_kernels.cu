@@ -23,6 +23,7 @@
 #include <mutex>
 
 #include "eval_mm.cuh"
+#include "near.cuh"
 
 namespace fmm {
 
@@ -151,29 +152,6 @@ __device__ __forceinline__ double2 tab_get(const double2 *tab, int stride, int n
 // out, so that every instantiation rounds alike.
 constexpr int kP2PThreads = 128;      // direct sums
 constexpr int kNearWarps = 2;
-
-// 1/sqrt(x) for ordinary x: the hardware's approximation (relative error below
-// 2^-19) and one step of Halley's iteration, y (1 + e/2 + 3 e^2/8) with
-// e = 1 - x y^2, which cubes the error.  Zeros, infinities, NaN and numbers near
-// the ends of the range need the library function: `odd` collects the largest
-// position of the exponent above the ordinary range's start, so that a warp tests
-// it once for all its pairs; with LIB every such number takes the library function.
-constexpr unsigned kRsqrtLow = 0x03000000u, kRsqrtSpan = 0x79000000u;   // 2^-975 .. 2^961
-template <bool LIB>
-__device__ __forceinline__ double rsqrt_near(double x, unsigned &odd)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    y = fma(y * e, fma(e, 0.375, 0.5), y);
-    const unsigned at = (unsigned)__double2hiint(x) - kRsqrtLow;
-    if (LIB) {
-        if (at > kRsqrtSpan) y = rsqrt(x);
-    } else {
-        odd = max(odd, at);
-    }
-    return y;
-}
 
 // Source record: x, y, z, [q], [d, v, -d v (re), -d v (im)], padded to a stride
 // whose 16-byte parts fall into different banks for consecutive sources.
