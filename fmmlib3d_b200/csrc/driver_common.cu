@@ -206,6 +206,7 @@ SideStreams &side_streams()
         cudaStreamCreateWithFlags(&ss.copy, cudaStreamNonBlocking);
         cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ss.join, cudaEventDisableTiming);
+        cudaEventCreateWithFlags(&ss.mid, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ss.copied, cudaEventDisableTiming);
         ss.dev = dev;
     }

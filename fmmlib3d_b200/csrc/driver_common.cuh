@@ -117,7 +117,7 @@ struct Timer {
 // fork / join events between it and the call's stream (made once per thread).
 struct SideStreams {
     cudaStream_t far = nullptr, copy = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr, copied = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, mid = nullptr, copied = nullptr;
     int dev = -1;
 };
 SideStreams &side_streams();

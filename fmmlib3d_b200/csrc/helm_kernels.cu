@@ -1359,15 +1359,14 @@ __global__ void __launch_bounds__(32 * kHL2PWarps) k_hl2p(const int *leaves, Tre
     }
 }
 
-void launch_heval(const int *leaves, int nleaves, const TreeView &tv, const double *sx, const double *sy,
-                  const double *sz, const double *tx, const double *ty, const double *tz, HLevels lv, int NC,
-                  double2 zk, const double2 *mpole, const double2 *local, OutSoA outs, OutSoA outt, int do_src,
-                  int do_trg, cudaStream_t s, Status &st)
+// The leaves' own local expansions.
+void launch_hl2p(const int *leaves, int nleaves, const TreeView &tv, const double *sx, const double *sy,
+                 const double *sz, const double *tx, const double *ty, const double *tz, HLevels lv, int NC, double2 zk,
+                 const double2 *local, OutSoA outs, OutSoA outt, int do_src, int do_trg, cudaStream_t s, Status &st)
 {
     if (nleaves == 0 || !st.ok() || (!do_src && !do_trg)) return;
     htab_init(s, st);
     int pm = max_p(lv);
-    // L2P (the leaves' own local expansions) first, then M2P of list 3
     size_t sm = sizeof(double2) * ((size_t)(pm + 1) * (pm + 1) + (size_t)(pm + 2) * kHEvalThreads);
     if (hl2p_smem(pm) <= 100 * 1024) {
         const size_t sl = hl2p_smem(pm);
@@ -1377,34 +1376,54 @@ void launch_heval(const int *leaves, int nleaves, const TreeView &tv, const doub
     } else if (sm <= 226 * 1024) {
         FMM_TRY(st, smem_allow(k_heval<kHEvalThreads>, (int)sm));
         k_heval<kHEvalThreads><<<dim3(nleaves, 2), kHEvalThreads, sm, s>>>(leaves, tv, sx, sy, sz, tx, ty, tz, lv,
-                                                                           NC, zk, mpole, local, outs, outt, do_src,
+                                                                           NC, zk, nullptr, local, outs, outt, do_src,
                                                                            do_trg, 0);
     } else {
         sm = sizeof(double2) * ((size_t)(pm + 1) * (pm + 1) + (size_t)(pm + 2) * 32);
         FMM_TRY(st, smem_allow(k_heval<32>, (int)sm));
-        k_heval<32><<<dim3(nleaves, 8), 32, sm, s>>>(leaves, tv, sx, sy, sz, tx, ty, tz, lv, NC, zk, mpole, local,
+        k_heval<32><<<dim3(nleaves, 8), 32, sm, s>>>(leaves, tv, sx, sy, sz, tx, ty, tz, lv, NC, zk, nullptr, local,
                                                      outs, outt, do_src, do_trg, 0);
     }
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
-    // M2P work items: (leaf, chunk of points, group of list-3 boxes)
-    DBuf<int> cnt, off;
-    if (!cnt.alloc(nleaves, s, st) || !off.alloc(nleaves, s, st)) return;
+}
+
+// M2P work items: (leaf, chunk of points, group of list-3 boxes)
+void hm2p_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, HM2PItems &I,
+                  cudaStream_t s, Status &st)
+{
+    I.n = 0;
+    if (nleaves == 0 || !st.ok() || (!do_src && !do_trg)) return;
+    DBuf<int> cnt;
+    if (!cnt.alloc(nleaves, s, st) || !I.off.alloc(nleaves, s, st)) return;
     k_hm2p_count<<<div_up(nleaves, 256), 256, 0, s>>>(leaves, nleaves, tv, do_src, do_trg, cnt.p);
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
-    int nitems = 0;
-    scan_exclusive_int(cnt.p, off.p, nleaves, s, st, &nitems);
-    if (!st.ok() || nitems == 0) return;
-    DBuf<double> part;
-    if (!part.alloc((size_t)nitems * 8 * kHM2PThreads, s, st)) return;
-    sm = sizeof(double2) * (size_t)(pm + 1) * (pm + 1);
+    scan_exclusive_int(cnt.p, I.off.p, nleaves, s, st, &I.n);
+    if (st.ok() && I.n > 0) I.part.alloc((size_t)I.n * 8 * kHM2PThreads, s, st);
+}
+
+void launch_hm2p(const int *leaves, int nleaves, const HM2PItems &I, const TreeView &tv, const double *sx,
+                 const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, HLevels lv,
+                 int NC, double2 zk, const double2 *mpole, int do_src, int do_trg, cudaStream_t s, Status &st)
+{
+    if (I.n == 0 || !st.ok()) return;
+    htab_init(s, st);
+    const int pm = max_p(lv);
+    const size_t sm = sizeof(double2) * (size_t)(pm + 1) * (pm + 1);
     FMM_TRY(st, smem_allow(k_hm2p<kHM2PThreads>, (int)sm));
-    k_hm2p<kHM2PThreads><<<nitems, kHM2PThreads, sm, s>>>(leaves, nleaves, off.p, tv, sx, sy, sz, tx, ty, tz, lv, NC,
-                                                          zk, mpole, do_src, do_trg, part.p);
+    k_hm2p<kHM2PThreads><<<I.n, kHM2PThreads, sm, s>>>(leaves, nleaves, I.off.p, tv, sx, sy, sz, tx, ty, tz, lv, NC, zk,
+                                                       mpole, do_src, do_trg, I.part.p);
     FMM_COUNT_LAUNCH();
-    k_hm2p_add<kHM2PThreads><<<dim3(nleaves, 4), kHM2PThreads, 0, s>>>(leaves, off.p, tv, outs, outt, do_src, do_trg,
-                                                                       part.p);
+    FMM_LAUNCH_CHECK(st);
+}
+
+void launch_hm2p_add(const int *leaves, int nleaves, const HM2PItems &I, const TreeView &tv, OutSoA outs, OutSoA outt,
+                     int do_src, int do_trg, cudaStream_t s, Status &st)
+{
+    if (I.n == 0 || !st.ok()) return;
+    k_hm2p_add<kHM2PThreads><<<dim3(nleaves, 4), kHM2PThreads, 0, s>>>(leaves, I.off.p, tv, outs, outt, do_src, do_trg,
+                                                                       I.part.p);
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
 }

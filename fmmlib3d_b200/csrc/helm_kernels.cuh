@@ -66,10 +66,24 @@ void launch_hform(bool irreg, const int *boxes, int nboxes, const TreeView &tv, 
                   Status &st);
 
 // L2P at leaves of level >= 2 and M2P from list-3 boxes, at sources and targets.
-void launch_heval(const int *leaves, int nleaves, const TreeView &tv, const double *sx, const double *sy,
-                  const double *sz, const double *tx, const double *ty, const double *tz, HLevels lv, int NC,
-                  double2 zk, const double2 *mpole, const double2 *local, OutSoA outs, OutSoA outt, int do_src,
-                  int do_trg, cudaStream_t s, Status &st);
+void launch_hl2p(const int *leaves, int nleaves, const TreeView &tv, const double *sx, const double *sy,
+                 const double *sz, const double *tx, const double *ty, const double *tz, HLevels lv, int NC, double2 zk,
+                 const double2 *local, OutSoA outs, OutSoA outt, int do_src, int do_trg, cudaStream_t s, Status &st);
+
+// Work items of the list-3 multipoles (host-synchronising), their sums, and the
+// addition of these to the outputs.
+struct HM2PItems {
+    DBuf<int> off;
+    DBuf<double> part;
+    int n = 0;
+};
+void hm2p_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, HM2PItems &I,
+                  cudaStream_t s, Status &st);
+void launch_hm2p(const int *leaves, int nleaves, const HM2PItems &I, const TreeView &tv, const double *sx,
+                 const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, HLevels lv,
+                 int NC, double2 zk, const double2 *mpole, int do_src, int do_trg, cudaStream_t s, Status &st);
+void launch_hm2p_add(const int *leaves, int nleaves, const HM2PItems &I, const TreeView &tv, OutSoA outs, OutSoA outt,
+                     int do_src, int do_trg, cudaStream_t s, Status &st);
 
 // kind 0 = M2M, 1 = M2L, 2 = L2L by rotation, z-shift operator, rotation.
 void launch_htranslate(int kind, const Tile *tiles, int ntiles, const int *grouped, const HSlot *slots,
