@@ -472,7 +472,7 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
             if (k.m2l_kt % 16 || k.m2l_kt < 16 || k.m2l_kt > kTcTileTargetsMax) return 2;
         } else if (S.mixed) {
             if (k.m2l_kt != kDenseTileTargets) return 2;
-        } else if (S.dense) {
+        } else if (S.dense && S.fold) {
             if (k.m2l_kt != 16 && k.m2l_kt != kDenseTileTargets) return 2;
         } else {
             const int nbuf = (k.m2l_kt == 8 && NC <= 3 * 256) ? 2 : 3;
@@ -504,7 +504,7 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
     // M2L tile size (automatic): the largest whose tile count fills the GPU (two
     // CTAs per SM per 64-row block); smaller tiles only add CTAs, every target's
     // sums are unchanged
-    int m2l_kt = S.tcm2l ? kTcTileTargets : S.dense ? kDenseTileTargets : plan->kt_m2l;
+    int m2l_kt = S.tcm2l ? kTcTileTargets : S.dense && (S.fold || S.mixed) ? kDenseTileTargets : plan->kt_m2l;
     if (k.m2l_kt) {
         m2l_kt = k.m2l_kt;
     } else if (S.tcm2l) {
@@ -743,7 +743,9 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
     // near field and every other pass stay FP64
     if (S.tri && form == 1 && iprec <= 1 && plan->dense && sw(kSwTensorM2L) > 0) S.dense = S.tcm2l = true;
     const int m2l_mode = sw(kSwM2LMode);
-    S.fold = plan->folded && !S.mixed && !S.tcm2l && m2l_mode != 1 && m2l_mode != 3;
+    // (the folded kernel indexes the multipoles with 32 bits)
+    S.fold = plan->folded && !S.mixed && !S.tcm2l && m2l_mode != 1 && m2l_mode != 3 &&
+             (unsigned long long)(T.nboxes + 1) * K < 0xffffffffull;
     if (S.fold && T.nlev >= 2 && !fold_prepare(plan->fold, S.fw, T.nboxes, T.nboxes - T.lev_start[2], s, st)) {
         g_ti.err = cudaGetErrorString(st.err);
         return 16;

@@ -21,10 +21,10 @@
 // k_m2l_fold: a CTA owns 16 consecutive target boxes (32 columns: 16 targets x
 // 2 right-hand sides) and all their coefficients; warp w owns the rows of
 // parity class w (of half of it for high orders) in DMMA accumulators.  Per
-// batch all warps stage X (one 36-row slot per parity class: 83 KB; two CTAs
-// per SM fill each other's staging gaps up to order 14), then
+// batch all warps stage X (36 rows per parity class: 83 KB; two CTAs per SM fill
+// each other's staging gaps up to order 14), then
 // each warp multiplies its operator fragments, read from L2 in the lane order
-// of the MMA and each used for all 32 columns, with its slot.  Offset classes
+// of the MMA and each used for all 32 columns, with its rows.  Offset classes
 // that no target of the tile has a source in are skipped.
 // The sums of a target are formed in 8 fixed groups of batches, added in
 // order; a small problem runs one CTA per (tile, group) and adds the groups
@@ -46,7 +46,7 @@ constexpr int kFoldSplitTiles = 296;            // fewer tiles than this: one CT
 // ---------------------------------------------------------------- operators
 struct FoldBlock {
     long long off;
-    int k4, rb, off_id, alpha, beta, na, nb, work0;
+    int k4, rb, off_id, alpha, beta, na, nb, k0;
 };
 
 // T_D[(j, m)][(n, mc)] = e^{i (mc - m) phi} sum_k D^j[m][k] Z(j, k, n) D^n[mc][k],
@@ -82,7 +82,7 @@ __global__ void k_fold_ops(const FoldBlock *blocks, const FoldOffset *offs, cons
     const double *Rm = rot + rot_class_size(p) * o.cls;
     for (int e = threadIdx.x; e < B.k4 * B.rb * 32; e += blockDim.x) {
         const int lane = e & 31, rb = (e >> 5) % B.rb, ks = (e >> 5) / B.rb;
-        const int row = rb * 8 + (lane >> 2), col = ks * 4 + (lane & 3);
+        const int row = rb * 8 + (lane >> 2), col = B.k0 + ks * 4 + (lane & 3);
         double v = 0;
         if (row < B.na && col < B.nb) {
             const int4 r = kmap[base[B.alpha] + row], c = kmap[base[B.beta] + col];
@@ -128,97 +128,97 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
         for (int m = 0; m <= n; m++)
             rmap.push_back(make_int4(eidx(n, m), eidx(n, -m), kc[n * (p + 1) + m], m ? ksn[n * (p + 1) + m] : -1));
 
-    // operator blocks and their fragments
+    // Segments (offset class, round of column classes, K range) packed into batches.  The
+    // segments of one offset class in a batch are a run: their operand rows follow each other in
+    // every parity class's slot, and so do the K steps of its operator fragments, so
+    // that a warp multiplies a run in one loop.
+    F.tile = F.rows <= 5 ? 16 : 8;
     std::vector<FoldBlock> blocks;
-    std::vector<long long> aoff((size_t)kFoldClasses * 64, -1);
     std::vector<int4> cls;
-    long long tot = 0;
-    for (int q = 0; q < kFoldClasses; q++) {
-        const FoldOffset &o = off[q];
-        const int z = (o.a == 0) | (o.b == 0) << 1 | (o.c == 0) << 2;
-        cls.push_back(make_int4(o.a, o.b, o.c, 7 ^ z));
-        for (int al = 0; al < 8; al++)
-            for (int be = 0; be < 8; be++) {
-                const int na = cnt[al][o.pt], nb = cnt[be][o.pt];
-                if (((al ^ be) & z) || na == 0 || nb == 0) continue;
-                FoldBlock b;
-                b.off = tot; b.k4 = div_up(nb, 4); b.rb = div_up(na, 8); b.off_id = q;
-                b.alpha = al; b.beta = be; b.na = na; b.nb = nb; b.work0 = 0;
-                aoff[(size_t)q * 64 + al * 8 + be] = tot;
-                tot += (long long)b.k4 * b.rb * 32;
-                blocks.push_back(b);
-            }
-    }
-    // segments (offset class, round of column classes, K range) packed into batches
     std::vector<FoldTask> tasks;
     std::vector<FoldBatch> batches;
-    std::vector<int> seg_cls;
-    std::vector<int4> wseg;
+    std::vector<int2> runs;
     std::vector<double> cost;
-    int fill[8] = {};
+    long long tot = 0;
+    int fill = 0;
+    struct Seg { int rb, k0, depth; };
+    std::vector<Seg> open_;
+    int open_cls = -1, open_row = 0;
+    auto close_run = [&]() {
+        if (open_.empty()) return;
+        const FoldOffset &o = off[open_cls];
+        const int z = 7 ^ cls[open_cls].w;
+        int depth = 0;
+        double most = 0;
+        for (const Seg &g : open_) depth += g.depth;
+        for (int al = 0; al < 8; al++) {
+            const int na = cnt[al][o.pt], rb = div_up(na, 8);
+            runs.push_back(na ? make_int2((int)(tot / 32), depth / 4 | rb << 4 | open_row << 8 | open_cls << 16)
+                              : make_int2(0, open_cls << 16));
+            if (!na) continue;
+            for (const Seg &g : open_) {
+                const int be = (al & z) | g.rb;
+                FoldBlock b;
+                b.off = tot; b.k4 = g.depth / 4; b.rb = rb; b.off_id = open_cls; b.alpha = al; b.beta = be; b.na = na;
+                b.nb = cnt[be][o.pt]; b.k0 = g.k0;
+                blocks.push_back(b);
+                tot += (long long)b.k4 * b.rb * 32;
+            }
+            most = std::max(most, depth / 4.0 * rb);
+        }
+        batches.back().nrun++;
+        cost.back() += most;
+        open_.clear();
+    };
     for (int q = 0; q < kFoldClasses; q++) {
         const FoldOffset &o = off[q];
-        const int free_ = cls[q].w, z = 7 ^ free_;
+        const int z = (o.a == 0) | (o.b == 0) << 1 | (o.c == 0) << 2, free_ = 7 ^ z;
+        cls.push_back(make_int4(o.a, o.b, o.c, free_));
         int axis[3], bits = 0;
         for (int i = 0; i < 3; i++)
             if (free_ >> i & 1) axis[bits++] = i;
-        auto spread = [&](int j) {
-            int g = 0;
-            for (int i = 0; i < bits; i++) g |= (j >> i & 1) << axis[i];
-            return g;
-        };
         int most = 0;
         for (int c = 0; c < 8; c++) most = std::max(most, cnt[c][o.pt]);
+        const int kcap = bits == 1 ? 32 : kFoldCap;   // (four column classes a round: 32 tasks)
+        open_cls = q;
         for (int r = 0; r < 1 << bits; r++)
-            for (int k0 = 0; k0 < most; k0 += kFoldCap) {
-                const int rb = spread(r);
-                int depth[8];   // operand rows of row class al: column class (al & z) | rb
-                bool fits = true, any = false;
-                for (int al = 0; al < 8; al++) {
-                    const int nb = cnt[(al & z) | rb][o.pt] - k0, na = cnt[al][o.pt];
-                    depth[al] = nb > 0 && na > 0 ? 4 * div_up(std::min(nb, kFoldCap), 4) : 0;
-                    any |= depth[al] > 0;
-                    fits &= fill[al] + depth[al] <= kFoldCap;
+            for (int k0 = 0; k0 < most; k0 += kcap) {
+                int rb = 0;   // the round's column classes: these bits on the free axes, any on the others
+                for (int i = 0; i < bits; i++) rb |= (r >> i & 1) << axis[i];
+                int depth = 0, ntask = 0;
+                for (int be = 0; be < 8; be++) {
+                    const int nb = (be & free_) == rb ? std::min(cnt[be][o.pt] - k0, kcap) : 0;
+                    if (nb <= 0) continue;
+                    depth = std::max(depth, 4 * div_up(nb, 4));
+                    ntask += div_up(nb, 4);
                 }
-                if (!any) continue;
-                if (batches.empty() || !fits) {
-                    batches.push_back({(int)tasks.size(), 0, (int)seg_cls.size(), 0});
-                    cost.push_back(8.0);   // staging latency of a batch, in K steps of one row block
-                    std::fill(fill, fill + 8, 0);
+                if (depth == 0) continue;
+                if (batches.empty() || fill + depth > kFoldCap || batches.back().ntask + ntask > kFoldMaxTask ||
+                    (open_.empty() && batches.back().nrun == kFoldMaxRun)) {
+                    close_run();
+                    batches.push_back({(int)tasks.size(), 0, (int)runs.size() / 8, 0});
+                    cost.push_back(8.0);   // latency of a batch, in K steps of one row block
+                    fill = 0;
                 }
-                double most_steps = 0;
-                for (int al = 0; al < 8; al++) {
-                    const int be = (al & z) | rb, nrb = div_up(cnt[al][o.pt], 8);
-                    wseg.push_back(depth[al] ? make_int4((int)(aoff[(size_t)q * 64 + al * 8 + be] / 32) + k0 / 4 * nrb,
-                                                         depth[al] / 4, nrb, fill[al])
-                                             : make_int4(0, 0, 0, 0));
-                    most_steps = std::max(most_steps, depth[al] / 4.0 * nrb);
-                }
-                // staging tasks: the round's column classes, 4 coefficients each
+                if (open_.empty()) open_row = fill;
+                open_.push_back({rb, k0, depth});
+                // staging tasks: the round's column classes, 4 coefficients each, zeros up to the depth
                 for (int be = 0; be < 8; be++) {
                     if ((be & free_) != rb) continue;
-                    const int nb = std::min(cnt[be][o.pt] - k0, kFoldCap);
+                    const int nb = std::max(0, std::min(cnt[be][o.pt] - k0, kcap));
                     for (int k = 0; k < nb; k += 4) {
                         FoldTask t = {};
-                        t.src0 = base[be] + k0 + k;
-                        t.cls = (unsigned char)q; t.n = (unsigned char)std::min(4, nb - k);
-                        t.bits = (unsigned char)bits; t.beta = (unsigned char)be;
-                        for (int i = 0; i < bits; i++) t.axis[i] = (unsigned char)axis[i];
-                        bool used = false;
-                        for (int j = 0; j < 1 << bits; j++) {
-                            const int al = be ^ spread(j);
-                            t.row[j] = depth[al] ? (unsigned char)(fill[al] + k) : 255;
-                            used |= depth[al] > 0;
-                        }
-                        if (used) tasks.push_back(t);
+                        t.src0 = (unsigned short)(base[be] + k0 + k);
+                        t.cls = (unsigned char)q;
+                        t.n_beta_free = (unsigned char)((std::min(4, nb - k) - 1) | be << 2 | free_ << 5);
+                        t.row = (unsigned short)(fill + k);
+                        tasks.push_back(t);
                     }
                 }
-                for (int al = 0; al < 8; al++) fill[al] += depth[al];
-                seg_cls.push_back(q);
-                batches.back().nseg++;
                 batches.back().ntask = (int)tasks.size() - batches.back().task0;
-                cost.back() += most_steps;
+                fill += depth;
             }
+        close_run();
     }
     F.nbatch = (int)batches.size();
     double all = 0, run = 0;
@@ -238,14 +238,14 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
     };
     std::vector<FoldOffset> offs(off, off + kFoldClasses);
     put(F.kmap, kmap); put(F.rmap, rmap); put(F.base, base); put(F.group, group); put(F.cls, cls); put(F.tasks, tasks);
-    put(F.batches, batches); put(F.seg_cls, seg_cls); put(F.wseg, wseg); put(dblocks, blocks); put(doffs, offs);
+    put(F.batches, batches); put(F.runs, runs); put(dblocks, blocks); put(doffs, offs);
     F.A.alloc(tot, s, st);
     if (!st.ok()) return false;
     k_fold_ops<<<(unsigned)blocks.size(), 128, 0, s>>>(dblocks.p, doffs.p, F.kmap.p, F.base.p, p, rot, dc, lddc,
                                                        F.A.p); FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
     FMM_TRY(st, cudaStreamSynchronize(s));
-    F.kmap.s = F.rmap.s = F.base.s = F.group.s = F.cls.s = F.tasks.s = F.batches.s = F.seg_cls.s = F.wseg.s = F.A.s = nullptr;
+    F.kmap.s = F.rmap.s = F.base.s = F.group.s = F.cls.s = F.tasks.s = F.batches.s = F.runs.s = F.A.s = nullptr;
     return st.ok();
 }
 
@@ -289,8 +289,7 @@ struct FoldView {
     const int4 *cls;
     const FoldTask *tasks;
     const FoldBatch *batches;
-    const int *seg_cls;
-    const int4 *wseg;
+    const int2 *runs;
     const double *A;
     const int *group;
     int K;
@@ -298,15 +297,19 @@ struct FoldView {
 
 // Stage one task for the 8 targets of this lane group: BITS reflections.
 template <int BITS, int NT>
-__device__ __forceinline__ void fold_stage(const FoldTask &t, const int *idx, int tl, int kk, int K,
-                                           const double2 *mr, double *X)
+__device__ __forceinline__ void fold_stage(const FoldTask &t, const unsigned *idx, int tl, int kk, const double2 *mr,
+                                           double *X)
 {
     constexpr int NS = 1 << BITS;
+    const int n = (t.n_beta_free & 3) + 1, beta = t.n_beta_free >> 2 & 7, fr = t.n_beta_free >> 5;
+    const int lo = fr & -fr, hi = fr ^ lo;   // the axes of bits 0 and 1 (one or two reflections)
+    const unsigned at = t.src0 + kk, none = kk < n ? 0 : ~0u;
+    const unsigned *id = idx + t.cls * 8 * NT + tl;
     double2 v[NS];
 #pragma unroll
     for (int g = 0; g < NS; g++) {
-        const int b = idx[(t.cls * 8 + g) * NT + tl];
-        v[g] = b >= 0 && kk < t.n ? __ldg(mr + (size_t)b * K + t.src0 + kk) : cmk(0, 0);
+        const unsigned b = id[g * NT] | none;
+        v[g] = b != ~0u ? __ldg(mr + (b + at)) : cmk(0, 0);
     }
     // sums over the reflections with the signs of every character
 #pragma unroll
@@ -318,58 +321,91 @@ __device__ __forceinline__ void fold_stage(const FoldTask &t, const int *idx, in
                 v[g] = cadd(a, b);
                 v[g | h] = csub(a, b);
             }
+    double *x = X + (t.row + kk) * kFoldLd<NT> + 2 * tl;
 #pragma unroll
     for (int c = 0; c < NS; c++) {
-        int sp = 0;
-#pragma unroll
-        for (int i = 0; i < BITS; i++) sp |= (c >> i & 1) << t.axis[i];
-        if (t.row[c] != 255)
-            *reinterpret_cast<double2 *>(X + ((t.beta ^ sp) * kFoldCap + t.row[c] + kk) * kFoldLd<NT> + 2 * tl) = v[c];
+        const int sp = BITS == 3 ? c : (c & 1 ? lo : 0) | (c & 2 ? hi : 0);
+        *reinterpret_cast<double2 *>(x + (beta ^ sp) * (kFoldCap * kFoldLd<NT>)) = v[c];
     }
 }
 
+// R row blocks x NT / 4 column blocks over k4 K steps.  The operator fragments of U
+// steps are loaded while the U steps before are multiplied (U = 0: step by step), as
+// far as the registers left by the sums allow.
 template <int R, int RT, int NT>
-__device__ __forceinline__ void fold_mma(double (&acc)[RT][NT / 4][2], const double *A, int astep, int k4,
+__device__ __forceinline__ void fold_mma(double (&acc)[RT][NT / 4][2], const double *A, int astep, int rstep, int k4,
                                          const double *X)
 {
-    for (int ks = 0; ks < k4; ks++) {
-        double a[R], b[NT / 4];
+    constexpr int U = R == 1 ? 3 : R <= 3 ? 1 : 0, V = U ? U : 1;
+    double cur[V][R], nxt[V][R];
+    if (U) {
 #pragma unroll
-        for (int r = 0; r < R; r++) a[r] = __ldg(A + 32 * r);
+        for (int u = 0; u < V; u++)
 #pragma unroll
-        for (int c = 0; c < NT / 4; c++) b[c] = X[8 * c];
-        A += astep;
-        X += 4 * kFoldLd<NT>;
+            for (int r = 0; r < R; r++) cur[u][r] = u < k4 ? __ldg(A + u * astep + rstep * r) : 0;
+    }
+    for (int k0 = 0; k0 < k4; k0 += V) {
+        if (U) {
+            A += V * astep;
 #pragma unroll
-        for (int r = 0; r < R; r++)
+            for (int u = 0; u < V; u++)
 #pragma unroll
-            for (int c = 0; c < NT / 4; c++) dmma(acc[r][c][0], acc[r][c][1], a[r], b[c]);
+                for (int r = 0; r < R; r++) nxt[u][r] = k0 + V + u < k4 ? __ldg(A + u * astep + rstep * r) : 0;
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) cur[0][r] = __ldg(A + rstep * r);
+            A += astep;
+        }
+#pragma unroll
+        for (int u = 0; u < V; u++) {
+            if (k0 + u >= k4) break;
+            double b[NT / 4];
+#pragma unroll
+            for (int c = 0; c < NT / 4; c++) b[c] = X[8 * c];
+            X += 4 * kFoldLd<NT>;
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int c = 0; c < NT / 4; c++) dmma(acc[r][c][0], acc[r][c][1], cur[u][r], b[c]);
+        }
+        if (U) {
+#pragma unroll
+            for (int u = 0; u < V; u++)
+#pragma unroll
+                for (int r = 0; r < R; r++) cur[u][r] = nxt[u][r];
+        }
     }
 }
 
 template <int R, int RT, int NT>
-__device__ __forceinline__ void fold_mma_n(int n, double (&acc)[RT][NT / 4][2], const double *A, int astep,
+__device__ __forceinline__ void fold_mma_n(int n, double (&acc)[RT][NT / 4][2], const double *A, int astep, int rstep,
                                            int k4, const double *X)
 {
     if constexpr (R > 0) {
-        if (n == R) fold_mma<R, RT, NT>(acc, A, astep, k4, X);
-        else fold_mma_n<R - 1, RT, NT>(n, acc, A, astep, k4, X);
+        if (n == R) fold_mma<R, RT, NT>(acc, A, astep, rstep, k4, X);
+        else fold_mma_n<R - 1, RT, NT>(n, acc, A, astep, rstep, k4, X);
     }
 }
 
-// RS warps per parity class, each with up to RT 8-row blocks of it.
+// RS warps per parity class, which take its row blocks in turn, up to RT each.
+// Descriptors are read a batch ahead, one per lane, and handed round by shuffles: read
+// where they are used, each costs a trip to L2 per warp.
 template <int RS, int RT, int NT, int CTAS>
 __global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeView tv, int first, int count,
                                                           const double2 *mr, double2 *lr, int slots, int prune)
 {
+    constexpr int NTHR = 256 * RS, NW = 8 * RS, H = NT / 8;
     extern __shared__ double fold_sm[];
-    double *X = fold_sm;                                               // [8][kFoldCap][kFoldLd]
-    int *idx = reinterpret_cast<int *>(X + 8 * kFoldCap * kFoldLd<NT>);    // source boxes [class][reflection][target]
+    double *X = fold_sm;                                                          // [8][kFoldCap][kFoldLd]
+    unsigned *idx = reinterpret_cast<unsigned *>(X + 8 * kFoldCap * kFoldLd<NT>); // first coefficient of the source
+                                                                                  // boxes [class][reflection][target]
     __shared__ unsigned present[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int al = warp & 7, rs = warp >> 3;
     const int t0 = blockIdx.x * NT;
     if (tid < 2) present[tid] = 0;
+    // rows that a class does not fill meet zeros of the operator: they have to be finite
+    for (int i = tid; i < 8 * kFoldCap * kFoldLd<NT>; i += NTHR) X[i] = 0;
     __syncthreads();
     {
         // tid % NT is the target throughout
@@ -377,7 +413,7 @@ __global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeVie
         const int b = t0 + t < count ? first + t0 + t : -1;
         const bool use = b >= 0 && !(prune && tv.ntrg[b] == 0);
         const int o = use ? tv.octant[b] : 0, P = use ? tv.parent[b] : -1;
-        for (int e = tid / NT; e < kFoldClasses * 8; e += 256 * RS / NT) {
+        for (int e = tid / NT; e < kFoldClasses * 8; e += NTHR / NT) {
             const int q = e >> 3, j = e & 7;
             const int4 c = f.cls[q];
             int src = -1;
@@ -401,52 +437,28 @@ __global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeVie
                 src = C >= 0 ? tv.child[8L * C + oct] : -1;
                 if (src >= 0 && tv.nsrc[src] == 0) src = -1;
             }
-            idx[e * NT + t] = src;
+            idx[e * NT + t] = src >= 0 ? (unsigned)src * (unsigned)f.K : ~0u;
             if (src >= 0) atomicOr(&present[q >> 5], 1u << (q & 31));
         }
     }
     __syncthreads();
     const unsigned long long have = present[0] | (unsigned long long)present[1] << 32;
-    double acc[RT][NT / 4][2];
     const int g0 = slots > 1 ? blockIdx.y : 0, g1 = slots > 1 ? g0 + 1 : kFoldGroups;
-    for (int g = g0; g < g1; g++) {
+    const int bend = f.group[g1];
+    double acc[RT][NT / 4][2];
+    auto clear = [&]() {
 #pragma unroll
         for (int r = 0; r < RT; r++)
 #pragma unroll
             for (int c = 0; c < NT / 4; c++) acc[r][c][0] = acc[r][c][1] = 0;
-        bool any = false;
-        for (int bi = f.group[g]; bi < f.group[g + 1]; bi++) {
-            const FoldBatch B = f.batches[bi];
-            bool need = false;
-            for (int sg = 0; sg < B.nseg; sg++) need |= have >> f.seg_cls[B.seg0 + sg] & 1;
-            if (!need) continue;
-            any = true;
-            __syncthreads();
-            for (int ti = warp; ti < NT / 8 * B.ntask; ti += 8 * RS) {
-                const FoldTask t = f.tasks[B.task0 + ti / (NT / 8)];
-                if (!(have >> t.cls & 1)) continue;
-                const int tl = ti % (NT / 8) * 8 + (lane & 7), kk = lane >> 3;
-                if (t.bits == 3) fold_stage<3, NT>(t, idx, tl, kk, f.K, mr, X);
-                else if (t.bits == 2) fold_stage<2, NT>(t, idx, tl, kk, f.K, mr, X);
-                else fold_stage<1, NT>(t, idx, tl, kk, f.K, mr, X);
-            }
-            __syncthreads();
-            for (int sg = 0; sg < B.nseg; sg++) {
-                if (!(have >> f.seg_cls[B.seg0 + sg] & 1)) continue;
-                const int4 w = f.wseg[(B.seg0 + sg) * 8 + al];
-                // this warp's row blocks of the class
-                const int r0 = rs * RT, nr = min(w.z - r0, RT);
-                if (w.y == 0 || nr <= 0) continue;
-                fold_mma_n<RT, RT, NT>(nr, acc, f.A + (size_t)w.x * 32 + r0 * 32 + lane, w.z * 32, w.y,
-                                   X + (al * kFoldCap + w.w + (lane & 3)) * kFoldLd<NT> + (lane >> 2));
-            }
-        }
-        // the group's sums: lane l holds both right-hand sides of target 4 c + l % 4, row 8 r + l / 4
-        if (!any && slots == 1 && g > 0) continue;
+    };
+    // a group's sums: lane l holds both right-hand sides of target 4 c + l % 4, row 8 r + l / 4
+    auto flush = [&](int g, bool any) {
+        if (!any && slots == 1 && g > 0) return;
         const int na = f.base[8 + al];
 #pragma unroll
         for (int r = 0; r < RT; r++) {
-            const int row = (rs * RT + r) * 8 + (lane >> 2);
+            const int row = (r * RS + rs) * 8 + (lane >> 2);
 #pragma unroll
             for (int c = 0; c < NT / 4; c++) {
                 const int t = t0 + 4 * c + (lane & 3);
@@ -456,16 +468,74 @@ __global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeVie
                 *o = slots > 1 || g == 0 ? v : cadd(*o, v);
             }
         }
+        clear();
+    };
+    // descriptors of a batch: task `lane`, and run `lane` of this warp's class
+    int ntask = 0, nrun = 0;
+    int2 task = make_int2(0, 0), run = task;
+    auto fetch = [&](int b) {
+        if (b >= bend) return;
+        const FoldBatch B = f.batches[b];
+        ntask = B.ntask;
+        nrun = B.nrun;
+        if (lane < B.ntask) task = reinterpret_cast<const int2 *>(f.tasks + B.task0)[lane];
+        if (lane < B.nrun) run = f.runs[(B.run0 + lane) * 8 + al];
+    };
+    clear();
+    int g = g0;
+    bool any = false;
+    fetch(f.group[g0]);
+    for (int bi = f.group[g0]; bi < bend; bi++) {
+        while (bi >= f.group[g + 1]) {
+            flush(g++, any);
+            any = false;
+        }
+        const int2 ru = run;
+        const int nr_ = nrun;
+        // (run 0's class, and so on, are the same in every warp)
+        const bool need = __any_sync(0xffffffffu, lane < nr_ && (have >> (ru.y >> 16) & 1));
+        if (need) {
+            any = true;
+            __syncthreads();
+            for (int u = warp; u < H * ntask; u += NW) {
+                const int x0 = __shfl_sync(0xffffffffu, task.x, u / H), y0 = __shfl_sync(0xffffffffu, task.y, u / H);
+                FoldTask t;
+                t.src0 = (unsigned short)(x0 & 0xffff);
+                t.cls = (unsigned char)(x0 >> 16 & 0xff);
+                t.n_beta_free = (unsigned char)((unsigned)x0 >> 24);
+                t.row = (unsigned short)(y0 & 0xffff);
+                if (!(have >> t.cls & 1)) continue;
+                const int tl = u % H * 8 + (lane & 7), kk = lane >> 3, bits = __popc(t.n_beta_free >> 5);
+                if (bits == 3) fold_stage<3, NT>(t, idx, tl, kk, mr, X);
+                else if (bits == 2) fold_stage<2, NT>(t, idx, tl, kk, mr, X);
+                else fold_stage<1, NT>(t, idx, tl, kk, mr, X);
+            }
+        }
+        fetch(bi + 1);
+        if (!need) continue;
+        __syncthreads();
+        for (int i = 0; i < nr_; i++) {
+            const int a = __shfl_sync(0xffffffffu, ru.x, i), w = __shfl_sync(0xffffffffu, ru.y, i);
+            if (!(have >> (w >> 16) & 1)) continue;
+            const int k4 = w & 15, rb = w >> 4 & 15, row = w >> 8 & 255;
+            const int nr = (rb - rs + RS - 1) / RS;   // this warp's row blocks of the class
+            if (nr > 0)
+                fold_mma_n<RT, RT, NT>(nr, acc, f.A + ((size_t)a + rs) * 32 + lane, rb * 32, RS * 32, k4,
+                                       X + (al * kFoldCap + row + (lane & 3)) * kFoldLd<NT> + (lane >> 2));
+        }
+    }
+    for (; g < g1; g++) {
+        flush(g, any);
+        any = false;
     }
 }
 
 bool fold_prepare(const FoldPlan &F, FoldWork &W, int nboxes, int count, cudaStream_t s, Status &st)
 {
     if (count <= 0) return true;
-    W.tile = F.rows <= 5 ? 16 : 8;
-    W.slots = div_up(count, W.tile) < kFoldSplitTiles ? kFoldGroups : 1;
+    W.slots = div_up(count, F.tile) < kFoldSplitTiles ? kFoldGroups : 1;
     // at most 1 GB of sums at a time
-    const long long most = std::max<long long>((1LL << 30) / (16LL * F.K * W.slots) / W.tile, 1) * W.tile;
+    const long long most = std::max<long long>((1LL << 30) / (16LL * F.K * W.slots) / F.tile, 1) * F.tile;
     W.chunk = (int)std::min<long long>(count, W.slots > 1 ? count : most);
     return W.mr.alloc((size_t)nboxes * F.K, s, st) && W.lr.alloc((size_t)W.chunk * F.K * W.slots, s, st);
 }
@@ -494,8 +564,8 @@ void launch_m2l_fold(const FoldPlan &F, const FoldWork &W, const TreeView &tv, i
     const long long n = (long long)nboxes * F.K;
     k_fold_real<<<div_up(n, 256), 256, 0, s>>>(n, F.K, F.kmap.p, in, W.mr.p); FMM_COUNT_LAUNCH();
     FoldView f;
-    f.base = F.base.p; f.cls = F.cls.p; f.tasks = F.tasks.p; f.batches = F.batches.p; f.seg_cls = F.seg_cls.p;
-    f.wseg = F.wseg.p; f.A = F.A.p; f.group = F.group.p; f.K = F.K;
+    f.base = F.base.p; f.cls = F.cls.p; f.tasks = F.tasks.p; f.batches = F.batches.p; f.runs = F.runs.p;
+    f.A = F.A.p; f.group = F.group.p; f.K = F.K;
     // row blocks of the largest parity class: orders <= 6, <= 9, <= 14, above
     if (F.rows <= 1) launch_fold_t<1, 1, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);
     else if (F.rows <= 2) launch_fold_t<1, 2, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);

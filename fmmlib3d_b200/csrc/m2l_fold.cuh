@@ -17,24 +17,25 @@ struct FoldOffset {
 };
 
 // Staging of 4 consecutive coefficients of one parity class: source
-// coefficients from `src0` on, `n` of them valid, combined over the
-// 2^bits reflections of offset class `cls` into the operand rows `row[j]` of
-// parity classes beta ^ spread(j).
-struct __align__(16) FoldTask {
-    int src0;
-    unsigned char cls, n, bits, beta;
-    unsigned char axis[4];    // axis[i]: coordinate axis of reflection bit i
-    unsigned char row[8];
-    int pad[3];
+// coefficients from `src0` on, `n` of them valid, combined over the reflections
+// of offset class `cls` (coordinate axes `free`, a bit each) into the operand rows from
+// `row` on of the parity classes beta ^ (j spread over the axes).
+struct __align__(8) FoldTask {
+    unsigned short src0;
+    unsigned char cls, n_beta_free;   // n - 1 (2 bits), beta (3 bits), free (3 bits)
+    unsigned short row, pad;
 };
 
-// A batch: the segments whose operands share one filling of shared memory.
+// A batch: the tasks and runs (offset classes) that share one filling of shared memory.
 struct FoldBatch {
-    int task0, ntask, seg0, nseg;
+    int task0, ntask, run0, nrun;
 };
+constexpr int kFoldMaxTask = 32, kFoldMaxRun = 16;   // of a batch (a task and a run per lane)
 
 struct FoldPlan {
-    int p = 0, K = 0, nbatch = 0, rows = 0;   // rows: 8-row blocks of the largest parity class
+    int p = 0, K = 0, nbatch = 0;
+    int rows = 0;             // 8-row blocks of the largest parity class
+    int tile = 16;            // targets per CTA
     DBuf<int4> kmap;          // real coefficient -> (n, m), (n, -m), 1 for the sine part
     DBuf<int4> rmap;          // (n, m >= 0) -> (n, m), (n, -m), cosine and sine coefficients
     DBuf<int> base;           // first coefficient and count of every parity class
@@ -42,8 +43,7 @@ struct FoldPlan {
     DBuf<int4> cls;           // offset classes: a, b, c, reflection bits
     DBuf<FoldTask> tasks;
     DBuf<FoldBatch> batches;
-    DBuf<int> seg_cls;
-    DBuf<int4> wseg;          // (segment, parity class): operator fragment, K steps, row blocks, operand row
+    DBuf<int2> runs;          // (run, parity class): operator fragment; K steps, row blocks, first operand row, class
     DBuf<double> A;           // operator fragments
 };
 
@@ -56,7 +56,7 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
 // first + count - 1 (boxes of level >= 2).
 struct FoldWork {
     DBuf<double2> mr, lr;
-    int slots = 1, chunk = 0, tile = 16;   // tile: targets per CTA
+    int slots = 1, chunk = 0;
 };
 bool fold_prepare(const FoldPlan &F, FoldWork &W, int nboxes, int count, cudaStream_t s, Status &st);
 void launch_m2l_fold(const FoldPlan &F, const FoldWork &W, const TreeView &tv, int nboxes, int first, int count,
