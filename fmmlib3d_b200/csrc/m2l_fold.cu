@@ -167,6 +167,7 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
             most = std::max(most, depth / 4.0 * rb);
         }
         batches.back().nrun++;
+        batches.back().classes |= 1ull << open_cls;
         cost.back() += most;
         open_.clear();
     };
@@ -196,7 +197,7 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
                 if (batches.empty() || fill + depth > kFoldCap || batches.back().ntask + ntask > kFoldMaxTask ||
                     (open_.empty() && batches.back().nrun == kFoldMaxRun)) {
                     close_run();
-                    batches.push_back({(int)tasks.size(), 0, (int)runs.size() / 8, 0});
+                    batches.push_back({(int)tasks.size(), 0, (int)runs.size() / 8, 0, 0});
                     cost.push_back(8.0);   // latency of a batch, in K steps of one row block
                     fill = 0;
                 }
@@ -295,23 +296,37 @@ struct FoldView {
     int K;
 };
 
-// Stage one task for the 8 targets of this lane group: BITS reflections.
-template <int BITS, int NT>
-__device__ __forceinline__ void fold_stage(const FoldTask &t, const unsigned *idx, int tl, int kk, const double2 *mr,
-                                           double *X)
+__device__ __forceinline__ FoldTask fold_task(int x, int y)
 {
-    constexpr int NS = 1 << BITS;
-    const int n = (t.n_beta_free & 3) + 1, beta = t.n_beta_free >> 2 & 7, fr = t.n_beta_free >> 5;
-    const int lo = fr & -fr, hi = fr ^ lo;   // the axes of bits 0 and 1 (one or two reflections)
-    const unsigned at = t.src0 + kk, none = kk < n ? 0 : ~0u;
+    FoldTask t;
+    t.src0 = (unsigned short)(x & 0xffff);
+    t.cls = (unsigned char)(x >> 16 & 0xff);
+    t.n_beta_free = (unsigned char)((unsigned)x >> 24);
+    t.row = (unsigned short)(y & 0xffff);
+    return t;
+}
+
+// Staging of one task for the 8 targets of this lane group, BITS reflections: the
+// sources' coefficients, then their sums with the signs of every character into X.
+template <int BITS, int NT>
+__device__ __forceinline__ void fold_load(const FoldTask &t, const unsigned *idx, int tl, int kk, const double2 *mr,
+                                          double2 (&v)[8])
+{
+    const unsigned at = t.src0 + kk, none = kk < (t.n_beta_free & 3) + 1 ? 0 : ~0u;
     const unsigned *id = idx + t.cls * 8 * NT + tl;
-    double2 v[NS];
 #pragma unroll
-    for (int g = 0; g < NS; g++) {
+    for (int g = 0; g < 1 << BITS; g++) {
         const unsigned b = id[g * NT] | none;
         v[g] = b != ~0u ? __ldg(mr + (b + at)) : cmk(0, 0);
     }
-    // sums over the reflections with the signs of every character
+}
+
+template <int BITS, int NT>
+__device__ __forceinline__ void fold_store(const FoldTask &t, int tl, int kk, double2 (&v)[8], double *X)
+{
+    constexpr int NS = 1 << BITS;
+    const int beta = t.n_beta_free >> 2 & 7, fr = t.n_beta_free >> 5;
+    const int lo = fr & -fr, hi = fr ^ lo;   // the axes of bits 0 and 1 (one or two reflections)
 #pragma unroll
     for (int h = 1; h < NS; h <<= 1)
 #pragma unroll
@@ -327,6 +342,23 @@ __device__ __forceinline__ void fold_stage(const FoldTask &t, const unsigned *id
         const int sp = BITS == 3 ? c : (c & 1 ? lo : 0) | (c & 2 ? hi : 0);
         *reinterpret_cast<double2 *>(x + (beta ^ sp) * (kFoldCap * kFoldLd<NT>)) = v[c];
     }
+}
+
+template <int NT>
+__device__ __forceinline__ void fold_load_n(int bits, const FoldTask &t, const unsigned *idx, int tl, int kk,
+                                            const double2 *mr, double2 (&v)[8])
+{
+    if (bits == 3) fold_load<3, NT>(t, idx, tl, kk, mr, v);
+    else if (bits == 2) fold_load<2, NT>(t, idx, tl, kk, mr, v);
+    else fold_load<1, NT>(t, idx, tl, kk, mr, v);
+}
+
+template <int NT>
+__device__ __forceinline__ void fold_store_n(int bits, const FoldTask &t, int tl, int kk, double2 (&v)[8], double *X)
+{
+    if (bits == 3) fold_store<3, NT>(t, tl, kk, v, X);
+    else if (bits == 2) fold_store<2, NT>(t, tl, kk, v, X);
+    else fold_store<1, NT>(t, tl, kk, v, X);
 }
 
 // R row blocks x NT / 4 column blocks over k4 K steps.  The operator fragments of U
@@ -387,28 +419,36 @@ __device__ __forceinline__ void fold_mma_n(int n, double (&acc)[RT][NT / 4][2], 
     }
 }
 
-// RS warps per parity class, which take its row blocks in turn, up to RT each.
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// Warps 0 .. 7 multiply, one parity class each (up to RT row blocks); the SW warps after
+// them stage the next batch into the other of two buffers meanwhile, two tasks' loads
+// in flight each.  Named barriers 1, 2 (a buffer is full) and 3, 4 (free again): both
+// sides walk the same list of batches, so every arrival meets one wait.
 // Descriptors are read a batch ahead, one per lane, and handed round by shuffles: read
 // where they are used, each costs a trip to L2 per warp.
-template <int RS, int RT, int NT, int CTAS>
-__global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeView tv, int first, int count,
-                                                          const double2 *mr, double2 *lr, int slots, int prune)
+template <int RT, int NT, int SW>
+__global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeView tv, int first, int count,
+                                                            const double2 *mr, double2 *lr, int slots, int prune)
 {
-    constexpr int NTHR = 256 * RS, NW = 8 * RS, H = NT / 8;
+    constexpr int NTHR = 256 + 32 * SW, H = NT / 8, XBUF = 8 * kFoldCap * kFoldLd<NT>;
     extern __shared__ double fold_sm[];
-    double *X = fold_sm;                                                          // [8][kFoldCap][kFoldLd]
-    unsigned *idx = reinterpret_cast<unsigned *>(X + 8 * kFoldCap * kFoldLd<NT>); // first coefficient of the source
-                                                                                  // boxes [class][reflection][target]
+    double *X = fold_sm;                                         // two buffers [8][kFoldCap][kFoldLd]
+    unsigned *idx = reinterpret_cast<unsigned *>(X + 2 * XBUF);  // first coefficient of the source
+                                                                 // boxes [class][reflection][target]
+    short *order = reinterpret_cast<short *>(idx + kFoldClasses * 8 * NT);   // batches with sources
     __shared__ unsigned present[2];
+    __shared__ int norder;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int al = warp & 7, rs = warp >> 3;
     const int t0 = blockIdx.x * NT;
     if (tid < 2) present[tid] = 0;
     // rows that a class does not fill meet zeros of the operator: they have to be finite
-    for (int i = tid; i < 8 * kFoldCap * kFoldLd<NT>; i += NTHR) X[i] = 0;
+    for (int i = tid; i < 2 * XBUF; i += NTHR) X[i] = 0;
     __syncthreads();
     {
         // tid % NT is the target throughout
+        static_assert(NTHR % NT == 0, "");
         const int t = tid & (NT - 1);
         const int b = t0 + t < count ? first + t0 + t : -1;
         const bool use = b >= 0 && !(prune && tv.ntrg[b] == 0);
@@ -444,7 +484,57 @@ __global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeVie
     __syncthreads();
     const unsigned long long have = present[0] | (unsigned long long)present[1] << 32;
     const int g0 = slots > 1 ? blockIdx.y : 0, g1 = slots > 1 ? g0 + 1 : kFoldGroups;
-    const int bend = f.group[g1];
+    const int bbeg = f.group[g0], bend = f.group[g1];
+    if (warp == 0) {
+        int n = 0;
+        for (int b0 = bbeg; b0 < bend; b0 += 32) {
+            const bool need = b0 + lane < bend && (f.batches[b0 + lane].classes & have);
+            const unsigned m = __ballot_sync(0xffffffffu, need);
+            if (need) order[n + __popc(m & ((1u << lane) - 1))] = (short)(b0 + lane);
+            n += __popc(m);
+        }
+        if (lane == 0) norder = n;
+    }
+    __syncthreads();
+    const int N = norder;
+    if (warp >= 8) {
+        // ---- staging
+        const int w = warp - 8, kk = lane >> 3;
+        int ntask = 0;
+        int2 task = make_int2(0, 0);
+        auto fetch = [&](int n) {
+            if (n >= N) return;
+            const FoldBatch B = f.batches[order[n]];
+            ntask = B.ntask;
+            if (lane < B.ntask) task = reinterpret_cast<const int2 *>(f.tasks + B.task0)[lane];
+        };
+        fetch(0);
+        for (int n = 0; n < N; n++) {
+            const int2 cur = task;
+            const int units = H * ntask;
+            fetch(n + 1);
+            if (n >= 2) bar_sync(3 + (n & 1), NTHR);
+            double *x = X + (n & 1) * XBUF;
+            for (int u = w; u < units; u += 2 * SW) {
+                const int u1 = u + SW;
+                const FoldTask a = fold_task(__shfl_sync(0xffffffffu, cur.x, u / H), __shfl_sync(0xffffffffu, cur.y, u / H));
+                const FoldTask b = fold_task(__shfl_sync(0xffffffffu, cur.x, u1 / H & 31),
+                                             __shfl_sync(0xffffffffu, cur.y, u1 / H & 31));
+                const bool ua = have >> a.cls & 1, ub = u1 < units && (have >> b.cls & 1);
+                const int ta = u % H * 8 + (lane & 7), tb = u1 % H * 8 + (lane & 7);
+                const int ba = __popc(a.n_beta_free >> 5), bb = __popc(b.n_beta_free >> 5);
+                double2 va[8], vb[8];
+                if (ua) fold_load_n<NT>(ba, a, idx, ta, kk, mr, va);
+                if (ub) fold_load_n<NT>(bb, b, idx, tb, kk, mr, vb);
+                if (ua) fold_store_n<NT>(ba, a, ta, kk, va, x);
+                if (ub) fold_store_n<NT>(bb, b, tb, kk, vb, x);
+            }
+            bar_arrive(1 + (n & 1), NTHR);
+        }
+        return;
+    }
+    // ---- products
+    const int al = warp;
     double acc[RT][NT / 4][2];
     auto clear = [&]() {
 #pragma unroll
@@ -458,7 +548,7 @@ __global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeVie
         const int na = f.base[8 + al];
 #pragma unroll
         for (int r = 0; r < RT; r++) {
-            const int row = (r * RS + rs) * 8 + (lane >> 2);
+            const int row = r * 8 + (lane >> 2);
 #pragma unroll
             for (int c = 0; c < NT / 4; c++) {
                 const int t = t0 + 4 * c + (lane & 3);
@@ -470,59 +560,36 @@ __global__ void __launch_bounds__(256 * RS, CTAS) k_m2l_fold(FoldView f, TreeVie
         }
         clear();
     };
-    // descriptors of a batch: task `lane`, and run `lane` of this warp's class
-    int ntask = 0, nrun = 0;
-    int2 task = make_int2(0, 0), run = task;
-    auto fetch = [&](int b) {
-        if (b >= bend) return;
-        const FoldBatch B = f.batches[b];
-        ntask = B.ntask;
+    int nrun = 0;
+    int2 run = make_int2(0, 0);
+    auto fetch = [&](int n) {
+        if (n >= N) return;
+        const FoldBatch B = f.batches[order[n]];
         nrun = B.nrun;
-        if (lane < B.ntask) task = reinterpret_cast<const int2 *>(f.tasks + B.task0)[lane];
         if (lane < B.nrun) run = f.runs[(B.run0 + lane) * 8 + al];
     };
     clear();
     int g = g0;
     bool any = false;
-    fetch(f.group[g0]);
-    for (int bi = f.group[g0]; bi < bend; bi++) {
-        while (bi >= f.group[g + 1]) {
+    fetch(0);
+    for (int n = 0; n < N; n++) {
+        while (order[n] >= f.group[g + 1]) {
             flush(g++, any);
             any = false;
         }
+        any = true;
         const int2 ru = run;
-        const int nr_ = nrun;
-        // (run 0's class, and so on, are the same in every warp)
-        const bool need = __any_sync(0xffffffffu, lane < nr_ && (have >> (ru.y >> 16) & 1));
-        if (need) {
-            any = true;
-            __syncthreads();
-            for (int u = warp; u < H * ntask; u += NW) {
-                const int x0 = __shfl_sync(0xffffffffu, task.x, u / H), y0 = __shfl_sync(0xffffffffu, task.y, u / H);
-                FoldTask t;
-                t.src0 = (unsigned short)(x0 & 0xffff);
-                t.cls = (unsigned char)(x0 >> 16 & 0xff);
-                t.n_beta_free = (unsigned char)((unsigned)x0 >> 24);
-                t.row = (unsigned short)(y0 & 0xffff);
-                if (!(have >> t.cls & 1)) continue;
-                const int tl = u % H * 8 + (lane & 7), kk = lane >> 3, bits = __popc(t.n_beta_free >> 5);
-                if (bits == 3) fold_stage<3, NT>(t, idx, tl, kk, mr, X);
-                else if (bits == 2) fold_stage<2, NT>(t, idx, tl, kk, mr, X);
-                else fold_stage<1, NT>(t, idx, tl, kk, mr, X);
-            }
-        }
-        fetch(bi + 1);
-        if (!need) continue;
-        __syncthreads();
-        for (int i = 0; i < nr_; i++) {
+        const int nr = nrun;
+        fetch(n + 1);
+        bar_sync(1 + (n & 1), NTHR);
+        const double *x = X + (n & 1) * XBUF + (al * kFoldCap + (lane & 3)) * kFoldLd<NT> + (lane >> 2);
+        for (int i = 0; i < nr; i++) {
             const int a = __shfl_sync(0xffffffffu, ru.x, i), w = __shfl_sync(0xffffffffu, ru.y, i);
             if (!(have >> (w >> 16) & 1)) continue;
             const int k4 = w & 15, rb = w >> 4 & 15, row = w >> 8 & 255;
-            const int nr = (rb - rs + RS - 1) / RS;   // this warp's row blocks of the class
-            if (nr > 0)
-                fold_mma_n<RT, RT, NT>(nr, acc, f.A + ((size_t)a + rs) * 32 + lane, rb * 32, RS * 32, k4,
-                                       X + (al * kFoldCap + row + (lane & 3)) * kFoldLd<NT> + (lane >> 2));
+            if (rb > 0) fold_mma_n<RT, RT, NT>(rb, acc, f.A + (size_t)a * 32 + lane, rb * 32, 32, k4, x + row * kFoldLd<NT>);
         }
+        if (n + 2 < N) bar_arrive(3 + (n & 1), NTHR);
     }
     for (; g < g1; g++) {
         flush(g, any);
@@ -540,16 +607,17 @@ bool fold_prepare(const FoldPlan &F, FoldWork &W, int nboxes, int count, cudaStr
     return W.mr.alloc((size_t)nboxes * F.K, s, st) && W.lr.alloc((size_t)W.chunk * F.K * W.slots, s, st);
 }
 
-template <int RS, int RT, int NT, int CTAS>
+template <int RT, int NT, int SW>
 static void launch_fold_t(const FoldPlan &F, const FoldView &f, const FoldWork &W, const TreeView &tv, int first,
                           int count, double2 *out, int prune, cudaStream_t s, Status &st)
 {
-    constexpr size_t sm = sizeof(double) * 8 * kFoldCap * kFoldLd<NT> + sizeof(int) * kFoldClasses * 8 * NT;
-    FMM_TRY(st, smem_allow(k_m2l_fold<RS, RT, NT, CTAS>, sm));
+    const size_t sm = sizeof(double) * 2 * 8 * kFoldCap * kFoldLd<NT> + sizeof(int) * kFoldClasses * 8 * NT +
+                      sizeof(short) * F.nbatch;
+    FMM_TRY(st, smem_allow(k_m2l_fold<RT, NT, SW>, sm));
     const int nr = (F.p + 1) * (F.p + 2) / 2;
     for (int c0 = 0; c0 < count && st.ok(); c0 += W.chunk) {
         const int n = std::min(W.chunk, count - c0);
-        k_m2l_fold<RS, RT, NT, CTAS><<<dim3(div_up(n, NT), W.slots), 256 * RS, sm, s>>>(
+        k_m2l_fold<RT, NT, SW><<<dim3(div_up(n, NT), W.slots), 256 + 32 * SW, sm, s>>>(
             f, tv, first + c0, n, W.mr.p, W.lr.p, W.slots, prune); FMM_COUNT_LAUNCH();
         k_fold_add<<<div_up((long)n * nr, 256), 256, 0, s>>>(n, nr, F.K, W.slots, F.rmap.p, W.lr.p,
                                                              out + (size_t)(first + c0) * F.K); FMM_COUNT_LAUNCH();
@@ -567,10 +635,10 @@ void launch_m2l_fold(const FoldPlan &F, const FoldWork &W, const TreeView &tv, i
     f.base = F.base.p; f.cls = F.cls.p; f.tasks = F.tasks.p; f.batches = F.batches.p; f.runs = F.runs.p;
     f.A = F.A.p; f.group = F.group.p; f.K = F.K;
     // row blocks of the largest parity class: orders <= 6, <= 9, <= 14, above
-    if (F.rows <= 1) launch_fold_t<1, 1, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);
-    else if (F.rows <= 2) launch_fold_t<1, 2, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);
-    else if (F.rows <= 5) launch_fold_t<1, 5, 16, 2>(F, f, W, tv, first, count, out, prune, s, st);
-    else launch_fold_t<2, 7, 8, 1>(F, f, W, tv, first, count, out, prune, s, st);
+    if (F.rows <= 1) launch_fold_t<1, 16, 8>(F, f, W, tv, first, count, out, prune, s, st);
+    else if (F.rows <= 2) launch_fold_t<2, 16, 8>(F, f, W, tv, first, count, out, prune, s, st);
+    else if (F.rows <= 5) launch_fold_t<5, 16, 8>(F, f, W, tv, first, count, out, prune, s, st);
+    else launch_fold_t<14, 8, 4>(F, f, W, tv, first, count, out, prune, s, st);
 }
 
 }  // namespace fmm

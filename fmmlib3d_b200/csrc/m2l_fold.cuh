@@ -29,6 +29,7 @@ struct __align__(8) FoldTask {
 // A batch: the tasks and runs (offset classes) that share one filling of shared memory.
 struct FoldBatch {
     int task0, ntask, run0, nrun;
+    unsigned long long classes;   // offset classes of its runs
 };
 constexpr int kFoldMaxTask = 32, kFoldMaxRun = 16;   // of a batch (a task and a run per lane)
 
