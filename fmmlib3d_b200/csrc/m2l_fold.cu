@@ -19,12 +19,12 @@
 // rotate, all of them in matrix products.
 //
 // k_m2l_fold: a CTA owns 16 consecutive target boxes (32 columns: 16 targets x
-// 2 right-hand sides) and all their coefficients; warp w owns the rows of
-// parity class w (of half of it for high orders) in DMMA accumulators.  Per
-// batch all warps stage X (36 rows per parity class: 83 KB; two CTAs per SM fill
-// each other's staging gaps up to order 14), then
-// each warp multiplies its operator fragments, read from L2 in the lane order
-// of the MMA and each used for all 32 columns, with its rows.  Offset classes
+// 2 right-hand sides; 8 at order 26) and all their coefficients; warp w < 8 owns the rows of
+// parity class w in DMMA accumulators.  Per
+// batch other warps stage X (32 rows per parity class, 74 KB, two buffers) and bring
+// the batch's operator fragments into L1; each
+// warp multiplies its fragments, in the lane order of the MMA and each used for
+// all 32 columns, with its rows.  Offset classes
 // that no target of the tile has a source in are skipped.
 // The sums of a target are formed in 8 fixed groups of batches, added in
 // order; a small problem runs one CTA per (tile, group) and adds the groups
@@ -36,7 +36,7 @@
 
 namespace fmm {
 
-constexpr int kFoldCap = 36;                    // operand rows per parity class and batch
+constexpr int kFoldCap = 32;                    // operand rows per parity class and batch
 // Row stride of the operands of NT targets: = 4 mod 16 doubles, so that the 4 x 4
 // lanes of a half warp reading a fragment meet different banks.
 template <int NT>
@@ -170,6 +170,7 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
         batches.back().classes |= 1ull << open_cls;
         cost.back() += most;
         open_.clear();
+        batches.back().na = (int)(tot / 32) - batches.back().a0;
     };
     for (int q = 0; q < kFoldClasses; q++) {
         const FoldOffset &o = off[q];
@@ -197,7 +198,7 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
                 if (batches.empty() || fill + depth > kFoldCap || batches.back().ntask + ntask > kFoldMaxTask ||
                     (open_.empty() && batches.back().nrun == kFoldMaxRun)) {
                     close_run();
-                    batches.push_back({(int)tasks.size(), 0, (int)runs.size() / 8, 0, 0});
+                    batches.push_back({(int)tasks.size(), 0, (int)runs.size() / 8, 0, 0, (int)(tot / 32), 0});
                     cost.push_back(8.0);   // latency of a batch, in K steps of one row block
                     fill = 0;
                 }
@@ -361,48 +362,62 @@ __device__ __forceinline__ void fold_store_n(int bits, const FoldTask &t, int tl
     else fold_store<1, NT>(t, tl, kk, v, X);
 }
 
-// R row blocks x NT / 4 column blocks over k4 K steps.  The operator fragments of U
-// steps are loaded while the U steps before are multiplied (U = 0: step by step), as
-// far as the registers left by the sums allow.
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// One K step: R row blocks x NT / 4 column blocks.
 template <int R, int RT, int NT>
-__device__ __forceinline__ void fold_mma(double (&acc)[RT][NT / 4][2], const double *A, int astep, int rstep, int k4,
-                                         const double *X)
+__device__ __forceinline__ void fold_step(double (&acc)[RT][NT / 4][2], const double *A, const double *X)
 {
-    constexpr int U = R == 1 ? 3 : R <= 3 ? 1 : 0, V = U ? U : 1;
-    double cur[V][R], nxt[V][R];
-    if (U) {
+    double a[R], b[NT / 4];
 #pragma unroll
-        for (int u = 0; u < V; u++)
+    for (int r = 0; r < R; r++) a[r] = __ldg(A + 32 * r);
 #pragma unroll
-            for (int r = 0; r < R; r++) cur[u][r] = u < k4 ? __ldg(A + u * astep + rstep * r) : 0;
-    }
-    for (int k0 = 0; k0 < k4; k0 += V) {
-        if (U) {
-            A += V * astep;
+    for (int c = 0; c < NT / 4; c++) b[c] = X[8 * c];
 #pragma unroll
-            for (int u = 0; u < V; u++)
+    for (int r = 0; r < R; r++)
 #pragma unroll
-                for (int r = 0; r < R; r++) nxt[u][r] = k0 + V + u < k4 ? __ldg(A + u * astep + rstep * r) : 0;
-        } else {
-#pragma unroll
-            for (int r = 0; r < R; r++) cur[0][r] = __ldg(A + rstep * r);
-            A += astep;
-        }
-#pragma unroll
-        for (int u = 0; u < V; u++) {
-            if (k0 + u >= k4) break;
-            double b[NT / 4];
-#pragma unroll
-            for (int c = 0; c < NT / 4; c++) b[c] = X[8 * c];
+        for (int c = 0; c < NT / 4; c++) dmma(acc[r][c][0], acc[r][c][1], a[r], b[c]);
+}
+
+// R row blocks over k4 K steps (the fragments are in L1 by then).  Few row blocks: the
+// fragments of the next U steps are loaded while U steps are multiplied.
+template <int R, int RT, int NT>
+__device__ __forceinline__ void fold_mma(double (&acc)[RT][NT / 4][2], const double *A, int k4, const double *X)
+{
+    if constexpr (R > 3) {
+        for (int k = 0; k < k4; k++) {
+            fold_step<R, RT, NT>(acc, A, X);
+            A += 32 * R;
             X += 4 * kFoldLd<NT>;
-#pragma unroll
-            for (int r = 0; r < R; r++)
-#pragma unroll
-                for (int c = 0; c < NT / 4; c++) dmma(acc[r][c][0], acc[r][c][1], cur[u][r], b[c]);
         }
-        if (U) {
+    } else {
+        constexpr int U = R == 1 ? 3 : 1;
+        double cur[U][R], nxt[U][R];
 #pragma unroll
-            for (int u = 0; u < V; u++)
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int r = 0; r < R; r++) cur[u][r] = u < k4 ? __ldg(A + 32 * (u * R + r)) : 0;
+        for (int k0 = 0; k0 < k4; k0 += U) {
+            A += 32 * U * R;
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int r = 0; r < R; r++) nxt[u][r] = k0 + U + u < k4 ? __ldg(A + 32 * (u * R + r)) : 0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (k0 + u >= k4) break;
+                double b[NT / 4];
+#pragma unroll
+                for (int c = 0; c < NT / 4; c++) b[c] = X[8 * c];
+                X += 4 * kFoldLd<NT>;
+#pragma unroll
+                for (int r = 0; r < R; r++)
+#pragma unroll
+                    for (int c = 0; c < NT / 4; c++) dmma(acc[r][c][0], acc[r][c][1], cur[u][r], b[c]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
 #pragma unroll
                 for (int r = 0; r < R; r++) cur[u][r] = nxt[u][r];
         }
@@ -410,17 +425,13 @@ __device__ __forceinline__ void fold_mma(double (&acc)[RT][NT / 4][2], const dou
 }
 
 template <int R, int RT, int NT>
-__device__ __forceinline__ void fold_mma_n(int n, double (&acc)[RT][NT / 4][2], const double *A, int astep, int rstep,
-                                           int k4, const double *X)
+__device__ __forceinline__ void fold_mma_n(int n, double (&acc)[RT][NT / 4][2], const double *A, int k4, const double *X)
 {
     if constexpr (R > 0) {
-        if (n == R) fold_mma<R, RT, NT>(acc, A, astep, rstep, k4, X);
-        else fold_mma_n<R - 1, RT, NT>(n, acc, A, astep, rstep, k4, X);
+        if (n == R) fold_mma<R, RT, NT>(acc, A, k4, X);
+        else fold_mma_n<R - 1, RT, NT>(n, acc, A, k4, X);
     }
 }
-
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 // Warps 0 .. 7 multiply, one parity class each (up to RT row blocks); the SW warps after
 // them stage the next batch into the other of two buffers meanwhile, two tasks' loads
@@ -437,12 +448,15 @@ __global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeV
     double *X = fold_sm;                                         // two buffers [8][kFoldCap][kFoldLd]
     unsigned *idx = reinterpret_cast<unsigned *>(X + 2 * XBUF);  // first coefficient of the source
                                                                  // boxes [class][reflection][target]
-    short *order = reinterpret_cast<short *>(idx + kFoldClasses * 8 * NT);   // batches with sources
+    int4 *order = reinterpret_cast<int4 *>(idx + kFoldClasses * 8 * NT);   // batches with sources: number, first task,
+                                                                           // first run, tasks and runs; fragments
+    __shared__ int gend[kFoldGroups];
     __shared__ unsigned present[2];
     __shared__ int norder;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int t0 = blockIdx.x * NT;
     if (tid < 2) present[tid] = 0;
+    if (tid < kFoldGroups) gend[tid] = f.group[tid + 1];
     // rows that a class does not fill meet zeros of the operator: they have to be finite
     for (int i = tid; i < 2 * XBUF; i += NTHR) X[i] = 0;
     __syncthreads();
@@ -488,9 +502,16 @@ __global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeV
     if (warp == 0) {
         int n = 0;
         for (int b0 = bbeg; b0 < bend; b0 += 32) {
-            const bool need = b0 + lane < bend && (f.batches[b0 + lane].classes & have);
+            FoldBatch B = {};
+            if (b0 + lane < bend) B = f.batches[b0 + lane];
+            const bool need = B.classes & have;
             const unsigned m = __ballot_sync(0xffffffffu, need);
-            if (need) order[n + __popc(m & ((1u << lane) - 1))] = (short)(b0 + lane);
+            if (need)
+            {
+                int4 *o = order + 2 * (n + __popc(m & ((1u << lane) - 1)));
+                o[0] = make_int4(b0 + lane, B.task0, B.run0, B.ntask | B.nrun << 16);
+                o[1] = make_int4(B.a0, B.na, 0, 0);
+            }
             n += __popc(m);
         }
         if (lane == 0) norder = n;
@@ -504,15 +525,22 @@ __global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeV
         int2 task = make_int2(0, 0);
         auto fetch = [&](int n) {
             if (n >= N) return;
-            const FoldBatch B = f.batches[order[n]];
-            ntask = B.ntask;
-            if (lane < B.ntask) task = reinterpret_cast<const int2 *>(f.tasks + B.task0)[lane];
+            const int4 B = order[2 * n];
+            ntask = B.w & 0xffff;
+            if (lane < ntask) task = reinterpret_cast<const int2 *>(f.tasks + B.y)[lane];
         };
         fetch(0);
         for (int n = 0; n < N; n++) {
             const int2 cur = task;
             const int units = H * ntask;
             fetch(n + 1);
+            {
+                // this batch's fragments into L1
+                const int4 B = order[2 * n + 1];
+                const char *a = reinterpret_cast<const char *>(f.A + (size_t)B.x * 32);
+                for (int i = w * 32 + lane; i < 2 * B.y; i += 32 * SW)
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a + 128 * i));
+            }
             if (n >= 2) bar_sync(3 + (n & 1), NTHR);
             double *x = X + (n & 1) * XBUF;
             for (int u = w; u < units; u += 2 * SW) {
@@ -564,16 +592,16 @@ __global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeV
     int2 run = make_int2(0, 0);
     auto fetch = [&](int n) {
         if (n >= N) return;
-        const FoldBatch B = f.batches[order[n]];
-        nrun = B.nrun;
-        if (lane < B.nrun) run = f.runs[(B.run0 + lane) * 8 + al];
+        const int4 B = order[2 * n];
+        nrun = B.w >> 16;
+        if (lane < nrun) run = f.runs[(B.z + lane) * 8 + al];
     };
     clear();
     int g = g0;
     bool any = false;
     fetch(0);
     for (int n = 0; n < N; n++) {
-        while (order[n] >= f.group[g + 1]) {
+        while (order[2 * n].x >= gend[g]) {
             flush(g++, any);
             any = false;
         }
@@ -587,7 +615,8 @@ __global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeV
             const int a = __shfl_sync(0xffffffffu, ru.x, i), w = __shfl_sync(0xffffffffu, ru.y, i);
             if (!(have >> (w >> 16) & 1)) continue;
             const int k4 = w & 15, rb = w >> 4 & 15, row = w >> 8 & 255;
-            if (rb > 0) fold_mma_n<RT, RT, NT>(rb, acc, f.A + (size_t)a * 32 + lane, rb * 32, 32, k4, x + row * kFoldLd<NT>);
+            if (rb == 0) continue;
+            fold_mma_n<RT, RT, NT>(rb, acc, f.A + (size_t)a * 32 + lane, k4, x + row * kFoldLd<NT>);
         }
         if (n + 2 < N) bar_arrive(3 + (n & 1), NTHR);
     }
@@ -612,7 +641,7 @@ static void launch_fold_t(const FoldPlan &F, const FoldView &f, const FoldWork &
                           int count, double2 *out, int prune, cudaStream_t s, Status &st)
 {
     const size_t sm = sizeof(double) * 2 * 8 * kFoldCap * kFoldLd<NT> + sizeof(int) * kFoldClasses * 8 * NT +
-                      sizeof(short) * F.nbatch;
+                      2 * sizeof(int4) * F.nbatch;
     FMM_TRY(st, smem_allow(k_m2l_fold<RT, NT, SW>, sm));
     const int nr = (F.p + 1) * (F.p + 2) / 2;
     for (int c0 = 0; c0 < count && st.ok(); c0 += W.chunk) {

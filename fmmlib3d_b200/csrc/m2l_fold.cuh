@@ -30,6 +30,7 @@ struct __align__(8) FoldTask {
 struct FoldBatch {
     int task0, ntask, run0, nrun;
     unsigned long long classes;   // offset classes of its runs
+    int a0, na;                   // its operator fragments (32 doubles each)
 };
 constexpr int kFoldMaxTask = 32, kFoldMaxRun = 16;   // of a batch (a task and a run per lane)
 
