@@ -113,8 +113,8 @@ def parse_args(argv=None):
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--err-samples", type=int, default=1000)
     ap.add_argument("--m2l-mode", type=int, default=0, help="0 auto, 1 rotate-shift-rotate, 2 dense operators")
-    ap.add_argument("--tensor-m2l", type=int, default=1,
-                    help="mixed-form M2L: 0 FP32 CUDA cores, 1/2 tensor cores (tcgen05 split TF32)")
+    ap.add_argument("--tensor-m2l", type=int, default=3,
+                    help="mixed-form M2L: 0 FP32 CUDA cores, 1/2 tensor cores (tcgen05 split TF32), 3 FP64 tensor cores")
     ap.add_argument("--helm-n", type=int, default=1_000_000, help="sources of the Helmholtz workload (0: skip)")
     ap.add_argument("--helm-cpu-sample", type=int, default=1_000_000,
                     help="sources of the Helmholtz oracle call (parity and CPU baseline; capped at --helm-n)")
@@ -1012,12 +1012,12 @@ PEAK_SOURCE = {"fp64": "cuBLAS DGEMM 8192^3", "fp32": "cuBLAS SGEMM 8192^3 (TF32
                "tf32": "cuBLAS SGEMM 8192^3 with TF32 (tensor cores)"}
 
 
-def roofline_of(M, peaks, form, tensor_m2l=False, iprec=1):
+def roofline_of(M, peaks, form, tensor_m2l=False, iprec=1, fp64_m2l=False):
     """Roofline of the dominant pass (and of P2P and M2L separately) of one form, from the per-pass
     CUDA events of its timed steps.  P2P and M2L are compute passes: P2P on the CUDA cores (FP32 in
     the mixed form, FP64 otherwise), M2L on the tensor cores (TF32) when the mixed form runs it there.
     Peaks are cuBLAS GEMM rates measured in the same run (MEASURED_PEAKS.json holds HBM and bf16
-    figures only)."""
+    figures only).  fp64_m2l: the mixed form's M2L is the FP64 one."""
     keys = [k for k in M["passes"][0] if k not in ("total",)]
     mean = {k: float(np.mean([p[k] for p in M["passes"]])) for k in keys}
     # kernel times from the serialised step (each pass with the GPU to itself)
@@ -1028,12 +1028,12 @@ def roofline_of(M, peaks, form, tensor_m2l=False, iprec=1):
     if iprec > 1:
         form, tensor_m2l = "fp64", False
     cuda = "fp32" if form == "mixed" else "fp64"
-    # the FP64 rotate-shift-rotate M2L (orders <= 28) runs its products on the FP64 tensor cores (DMMA)
-    dmma = cuda == "fp64" and M.get("tuning", {}).get("form") == "fp64-rotation" and st.get("nterms", 99) <= 28
+    # the FP64 M2L (orders <= 28) runs its products on the FP64 tensor cores (DMMA)
+    dmma = not tensor_m2l and (cuda == "fp64" or fp64_m2l) and st.get("nterms", 99) <= 28
     per = {}
     p2p_flops = st["p2p_pairs"] * P2P_FLOPS_PER_PAIR
     m2l_fl = sum(cnt * m2l_flops(pt) for pt, cnt in st["m2l_pt_hist"].items())
-    for name, flops, bound in (("p2p", p2p_flops, cuda), ("m2l", m2l_fl, "tf32" if tensor_m2l else cuda)):
+    for name, flops, bound in (("p2p", p2p_flops, cuda), ("m2l", m2l_fl, "tf32" if tensor_m2l else "fp64" if dmma else cuda)):
         ach = flops / (alone[name] * 1e-3) / 1e12
         label = ("tensor" if bound == "tf32" else
                  "fp64 tensor cores (DMMA)" if (name == "m2l" and dmma) else bound + " CUDA cores")
@@ -1221,7 +1221,8 @@ def main(argv=None):
             "dtype": "f32/f64 mixed (P2P, M2L in f32; tree, recurrences, other passes f64)",
             "data": "synthetic (seeded uniform cube; charges, dipoles)", "config": config_of(args, ws),
             "errors": head["errors"], "gpu_launches": int(sum(H["launches"])), "clocks": H["clocks"], "e2e": e2e,
-            "roofline": roofline_of(H, R["peaks"], "mixed", tensor_m2l=args.tensor_m2l > 0, iprec=args.iprec),
+            "roofline": roofline_of(H, R["peaks"], "mixed", tensor_m2l=args.tensor_m2l in (1, 2), iprec=args.iprec,
+                                     fp64_m2l=args.tensor_m2l == 3),
             "forms": {"mixed": head, "fp64": dict(summary(R["forms"]["fp64"]),
                                                   roofline=roofline_of(R["forms"]["fp64"], R["peaks"], "fp64",
                                                                        iprec=args.iprec),

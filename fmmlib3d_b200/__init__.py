@@ -771,7 +771,8 @@ def set_precision_thread(mode):
 
 
 def set_tensor_m2l(mode):
-    """Mixed-form M2L: 0 FP32 CUDA cores, 1 (default) / 2 tensor cores (tcgen05, split TF32; staging variants)."""
+    """Mixed-form M2L: 0 FP32 CUDA cores, 1 / 2 tensor cores (tcgen05, split TF32; staging variants), 3 (default)
+    the FP64 form's folded operators on the FP64 tensor cores."""
     if _lib.fmm3d_set_tensor_m2l(int(mode)) != 0:
         raise ValueError("unknown tensor M2L mode %r" % (mode,))
 

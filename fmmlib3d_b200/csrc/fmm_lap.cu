@@ -119,12 +119,14 @@ enum Switch {
     kSwM2LMode = 0,    // 0 automatic, 1 rotate-shift-rotate (on the FP64 tensor cores up to order 28),
                        // 2 folded dense operators (up to order 26, as 0), 3 rotate-shift-rotate on the CUDA cores
     kSwPrecision = 1,  // 0 FP64 throughout, 1 mixed (FP32 P2P and M2L) for iprec <= 1
-    kSwTensorM2L = 2,  // mixed-form M2L: 0 FP32 CUDA cores, 1/2 tensor cores (stage variants 0/1)
+    kSwTensorM2L = 2,  // mixed-form M2L: 0 FP32 CUDA cores, 1/2 split TF32 on tcgen05 (stage variants 0/1), 3 the
+                       // FP64 form's folded operators on the FP64 tensor cores (default: 2.4 -> 0.9 ms at the
+                       // 200k cube beside an FP32 near field, and no rounding of the far field to FP32)
     kSwTcGroup = 3,    // tensor-core M2L: slots per TMEM sum (0: one sum per tile)
     kSwOverlap = 4,    // near field concurrent with the far-field passes
     kNumSw = 5
 };
-static std::atomic<int> g_sw[kNumSw] = {{0}, {0}, {1}, {1}, {1}};
+static std::atomic<int> g_sw[kNumSw] = {{0}, {0}, {3}, {1}, {1}};
 static thread_local int g_sw_thread[kNumSw] = {-1, -1, -1, -1, -1};
 static inline int sw(int k) { return g_sw_thread[k] >= 0 ? g_sw_thread[k] : g_sw[k].load(std::memory_order_relaxed); }
 static bool sw_valid(int k, int v)
@@ -132,7 +134,7 @@ static bool sw_valid(int k, int v)
     switch (k) {
     case kSwM2LMode: return v >= 0 && v <= 3;
     case kSwPrecision: return v == 0 || v == 1;
-    case kSwTensorM2L: return v >= 0 && v <= 2;
+    case kSwTensorM2L: return v >= 0 && v <= 3;
     case kSwTcGroup: return v >= 0;
     case kSwOverlap: return v == 0 || v == 1;
     }
@@ -744,8 +746,8 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
     if (S.tri && form == 1 && iprec <= 1 && plan->dense && sw(kSwTensorM2L) > 0) S.dense = S.tcm2l = true;
     const int m2l_mode = sw(kSwM2LMode);
     // (the folded kernel indexes the multipoles with 32 bits)
-    S.fold = plan->folded && !S.mixed && !S.tcm2l && m2l_mode != 1 && m2l_mode != 3 &&
-             (unsigned long long)(T.nboxes + 1) * K < 0xffffffffull;
+    S.fold = plan->folded && (unsigned long long)(T.nboxes + 1) * K < 0xffffffffull &&
+             (S.tcm2l ? sw(kSwTensorM2L) == 3 : !S.mixed && m2l_mode != 1 && m2l_mode != 3);
     if (S.fold && T.nlev >= 2 && !fold_prepare(plan->fold, S.fw, T.nboxes, T.nboxes - T.lev_start[2], s, st)) {
         g_ti.err = cudaGetErrorString(st.err);
         return 16;
@@ -785,7 +787,7 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
         S.tv_quad.nsrc = S.qnsrc.p;
     }
     S.ldm = K + (K & 1);
-    if (S.tcm2l && (!S.mp32.alloc((size_t)T.nboxes * S.ldm, s, st) || !S.tcerr.alloc(1, s, st))) {
+    if (S.tcm2l && !S.fold && (!S.mp32.alloc((size_t)T.nboxes * S.ldm, s, st) || !S.tcerr.alloc(1, s, st))) {
         g_ti.err = cudaGetErrorString(st.err);
         return 16;
     }
@@ -878,21 +880,20 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
                S.local.p, f, st);
     tm.mark_on(f);
     // STEP 4: M2L over list 2, all levels >= 2
-    if (S.tcm2l) {
+    if (S.fold) {
+        if (T.nlev >= 2)
+            launch_m2l_fold(plan->fold, S.fw, tv, T.nboxes, T.lev_start[2], T.nboxes - T.lev_start[2], S.mpole.p,
+                            S.local.p, prune, f, st);
+    } else if (S.tcm2l) {
         FMM_TRY(st, cudaMemsetAsync(S.tcerr.p, 0, sizeof(int), f));
         convert_mp_f32(T.nboxes, K, S.ldm, S.mpole.p, S.mp32.p, f, st);
-        const int tcv = S.knobs.tc_variant ? S.knobs.tc_variant - 1 : std::max(sw(kSwTensorM2L) - 1, 0);
+        const int tcv = S.knobs.tc_variant ? S.knobs.tc_variant - 1 : sw(kSwTensorM2L) == 2 ? 1 : 0;
         launch_m2l_tc(tcv, S.dtiles.p + S.m2l_a, S.m2l_n, T.grouped.p, plan->slots.p, plan->slot_toff.p,
                       plan->T32.p, tv, p, S.mp32.p, S.ldm, S.local.p, prune, 3, sw(kSwTcGroup), S.tcerr.p, S.m2l_kt, f,
                       st);
     } else if (S.mixed)
         launch_m2l_dense32(S.dtiles.p + S.m2l_a, S.m2l_n, T.grouped.p, plan->slots.p, plan->slot_toff.p,
                            plan->T32.p, tv, p, S.mpole.p, S.local.p, prune, f, st);
-    else if (S.fold) {
-        if (T.nlev >= 2)
-            launch_m2l_fold(plan->fold, S.fw, tv, T.nboxes, T.lev_start[2], T.nboxes - T.lev_start[2], S.mpole.p,
-                            S.local.p, prune, f, st);
-    }
     else if (sw(kSwM2LMode) != 3 && S.m2l_kt <= 8 && m2l_rot_dmma_supported(p))
         launch_m2l_rot_dmma(S.dtiles.p + S.m2l_a, S.m2l_n, T.grouped.p, plan->slots.p, tv, p, plan->rot.p,
                             plan->dc.p, plan->lddc, S.mpole.p, S.local.p, prune, f, st);
@@ -974,7 +975,7 @@ static void lap_stats(LapSetup &S, cudaStream_t s, Status &st)
 static int lap_finish(LapSetup &S, cudaStream_t s, Status &st)
 {
     int herr = 0;
-    if (S.tcm2l) FMM_TRY(st, cudaMemcpyAsync(&herr, S.tcerr.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (S.tcm2l && !S.fold) FMM_TRY(st, cudaMemcpyAsync(&herr, S.tcerr.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     FMM_TRY(st, cudaStreamSynchronize(s));
     if (!st.ok()) { g_ti.err = std::string(st.where ? st.where : "") + ": " + cudaGetErrorString(st.err); return 16; }
     if (herr) { g_ti.err = "tensor-core M2L: a wait expired"; return 16; }
@@ -990,7 +991,7 @@ static void lap_effective_knobs(const LapSetup &S, int *out)
 {
     out[0] = S.m2l_kt;
     out[1] = S.trans_kt;
-    out[2] = S.tcm2l ? (S.knobs.tc_variant ? S.knobs.tc_variant : std::max(sw(kSwTensorM2L), 1)) : 0;
+    out[2] = S.tcm2l ? (S.knobs.tc_variant ? S.knobs.tc_variant : sw(kSwTensorM2L) == 2 ? 2 : 1) : 0;
     out[3] = (sw(kSwOverlap) != 0 && S.knobs.overlap != 2) ? 1 : 2;
     out[4] = S.mixed ? (S.knobs.p2p_ept ? S.knobs.p2p_ept : 4) : 0;
     out[5] = lap_form(S);

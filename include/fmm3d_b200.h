@@ -373,9 +373,11 @@ int fmm3d_inject_tc_wait_expiry(int on);
 
 /* M2L of the mixed form (iprec <= 1, nterms <= 16) on the tensor cores:
  * 0 = FP32 CUDA cores, 1 or 2 = tcgen05 kind::tf32 with operands split into
- * TF32 pairs (three products per step, FP32 accumulation in TMEM; the
- * default is 1); 1 and 2 differ only in the shared-memory staging (K stage
- * 16 with three stages, K stage 32 with two).  No counterpart in the reference.  Returns 1 for an
+ * TF32 pairs (three products per step, FP32 accumulation in TMEM); 1 and 2
+ * differ only in the shared-memory staging (K stage 16 with three stages, K
+ * stage 32 with two); 3 (the default) = the FP64 form's M2L (dense operators
+ * folded over the reflections of the offsets, FP64 tensor cores), which runs
+ * beside the FP32 near field on another pipe.  No counterpart in the reference.  Returns 1 for an
  * unknown mode. */
 int fmm3d_set_tensor_m2l(int mode);
 
