@@ -34,6 +34,9 @@ __constant__ double c_ra[kTabN];   // a_nm at tidx(n,m)
 __constant__ double c_rb[kTabN];   // b_nm at tidx(n,m)
 __constant__ double c_cm[kTabP + 2];  // c_m
 __constant__ double c_sq[kTabP + 2];  // sqrt(2m+1)
+// Recurrence factors (a_nm, b_nm) at tidx(n, m), with (sqrt(2m+1), 0) at n = m + 1, in global memory:
+// copied to shared memory where every step of a column needs a pair.
+__device__ double2 g_rab[kTabN];
 
 void lap_init_constants(Status &st)
 {
@@ -41,6 +44,7 @@ void lap_init_constants(Status &st)
     std::lock_guard<std::mutex> lk(mu);
     static bool done = false;
     static double ra[kTabN], rb[kTabN], cm[kTabP + 2], sq[kTabP + 2];
+    static double2 rab[kTabN];
     if (!done) {
         for (int n = 0; n <= kTabP + 1; n++)
             for (int m = 0; m <= n; m++) {
@@ -56,6 +60,9 @@ void lap_init_constants(Status &st)
         cm[0] = 0;
         for (int m = 1; m <= kTabP + 1; m++) cm[m] = sqrt((2.0 * m - 1) / (2.0 * m));
         for (int m = 0; m <= kTabP + 1; m++) sq[m] = sqrt(2.0 * m + 1);
+        for (int n = 0; n <= kTabP + 1; n++)
+            for (int m = 0; m <= n; m++)
+                rab[tidx(n, m)] = n == m + 1 ? make_double2(sq[m], 0) : make_double2(ra[tidx(n, m)], rb[tidx(n, m)]);
         done = true;
     }
     int dev = 0;
@@ -66,6 +73,7 @@ void lap_init_constants(Status &st)
     FMM_TRY(st, cudaMemcpyToSymbol(c_rb, rb, sizeof(rb)));
     FMM_TRY(st, cudaMemcpyToSymbol(c_cm, cm, sizeof(cm)));
     FMM_TRY(st, cudaMemcpyToSymbol(c_sq, sq, sizeof(sq)));
+    FMM_TRY(st, cudaMemcpyToSymbol(g_rab, rab, sizeof(rab)));
     if (st.ok() && dev < 64) uploaded[dev] = true;
 }
 
@@ -761,16 +769,17 @@ template <int C>
 constexpr int kFmmLd = C + 4;
 constexpr int kFmmLdw = 12;   // row stride of the weights, = 12 mod 16
 
-template <bool IRREG, int NW, int C, int TPW>
-__global__ void __launch_bounds__(32 * NW) k_form_mm(const int *boxes, const int *l4s, const int *l4i, TreeView tv,
-                                                     PointsSoA src, int ifcharge, int p, double2 *coef)
+template <bool IRREG, int NW, int C, int TPW, int CTAS>
+__global__ void __launch_bounds__(32 * NW, CTAS) k_form_mm(const int *boxes, const int *l4s, const int *l4i, TreeView tv,
+                                                        PointsSoA src, int ifcharge, int p, double2 *coef)
 {
     constexpr int S = kFmmLd<C>, NT = 32 * NW, G = NT / C;
     extern __shared__ double fsm[];
     const int pt = IRREG ? p + 1 : p;                 // table degree
-    const int rows = (pt + 1) * (pt + 1), ntile = (rows + 7) / 8;
+    const int rows = (pt + 1) * (pt + 1), ntile = (rows + 7) / 8, ntri = (pt + 1) * (pt + 2) / 2;
     double *tab = fsm;                                // [8 ntile][S]
-    double *wt = tab + (size_t)8 * ntile * S;         // [C][kFmmLdw]
+    double2 *ab = reinterpret_cast<double2 *>(tab + (size_t)8 * ntile * S);   // recurrence factors
+    double *wt = reinterpret_cast<double *>(ab + ntri);                       // [C][kFmmLdw]
     int *pre = (int *)(wt + C * kFmmLdw);             // [kFormWin + 1]
     const int b = boxes[blockIdx.x];
     const int nsb = IRREG ? l4s[b + 1] - l4s[b] : 1;
@@ -784,6 +793,7 @@ __global__ void __launch_bounds__(32 * NW) k_form_mm(const int *boxes, const int
 #pragma unroll
     for (int i = 0; i < TPW; i++) acc[i][0] = acc[i][1] = 0;
     for (int i = rows * S + tid; i < 8 * ntile * S; i += NT) tab[i] = 0;
+    for (int i = tid; i < ntri; i += NT) ab[i] = g_rab[i];
     for (int w0 = 0; w0 < nsb; w0 += kFormWin) {
         const int nw = min(kFormWin, nsb - w0);
         __syncthreads();
@@ -804,32 +814,44 @@ __global__ void __launch_bounds__(32 * NW) k_form_mm(const int *boxes, const int
         }
         __syncthreads();
         const int total = pre[nw];
+        // the chunk's source of this thread: of concatenated position c0 + j, in the last window
+        // box with pre[k] <= pos (positions that fill the last K step repeat the last
+        // source, without weight); the next chunk's is read while this one is multiplied
+        double sx = 0, sy = 0, sz = 0, v[3] = {0, 0, 0};
+        double2 q = cmk(0, 0), d = cmk(0, 0);
+        auto fetch = [&](int c0) {
+            const int cn = min(C, total - c0);
+            if (cn <= 0 || j >= ((cn + 3) & ~3)) return;
+            const int pos = c0 + min(j, cn - 1);
+            int lo = 0, hi = nw - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (pre[mid] <= pos) lo = mid;
+                else hi = mid - 1;
+            }
+            const int jb = IRREG ? l4i[l4s[b] + w0 + lo] : b;
+            const int i = tv.src0[jb] + pos - pre[lo];
+            sx = src.x[i]; sy = src.y[i]; sz = src.z[i];
+            if (g == 0) {
+                q = ifcharge == 1 ? src.q[i] : cmk(0, 0);
+                d = src.dq[i];
+                v[0] = src.vz[i]; v[1] = src.vx[i]; v[2] = src.vy[i];
+            }
+        };
+        fetch(0);
         for (int c0 = 0; c0 < total; c0 += C) {
             const int cn = min(C, total - c0);
             __syncthreads();
             if (j < ((cn + 3) & ~3)) {
-                // the source of concatenated position c0 + j: last window box with pre[k] <= pos
-                // (positions that fill the last K step repeat the last source, without weight)
-                const int pos = c0 + min(j, cn - 1);
-                int lo = 0, hi = nw - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (pre[mid] <= pos) lo = mid;
-                    else hi = mid - 1;
-                }
-                const int jb = IRREG ? l4i[l4s[b] + w0 + lo] : b;
-                const int i = tv.src0[jb] + pos - pre[lo];
-                const double ux = (src.x[i] - cx) * is, uy = (src.y[i] - cy) * is, uz = (src.z[i] - cz) * is;
+                const double ux = (sx - cx) * is, uy = (sy - cy) * is, uz = (sz - cz) * is;
                 if (g == 0) {
-                    const double2 q = ifcharge == 1 ? src.q[i] : cmk(0, 0), d = cscal(is, src.dq[i]);
-                    const double v[3] = {src.vz[i], src.vx[i], src.vy[i]};
                     double *w = wt + j * kFmmLdw;
                     const bool in = j < cn;
                     w[0] = in ? q.x : 0; w[1] = in ? q.y : 0;
 #pragma unroll
                     for (int k = 0; k < 3; k++) {
-                        w[2 + 2 * k] = in ? d.x * v[k] : 0;
-                        w[3 + 2 * k] = in ? d.y * v[k] : 0;
+                        w[2 + 2 * k] = in ? is * d.x * v[k] : 0;
+                        w[3 + 2 * k] = in ? is * d.y * v[k] : 0;
                     }
                 }
                 const double r2 = ux * ux + uy * uy + uz * uz;
@@ -843,20 +865,26 @@ __global__ void __launch_bounds__(32 * NW) k_form_mm(const int *boxes, const int
                     }
                     if (m % G != g) continue;
                     double2 h0 = diag, h1 = cmk(0, 0);
-                    for (int n = m; n <= pt; n++) {
-                        if (n > m) {
-                            const double a = (n == m + 1 ? c_sq[m] : c_ra[tidx(n, m)]) * zz, bb = c_rb[tidx(n, m)] * rr;
-                            const double2 h = cmk(a * h0.x - bb * h1.x, a * h0.y - bb * h1.y);
-                            h1 = h0;
-                            h0 = h;
-                        }
-                        double *t = tab + (size_t)(m ? n * n + 2 * m - 1 : n * n) * S + j;
-                        t[0] = h0.x;
-                        if (m) t[S] = h0.y;
+                    double *t = tab + (size_t)(m ? m * m + 2 * m - 1 : 0) * S + j;
+                    t[0] = h0.x;
+                    if (m) t[S] = h0.y;
+                    int at = tidx(m, m);
+#pragma unroll 2
+                    for (int n = m + 1; n <= pt; n++) {
+                        at += n;                      // tidx(n, m)
+                        t += (2 * n - 1) * S;         // row n^2 + ...
+                        const double2 f = ab[at];
+                        const double a = f.x * zz, bb = f.y * rr;
+                        const double2 h = cmk(a * h0.x - bb * h1.x, a * h0.y - bb * h1.y);
+                        h1 = h0;
+                        h0 = h;
+                        t[0] = h.x;
+                        if (m) t[S] = h.y;
                     }
                 }
             }
             __syncthreads();
+            fetch(c0 + C);
             double bf[C / 4];
 #pragma unroll
             for (int ks = 0; ks < C / 4; ks++) bf[ks] = 4 * ks < cn ? wt[(4 * ks + (lane & 3)) * kFmmLdw + (lane >> 2)] : 0;
@@ -938,14 +966,14 @@ __global__ void __launch_bounds__(32 * NW) k_form_mm(const int *boxes, const int
     }
 }
 
-template <bool IRREG, int NW, int C, int TPW>
+template <bool IRREG, int NW, int C, int TPW, int CTAS>
 static void launch_form_mm(const int *boxes, int nboxes, const TreeView &tv, const PointsSoA &src, int ifcharge, int p,
                            double2 *coef, cudaStream_t s, Status &st)
 {
     const int pt = IRREG ? p + 1 : p, ntile = ((pt + 1) * (pt + 1) + 7) / 8;
-    const size_t sm = sizeof(double) * ((size_t)8 * ntile * kFmmLd<C> + C * kFmmLdw) + sizeof(int) * (kFormWin + 1);
-    FMM_TRY(st, smem_allow(k_form_mm<IRREG, NW, C, TPW>, sm));
-    k_form_mm<IRREG, NW, C, TPW><<<nboxes, 32 * NW, sm, s>>>(boxes, IRREG ? tv.l4_start : nullptr,
+    const size_t sm = sizeof(double) * ((size_t)8 * ntile * kFmmLd<C> + (pt + 1) * (pt + 2) + C * kFmmLdw) + sizeof(int) * (kFormWin + 1);
+    FMM_TRY(st, smem_allow(k_form_mm<IRREG, NW, C, TPW, CTAS>, sm));
+    k_form_mm<IRREG, NW, C, TPW, CTAS><<<nboxes, 32 * NW, sm, s>>>(boxes, IRREG ? tv.l4_start : nullptr,
                                                              IRREG ? tv.l4_idx : nullptr, tv, src, ifcharge, p,
                                                              coef); FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
@@ -959,9 +987,9 @@ static bool form_mm(const int *boxes, int nboxes, const TreeView &tv, const Poin
 {
     const int pt = IRREG ? p + 1 : p, ntile = ((pt + 1) * (pt + 1) + 7) / 8;
     if (pt > 29) return false;
-    if (ntile <= 16) launch_form_mm<IRREG, 4, 32, 4>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
-    else if (ntile <= 32) launch_form_mm<IRREG, 4, 32, 8>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
-    else launch_form_mm<IRREG, 8, 16, 15>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
+    if (ntile <= 16) launch_form_mm<IRREG, 4, 32, 4, 4>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
+    else if (ntile <= 32) launch_form_mm<IRREG, 8, 32, 4, 2>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
+    else launch_form_mm<IRREG, 16, 16, 8, 1>(boxes, nboxes, tv, src, ifcharge, p, coef, s, st);
     return true;
 }
 
