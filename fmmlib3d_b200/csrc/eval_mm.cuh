@@ -51,6 +51,17 @@ __host__ __device__ inline size_t emm_smem(int nmax, int nc)
     return s * 8 * 8 * nc + s * 8 + nmax + 1 + (s + 1) / 2;
 }
 
+// What the steps of an order need beside the coefficients, on the device (made once
+// per order): recurrence factors and degrees of the steps, diagonal factors, and
+// the ladder factors of the columns, [step][q][2 signs of m][NF], for local
+// expansions and for multipoles.
+struct EmmTab {
+    const double2 *ab;
+    const double *cm;
+    const int *step;
+    const double *fac[2];   // multipole, local
+};
+
 struct EmmShared {
     double *B;      // [step][part][q][8 nc], columns rotated so that the half warp's rows meet different banks
     double2 *ab;    // [step][q]: recurrence factors of (n, m = 4 t + q)
@@ -66,9 +77,25 @@ __device__ __forceinline__ int emm_col(int step, int part, int q, int col)
     return ((step * 2 + part) * 4 + q) * (8 * NC) + c;
 }
 
-// Carves the shared memory and fills the tables that depend on nmax alone.
+// Recurrence factors of step i / 4, q = i % 4 at maximum degree nmax; returns n | t << 16.
+__device__ __forceinline__ int emm_factors(int i, int nmax, double2 &ab)
+{
+    int s = i >> 2, t = 0;
+    while (s >= nmax - 4 * t + 1) s -= nmax - 4 * t++ + 1;
+    const int n = 4 * t + s, m = 4 * t + (i & 3);
+    ab = make_double2(0, 0);
+    if (n == m + 1) ab.x = sqrt(2.0 * m + 1);
+    else if (n > m) {
+        const double den = sqrt((double)(n - m) * (n + m));
+        ab.x = (2.0 * n - 1) / den;
+        ab.y = sqrt((double)(n + m - 1) * (n - m - 1)) / den;
+    }
+    return n | t << 16;
+}
+
+// Carves the shared memory and copies the tables.
 template <int NC>
-__device__ __forceinline__ EmmShared emm_init(double *sm, int nmax)
+__device__ __forceinline__ EmmShared emm_init(double *sm, int nmax, const EmmTab &tab)
 {
     EmmShared E;
     E.nmax = nmax;
@@ -77,26 +104,16 @@ __device__ __forceinline__ EmmShared emm_init(double *sm, int nmax)
     E.ab = reinterpret_cast<double2 *>(sm + (size_t)E.nstep * 64 * NC);
     E.cm = reinterpret_cast<double *>(E.ab + E.nstep * 4);
     E.step = reinterpret_cast<int *>(E.cm + nmax + 1);
-    for (int m = threadIdx.x; m <= nmax; m += blockDim.x) E.cm[m] = m ? sqrt((2.0 * m - 1) / (2.0 * m)) : 0.0;
-    for (int i = threadIdx.x; i < E.nstep * 4; i += blockDim.x) {
-        int s = i >> 2, t = 0;
-        while (s >= nmax - 4 * t + 1) s -= nmax - 4 * t++ + 1;
-        const int n = 4 * t + s, m = 4 * t + (i & 3);
-        double a = 0, b = 0;
-        if (n == m + 1) a = sqrt(2.0 * m + 1);
-        else if (n > m) {
-            const double den = sqrt((double)(n - m) * (n + m));
-            a = (2.0 * n - 1) / den;
-            b = sqrt((double)(n + m - 1) * (n - m - 1)) / den;
-        }
-        E.ab[i] = make_double2(a, b);
-        if ((i & 3) == 0) E.step[i >> 2] = n | t << 16;
-    }
+    for (int m = threadIdx.x; m <= nmax; m += blockDim.x) E.cm[m] = tab.cm[m];
+    for (int i = threadIdx.x; i < E.nstep * 4; i += blockDim.x) E.ab[i] = tab.ab[i];
+    for (int i = threadIdx.x; i < E.nstep; i += blockDim.x) E.step[i] = tab.step[i];
     return E;
 }
 
-// Stages the columns of one expansion.  quantity(n, mu, v) writes the 4 NC
-// coefficients of (n, mu) of every quantity (zero outside the quantity's degrees).
+// Stages the columns of one expansion.  quantity(i, sign, n, mu, v) writes the 4 NC
+// coefficients of (n, mu) of every quantity (zero outside the quantity's degrees); i is the
+// step and q, sign 1 for negative mu.
+
 template <int NC, class Q>
 __device__ __forceinline__ void emm_stage(const EmmShared &E, const Q &quantity)
 {
@@ -106,8 +123,8 @@ __device__ __forceinline__ void emm_stage(const EmmShared &E, const Q &quantity)
 #pragma unroll
         for (int k = 0; k < 4 * NC; k++) u[k] = v[k] = cmk(0, 0);
         if (m <= n) {
-            quantity(n, m, u);
-            if (m) quantity(n, -m, v);
+            quantity(i, 0, n, m, u);
+            if (m) quantity(i, 1, n, -m, v);
         }
 #pragma unroll
         for (int k = 0; k < 4 * NC; k++) {
@@ -204,16 +221,16 @@ __device__ __forceinline__ int emm_leaf(const int *off, int nleaves, int item)
 // One work item: leaf, chunk of 128 points (32 per warp, as two pairs of 8-point
 // rows) and group of up to 8 expansions.  order(d) is the degree of the harmonics of
 // a local expansion (d = 0) or a multipole; scale(side, k) the factor of quantity k;
-// quantity(loc, coef, n, mu, v) the columns; store(e, k, value) takes the sum of
+// quantity(loc, coef, i, sign, n, mu, v) the columns; store(e, k, value) takes the sum of
 // quantity k at point e of the leaf.
 template <int NC, class Deg, class Scale, class Quant, class Store>
-__device__ __forceinline__ void emm_item(double *sm, int nmax, const TreeView &tv, int b, int grp, int e0, int ne,
+__device__ __forceinline__ void emm_item(double *sm, int nmax, const EmmTab &tab, const TreeView &tv, int b, int grp, int e0, int ne,
                                          int ns, const double *sx, const double *sy, const double *sz,
                                          const double *tx, const double *ty, const double *tz, int K,
                                          const double2 *mpole, const double2 *local, const Deg &degree,
                                          const Scale &scale, const Quant &quantity, const Store &store)
 {
-    const EmmShared E = emm_init<NC>(sm, nmax);
+    const EmmShared E = emm_init<NC>(sm, nmax, tab);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3;
     const int s0 = tv.src0[b], t0 = tv.trg0[b], l3a = tv.l3_start[b];
     const bool has_local = tv.level[b] >= 2;
@@ -239,7 +256,7 @@ __device__ __forceinline__ void emm_item(double *sm, int nmax, const TreeView &t
         const double2 *coef = (loc ? local : mpole) + (size_t)c * K;
         const double cx = tv.center[3L * c], cy = tv.center[3L * c + 1], cz = tv.center[3L * c + 2];
         __syncthreads();
-        emm_stage<NC>(E, [&](int n, int mu, double2 *v) { quantity(loc, coef, n, mu, v); });
+        emm_stage<NC>(E, [&](int i, int sign, int n, int mu, double2 *v) { quantity(loc, coef, i, sign, n, mu, v); });
         __syncthreads();
 #pragma unroll
         for (int h = 0; h < 2; h++) {

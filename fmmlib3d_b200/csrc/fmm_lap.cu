@@ -103,6 +103,7 @@ struct LapPlan {
     // FP64 M2L operators folded over the reflections of the offsets (p <= kFoldMaxP)
     bool folded = false;
     FoldPlan fold;
+    EmmTables emm, emm_hess;   // evaluation by matrix products
     // mixed form: dense M2L operators rounded to FP32 (p <= kDenseMaxP), one per
     // list-2 offset, and the operator offset of every M2L slot
     bool dense = false;
@@ -249,6 +250,10 @@ static std::shared_ptr<LapPlan> get_plan(int p, double eps, cudaStream_t s, Stat
     const int m2l_nbuf = NC <= 3 * 256 ? 2 : 3;
     P->kt_m2l = 8;
     while (P->kt_m2l > 1 && (size_t)m2l_nbuf * P->kt_m2l * NC * 16 > 200 * 1024) P->kt_m2l /= 2;
+    build_emm_tables(p, P->emm, s, st);
+    build_emm_hess_tables(p, P->emm_hess, s, st);
+    FMM_TRY(st, cudaStreamSynchronize(s));
+    if (!st.ok()) return nullptr;
     if (p <= kFoldMaxP) {
         // the 56 offsets with no negative component: those of the octant-0 targets
         FoldOffset off[kFoldClasses];
@@ -914,9 +919,9 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     }
     tm.mark();
     // STEPS 6, 7: M2P from list 3 and L2P (add the far field to the outputs)
-    launch_eval(T.leaves.p, T.nleaves, S.ev, S.tv_far, S.sx.p, S.sy.p, S.sz.p, S.tx.p, S.ty.p, S.tz.p, p,
+    launch_eval(T.leaves.p, T.nleaves, S.ev, plan->emm, S.tv_far, S.sx.p, S.sy.p, S.sz.p, S.tx.p, S.ty.p, S.tz.p, p,
                 S.mpole.p, S.local.p, S.os, S.ot, S.do_src, S.do_trg, s, st);
-    launch_eval_hess(T.leaves.p, T.nleaves, S.ev, S.tv_far, S.sx.p, S.sy.p, S.sz.p, S.tx.p, S.ty.p, S.tz.p, p,
+    launch_eval_hess(T.leaves.p, T.nleaves, S.ev, plan->emm_hess, S.tv_far, S.sx.p, S.sy.p, S.sz.p, S.tx.p, S.ty.p, S.tz.p, p,
                      S.mpole.p, S.local.p, S.hs, S.ht, S.do_src, S.do_trg, hsrc, htrg, s, st);
     tm.mark();
     if (tm.on) {

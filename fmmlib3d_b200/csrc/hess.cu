@@ -366,6 +366,48 @@ __global__ void __launch_bounds__(kEvalHThreads) k_eval_hess(const int *leaves, 
     }
 }
 
+// Where derivative array q = 4 + c takes its coefficient for (n, mu) from: degree n + 2
+// (local) or n - 2 (multipole), order mu + kHessShift[c].
+__device__ __forceinline__ int hess_shift(int c) { return c == 1 ? -2 : c == 2 ? 2 : c == 3 ? -1 : c == 4 ? 1 : 0; }
+
+// Factors of the five second-derivative arrays (kinds 4 .. 8), by step, q and sign of m
+// (0: no such coefficient).
+__global__ void k_emm_hess_tables(int p, int nstep, double2 *ab, double *cm, int *step, double *fm, double *fl)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, nmax = p + 2;
+    if (i <= nmax) cm[i] = i ? sqrt((2.0 * i - 1) / (2.0 * i)) : 0.0;
+    if (i >= nstep * 4) return;
+    double2 f;
+    const int st = emm_factors(i, nmax, f), n = st & 0xffff, m = 4 * (st >> 16) + (i & 3);
+    ab[i] = f;
+    if ((i & 3) == 0) step[i >> 2] = st;
+    for (int sg = 0; sg < 2; sg++)
+        for (int c = 0; c < 5; c++)
+            for (int loc = 0; loc < 2; loc++) {
+                int lo, hi;
+                kind_range(loc, p, 4, lo, hi);
+                // deriv_coef of an expansion of ones is the factor
+                double v = 0;
+                if (m <= n && n >= lo && n <= hi)
+                    v = deriv_coef(loc, p, 4 + c, n, sg ? -m : m, [](int, int) { return cmk(1, 0); }).x;
+                (loc ? fl : fm)[(2 * i + sg) * 5 + c] = v;
+            }
+}
+
+void build_emm_hess_tables(int p, EmmTables &E, cudaStream_t s, Status &st)
+{
+    if (sizeof(double) * emm_smem(p + 2, 2) > kEmmSmemMax) return;
+    const int ns = emm_steps(p + 2);
+    if (!E.ab.alloc(4 * ns, s, st) || !E.cm.alloc(p + 3, s, st) || !E.step.alloc(ns, s, st) ||
+        !E.fac[0].alloc(40 * ns, s, st) || !E.fac[1].alloc(40 * ns, s, st))
+        return;
+    k_emm_hess_tables<<<(4 * ns + p + 3 + 127) / 128, 128, 0, s>>>(p, ns, E.ab.p, E.cm.p, E.step.p, E.fac[0].p,
+                                                                   E.fac[1].p); FMM_COUNT_LAUNCH();
+    FMM_LAUNCH_CHECK(st);
+    E.ab.s = E.cm.s = E.step.s = E.fac[0].s = E.fac[1].s = nullptr;   // kept for the life of the process
+    E.ready = st.ok();
+}
+
 // Hessians of one work item in matrix products (eval_mm.cuh): six complex
 // quantities in two column blocks.  Balanced like the potentials' pass: on a
 // Plummer ball of 40k + 25k points, where one leaf has dozens of list-3 boxes,
@@ -376,7 +418,7 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_hess_mm(const int *leaves
                                                                const double *ty, const double *tz, int p,
                                                                const double2 *mpole, const double2 *local,
                                                                HessSoA hs, HessSoA ht, int do_src, int do_trg,
-                                                               int hsrc, int htrg, double *part)
+                                                               int hsrc, int htrg, double *part, EmmTab tab)
 {
     extern __shared__ double hmm_sm[];
     const int l = emm_leaf(off, nleaves, blockIdx.x), b = leaves[l];
@@ -387,17 +429,18 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_hess_mm(const int *leaves
     // chunks of points that want no Hessians
     if ((!hsrc && e0 + kEvalThreads <= ns) || (!htrg && e0 >= ns)) return;
     emm_item<2>(
-        hmm_sm, p + 2, tv, b, grp, e0, ne, ns, sx, sy, sz, tx, ty, tz, (p + 1) * (p + 1), mpole, local,
+        hmm_sm, p + 2, tab, tv, b, grp, e0, ne, ns, sx, sy, sz, tx, ty, tz, (p + 1) * (p + 1), mpole, local,
         [&](bool loc) { return loc ? p - 2 : p + 2; },
         [](double is, int) { return is * is * is; },
-        [&](bool loc, const double2 *C, int n, int mu, double2 *v) {
-            int lo, hi;
-            kind_range(loc, p, 4, lo, hi);
-            if (n < lo || n > hi) return;
+        [&](bool loc, const double2 *C, int i, int sign, int n, int mu, double2 *v) {
+            const double *f = tab.fac[loc] + (2 * i + sign) * 5;
+            const double2 *c0 = C + (loc ? eidx(n + 2, mu) : eidx(n - 2, mu));
             double2 a[kNumKinds], h[6];
 #pragma unroll
-            for (int q = 4; q < kNumKinds; q++)
-                a[q] = deriv_coef(loc, p, q, n, mu, [&](int k, int m) { return C[eidx(k, m)]; });
+            for (int c = 0; c < 5; c++) {
+                const double x = __ldg(f + c);
+                a[4 + c] = x != 0 ? cscal(x, c0[hess_shift(c)]) : cmk(0, 0);
+            }
 #pragma unroll
             for (int c = 0; c < 6; c++) h[c] = cmk(0, 0);
             hess_from_ladders(a, 1.0, h);
@@ -444,21 +487,22 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_hess_add(const int *leave
 
 static constexpr size_t kHessSmemMax = 200 * 1024;
 
-void launch_eval_hess(const int *leaves, int nleaves, const EvalItems &E, const TreeView &tv, const double *sx,
+void launch_eval_hess(const int *leaves, int nleaves, const EvalItems &E, const EmmTables &tab, const TreeView &tv, const double *sx,
                       const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, int p,
                       const double2 *mpole, const double2 *local, HessSoA hs, HessSoA ht, int do_src, int do_trg,
                       int hsrc, int htrg, cudaStream_t s, Status &st)
 {
     if (nleaves == 0 || !st.ok() || !(hsrc || htrg)) return;
     if (p > kHessMaxP) { st.err = cudaErrorInvalidValue; st.where = "Hessian: expansion order above the table"; return; }
-    const size_t mm = sizeof(double) * emm_smem(p + 2, 2);
-    if (mm <= kEmmSmemMax) {
+    if (tab.ready) {
         if (E.nitems == 0) return;
+        const size_t mm = sizeof(double) * emm_smem(p + 2, 2);
+        const EmmTab t = {tab.ab.p, tab.cm.p, tab.step.p, {tab.fac[0].p, tab.fac[1].p}};
         FMM_TRY(st, smem_allow(k_eval_hess_mm, mm));
         if (!st.ok()) return;
         k_eval_hess_mm<<<E.nitems, kEvalThreads, mm, s>>>(leaves, nleaves, E.off.p, E.soff.p, tv, sx, sy, sz, tx, ty,
                                                           tz, p, mpole, local, hs, ht, do_src, do_trg, hsrc, htrg,
-                                                          E.hpart.p); FMM_COUNT_LAUNCH();
+                                                          E.hpart.p, t); FMM_COUNT_LAUNCH();
         if (E.nscratch > 0) {
             k_eval_hess_add<<<dim3(nleaves, 2), kEvalThreads, 0, s>>>(leaves, E.soff.p, tv, hs, ht, do_src, do_trg,
                                                                       hsrc, htrg, E.hpart.p); FMM_COUNT_LAUNCH();

@@ -27,7 +27,7 @@ void launch_p2p_hess(const int *leaves, int nleaves, const TreeView &tv, const P
 
 // Far field: the Hessians of the leaf's local expansion and of its list-3
 // multipoles, added to hs / ht.
-void launch_eval_hess(const int *leaves, int nleaves, const EvalItems &E, const TreeView &tv, const double *sx,
+void launch_eval_hess(const int *leaves, int nleaves, const EvalItems &E, const EmmTables &tab, const TreeView &tv, const double *sx,
                       const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, int p,
                       const double2 *mpole, const double2 *local, HessSoA hs, HessSoA ht, int do_src, int do_trg,
                       int hsrc, int htrg, cudaStream_t s, Status &st);

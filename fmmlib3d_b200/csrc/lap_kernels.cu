@@ -863,7 +863,8 @@ __global__ void __launch_bounds__(32 * NW, CTAS) k_form_mm(const int *boxes, con
                         const double cc = -c_cm[m] * ir2;
                         diag = cmk(cc * (ux * diag.x + uy * diag.y), cc * (ux * diag.y - uy * diag.x));
                     }
-                    if (m % G != g) continue;
+                    // (columns dealt back and forth: a long one and a short one for each thread)
+                    if ((m / G & 1 ? G - 1 - m % G : m % G) != g) continue;
                     double2 h0 = diag, h1 = cmk(0, 0);
                     double *t = tab + (size_t)(m ? m * m + 2 * m - 1 : 0) * S + j;
                     t[0] = h0.x;
@@ -1181,24 +1182,59 @@ __global__ void k_eval_count(const int *leaves, int nleaves, TreeView tv, int do
     scnt[l] = nbx > kEvalGroup ? items : 0;
 }
 
-// Gradient coefficients of (k, mu) of an order-p expansion C: d/dz, D+ and D-.
-__device__ __forceinline__ void grad_coefs(bool loc, int p, const double2 *C, int k, int mu, double2 &z, double2 &dp,
-                                           double2 &dm)
+// Factors of the gradient arrays at (k, mu): d/dz, D+ and D- of an order-p
+// expansion take its coefficients (k', mu), (k', mu - 1) and (k', mu + 1), k' = k + 1
+// for a local expansion and k - 1 for a multipole, times these (0: no such coefficient).
+__device__ void grad_factors(bool loc, int p, int k, int mu, double *f)
 {
-    z = dp = dm = cmk(0, 0);
+    f[0] = f[1] = f[2] = 0;
     if (loc) {
         if (k >= p) return;
-        z = cscal(sqrt((double)(k + 1 + mu) * (k + 1 - mu)), C[eidx(k + 1, mu)]);
-        dp = cscal((mu <= 0 ? -1.0 : 1.0) * sqrt((double)(k + 2 - mu) * (k + 1 - mu)), C[eidx(k + 1, mu - 1)]);
-        dm = cscal((mu >= 0 ? -1.0 : 1.0) * sqrt((double)(k + 2 + mu) * (k + 1 + mu)), C[eidx(k + 1, mu + 1)]);
+        f[0] = sqrt((double)(k + 1 + mu) * (k + 1 - mu));
+        f[1] = (mu <= 0 ? -1.0 : 1.0) * sqrt((double)(k + 2 - mu) * (k + 1 - mu));
+        f[2] = (mu >= 0 ? -1.0 : 1.0) * sqrt((double)(k + 2 + mu) * (k + 1 + mu));
     } else {
         if (k < 1) return;
-        if (abs(mu) <= k - 1) z = cscal(-sqrt((double)(k + mu) * (k - mu)), C[eidx(k - 1, mu)]);
-        if (abs(mu - 1) <= k - 1)
-            dp = cscal((mu <= 0 ? -1.0 : 1.0) * sqrt((double)(k + mu - 1) * (k + mu)), C[eidx(k - 1, mu - 1)]);
-        if (abs(mu + 1) <= k - 1)
-            dm = cscal((mu >= 0 ? -1.0 : 1.0) * sqrt((double)(k - mu - 1) * (k - mu)), C[eidx(k - 1, mu + 1)]);
+        if (abs(mu) <= k - 1) f[0] = -sqrt((double)(k + mu) * (k - mu));
+        if (abs(mu - 1) <= k - 1) f[1] = (mu <= 0 ? -1.0 : 1.0) * sqrt((double)(k + mu - 1) * (k + mu));
+        if (abs(mu + 1) <= k - 1) f[2] = (mu >= 0 ? -1.0 : 1.0) * sqrt((double)(k - mu - 1) * (k - mu));
     }
+}
+
+__global__ void k_emm_tables(int p, int nstep, double2 *ab, double *cm, int *step, double *fm, double *fl)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, nmax = p + 1;
+    if (i <= nmax) cm[i] = i ? sqrt((2.0 * i - 1) / (2.0 * i)) : 0.0;
+    if (i >= nstep * 4) return;
+    double2 f;
+    const int st = emm_factors(i, nmax, f), n = st & 0xffff, m = 4 * (st >> 16) + (i & 3);
+    ab[i] = f;
+    if ((i & 3) == 0) step[i >> 2] = st;
+    for (int sg = 0; sg < 2; sg++) {
+        double z[6] = {0, 0, 0, 0, 0, 0};
+        if (m <= n) {
+            grad_factors(false, p, n, sg ? -m : m, z);
+            grad_factors(true, p, n, sg ? -m : m, z + 3);
+        }
+        for (int c = 0; c < 3; c++) {
+            fm[(2 * i + sg) * 3 + c] = z[c];
+            fl[(2 * i + sg) * 3 + c] = z[3 + c];
+        }
+    }
+}
+
+void build_emm_tables(int p, EmmTables &E, cudaStream_t s, Status &st)
+{
+    if (sizeof(double) * emm_smem(p + 1, 1) > kEmmSmemMax) return;
+    const int ns = emm_steps(p + 1);
+    if (!E.ab.alloc(4 * ns, s, st) || !E.cm.alloc(p + 2, s, st) || !E.step.alloc(ns, s, st) ||
+        !E.fac[0].alloc(24 * ns, s, st) || !E.fac[1].alloc(24 * ns, s, st))
+        return;
+    k_emm_tables<<<div_up(4 * ns + p + 2, 128), 128, 0, s>>>(p, ns, E.ab.p, E.cm.p, E.step.p, E.fac[0].p, E.fac[1].p);
+    FMM_COUNT_LAUNCH();
+    FMM_LAUNCH_CHECK(st);
+    E.ab.s = E.cm.s = E.step.s = E.fac[0].s = E.fac[1].s = nullptr;   // kept for the life of the process
+    E.ready = st.ok();
 }
 
 // Potential and field of a work item in matrix products (eval_mm.cuh): the 8
@@ -1209,7 +1245,8 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_mm(const int *leaves, int
                                                           const double *sy, const double *sz, const double *tx,
                                                           const double *ty, const double *tz, int p,
                                                           const double2 *mpole, const double2 *local, OutSoA outs,
-                                                          OutSoA outt, int do_src, int do_trg, double *part)
+                                                          OutSoA outt, int do_src, int do_trg, double *part,
+                                                          EmmTab tab)
 {
     extern __shared__ double emm_sm[];
     const int l = emm_leaf(off, nleaves, blockIdx.x), b = leaves[l];
@@ -1218,13 +1255,16 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_mm(const int *leaves, int
     const int local_item = blockIdx.x - off[l], ck = local_item / ngr, grp = local_item - ck * ngr;
     const int s0 = tv.src0[b], t0 = tv.trg0[b];
     emm_item<1>(
-        emm_sm, p + 1, tv, b, grp, ck * kEvalThreads, ne, ns, sx, sy, sz, tx, ty, tz, (p + 1) * (p + 1), mpole, local,
+        emm_sm, p + 1, tab, tv, b, grp, ck * kEvalThreads, ne, ns, sx, sy, sz, tx, ty, tz, (p + 1) * (p + 1), mpole, local,
         [&](bool loc) { return loc ? p : p + 1; },
         [](double is, int k) { return k ? is * is : is; },
-        [&](bool loc, const double2 *C, int n, int mu, double2 *v) {
+        [&](bool loc, const double2 *C, int i, int sign, int n, int mu, double2 *v) {
             if (n <= p) v[0] = C[eidx(n, mu)];
-            double2 z, dp, dm;
-            grad_coefs(loc, p, C, n, mu, z, dp, dm);
+            const double *f = tab.fac[loc] + (2 * i + sign) * 3;
+            const double f0 = __ldg(f), f1 = __ldg(f + 1), f2 = __ldg(f + 2);
+            const double2 *c = C + (loc ? eidx(n + 1, mu) : eidx(n - 1, mu));
+            const double2 z = f0 != 0 ? cscal(f0, c[0]) : cmk(0, 0), dp = f1 != 0 ? cscal(f1, c[-1]) : cmk(0, 0),
+                          dm = f2 != 0 ? cscal(f2, c[1]) : cmk(0, 0);
             const double2 d = csub(dp, dm);
             v[1] = cscal(0.5, cadd(dp, dm));             // d/dx = (D+ + D-) / 2
             v[2] = cmk(0.5 * d.y, -0.5 * d.x);           // d/dy = (D+ - D-) / 2i
@@ -1392,17 +1432,18 @@ int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int d
     return E.nitems;
 }
 
-void launch_eval(const int *leaves, int nleaves, const EvalItems &E, const TreeView &tv, const double *sx,
+void launch_eval(const int *leaves, int nleaves, const EvalItems &E, const EmmTables &tab, const TreeView &tv, const double *sx,
                  const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, int p,
                  const double2 *mpole, const double2 *local, OutSoA outs, OutSoA outt, int do_src, int do_trg,
                  cudaStream_t s, Status &st)
 {
     if (nleaves == 0 || E.nitems == 0 || !st.ok()) return;
-    const size_t mm = sizeof(double) * emm_smem(p + 1, 1);
-    if (mm <= kEmmSmemMax) {
+    if (tab.ready) {
+        const size_t mm = sizeof(double) * emm_smem(p + 1, 1);
+        const EmmTab t = {tab.ab.p, tab.cm.p, tab.step.p, {tab.fac[0].p, tab.fac[1].p}};
         FMM_TRY(st, smem_allow(k_eval_mm, mm));
         k_eval_mm<<<E.nitems, kEvalThreads, mm, s>>>(leaves, nleaves, E.off.p, E.soff.p, tv, sx, sy, sz, tx, ty, tz, p,
-                                                     mpole, local, outs, outt, do_src, do_trg, E.part.p);
+                                                     mpole, local, outs, outt, do_src, do_trg, E.part.p, t);
     } else {
         const size_t arr = (size_t)(p + 2) * (p + 2) * sizeof(double2);
         FMM_TRY(st, smem_allow(k_eval, 2 * arr));

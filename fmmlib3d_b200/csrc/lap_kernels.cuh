@@ -64,6 +64,17 @@ void launch_p2m(const int *boxes, int nboxes, const TreeView &tv, const PointsSo
 void launch_p2l(const int *boxes, int nboxes, const TreeView &tv, const PointsSoA &src, int ifcharge,
                 int ifdipole, int p, double2 *local, cudaStream_t s, Status &st);
 
+// Tables of the evaluation by matrix products (eval_mm.cuh) of one order: the
+// potential and field (hess 0), or the Hessians.
+struct EmmTables {
+    DBuf<double2> ab;
+    DBuf<double> cm, fac[2];
+    DBuf<int> step;
+    bool ready = false;   // false: the order's columns do not fit shared memory
+};
+void build_emm_tables(int p, EmmTables &E, cudaStream_t s, Status &st);
+void build_emm_hess_tables(int p, EmmTables &E, cudaStream_t s, Status &st);
+
 // Work items of the evaluation pass (L2P + M2P): item offsets per leaf, scratch
 // offsets of the leaves with more than one group of source expansions, and the
 // scratch.  Built with the tree (host-synchronising); the launch then only
@@ -75,7 +86,7 @@ struct EvalItems {
 };
 int eval_items_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, int hess,
                        EvalItems &E, cudaStream_t s, Status &st);
-void launch_eval(const int *leaves, int nleaves, const EvalItems &E, const TreeView &tv, const double *sx,
+void launch_eval(const int *leaves, int nleaves, const EvalItems &E, const EmmTables &tab, const TreeView &tv, const double *sx,
                  const double *sy, const double *sz, const double *tx, const double *ty, const double *tz, int p,
                  const double2 *mpole, const double2 *local, OutSoA outs, OutSoA outt, int do_src, int do_trg,
                  cudaStream_t s, Status &st);
