@@ -64,7 +64,9 @@ void hess_init_constants(Status &st)
 }
 
 // ---------------------------------------------------------------- near field
-constexpr int kP2PHThreads = 128;
+// One warp per (leaf, run of 32 points): with a CTA of 128 per leaf most of its lanes idled
+// and the largest leaves of an adaptive tree held the pass (1.4 ms at a Plummer ball of 40k + 25k).
+constexpr int kP2PHThreads = 32, kP2PHRuns = 8;
 
 template <bool CHG, bool DIP>
 __global__ void __launch_bounds__(kP2PHThreads) k_p2p_hess(const int *leaves, TreeView tv, PointsSoA src,
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(kP2PHThreads) k_p2p_hess(const int *leaves, Tr
     const int t0 = tv.trg0[b], nt = do_trg ? tv.ntrg[b] : 0;
     const int ne = ns + nt;
     const int l1a = tv.l1_start[b], nl = 1 + tv.l1_start[b + 1] - l1a;
-    for (int e0 = 0; e0 < ne; e0 += kP2PHThreads) {
+    for (int e0 = blockIdx.y * kP2PHThreads; e0 < ne; e0 += gridDim.y * kP2PHThreads) {
         const int e = e0 + threadIdx.x;
         const bool act = e < ne;
         const bool is_src = e < ns;
@@ -108,14 +110,16 @@ __global__ void __launch_bounds__(kP2PHThreads) k_p2p_hess(const int *leaves, Tr
                 __syncthreads();
                 if (!act) continue;
                 const int selfk = self - (js0 + c0);
+                // the self pair adds exact zeros (no strength, unit distance)
+#pragma unroll 2
                 for (int k = 0; k < cn; k++) {
-                    if (k == selfk) continue;
+                    const bool me = k == selfk;
                     const double dx = ex - sx[k], dy = ey - sy[k], dz = ez - sz[k];
-                    const double r2 = dx * dx + dy * dy + dz * dz;
+                    const double r2 = me ? 1.0 : dx * dx + dy * dy + dz * dz;
                     const double ri = rsqrt(r2), ri2 = ri * ri, ri5 = ri2 * ri2 * ri;
                     if (CHG) {
                         // q (3 d d^T - r^2 I) / r^5
-                        const double2 q = sq[k];
+                        const double2 q = me ? cmk(0, 0) : sq[k];
                         const double t[6] = {(3 * dx * dx - r2) * ri5, (3 * dy * dy - r2) * ri5,
                                              (3 * dz * dz - r2) * ri5, 3 * dx * dy * ri5,
                                              3 * dx * dz * ri5, 3 * dy * dz * ri5};
@@ -124,7 +128,7 @@ __global__ void __launch_bounds__(kP2PHThreads) k_p2p_hess(const int *leaves, Tr
                     }
                     if (DIP) {
                         // 3 ds [ (v.d)(5 d d^T / r^2 - I) - (v d^T + d v^T) ] / r^5
-                        const double2 d = sd[k];
+                        const double2 d = me ? cmk(0, 0) : sd[k];
                         const double vx = svx[k], vy = svy[k], vz = svz[k];
                         const double dot = dx * vx + dy * vy + dz * vz;
                         const double f = 5 * dot * ri2, c3 = 3 * ri5;
@@ -154,11 +158,11 @@ void launch_p2p_hess(const int *leaves, int nleaves, const TreeView &tv, const P
     if (nleaves == 0 || !st.ok() || !(do_src || do_trg)) return;
     const bool c = ifcharge == 1, d = ifdipole == 1;
     if (c && d)
-        k_p2p_hess<true, true><<<nleaves, kP2PHThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, hs, ht, do_src, do_trg);
+        k_p2p_hess<true, true><<<dim3(nleaves, kP2PHRuns), kP2PHThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, hs, ht, do_src, do_trg);
     else if (c)
-        k_p2p_hess<true, false><<<nleaves, kP2PHThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, hs, ht, do_src, do_trg);
+        k_p2p_hess<true, false><<<dim3(nleaves, kP2PHRuns), kP2PHThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, hs, ht, do_src, do_trg);
     else if (d)
-        k_p2p_hess<false, true><<<nleaves, kP2PHThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, hs, ht, do_src, do_trg);
+        k_p2p_hess<false, true><<<dim3(nleaves, kP2PHRuns), kP2PHThreads, 0, s>>>(leaves, tv, src, tx, ty, tz, hs, ht, do_src, do_trg);
     else
         return;
     FMM_COUNT_LAUNCH();
