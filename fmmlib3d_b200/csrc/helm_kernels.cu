@@ -623,15 +623,20 @@ __device__ __forceinline__ PtGeo pt_geo(double dx, double dy, double dz)
     return g;
 }
 
-// P2M / P2L.  CTA per receiving box and range of 1024 coefficients, each
-// thread owning up to kHFormPer coefficients in registers.  Sources are taken in chunks of CH: per chunk
-// the sources' radial functions, e^{-i m phi} powers, diagonal Legendre
+// P2M / P2L.  CTA per receiving box and range of 768 pairs of coefficients (n, m) and
+// (n, -m), each thread owning up to kHFormPer pairs in registers.  Sources are taken in chunks of CH: per chunk
+// the sources' weights per degree, e^{-i m phi} powers, diagonal Legendre
 // values and full Legendre tables (2s form, one column per (source, m) task)
 // are built in shared memory, then every thread adds the chunk's
-// contributions to its coefficients.  The sum is multiplied by ik at the end
+// contributions to its pairs.  With the source's strengths multiplied into the
+// radial functions, W1 = q f + d (v . r-hat) k f', W2 = d (v . theta-hat) f / r and
+// W3 = d (v . phi-hat) f / r, both coefficients of a pair take one product
+// A = Y W1 - D W2, B = m Y W3:  e^{-im phi} (A - iB) and e^{im phi} (A + iB).
+// That is 6 operations a pair and source with charges (18 with dipoles) against 20
+// (60) with one thread per coefficient: P2L 13.4 and P2M 4.3 ms before at the 1M sphere.  The sum is multiplied by ik at the end
 // (h3dformmp_add_trunc / h3dformta_add_trunc, src/helmrouts3d.f:2972, 3299;
 // dipoles h3dformmp_dp_add_trunc :3580, h3dformta_dp_add_trunc :3978).
-constexpr int kHFormThreads = 256, kHFormPer = 4;
+constexpr int kHFormThreads = 256, kHFormPer = 3;
 // Source set-up in batches of kHFormSetA x kHFormSetCH (32) sources, tables per kHFormSetCH.
 constexpr int kHFormSetCH = 8, kHFormSetA = 4;
 
@@ -659,29 +664,30 @@ __global__ void __launch_bounds__(kHFormThreads) k_hform(const int *boxes, TreeV
     if (IRREG && tv.l4_start[b + 1] == tv.l4_start[b]) return;
     const int p = lv.p[lev];
     const double sc = lv.sc[lev];
-    const int W = p + 2, P1 = p + 1, TS = (p + 1) * (p + 2) / 2, K = (p + 1) * (p + 1);
+    const int W = p + 2, P1 = p + 1, TS = (p + 1) * (p + 2) / 2;
     // per-source arrays for AX CH sources (set up together in phase A), the
     // Legendre tables for CH (phases B and C run on AX sub-chunks in turn)
-    double2 *F = (double2 *)hsd;                 // [AX CH][W]
+    double2 *F = (double2 *)hsd;                 // [AX CH][W]    radial functions, then W1
     double2 *Em = F + AX * CH * W;               // [AX CH][P1]   e^{-i m phi}
     double *Dg = (double *)(Em + AX * CH * P1);  // [AX CH][P1]   diagonal Y_m^m (2s form)
     double *Y = Dg + AX * CH * P1;               // [CH][TS]
     double *Sc = Y + CH * TS;                    // [AX CH][16]   per-source scalars
     double *D = Sc + AX * CH * 16;               // [CH][TS]      (dipoles)
-    double2 *Fd = (double2 *)(D + (DIP ? CH * TS : 0));  // [AX CH][P1]
-    double2 *Fu = Fd + (DIP ? AX * CH * P1 : 0);         // [AX CH][P1]
-    const int e0 = blockIdx.y * kHFormThreads * kHFormPer;  // this CTA's coefficient range
-    if (e0 >= K) return;
-    double2 acc[kHFormPer];
+    double2 *W2 = (double2 *)(D + (DIP ? CH * TS : 0));  // [AX CH][P1]
+    double2 *W3 = W2 + (DIP ? AX * CH * P1 : 0);         // [AX CH][P1]
+    const int e0 = blockIdx.y * kHFormThreads * kHFormPer;  // this CTA's range of pairs
+    if (e0 >= TS) return;
+    double2 accp[kHFormPer], accm[kHFormPer];   // (n, m) and (n, -m)
     int en[kHFormPer], em_[kHFormPer];
 #pragma unroll
     for (int q = 0; q < kHFormPer; q++) {
-        acc[q] = cmk(0, 0);
-        int e = e0 + threadIdx.x + q * kHFormThreads;
-        int n = 0;
-        while ((n + 1) * (n + 1) <= e) n++;
-        en[q] = e < K ? n : -1;
-        em_[q] = e - n * n - n;
+        accp[q] = accm[q] = cmk(0, 0);
+        const int u = e0 + threadIdx.x + q * kHFormThreads;
+        int n = (int)((sqrtf(8.0f * u + 1.0f) - 1.0f) * 0.5f);
+        while (tidx(n, 0) > u) n--;
+        while (tidx(n + 1, 0) <= u) n++;
+        en[q] = u < TS ? n : -1;
+        em_[q] = u - tidx(n, 0);
     }
     const double *c = tv.center + 3L * b;
     const int nsb = IRREG ? tv.l4_start[b + 1] - tv.l4_start[b] : 1;
@@ -719,27 +725,35 @@ __global__ void __launch_bounds__(kHFormThreads) k_hform(const int *boxes, TreeV
                 }
                 double *S = Sc + j * 16;
                 const double2 qv = (CHG && ok) ? src.q[i] : cmk(0, 0), dv = (DIP && ok) ? src.dq[i] : cmk(0, 0);
-                S[0] = g.ct; S[1] = g.st; S[2] = qv.x; S[3] = qv.y; S[4] = dv.x; S[5] = dv.y;
-                if (DIP) {
+                S[0] = g.ct; S[1] = g.st;
+                if (!DIP) {
+                    for (int n = 0; n <= p; n++) f[n] = cmul(qv, f[n]);
+                } else {
                     const double vx = src.vx[i], vy = src.vy[i], vz = src.vz[i];
-                    S[6] = vx * g.st * g.cp + vy * g.st * g.sp + vz * g.ct;  // v . r-hat
-                    S[7] = vx * g.ct * g.cp + vy * g.ct * g.sp - vz * g.st;  // v . theta-hat
-                    S[8] = -vx * g.sp + vy * g.cp;                           // v . phi-hat
+                    const double2 dr = cscal(vx * g.st * g.cp + vy * g.st * g.sp + vz * g.ct, dv),   // d v . r-hat
+                                  dt = cscal(vx * g.ct * g.cp + vy * g.ct * g.sp - vz * g.st, dv),   // d v . theta-hat
+                                  dp = cscal(-vx * g.sp + vy * g.cp, dv);                            // d v . phi-hat
                     // radial derivative (times k) and the 1/r angular radial factor
                     const double2 zi = IRREG && ok ? cdiv(cmk(1, 0), z) : cmk(0, 0);
+                    double2 fm = cmk(0, 0);   // f[n - 1]
                     for (int n = 0; n <= p; n++) {
+                        const double2 fn = f[n], fp = f[n + 1];
                         double2 fd, fu;
                         if (IRREG) {
-                            fd = n == 0 ? cscal(-1.0 / sc, f[1]) : csub(cscal(sc, f[n - 1]), cmul(cscal(n + 1.0, zi), f[n]));
-                            fu = ok ? cscal(1.0 / g.r, f[n]) : cmk(0, 0);
+                            fd = n == 0 ? cscal(-1.0 / sc, fp) : csub(cscal(sc, fm), cmul(cscal(n + 1.0, zi), fn));
+                            fu = ok ? cscal(1.0 / g.r, fn) : cmk(0, 0);
                         } else {
                             double d1 = n / (2 * n + 1.0), d2 = 1.0 - d1;
-                            fd = n == 0 ? cscal(-sc, f[1]) : csub(cscal(d1 / sc, f[n - 1]), cscal(d2 * sc, f[n + 1]));
+                            fd = n == 0 ? cscal(-sc, fp) : csub(cscal(d1 / sc, fm), cscal(d2 * sc, fp));
                             fu = n == 0 ? cmk(0, 0)
-                                        : cscal(1.0 / (2 * n + 1.0), cmul(zk, cadd(cscal(sc, f[n + 1]), cscal(1.0 / sc, f[n - 1]))));
+                                        : cscal(1.0 / (2 * n + 1.0), cmul(zk, cadd(cscal(sc, fp), cscal(1.0 / sc, fm))));
                         }
-                        Fd[j * P1 + n] = cmul(fd, zk);
-                        Fu[j * P1 + n] = fu;
+                        double2 w = cmul(dr, cmul(fd, zk));
+                        if (CHG) cfma(w, qv, fn);
+                        f[n] = w;
+                        W2[j * P1 + n] = cmul(dt, fu);
+                        W3[j * P1 + n] = cmul(dp, fu);
+                        fm = fn;
                     }
                 }
             }
@@ -750,7 +764,7 @@ __global__ void __launch_bounds__(kHFormThreads) k_hform(const int *boxes, TreeV
                 if (sub > 0) __syncthreads();   // the previous sub-chunk's tables are read
                 const double2 *Fs = F + jb * W, *Ems = Em + jb * P1;
                 const double *Dgs = Dg + jb * P1, *Scs = Sc + jb * 16;
-                const double2 *Fds = Fd + (DIP ? jb * P1 : 0), *Fus = Fu + (DIP ? jb * P1 : 0);
+                const double2 *W2s = W2 + (DIP ? jb * P1 : 0), *W3s = W3 + (DIP ? jb * P1 : 0);
                 // phase B: Legendre columns, one (source, m) task per thread
                 for (int task = threadIdx.x; task < nb * P1; task += kHFormThreads) {
                     const int j = task / P1, m = task % P1;
@@ -768,35 +782,38 @@ __global__ void __launch_bounds__(kHFormThreads) k_hform(const int *boxes, TreeV
                     }
                 }
                 __syncthreads();
-                // phase C: accumulate into this thread's coefficients
-    #pragma unroll
+                // phase C: accumulate into this thread's pairs
+#pragma unroll
                 for (int q = 0; q < kHFormPer; q++) {
                     const int n = en[q];
                     if (n < 0) continue;
-                    const int m = em_[q], am = m < 0 ? -m : m, ti = tidx(n, am);
-                    for (int j = 0; j < nb; j++) {
-                        const double *S = Scs + j * 16;
-                        const double st = S[1];
-                        double2 E = Ems[j * P1 + am];
-                        if (m < 0) E = cconj(E);
-                        const double ys = Y[j * TS + ti];
-                        if (CHG) {
-                            const double yr = am == 0 ? ys : ys * st;
-                            cfma(acc[q], cmul(cmk(S[2], S[3]), cscal(yr, Fs[j * W + n])), E);
+                    const int m = em_[q], ti = tidx(n, m);
+                    if (!DIP) {
+                        // W e^{-im phi} and W e^{im phi} from four real sums
+                        double c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+                        for (int j = 0; j < nb; j++) {
+                            const double2 E = Ems[j * P1 + m], w = Fs[j * W + n];
+                            const double ys = Y[j * TS + ti], y = m == 0 ? ys : ys * Scs[j * 16 + 1];
+                            const double tx = y * w.x, ty = y * w.y;
+                            c0 = fma(tx, E.x, c0);
+                            c1 = fma(ty, E.y, c1);
+                            c2 = fma(tx, E.y, c2);
+                            c3 = fma(ty, E.x, c3);
                         }
-                        if (DIP) {
-                            const double dd = D[j * TS + ti];
-                            const double2 fd = Fds[j * P1 + n], fu = Fus[j * P1 + n];
-                            double2 A, B = cmk(0, 0);
-                            if (am == 0) A = csub(cscal(ys * S[6], fd), cscal(dd * st * S[7], fu));
-                            else {
-                                A = csub(cscal(ys * st * S[6], fd), cscal(dd * S[7], fu));
-                                B = cscal((m > 0 ? am : -am) * ys * S[8], fu);
-                            }
-                            // ds E (A - i sgn(m) B)
-                            const double2 AB = cmk(A.x + B.y, A.y - B.x);
-                            cfma(acc[q], cmul(cmk(S[4], S[5]), AB), E);
+                        accp[q] = cadd(accp[q], cmk(c0 - c1, c2 + c3));
+                        accm[q] = cadd(accm[q], cmk(c0 + c1, c3 - c2));
+                    } else {
+                        double2 ap = accp[q], am = accm[q];
+                        for (int j = 0; j < nb; j++) {
+                            const double2 E = Ems[j * P1 + m], w1 = Fs[j * W + n], w2 = W2s[j * P1 + n], w3 = W3s[j * P1 + n];
+                            const double st = Scs[j * 16 + 1], ys = Y[j * TS + ti], dd = D[j * TS + ti];
+                            const double y = m == 0 ? ys : ys * st, d = m == 0 ? dd * st : dd, z = m * ys;
+                            const double2 A = cmk(fma(y, w1.x, -(d * w2.x)), fma(y, w1.y, -(d * w2.y)));
+                            cfma(ap, cmk(fma(z, w3.y, A.x), fma(-z, w3.x, A.y)), E);
+                            cfma(am, cmk(fma(-z, w3.y, A.x), fma(z, w3.x, A.y)), cconj(E));
                         }
+                        accp[q] = ap;
+                        accm[q] = am;
                     }
                 }
             }
@@ -806,8 +823,10 @@ __global__ void __launch_bounds__(kHFormThreads) k_hform(const int *boxes, TreeV
     const double2 ik = cmk(-zk.y, zk.x);
 #pragma unroll
     for (int q = 0; q < kHFormPer; q++) {
-        const int e = e0 + threadIdx.x + q * kHFormThreads;
-        if (e < K) o[e] = cadd(o[e], cmul(acc[q], ik));
+        const int n = en[q], m = em_[q];
+        if (n < 0) continue;
+        o[eidx(n, m)] = cadd(o[eidx(n, m)], cmul(accp[q], ik));
+        if (m) o[eidx(n, -m)] = cadd(o[eidx(n, -m)], cmul(accm[q], ik));
     }
 }
 
@@ -827,7 +846,7 @@ void launch_hform(bool irreg, const int *boxes, int nboxes, const TreeView &tv, 
     if (!c && !d) return;
     htab_init(s, st);
     const int pm = max_p(lv);
-    const dim3 grid(nboxes, div_up((pm + 1) * (pm + 1), kHFormThreads * kHFormPer));
+    const dim3 grid(nboxes, div_up((pm + 1) * (pm + 2) / 2, kHFormThreads * kHFormPer));
 #define FMM_HF2(IR, C, D, CHV, AXV)                                                                           \
     do {                                                                                                      \
         size_t sm = sizeof(double) * HFormSmem<CHV, D, AXV>::doubles(pm);                                    \
