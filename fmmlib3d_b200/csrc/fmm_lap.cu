@@ -436,6 +436,19 @@ static std::string lap_signature(const LapSetup &S)
     return b;
 }
 
+// Near field beside the far field (knob 0): unless both are long and bound by the FP64
+// pipe.  Above order 16 a leaf holds 400 or more sources, so a run of the near
+// field takes about half a millisecond, and a far-field CTA, which needs a whole
+// multiprocessor, waits for the runs on it to end: 1M + 1M cube at order 26 (4,096
+// leaves) 49.6 ms beside each other, 47.0 one after the other; 2M + 2M cube at order
+// 14 31.6 / 32.0.  Small problems (fewer leaves than 16 warps on every
+// multiprocessor) gain from it at every order.
+static bool lap_overlap(const LapSetup &S)
+{
+    if (sw(kSwOverlap) == 0 || S.knobs.overlap == 2) return false;
+    return S.knobs.overlap == 1 || S.mixed || S.p <= 16 || S.T.nleaves < 16 * 148;
+}
+
 // form code reported with the knobs: 0 FP64 rotations, 1 FP64 dense, 2 mixed CUDA-core M2L, 3 mixed tensor-core M2L
 static int lap_form(const LapSetup &S) { return S.tcm2l ? 3 : S.mixed ? 2 : S.dense ? 1 : 0; }
 
@@ -841,7 +854,7 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     // stream, far field first, with the same arithmetic.
     SideStreams &ss = side_streams();
     // fmm3d_set_overlap(0) forces the passes in order (per-pass timing); else the knob decides
-    const bool overlap = sw(kSwOverlap) != 0 && S.knobs.overlap != 2;
+    const bool overlap = lap_overlap(S);
     const cudaStream_t f = overlap ? ss.far : s;
     if (overlap) {
         FMM_TRY(st, cudaEventRecord(ss.fork, s));
@@ -997,7 +1010,7 @@ static void lap_effective_knobs(const LapSetup &S, int *out)
     out[0] = S.m2l_kt;
     out[1] = S.trans_kt;
     out[2] = S.tcm2l ? (S.knobs.tc_variant ? S.knobs.tc_variant : sw(kSwTensorM2L) == 2 ? 2 : 1) : 0;
-    out[3] = (sw(kSwOverlap) != 0 && S.knobs.overlap != 2) ? 1 : 2;
+    out[3] = lap_overlap(S) ? 1 : 2;
     out[4] = S.mixed ? (S.knobs.p2p_ept ? S.knobs.p2p_ept : 4) : 0;
     out[5] = lap_form(S);
     out[6] = S.knobs_from_cache ? 1 : 0;
