@@ -372,10 +372,11 @@ static int helm_fmm_device(int iprec, double2 zk, int ns, const double *d_src, i
         rp = get_hrot(pmax, s, st);   // (its first use waits for the stream: before the near field)
         hm2p_prepare(T.leaves.p, T.nleaves, tv, do_src, do_trg, m2p, s, st);
     }
-    // The near field (STEP 8) and then the list-3 multipoles run on the call's stream
-    // while the operators of the far field are made (half a millisecond of host
-    // work) and its passes run on a high-priority side stream: those are bound by
+    // The near field (STEP 8) and then the list-3 multipoles run on the call's stream;
+    // the far field's passes run on a high-priority side stream: those are bound by
     // latency and barriers (16-42% of the issue slots), the near field by the FP64 pipe.
+    // What needs no translation operators (P2M, P2L) starts before the host makes them
+    // (half a millisecond): a cube of 10k + 5k 3.94 -> 3.5 ms.
     // With per-pass timing everything runs on the call's stream, in order.  The
     // far field's own buffers are allocated on its stream.
     SideStreams &ss = side_streams();
@@ -400,9 +401,21 @@ static int helm_fmm_device(int iprec, double2 zk, int ns, const double *d_src, i
             launch_hp2p(T.leaves.p, T.nleaves, tv, P, tx.p, ty.p, tz.p, zk, os, ot, ifcharge, ifdipole, ifpot, iffld,
                         do_trg ? ifpottarg : 0, do_trg ? iffldtarg : 0, s, st);
     };
+    // STEP 1: P2M at leaves of level >= 2 (src/hfmm3dpart.f:696-760)
+    auto form_mp = [&]() {
+        launch_hform(false, T.leaves.p, T.nleaves, tri ? tv_quad : tv, tri ? Pq : P, ifcharge, ifdipole, lv, NC, zk,
+                     mpole.p, f, st);
+    };
+    // STEP 2: P2L into boxes with a list 4 (src/hfmm3dpart.f:775-846)
+    auto list4 = [&]() {
+        launch_hform(true, T.grouped.p, T.nboxes, tri ? tv_quad : tv, tri ? Pq : P, ifcharge, ifdipole, lv, NC, zk,
+                     local.p, f, st);
+    };
     if (overlap) {
         FMM_TRY(st, cudaEventRecord(ss.fork, s));
         FMM_TRY(st, cudaStreamWaitEvent(f, ss.fork, 0));
+        form_mp();
+        list4();
         near_field();
     }
     if (far) {
@@ -528,9 +541,7 @@ static int helm_fmm_device(int iprec, double2 zk, int ns, const double *d_src, i
     }
     tm.mark();
     if (far) {
-        // STEP 1: P2M at leaves of level >= 2 (src/hfmm3dpart.f:696-760)
-        launch_hform(false, T.leaves.p, T.nleaves, tri ? tv_quad : tv, tri ? Pq : P, ifcharge, ifdipole, lv, NC, zk,
-                     mpole.p, f, st);
+        if (!overlap) form_mp();
         tm.mark();
         // STEP 3: M2M, levels nlev-1 .. 2
         for (auto &r : m2m_rng)
@@ -539,9 +550,7 @@ static int helm_fmm_device(int iprec, double2 zk, int ns, const double *d_src, i
         tm.mark();
         // the multipoles are complete
         if (overlap) FMM_TRY(st, cudaEventRecord(ss.mid, f));
-        // STEP 2: P2L into boxes with a list 4 (src/hfmm3dpart.f:775-846)
-        launch_hform(true, T.grouped.p, T.nboxes, tri ? tv_quad : tv, tri ? Pq : P, ifcharge, ifdipole, lv, NC, zk,
-                     local.p, f, st);
+        if (!overlap) list4();
         tm.mark();
         // STEP 4: M2L over list 2
         launch_htranslate(1, dtiles.p + m2l_a, m2l_n, T.grouped.p, dslots.p, tv, pmax, rp->rot.p, Z.p, mpole.p,

@@ -863,7 +863,9 @@ void launch_hform(bool irreg, const int *boxes, int nboxes, const TreeView &tv, 
     // B and C walk the four sub-chunks in order, so no sum changes order).
 #define FMM_HF_FIT(IR, C, D, CHV)                                                                             \
     do {                                                                                                      \
-        if (sizeof(double) * HFormSmem<kHFormSetCH, D, kHFormSetA>::doubles(pm) <= 110 * 1024)               \
+        if (sizeof(double) * HFormSmem<kHFormSetCH, D, 2 * kHFormSetA>::doubles(pm) <= 110 * 1024)           \
+            FMM_HF2(IR, C, D, kHFormSetCH, 2 * kHFormSetA);                                                   \
+        else if (sizeof(double) * HFormSmem<kHFormSetCH, D, kHFormSetA>::doubles(pm) <= 110 * 1024)          \
             FMM_HF2(IR, C, D, kHFormSetCH, kHFormSetA);                                                       \
         else if (sizeof(double) * HFormSmem<CHV, D>::doubles(pm) <= 226 * 1024) FMM_HF(IR, C, D, CHV);      \
         else if (sizeof(double) * HFormSmem<4, D>::doubles(pm) <= 226 * 1024) FMM_HF(IR, C, D, 4);          \
@@ -1035,7 +1037,9 @@ __global__ void __launch_bounds__(T) k_heval(const int *leaves, TreeView tv, con
 // degrees from the pair (f_{m-1}, f_m) that the previous order's run passed, so
 // every value is the one hank_dev stores and shared memory holds only the staged
 // multipole.
-constexpr int kHM2PGroup = 16;
+// Groups of 4: with 16 an SM had 5.5 warps on average (16.8 -> 15.5 ms with the local
+// expansions at the 1M sphere, 0.88 -> 0.55 ms at a cube of 10k + 5k).
+constexpr int kHM2PGroup = 4;
 
 __global__ void k_hm2p_count(const int *leaves, int nleaves, TreeView tv, int do_src, int do_trg, int *cnt)
 {
