@@ -6,8 +6,8 @@ M = 2,000,000 separate targets, both uniform in the unit cube; complex charges
 and dipole strengths with parts uniform in [-1, 1]; dipole directions uniform on
 the unit sphere; iprec = 1; potential and field at sources and targets.
 Inputs are seeded synthetic data (no dataset is involved).  The step runs in
-two arithmetic forms: "mixed" (FP32 compensated P2P and M2L on the tensor
-cores with operands split into TF32 pairs, FP64 elsewhere; the headline) and
+two arithmetic forms: "mixed" (FP32 compensated P2P, FP64 elsewhere, the M2L on
+the FP64 tensor cores unless --tensor-m2l says otherwise; the headline) and
 "fp64" (the reference's arithmetic throughout), both reported.
 
   value     points/s = (N + M) * steps / device time of the mixed form, inputs
@@ -19,8 +19,8 @@ cores with operands split into TF32 pairs, FP64 elsewhere; the headline) and
   roofline  the dominant pass of the step and (roofline.passes) P2P and M2L,
             from the library's per-pass CUDA events of one extra step with the
             passes serialised, against GEMM rates measured in the same run
-            (cuBLAS 8192^3: FP32 CUDA cores for the mixed P2P, TF32 tensor cores
-            for the mixed M2L, FP64 for the fp64 form) -- MEASURED_PEAKS.json
+            (cuBLAS 8192^3: FP32 CUDA cores for the mixed P2P, FP64 for the M2L
+            and the fp64 form, TF32 for --tensor-m2l 1 or 2) -- MEASURED_PEAKS.json
             holds only HBM and bf16 figures.
   errors    relative L2 error vs the FP64 direct sum at 1,000 seeded sources
             (self excluded) and 1,000 seeded targets, per output.
@@ -112,7 +112,7 @@ def parse_args(argv=None):
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--err-samples", type=int, default=1000)
-    ap.add_argument("--m2l-mode", type=int, default=0, help="0 auto, 1 rotate-shift-rotate, 2 dense operators")
+    ap.add_argument("--m2l-mode", type=int, default=0, help="0 auto, 1 rotate-shift-rotate, 2 folded dense operators")
     ap.add_argument("--tensor-m2l", type=int, default=3,
                     help="mixed-form M2L: 0 FP32 CUDA cores, 1/2 tensor cores (tcgen05 split TF32), 3 FP64 tensor cores")
     ap.add_argument("--helm-n", type=int, default=1_000_000, help="sources of the Helmholtz workload (0: skip)")
@@ -312,7 +312,8 @@ def run_triangles(args, R, k=7, iprec=1, zk=None):
                         "pass_ms": {kk: round(v, 3) for kk, v in passes_mixed.items()},
                         "errors": {"pot": float("%.3e" % float(torch.linalg.norm(mp - dp) / torch.linalg.norm(dp))),
                                    "fld": float("%.3e" % float(torch.linalg.norm(mf - df) / torch.linalg.norm(df)))},
-                        "form": "M2L on the tensor cores (split TF32); near field and other passes FP64"}
+                        "form": "all passes FP64 (M2L on the FP64 tensor cores)" if args.tensor_m2l == 3 else
+                        "M2L on the tensor cores (split TF32); near field and other passes FP64"}
     if R["rank"] == 0 and not args.no_cpu:
         forms["fp64"] = {"pot": gp.cpu().numpy(), "fld": gf.cpu().numpy()}
         if m_pot is not None:
@@ -1218,7 +1219,8 @@ def main(argv=None):
     line = {"metric": METRIC, "value": head["value"], "unit": UNIT, "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": head["ms_per_step"], "p50_ms": head["p50_ms"],
             "p99_ms": head["p99_ms"], "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32/f64 mixed (P2P, M2L in f32; tree, recurrences, other passes f64)",
+            "dtype": "f32/f64 mixed (P2P in f32%s; tree, recurrences, other passes f64)"
+                     % (", M2L in f64" if args.tensor_m2l == 3 else ", M2L in f32"),
             "data": "synthetic (seeded uniform cube; charges, dipoles)", "config": config_of(args, ws),
             "errors": head["errors"], "gpu_launches": int(sum(H["launches"])), "clocks": H["clocks"], "e2e": e2e,
             "roofline": roofline_of(H, R["peaks"], "mixed", tensor_m2l=args.tensor_m2l in (1, 2), iprec=args.iprec,

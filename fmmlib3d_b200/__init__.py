@@ -754,12 +754,13 @@ def set_stats(on=True):
 
 
 def set_m2l_mode(mode):
-    """0 automatic, 1 rotate-shift-rotate, 2 dense per-offset operators (nterms <= 16)."""
+    """FP64 M2L: 0 automatic and 2 folded dense operators (nterms <= 26; rotations above), 1 rotate-shift-rotate,
+    3 rotate-shift-rotate on the CUDA cores."""
     _lib.fmm3d_set_m2l_mode(int(mode))
 
 
 def set_precision(mode):
-    """0 FP64 throughout (default), 1 mixed FP32 P2P/M2L for iprec <= 1."""
+    """0 FP64 throughout (default), 1 mixed (FP32 P2P) for iprec <= 1."""
     _lib.fmm3d_set_precision(int(mode))
 
 

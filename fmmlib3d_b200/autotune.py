@@ -1,8 +1,8 @@
 """Autotuner of the Laplace passes' launch shapes, with a JSON cache.
 
 Knobs (``TUNING_KNOBS``, 0 = automatic):
-  m2l_kt      M2L targets per tile (tensor-core form 16..256; FP64 dense operators 16 or 64;
-              rotations 1, 2, 4, 8)
+  m2l_kt      M2L targets per tile (tensor-core form 16..256; rotations 1, 2, 4, 8; the folded
+              FP64 operators' tile is the kernel's own: 16 or 64 are taken without effect)
   trans_kt    M2M / L2L targets per tile (1, 2, 4, 8)
   tc_variant  tensor-core M2L shared-memory staging (1: K chunks of 16, three stages;
               2: K chunks of 32, two stages)

@@ -119,7 +119,7 @@ struct LapPlan {
 enum Switch {
     kSwM2LMode = 0,    // 0 automatic, 1 rotate-shift-rotate (on the FP64 tensor cores up to order 28),
                        // 2 folded dense operators (up to order 26, as 0), 3 rotate-shift-rotate on the CUDA cores
-    kSwPrecision = 1,  // 0 FP64 throughout, 1 mixed (FP32 P2P and M2L) for iprec <= 1
+    kSwPrecision = 1,  // 0 FP64 throughout, 1 mixed (FP32 P2P, M2L by kSwTensorM2L) for iprec <= 1
     kSwTensorM2L = 2,  // mixed-form M2L: 0 FP32 CUDA cores, 1/2 split TF32 on tcgen05 (stage variants 0/1), 3 the
                        // FP64 form's folded operators on the FP64 tensor cores (default: 2.4 -> 0.9 ms at the
                        // 200k cube beside an FP32 near field, and no rounding of the far field to FP32)
@@ -759,8 +759,8 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
     S.mixed = !S.tri && form == 1 && iprec <= 1 && plan->dense;
     S.dense = (plan->dense && sw(kSwM2LMode) != 1 && sw(kSwM2LMode) != 3) || S.mixed;
     S.tcm2l = S.mixed && sw(kSwTensorM2L) > 0;
-    // triangles in the mixed form: the M2L runs on the tensor cores (split TF32), the exact
-    // near field and every other pass stay FP64
+    // triangles in the mixed form: the M2L runs on the tensor cores (in FP64, or split TF32 where
+    // that is chosen), the exact near field and every other pass stay FP64
     if (S.tri && form == 1 && iprec <= 1 && plan->dense && sw(kSwTensorM2L) > 0) S.dense = S.tcm2l = true;
     const int m2l_mode = sw(kSwM2LMode);
     // (the folded kernel indexes the multipoles with 32 bits)
@@ -1907,7 +1907,7 @@ int fmm3d_set_precision_thread(int mode)
 
 int fmm3d_set_tensor_m2l(int mode)
 {
-    if (mode < 0 || mode > 2) return 1;
+    if (!sw_valid(kSwTensorM2L, mode)) return 1;
     g_sw[kSwTensorM2L] = mode;
     return 0;
 }

@@ -29,6 +29,16 @@
 // The sums of a target are formed in 8 fixed groups of batches, added in
 // order; a small problem runs one CTA per (tile, group) and adds the groups
 // afterwards, with the same result bit for bit.
+//
+// Bound: latency of the fragments and source rows in L2 (DMMA pipe 30% busy, long
+// scoreboard half of the stalls).  M2L pass, one B200, against the dense product per
+// offset that it replaced (orders <= 16) and rotate-shift-rotate (order 26):
+//   cube 2M + 2M, order 14   33.2 -> 6.0 ms     10k sphere, order 14    1.8 -> 0.07 ms
+//   100k sphere, order 14    2.6 -> 0.29 ms     cube 1M + 1M, order 26  11.5 -> 4.8 ms
+//   328k triangles, order 14 39.6 -> 8.3 ms
+// On the way: staging and products by the same 16 warps in turn 9.2 ms at the 2M cube;
+// staging by warps of their own 8.15; the next batch's fragments to L1 ahead of use 6.0.
+// (Fragments fetched into registers ahead: spills, 10.9 ms; raw rows by cp.async: 10.1.)
 #include <algorithm>
 
 #include "dmma.cuh"
@@ -41,7 +51,11 @@ constexpr int kFoldCap = 32;                    // operand rows per parity class
 // lanes of a half warp reading a fragment meet different banks.
 template <int NT>
 constexpr int kFoldLd = 2 * NT + 4;
-constexpr int kFoldSplitTiles = 296;            // fewer tiles than this: one CTA per group
+// Fewer tiles than this (two for each of 148 multiprocessors): one CTA per group.  M2L, one
+// CTA per tile against one per (tile, group): 4 tiles 0.35 / 0.062 ms, 111 tiles 0.36 /
+// 0.29, 292 tiles 0.78 / 0.80, 1,390 tiles 3.42 / 3.58, 2,330 tiles 6.0 / 6.5.
+// (Order 26, 585 tiles: 4.85 / 4.33, but the groups' sums take 437 MB instead of 55.)
+constexpr int kFoldSplitTiles = 296;
 
 // ---------------------------------------------------------------- operators
 struct FoldBlock {

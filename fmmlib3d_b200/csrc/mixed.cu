@@ -9,8 +9,8 @@
 // chunks.  The pair formulas are those of lpotfld3d /
 // lpotfld3d_dp (src/laprouts3d.f:1308-1368, 1962-2035).
 //
-// M2L in FP32 on the CUDA cores (k_m2l_dense32, used when the tensor-core
-// M2L of tc_m2l.cu is switched off): the dense per-offset operators
+// M2L in FP32 on the CUDA cores (k_m2l_dense32, used with fmm3d_set_tensor_m2l(0);
+// by default the mixed form takes the FP64 M2L of m2l_fold.cu): the dense per-offset operators
 // (m2l_dense.cu) rounded to FP32, box-scaled multipoles (all O(1)) rounded to
 // FP32 on load, FP32 accumulation, and the tile added to the FP64 local
 // expansion.

@@ -1,4 +1,6 @@
-// M2L on the Blackwell tensor cores (mixed form, nterms <= 16).
+// M2L on the Blackwell tensor cores (mixed form, nterms <= 16, with
+// fmm3d_set_tensor_m2l(1 or 2); the default there is m2l_fold.cu, which takes
+// 0.9 ms against 2.4 at a cube of 200k + 200k and 6.0 against 8.0 at 2M + 2M).
 //
 // The dense per-offset operators T_D (m2l_dense.cu) applied to gathered source
 // multipoles are products of complex matrices.  Here each CTA owns 64 complex

@@ -326,18 +326,18 @@ int fmm3d_last_timing(double *ms, int n);
  *  also holds the construction of that call's z-shift operators. */
 int fmm3d_set_stats(int on);
 
-/* M2L form: 0 automatic (dense per-offset operators for nterms <= 16,
- * rotate-shift-rotate otherwise), 1 always rotate-shift-rotate, 2 dense
- * where available, 3 rotate-shift-rotate on the CUDA cores (modes 0 and 1
- * run the rotations and z-shifts as FP64 tensor-core products up to order
- * 28).  All give the same results to rounding; the switch exists for testing
+/* M2L form: 0 automatic (dense operators folded over the reflections of the
+ * offsets, on the FP64 tensor cores, for nterms <= 26; rotate-shift-rotate
+ * otherwise), 1 always rotate-shift-rotate, 2 as 0, 3 rotate-shift-rotate on
+ * the CUDA cores (mode 1, and mode 0 above nterms 26, run the rotations and
+ * z-shifts as FP64 tensor-core products up to order 28).  All give the same results to rounding; the switch exists for testing
  * and measurement. */
 int fmm3d_set_m2l_mode(int mode);
 
 /* Arithmetic form of later calls (process-wide): 0 = FP64 throughout (the
  * default: the reference's arithmetic), 1 = mixed precision for iprec <= 1:
- * P2P in FP32 with TwoSum-compensated accumulation and M2L with FP32
- * operators, FP64 for the tree, geometry, recurrences, rotations and the
+ * P2P in FP32 with TwoSum-compensated accumulation, M2L as
+ * fmm3d_set_tensor_m2l says, FP64 for the tree, geometry, recurrences, rotations and the
  * other passes.  iprec >= 2 always runs FP64. */
 int fmm3d_set_precision(int mode);
 /* The same for the calling host thread only: 0 or 1 override the process-wide
@@ -453,7 +453,8 @@ int fmm3d_d3tstrcrem(int nsource, const double *d_source, int nbox, int ntarget,
 /* ---- Launch-shape tuning (no counterpart in the reference, whose only
  * tuning input is iprec).  Five knobs, 0 = automatic:
  *   [0] M2L targets per tile (tensor-core form 16..256 in steps of 16; FP64
- *       dense operators 16 or 64; FP32 CUDA-core form 64; rotations 1, 2, 4, 8),
+ *       dense operators 16 or 64 (the folded kernels' tile is their own: the
+ *       value is taken and has no effect there, in either form); FP32 CUDA-core form 64; rotations 1, 2, 4, 8),
  *   [1] M2M / L2L targets per tile (1, 2, 4, 8),
  *   [2] tensor-core M2L staging variant (1 or 2, as fmm3d_set_tensor_m2l),
  *   [3] 1 = near field concurrent with the far field, 2 = passes in order

@@ -57,3 +57,32 @@ def test_folded_m2l_matches_rotations(F, geom, n, m, iprec, self_out):
     for x, y in zip(a, b):
         assert np.all(np.isfinite(x))
         assert np.linalg.norm(x - y) <= 1e-12 * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("geom,n,iprec", [("cube", 20011, 1), ("plummer", 30011, 0), ("sphere", 9001, -1)])
+def test_mixed_form_with_the_folded_m2l(F, geom, n, iprec):
+    """The mixed form's FP64 M2L (the default there): error against the direct sum at most twice the
+    FP64 form's, or, where that is below the floor of the FP32 near field (1e-8), no worse than with
+    the FP32 M2L on the CUDA cores."""
+    import oracle as O
+    rng = np.random.default_rng(n)
+    src = geometry(geom, n, rng)
+    q = rng.uniform(-1, 1, n) + 1j * rng.uniform(-1, 1, n)
+    call = lambda: F.lfmm3dpartself(iprec, src, 1, q, 0, None, None, 1, 1)
+    full = call()
+    F.set_precision(1)
+    try:
+        F.set_tensor_m2l(0)
+        cuda = call()
+        F.set_tensor_m2l(3)
+        fold, again = call(), call()
+    finally:
+        F.set_tensor_m2l(3)
+        F.set_precision(0)
+    si = rng.choice(n, 400, replace=False)
+    exact = O.direct_at(src, src[si], si, q)
+    err = lambda a, d: np.linalg.norm(a[si] - d) / np.linalg.norm(d)
+    for k in (1, 2):
+        assert np.array_equal(fold[k], again[k])
+        e, e64, e32 = (err(x[k], exact[k - 1]) for x in (fold, full, cuda))
+        assert e <= 2 * e64 or (e < 1e-8 and e <= 1.02 * e32), (e, e64, e32)

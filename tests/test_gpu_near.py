@@ -65,3 +65,27 @@ def test_coincident_points_give_infinities_and_leave_the_others(F):
     keep = np.setdiff1d(np.arange(70), [7, 41])
     p0, f0 = O.direct_at(src, src[keep], keep, q)
     assert rel(pot[keep], p0) < 1e-13 and rel(fld[keep], f0) < 1e-13
+
+
+@pytest.mark.parametrize("charges,dipoles", [(True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("zk", [1e-6, 2.5, 3 + 0.5j, 0.7j, 3e5, 3e5 + 0.2j])
+@pytest.mark.parametrize("n,m", [(1, 1), (31, 33), (32, 32), (65, 97), (160, 3)])
+def test_helmholtz_one_leaf(F, n, m, zk, charges, dipoles):
+    """The Helmholtz near field alone.  The phase |k| r carries at most 16 roundings on both sides
+    together, so 16 eps |k| sqrt(3) is added to the bound; |k| = 3e5 has phases on both sides of
+    2^17, where the sine and cosine change from the polynomial to the library."""
+    rng = np.random.default_rng(1000 * n + m)
+    src, trg = rng.random((n, 3)), rng.random((m, 3))
+    q = rng.uniform(-1, 1, n) + 1j * rng.uniform(-1, 1, n) if charges else None
+    ds = rng.uniform(-1, 1, n) + 1j * rng.uniform(-1, 1, n) if dipoles else None
+    dv = rng.normal(size=(n, 3)) if dipoles else None
+    tol = 1e-13 + 16 * 2.0 ** -52 * abs(zk) * 3 ** 0.5
+    ier, pot, fld, pt, ft = F.hfmm3dparttarg(1, zk, src, int(charges), q, int(dipoles), ds, dv, 1, 1, trg, 1, 1)
+    assert ier == 0, F.last_error()
+    p0, f0 = O.hdirect_at(zk, src, src, np.arange(n), q, ds, dv)
+    p1, f1 = O.hdirect_at(zk, src, trg, None, q, ds, dv)
+    if n > 1:
+        assert rel(pot, p0) < tol and rel(fld, f0) < tol
+    else:
+        assert not np.any(pot) and not np.any(fld)
+    assert rel(pt, p1) < tol and rel(ft, f1) < tol
