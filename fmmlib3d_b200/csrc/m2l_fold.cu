@@ -27,14 +27,14 @@
 // all 32 columns, with its rows.  Offset classes
 // that no target of the tile has a source in are skipped.
 // The sums of a target are formed in 8 fixed groups of batches, added in
-// order; a small problem runs one CTA per (tile, group) and adds the groups
-// afterwards, with the same result bit for bit.
+// order; a small problem, or one above order 14, runs one CTA per (tile, group) and
+// adds the groups afterwards, with the same result bit for bit.
 //
 // Bound: latency of the fragments and source rows in L2 (DMMA pipe 30% busy, long
 // scoreboard half of the stalls).  M2L pass, one B200, against the dense product per
 // offset that it replaced (orders <= 16) and rotate-shift-rotate (order 26):
 //   cube 2M + 2M, order 14   33.2 -> 6.0 ms     10k sphere, order 14    1.8 -> 0.07 ms
-//   100k sphere, order 14    2.6 -> 0.29 ms     cube 1M + 1M, order 26  11.5 -> 4.8 ms
+//   100k sphere, order 14    2.6 -> 0.29 ms     cube 1M + 1M, order 26  11.5 -> 4.5 ms
 //   328k triangles, order 14 39.6 -> 8.3 ms
 // On the way: staging and products by the same 16 warps in turn 9.2 ms at the 2M cube;
 // staging by warps of their own 8.15; the next batch's fragments to L1 ahead of use 6.0.
@@ -54,7 +54,9 @@ constexpr int kFoldLd = 2 * NT + 4;
 // Fewer tiles than this (two for each of 148 multiprocessors): one CTA per group.  M2L, one
 // CTA per tile against one per (tile, group): 4 tiles 0.35 / 0.062 ms, 111 tiles 0.36 /
 // 0.29, 292 tiles 0.78 / 0.80, 1,390 tiles 3.42 / 3.58, 2,330 tiles 6.0 / 6.5.
-// (Order 26, 585 tiles: 4.85 / 4.33, but the groups' sums take 437 MB instead of 55.)
+// Tiles of 8 targets (above order 14, one CTA per multiprocessor) always run per group: eight
+// times the CTAs even out the tiles at a domain's faces.  Order 26: 585 tiles 4.83 /
+// 4.53, 4,681 tiles 38.9 / 35.7, with the groups' sums held to 256 MB at a time.
 constexpr int kFoldSplitTiles = 296;
 
 // ---------------------------------------------------------------- operators
@@ -643,10 +645,10 @@ __global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeV
 bool fold_prepare(const FoldPlan &F, FoldWork &W, int nboxes, int count, cudaStream_t s, Status &st)
 {
     if (count <= 0) return true;
-    W.slots = div_up(count, F.tile) < kFoldSplitTiles ? kFoldGroups : 1;
-    // at most 1 GB of sums at a time
-    const long long most = std::max<long long>((1LL << 30) / (16LL * F.K * W.slots) / F.tile, 1) * F.tile;
-    W.chunk = (int)std::min<long long>(count, W.slots > 1 ? count : most);
+    W.slots = F.tile == 8 || div_up(count, F.tile) < kFoldSplitTiles ? kFoldGroups : 1;
+    // at most 256 MB of sums at a time
+    const long long most = std::max<long long>((1LL << 28) / (16LL * F.K * W.slots) / F.tile, 1) * F.tile;
+    W.chunk = (int)std::min<long long>(count, most);
     return W.mr.alloc((size_t)nboxes * F.K, s, st) && W.lr.alloc((size_t)W.chunk * F.K * W.slots, s, st);
 }
 

@@ -45,6 +45,7 @@ def _call(F, iprec, src, q, trg, self_out):
     ("cube", 400003, 1000, 0, True),      # more than 296 tiles: all partial sums in one CTA
     ("plummer", 20000, 3000, 2, True),    # order 26
     ("sphere", 300007, 100, 2, False),
+    ("cube", 400003, 1000, 2, True),      # order 26, sums in two pieces
 ])
 def test_folded_m2l_matches_rotations(F, geom, n, m, iprec, self_out):
     rng = np.random.default_rng(n + m)
