@@ -385,7 +385,8 @@ struct LapSetup {
     DBuf<float2> mp32;
     DBuf<int> tcerr;
     DBuf<Tile> dtiles;
-    std::vector<std::pair<int, int>> m2m_rng, l2l_rng;  // per level: [first tile, count)
+    struct TileRange { int first, count, kt; };
+    std::vector<TileRange> m2m_rng, l2l_rng;  // per level: tiles [first, first + count) of kt targets
     int m2l_a = 0, m2l_n = 0, m2l_kt = 0, trans_kt = 0;
     // mixed form: list-3 boxes with few sources and the list-4 boxes of boxes with
     // few points are summed with the near field; tv_near is tv with list 1
@@ -515,11 +516,29 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
         }
     };
     const int tkt = k.trans_kt ? k.trans_kt : plan->kt;
-    std::vector<std::pair<int, int>> m2m, l2l;
+    // M2M / L2L tile size of a level (automatic): the largest with two tiles per
+    // multiprocessor, one target per tile if none has.  A tile is a serial chain of slots;
+    // targets in a tile share each operator's loads.  M2M / L2L with up to four targets
+    // everywhere -> by this rule -> one target everywhere (ms): cube 200k + 200k 0.204 / 0.095
+    // -> 0.134 / 0.081 -> 0.134 / 0.093; Plummer 40k 0.390 / 0.130 -> 0.245 / 0.073 -> the
+    // same; cube 2M + 2M 0.640 / 0.486 -> 0.568 / 0.470 -> 0.638 / 0.560.
+    const int want = 2 * device_sms();
+    auto ntiles = [&](int lev, int kt) {
+        int t = 0;
+        for (int o = 0; o < 8; o++) t += div_up(T.group_start[lev * 8 + o + 1] - T.group_start[lev * 8 + o], kt);
+        return t;
+    };
+    auto level_kt = [&](int lev) {
+        int kt = tkt;
+        while (!k.trans_kt && kt > 1 && ntiles(lev, kt) < want) kt /= 2;
+        return kt;
+    };
+    std::vector<LapSetup::TileRange> m2m, l2l;
     for (int l = T.nlev - 1; l >= 2; l--) {
         int a = ntile;
-        make_tiles(l, tkt, kSlotM2M, 0, 8);
-        m2m.push_back({a, ntile - a});
+        const int kt = level_kt(l);
+        make_tiles(l, kt, kSlotM2M, 0, 8);
+        m2m.push_back({a, ntile - a, kt});
     }
     // M2L tile size (automatic): the largest whose tile count fills the GPU (two
     // CTAs per SM per 64-row block); smaller tiles only add CTAs, every target's
@@ -528,16 +547,15 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
     if (k.m2l_kt) {
         m2l_kt = k.m2l_kt;
     } else if (S.tcm2l) {
-        const int rows = div_up(S.K, 64), want = 2 * device_sms();
-        auto ntiles = [&](int kt) {
+        const int rows = div_up(S.K, 64);
+        auto all_tiles = [&](int kt) {
             long t = 0;
-            for (int l = 2; l <= T.nlev; l++)
-                for (int o = 0; o < 8; o++) t += div_up(T.group_start[l * 8 + o + 1] - T.group_start[l * 8 + o], kt);
+            for (int l = 2; l <= T.nlev; l++) t += ntiles(l, kt);
             return t;
         };
         // (256-target tensor-core tiles run one CTA per SM and measured slower on every
         // workload tried; they are reached through the tuning knob only)
-        while (m2l_kt > 16 && ntiles(m2l_kt) * rows < want) m2l_kt /= 2;
+        while (m2l_kt > 16 && all_tiles(m2l_kt) * rows < want) m2l_kt /= 2;
     }
     const int m2l_a = ntile;
     // (the folded M2L takes runs of box ids; its tile is its own)
@@ -545,8 +563,9 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
     const int m2l_n = ntile - m2l_a;
     for (int l = 2; l <= T.nlev - 1; l++) {
         int a = ntile;
-        make_tiles(l + 1, tkt, kSlotL2L, 1, 1);
-        l2l.push_back({a, ntile - a});
+        const int kt = level_kt(l + 1);
+        make_tiles(l + 1, kt, kSlotL2L, 1, 1);
+        l2l.push_back({a, ntile - a, kt});
     }
     if ((size_t)ntile != S.dtiles.n && !S.dtiles.alloc(ntile, s, st)) return 16;
     if (!segs.empty()) {
@@ -890,8 +909,8 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     tm.mark_on(f);
     // STEP 3: M2M, levels nlev-1 .. 2
     for (auto &r : S.m2m_rng)
-        launch_translate(0, S.dtiles.p + r.first, r.second, T.grouped.p, plan->slots.p, tv, p, plan->rot.p,
-                         plan->dc.p, plan->lddc, S.mpole.p, S.mpole.p, prune, S.trans_kt, f, st);
+        launch_translate(0, S.dtiles.p + r.first, r.count, T.grouped.p, plan->slots.p, tv, p, plan->rot.p,
+                         plan->dc.p, plan->lddc, S.mpole.p, S.mpole.p, prune, r.kt, f, st);
     tm.mark_on(f);
     // STEP 2: P2L from list 4 (every box; boxes with an empty list add nothing)
     launch_p2l(T.grouped.p, T.nboxes, S.tri ? S.tv_quad : S.tv_far, S.tri ? S.Pq : P, S.ifcharge, S.ifdipole, p,
@@ -921,8 +940,8 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     tm.mark_on(f);
     // STEP 5: L2L, levels 2 .. nlev-1
     for (auto &r : S.l2l_rng)
-        launch_translate(2, S.dtiles.p + r.first, r.second, T.grouped.p, plan->slots.p, tv, p, plan->rot.p,
-                         plan->dc.p, plan->lddc, S.local.p, S.local.p, prune, S.trans_kt, f, st);
+        launch_translate(2, S.dtiles.p + r.first, r.count, T.grouped.p, plan->slots.p, tv, p, plan->rot.p,
+                         plan->dc.p, plan->lddc, S.local.p, S.local.p, prune, r.kt, f, st);
     tm.mark_on(f);
     if (overlap) {
         FMM_TRY(st, cudaEventRecord(ss.join, f));
