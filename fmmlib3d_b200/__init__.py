@@ -580,11 +580,12 @@ class LaplacePlan:
                                               ptr(pottarg), ptr(fldtarg), int(bool(use_graph)), _P(stream))
 
     def info(self):
-        out = np.zeros(10)
-        _lib.fmm3d_lfmm3d_plan_info(self._h, _ptr(out), 10)
+        out = np.zeros(11)
+        _lib.fmm3d_lfmm3d_plan_info(self._h, _ptr(out), 11)
         keys = ["nboxes", "nlev", "nleaves", "nterms", "nsource", "ntarget"]
         d = {k: int(out[i]) for i, k in enumerate(keys)}
         d["center"], d["size"] = out[6:9].copy(), float(out[9])
+        d["bytes"] = int(out[10])     # device memory held until close()
         return d
 
     def getb(self, ibox):

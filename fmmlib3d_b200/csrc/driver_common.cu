@@ -180,6 +180,7 @@ void staged_d2h(StageRing &ring, void *dst, const void *src, size_t bytes, cudaS
 thread_local ThreadInfo g_ti;
 thread_local int g_alloc_fail_countdown = 0;
 thread_local int g_alloc_fail_phase = 0;
+thread_local long long g_dbuf_bytes = 0;
 
 cudaStream_t thread_stream()
 {

@@ -103,6 +103,10 @@ inline void alloc_fail_point(int phase)
     }
 }
 
+// Bytes that this host thread's DBufs have allocated less those it has released: the
+// difference over a stretch of code is what that code keeps.
+extern thread_local long long g_dbuf_bytes;
+
 // Stream-ordered allocations from the device's default memory pool, so that
 // repeated calls reuse HBM without synchronising the device.
 template <typename T>
@@ -116,7 +120,10 @@ struct DBuf {
     ~DBuf() { release(); }
     void release()
     {
-        if (p) cudaFreeAsync(p, s);
+        if (p) {
+            cudaFreeAsync(p, s);
+            g_dbuf_bytes -= (long long)(sizeof(T) * n);
+        }
         p = nullptr;
         n = 0;
     }
@@ -132,6 +139,7 @@ struct DBuf {
         }
         FMM_TRY(st, cudaMallocAsync((void **)&p, sizeof(T) * count, stream));
         if (!st.ok()) { p = nullptr; n = 0; return false; }
+        g_dbuf_bytes += (long long)(sizeof(T) * n);
         return true;
     }
     bool zero(Status &st)

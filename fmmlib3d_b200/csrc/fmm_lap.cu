@@ -397,6 +397,7 @@ struct LapSetup {
     TuneKnobs knobs;          // as requested (0 = automatic); m2l_kt / trans_kt hold the values in use
     bool knobs_from_cache = false;
     std::string signature;
+    long long bytes = 0;      // device memory that this geometry holds (operator tables of the order apart)
     PointsSoA P;
     OutSoA os, ot;
     // Hessian outputs (dxx, dyy, dzz, dxy, dxz, dyz), set before lap_setup;
@@ -724,6 +725,7 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
     S.plan = get_plan(p, eps, s, st);
     if (!st.ok() || !S.plan) { g_ti.err = cudaGetErrorString(st.err); return 16; }
     auto &plan = S.plan;
+    const long long bytes0 = g_dbuf_bytes;
     S.iprec = iprec; S.p = p; S.K = (p + 1) * (p + 1); S.ns = ns; S.nt = nt;
     S.ifcharge = ifcharge; S.ifdipole = ifdipole; S.ifpot = ifpot; S.iffld = iffld;
     S.ifpottarg = ifpottarg; S.iffldtarg = iffldtarg;
@@ -829,6 +831,7 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
         return 16;
     }
     if (!st.ok()) { g_ti.err = cudaGetErrorString(st.err); return 16; }
+    S.bytes = g_dbuf_bytes - bytes0;
     return 0;
 }
 
@@ -1230,7 +1233,9 @@ int fmm3d_d3tstrcrem(int nsource, const double *d_source, int nbox, int ntarget,
     opt.minlevel = minlevel;
     opt.maxlevel = maxlevel;
     Status st;
+    const long long bytes0 = g_dbuf_bytes;
     build_tree(E->S.T, d_source, nsource, d_target, ntarget, nbox, s, st, opt);
+    E->S.bytes = g_dbuf_bytes - bytes0;
     FMM_TRY(st, cudaStreamSynchronize(s));
     if (!st.ok()) {
         g_ti.err = cudaGetErrorString(st.err);
@@ -1393,16 +1398,16 @@ int fmm3d_last_tuning(int *out, int n, char *sig, int nsig)
     return (int)g_last_signature.size() + 1;
 }
 
-// out[0..9] = nboxes, nlev, nleaves, nterms, nsource, ntarget, centre x, y, z, side of the root cube
-// (of the first instance for a batch)
+// out[0..10] = nboxes, nlev, nleaves, nterms, nsource, ntarget, centre x, y, z, side of the root cube
+// (of the first instance for a batch), bytes of device memory held
 int fmm3d_lfmm3d_plan_info(void *plan, double *out, int n)
 {
     if (!plan || !out) return 1;
     auto *E = (LapPlanExec *)plan;
     Tree &T = E->S.T;
-    const double v[10] = {(double)T.nboxes, (double)T.nlev, (double)T.nleaves, (double)E->S.p, (double)E->S.ns,
-                          (double)E->S.nt, T.center0[0], T.center0[1], T.center0[2], T.size};
-    for (int i = 0; i < n && i < 10; i++) out[i] = v[i];
+    const double v[11] = {(double)T.nboxes, (double)T.nlev, (double)T.nleaves, (double)E->S.p, (double)E->S.ns,
+                          (double)E->S.nt, T.center0[0], T.center0[1], T.center0[2], T.size, (double)E->S.bytes};
+    for (int i = 0; i < n && i < 11; i++) out[i] = v[i];
     return 0;
 }
 

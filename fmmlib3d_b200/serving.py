@@ -71,22 +71,28 @@ def projected_bytes(req):
     n = len(req.source)
     per_point = 24 + 16 + 64 + 24 + 16 + 64 + 64     # caller arrays, sorted copies, outputs, keys/sort
     nbox = _NBOX.get(req.iprec, 160)
-    boxes = 2.5 * max(n / nbox, 1) * 8 / 7 + 64
+    scratch = 64 << 20
     if req.kernel == "helmholtz":
+        boxes = 2.5 * max(n / nbox, 1) * 8 / 7 + 64
         p = 12 + 4 * abs(complex(req.zk)) + 4 * max(req.iprec, 0)   # generous order estimate
-        p = min(p, 60)
+        exps = boxes * 2 * (min(p, 60) + 1) ** 2 * 16
     else:
+        # a box just above nbox points leaves eight leaves: up to 8 leaves for each nbox points
+        boxes = 8 * max(n / nbox, 1) * 8 / 7 + 64
         p = {-2: 4, -1: 6, 0: 9, 1: 14, 2: 26, 3: 39}.get(req.iprec, 39)
-    exps = boxes * 2 * (p + 1) ** 2 * 16
-    return int(n * per_point + exps + boxes * 600 + (64 << 20))
+        exps = boxes * 2 * (p + 1) ** 2 * 16
+        if p <= 26:
+            # the folded M2L: the multipoles in its basis, and its targets' sums in up to eight
+            # groups, at most 256 MB of them
+            exps += boxes * (p + 1) ** 2 * 16
+            scratch += min(8 * boxes * (p + 1) ** 2 * 16, 256 << 20)
+    return int(n * per_point + exps + boxes * 600 + scratch)
 
 
 def plan_bytes(info):
-    """HBM held by a resident plan, from its built tree (LaplacePlan.info()): expansions and
-    box arrays per box, sorted coordinates, charges and output workspace per point, and the
-    server's charge / output buffers for the plan."""
-    p, nb, n = info["nterms"], info["nboxes"], info["nsource"] + info["ntarget"]
-    return int(nb * (2 * (p + 1) ** 2 * 16 + 600) + n * (24 + 16 + 64) + info["nsource"] * (24 + 16 + 64))
+    """HBM held by a resident plan: what the library counts for it (LaplacePlan.info()) and the
+    server's source, charge and output buffers for the plan."""
+    return int(info["bytes"] + info["nsource"] * (24 + 16 + 64))
 
 
 def transient_bytes(n):

@@ -427,7 +427,9 @@ int fmm3d_lfmm3d_plan_execute(void *plan, const double *d_charge, const double *
                               double *d_pot, double *d_fld, double *d_pottarg, double *d_fldtarg, int use_graph,
                               void *stream);
 int fmm3d_lfmm3d_plan_destroy(void *plan);
-/* out[0..9]: nboxes, nlev, nleaves, nterms, nsource, ntarget, root centre (3), root side. */
+/* out[0..10] (at most n of them): nboxes, nlev, nleaves, nterms, nsource, ntarget, root centre (3),
+ * root side, and the bytes of device memory that the plan holds until it is destroyed (its tree,
+ * coordinates, expansions and workspace; operator tables, shared by all calls of an order, apart). */
 int fmm3d_lfmm3d_plan_info(void *plan, double *out, int n);
 /* d3tgetb: box(20) (level; i, j, k; parent; children; first source (1-based in tree
  * order), count; first target, count; source and target type 0 empty / 1 leaf /

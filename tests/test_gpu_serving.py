@@ -127,3 +127,61 @@ def test_repeated_geometries_run_on_resident_plans():
             assert st["plans_built"] == 3 and st["plan_hits"] == 15 and st["plans_evicted"] == 0
         else:
             assert st["plans_evicted"] >= 1
+
+
+def _pool(attr):
+    """An attribute of the device's default memory pool (the pool the library allocates from), in bytes."""
+    from cuda.bindings import driver as drv
+    assert drv.cuInit(0)[0] == drv.CUresult.CUDA_SUCCESS
+    err, pool = drv.cuDeviceGetDefaultMemPool(0)
+    assert err == drv.CUresult.CUDA_SUCCESS
+    a = getattr(drv.CUmemPool_attribute, "CU_MEMPOOL_ATTR_USED_MEM_" + attr)
+    err, v = drv.cuMemPoolGetAttribute(pool, a)
+    assert err == drv.CUresult.CUDA_SUCCESS
+    if attr == "HIGH":   # and back to the current use
+        assert drv.cuMemPoolSetAttribute(pool, a, drv.cuuint64_t(0))[0] == drv.CUresult.CUDA_SUCCESS
+    return int(v)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape,n,iprec", [("sphere", 10000, 1), ("cube", 100000, 1), ("plummer", 100000, 2),
+                                           ("sphere", 1000000, 0), ("cube", 20000, 3)])
+def test_admission_covers_what_plans_hold_and_calls_take(shape, n, iprec, precision):
+    """The library's count of a plan's memory is what the pool has handed out for it, plan_bytes
+    covers it and the server's own buffers, and the projection of a request covers the peak of its
+    call.  The pool rounds each of a plan's fewer than 100 allocations up, by less than 512 bytes."""
+    import torch
+    import fmmlib3d_b200 as F
+    from fmmlib3d_b200.serving import Request, plan_bytes, projected_bytes
+    rng = np.random.default_rng(n + iprec)
+    src = rng.random((n, 3)) if shape == "cube" else rng.normal(size=(n, 3))
+    if shape != "cube":
+        src /= np.linalg.norm(src, axis=1)[:, None]
+    if shape == "plummer":
+        src *= (0.1 / np.sqrt(np.maximum(rng.random(n), 1e-9) ** (-2 / 3) - 1)).clip(0, 1)[:, None]
+    d_src = torch.from_numpy(src).cuda()
+    q = torch.ones((n, 2), dtype=torch.float64, device="cuda")
+    pot, fld = torch.empty((n, 2), dtype=torch.float64, device="cuda"), torch.empty((n, 6), dtype=torch.float64,
+                                                                                    device="cuda")
+    torch.cuda.synchronize()
+    F.set_precision(precision)
+    try:
+        F.LaplacePlan(iprec, d_src, 1, 0, 1, 1).close()    # the order's tables
+        torch.cuda.synchronize()
+        before = _pool("CURRENT")
+        plan = F.LaplacePlan(iprec, d_src, 1, 0, 1, 1)
+        torch.cuda.synchronize()
+        held, info = _pool("CURRENT") - before, plan.info()
+        plan.close()
+        torch.cuda.synchronize()
+        _pool("HIGH")
+        base = _pool("HIGH")
+        assert F.lfmm3dparttarg_device(iprec, d_src, q, None, None, pot, fld) == 0
+        torch.cuda.synchronize()
+        peak = _pool("HIGH") - base
+    finally:
+        F.set_precision(0)
+    arrays = n * (24 + 16 + 64)
+    assert info["bytes"] <= held < info["bytes"] + 100 * 512
+    assert plan_bytes(info) >= held + arrays - 100 * 512
+    assert projected_bytes(Request("laplace", src, None, iprec=iprec)) >= peak + arrays
