@@ -610,8 +610,8 @@ class LaplacePlan:
         return _lib.fmm3d_lfmm3d_plan_set_tuning(self._h, _ptr(a), len(a))
 
     def get_tuning(self):
-        """The knobs in use (0 where the form has none), the form and whether they came
-        from the tuning cache."""
+        """The knobs in use (0 where the form has none, and for M2M / L2L tiles chosen by level),
+        the form and whether they came from the tuning cache."""
         out = np.zeros(len(TUNING_KNOBS) + 2, np.int32)
         _lib.fmm3d_lfmm3d_plan_get_tuning(self._h, _ptr(out), len(out))
         return _tuning_dict(out)

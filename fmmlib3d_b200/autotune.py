@@ -3,7 +3,7 @@
 Knobs (``TUNING_KNOBS``, 0 = automatic):
   m2l_kt      M2L targets per tile (tensor-core form 16..256; rotations 1, 2, 4, 8; the folded
               FP64 operators' tile is the kernel's own: 16 or 64 are taken without effect)
-  trans_kt    M2M / L2L targets per tile (1, 2, 4, 8)
+  trans_kt    M2M / L2L targets per tile (1, 2, 4, 8; automatic: chosen level by level)
   tc_variant  tensor-core M2L shared-memory staging (1: K chunks of 16, three stages;
               2: K chunks of 32, two stages)
   overlap     1: near field concurrent with the far field; 2: all passes in order
@@ -42,7 +42,7 @@ def candidates(form):
         c.append(("m2l_kt", [16, 64]))
     elif form == "fp64-rotation":
         c.append(("m2l_kt", [1, 2, 4, 8]))
-    c.append(("trans_kt", [1, 2, 4, 8]))
+    c.append(("trans_kt", [0, 1, 2, 4, 8]))
     if form == "mixed-tc":
         c.append(("tc_variant", [1, 2]))
     if form.startswith("mixed"):

@@ -387,14 +387,14 @@ struct LapSetup {
     DBuf<Tile> dtiles;
     struct TileRange { int first, count, kt; };
     std::vector<TileRange> m2m_rng, l2l_rng;  // per level: tiles [first, first + count) of kt targets
-    int m2l_a = 0, m2l_n = 0, m2l_kt = 0, trans_kt = 0;
+    int m2l_a = 0, m2l_n = 0, m2l_kt = 0;
     // mixed form: list-3 boxes with few sources and the list-4 boxes of boxes with
     // few points are summed with the near field; tv_near is tv with list 1
     // replaced by the widened near list, tv_far with lists 3 and 4 by the rest
     DBuf<int> nl_start, nl_idx, fl_start, fl_idx, f4_start, f4_idx;
     TreeView tv_near, tv_far;
     int l3_direct = 0;        // source / point count up to which lists 3 / 4 go to the near field (0: none)
-    TuneKnobs knobs;          // as requested (0 = automatic); m2l_kt / trans_kt hold the values in use
+    TuneKnobs knobs;          // as requested (0 = automatic); m2l_kt holds the value in use
     bool knobs_from_cache = false;
     std::string signature;
     long long bytes = 0;      // device memory that this geometry holds (operator tables of the order apart)
@@ -582,7 +582,6 @@ static int lap_tiles(LapSetup &S, const TuneKnobs &k, cudaStream_t s, Status &st
     S.m2l_a = m2l_a;
     S.m2l_n = m2l_n;
     S.m2l_kt = m2l_kt;
-    S.trans_kt = tkt;
     S.knobs = k;
     return 0;
 }
@@ -1030,7 +1029,7 @@ thread_local int g_last_knobs[kNumKnobs + 2] = {};
 static void lap_effective_knobs(const LapSetup &S, int *out)
 {
     out[0] = S.m2l_kt;
-    out[1] = S.trans_kt;
+    out[1] = S.knobs.trans_kt;   // 0: by level
     out[2] = S.tcm2l ? (S.knobs.tc_variant ? S.knobs.tc_variant : sw(kSwTensorM2L) == 2 ? 2 : 1) : 0;
     out[3] = lap_overlap(S) ? 1 : 2;
     out[4] = S.mixed ? (S.knobs.p2p_ept ? S.knobs.p2p_ept : 4) : 0;
@@ -1367,7 +1366,7 @@ int fmm3d_lfmm3d_plan_set_tuning(void *plan, const int *knobs, int n)
 }
 
 // out[0..4] = knobs in use (m2l_kt, trans_kt, tc_variant, overlap, p2p_ept; 0 = not
-// applicable to this form), out[5] = form, out[6] = 1 if they came from the cache
+// applicable to this form, or trans_kt chosen by level), out[5] = form, out[6] = 1 if they came from the cache
 int fmm3d_lfmm3d_plan_get_tuning(void *plan, int *out, int n)
 {
     if (!plan || !out || n < kNumKnobs + 2) return 1;

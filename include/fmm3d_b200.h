@@ -457,7 +457,7 @@ int fmm3d_d3tstrcrem(int nsource, const double *d_source, int nbox, int ntarget,
  *   [0] M2L targets per tile (tensor-core form 16..256 in steps of 16; FP64
  *       dense operators 16 or 64 (the folded kernels' tile is their own: the
  *       value is taken and has no effect there, in either form); FP32 CUDA-core form 64; rotations 1, 2, 4, 8),
- *   [1] M2M / L2L targets per tile (1, 2, 4, 8),
+ *   [1] M2M / L2L targets per tile (1, 2, 4, 8; automatic: chosen level by level),
  *   [2] tensor-core M2L staging variant (1 or 2, as fmm3d_set_tensor_m2l),
  *   [3] 1 = near field concurrent with the far field, 2 = passes in order
  *       (fmm3d_set_overlap(0) forces the passes in order whatever the knob),
@@ -476,7 +476,8 @@ int fmm3d_tuning_cache_path(char *buf, int n);
 /* Set a plan's knobs (n >= 5).  Returns 0, 2 for a value this problem cannot
  * take (the plan keeps its previous knobs), 16 on a CUDA error. */
 int fmm3d_lfmm3d_plan_set_tuning(void *plan, const int *knobs, int n);
-/* out (n >= 7): the five knobs in use (0 where the form has no such knob), the
+/* out (n >= 7): the five knobs in use (0 where the form has no such knob, and for
+ * M2M / L2L tiles chosen by level), the
  * form (0 FP64 rotations, 1 FP64 dense operators, 2 mixed with CUDA-core M2L,
  * 3 mixed with tensor-core M2L) and 1 if the knobs came from the cache. */
 int fmm3d_lfmm3d_plan_get_tuning(void *plan, int *out, int n);

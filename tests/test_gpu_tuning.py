@@ -133,3 +133,18 @@ def test_tune_writes_the_cache_and_single_calls_use_it(F, tmp_path):
     assert plan2.get_tuning()["from_cache"]
     plan.close()
     plan2.close()
+
+
+def test_tuner_starts_from_the_tiles_chosen_by_level(F):
+    """The automatic M2M / L2L tiles differ by level: the knob reads 0, so that a search in which
+    nothing is kept ends with them and not with one size for every level."""
+    from fmmlib3d_b200 import autotune as A
+    n, m = 30000, 12000
+    src, trg, q, d, v = _problem(n, m, 56)
+    F.set_tuning_cache("")
+    plan = F.LaplacePlan(1, src, 1, 1, 1, 1, trg, 1, 1)
+    before = plan.get_tuning()
+    assert before["trans_kt"] == 0
+    res = A.tune(plan, q, d, v, *_outs(n, m), reps=1, min_gain=1.0, cache=False)
+    assert res["knobs"]["trans_kt"] == 0 and plan.get_tuning() == before
+    plan.close()
