@@ -517,6 +517,7 @@ def _tuning_dict(out):
     d = {k: int(out[i]) for i, k in enumerate(TUNING_KNOBS)}
     d["form"] = TUNING_FORMS[int(out[len(TUNING_KNOBS)])]
     d["from_cache"] = bool(out[len(TUNING_KNOBS) + 1])
+    d["folded"] = bool(out[len(TUNING_KNOBS) + 2])   # the M2L runs by the folded FP64 operators
     return d
 
 
@@ -540,7 +541,7 @@ def tuning_cache_path():
 
 def last_tuning():
     """(knobs dict, signature) of this thread's last single Laplace call."""
-    out = np.zeros(len(TUNING_KNOBS) + 2, np.int32)
+    out = np.zeros(len(TUNING_KNOBS) + 3, np.int32)
     buf = ctypes.create_string_buffer(1024)
     _lib.fmm3d_last_tuning(_ptr(out), len(out), buf, len(buf))
     return _tuning_dict(out), buf.value.decode()
@@ -611,8 +612,8 @@ class LaplacePlan:
 
     def get_tuning(self):
         """The knobs in use (0 where the form has none, and for M2M / L2L tiles chosen by level),
-        the form and whether they came from the tuning cache."""
-        out = np.zeros(len(TUNING_KNOBS) + 2, np.int32)
+        the form, whether they came from the tuning cache and whether the M2L is the folded one."""
+        out = np.zeros(len(TUNING_KNOBS) + 3, np.int32)
         _lib.fmm3d_lfmm3d_plan_get_tuning(self._h, _ptr(out), len(out))
         return _tuning_dict(out)
 

@@ -1,8 +1,8 @@
 """Autotuner of the Laplace passes' launch shapes, with a JSON cache.
 
 Knobs (``TUNING_KNOBS``, 0 = automatic):
-  m2l_kt      M2L targets per tile (tensor-core form 16..256; rotations 1, 2, 4, 8; the folded
-              FP64 operators' tile is the kernel's own: 16 or 64 are taken without effect)
+  m2l_kt      M2L targets per tile (tensor-core form 16..256; rotations 1, 2, 4, 8); the folded
+              FP64 operators' tile is the kernel's own: there the values are taken without effect
   trans_kt    M2M / L2L targets per tile (1, 2, 4, 8; automatic: chosen level by level)
   tc_variant  tensor-core M2L shared-memory staging (1: K chunks of 16, three stages;
               2: K chunks of 32, two stages)
@@ -33,17 +33,20 @@ from . import TUNING_KNOBS, set_tuning_cache, tuning_cache_path, tuning_reload  
 CACHE_FORMAT = "fmm3d_b200 tuning cache"
 
 
-def candidates(form):
-    """(knob, values) in search order for a form (as ``LaplacePlan.get_tuning()["form"]``)."""
+def candidates(form, folded=False):
+    """(knob, values) in search order for a form (as ``LaplacePlan.get_tuning()["form"]``); ``folded``
+    (there too): without the knobs of the M2L kernels that the folded operators replace."""
     c = []
-    if form == "mixed-tc":
+    if folded:
+        pass
+    elif form == "mixed-tc":
         c.append(("m2l_kt", [16, 32, 64, 128, 256]))
     elif form == "fp64-dense":
         c.append(("m2l_kt", [16, 64]))
     elif form == "fp64-rotation":
         c.append(("m2l_kt", [1, 2, 4, 8]))
     c.append(("trans_kt", [0, 1, 2, 4, 8]))
-    if form == "mixed-tc":
+    if form == "mixed-tc" and not folded:
         c.append(("tc_variant", [1, 2]))
     if form.startswith("mixed"):
         c.append(("p2p_ept", [1, 2, 4]))
@@ -123,7 +126,7 @@ def tune(plan, charge=None, dipstr=None, dipvec=None, pot=None, fld=None, pottar
     trials = [(dict(best), best_ms)]
     if log:
         log("start %s: %.3f ms" % (best, best_ms))
-    for knob, values in candidates(form):
+    for knob, values in candidates(form, start["folded"]):
         base = dict(best)
         for v in values:
             if v == base[knob]:

@@ -451,7 +451,8 @@ static bool lap_overlap(const LapSetup &S)
     return S.knobs.overlap == 1 || S.mixed || S.p <= 16 || S.T.nleaves < 16 * 148;
 }
 
-// form code reported with the knobs: 0 FP64 rotations, 1 FP64 dense, 2 mixed CUDA-core M2L, 3 mixed tensor-core M2L
+// form code reported with the knobs: 0 FP64 rotations, 1 FP64 dense, 2 mixed CUDA-core M2L, 3 mixed tensor-core M2L.
+// (0, 1 and 3 are also the forms of calls whose M2L is folded, at orders above 16, up to 16 and in the mixed form)
 static int lap_form(const LapSetup &S) { return S.tcm2l ? 3 : S.mixed ? 2 : S.dense ? 1 : 0; }
 
 // Tiles of one (level, octant) group and translation kind: boxes [a, bnd) of
@@ -1024,17 +1025,20 @@ static int lap_finish(LapSetup &S, cudaStream_t s, Status &st)
 // ---------------------------------------------------------------- the FMM, one call
 // knobs of the last single call on this thread (fmm3d_last_tuning)
 thread_local std::string g_last_signature;
-thread_local int g_last_knobs[kNumKnobs + 2] = {};
+constexpr int kNumTuningOut = kNumKnobs + 3;
+thread_local int g_last_knobs[kNumTuningOut] = {};
 
 static void lap_effective_knobs(const LapSetup &S, int *out)
 {
-    out[0] = S.m2l_kt;
+    // (the folded M2L has no tile or staging knob: what was asked for, without effect)
+    out[0] = S.fold ? S.knobs.m2l_kt : S.m2l_kt;
     out[1] = S.knobs.trans_kt;   // 0: by level
-    out[2] = S.tcm2l ? (S.knobs.tc_variant ? S.knobs.tc_variant : sw(kSwTensorM2L) == 2 ? 2 : 1) : 0;
+    out[2] = S.fold ? S.knobs.tc_variant : S.tcm2l ? (S.knobs.tc_variant ? S.knobs.tc_variant : sw(kSwTensorM2L) == 2 ? 2 : 1) : 0;
     out[3] = lap_overlap(S) ? 1 : 2;
     out[4] = S.mixed ? (S.knobs.p2p_ept ? S.knobs.p2p_ept : 4) : 0;
     out[5] = lap_form(S);
     out[6] = S.knobs_from_cache ? 1 : 0;
+    out[7] = S.fold ? 1 : 0;
 }
 
 static int lap_fmm_device(int iprec, int ns, const double *d_src, int ifcharge, const double *d_q, int ifdipole,
@@ -1366,14 +1370,17 @@ int fmm3d_lfmm3d_plan_set_tuning(void *plan, const int *knobs, int n)
 }
 
 // out[0..4] = knobs in use (m2l_kt, trans_kt, tc_variant, overlap, p2p_ept; 0 = not
-// applicable to this form, or trans_kt chosen by level), out[5] = form, out[6] = 1 if they came from the cache
+// applicable to this form, or trans_kt chosen by level), out[5] = form, out[6] = 1 if they came from the cache,
+// out[7] (if n allows) = 1 if the M2L runs by the folded FP64 operators
 int fmm3d_lfmm3d_plan_get_tuning(void *plan, int *out, int n)
 {
     if (!plan || !out || n < kNumKnobs + 2) return 1;
     auto *E = (LapPlanExec *)plan;
     if (!E->S.plan) return 4;   // a tree from fmm3d_d3tstrcrem: no FMM on it
     std::lock_guard<std::mutex> lk(E->mu);
-    lap_effective_knobs(E->S, out);
+    int v[kNumTuningOut];
+    lap_effective_knobs(E->S, v);
+    memcpy(out, v, sizeof(int) * std::min(n, kNumTuningOut));
     return 0;
 }
 
@@ -1392,7 +1399,7 @@ int fmm3d_lfmm3d_plan_signature(void *plan, char *buf, int n)
 // the knobs (as fmm3d_lfmm3d_plan_get_tuning) and signature of this thread's last single Laplace call
 int fmm3d_last_tuning(int *out, int n, char *sig, int nsig)
 {
-    if (out && n >= kNumKnobs + 2) memcpy(out, g_last_knobs, sizeof(int) * (kNumKnobs + 2));
+    if (out && n >= kNumKnobs + 2) memcpy(out, g_last_knobs, sizeof(int) * std::min(n, kNumTuningOut));
     if (sig && nsig > 0) snprintf(sig, (size_t)nsig, "%s", g_last_signature.c_str());
     return (int)g_last_signature.size() + 1;
 }

@@ -479,7 +479,9 @@ int fmm3d_lfmm3d_plan_set_tuning(void *plan, const int *knobs, int n);
 /* out (n >= 7): the five knobs in use (0 where the form has no such knob, and for
  * M2M / L2L tiles chosen by level), the
  * form (0 FP64 rotations, 1 FP64 dense operators, 2 mixed with CUDA-core M2L,
- * 3 mixed with tensor-core M2L) and 1 if the knobs came from the cache. */
+ * 3 mixed with tensor-core M2L), 1 if the knobs came from the cache, and, with
+ * n >= 8, 1 if the M2L runs by the folded FP64 operators (form 0 at orders 17 to
+ * 26, form 1 and form 3 by default), which have no tile or staging knob. */
 int fmm3d_lfmm3d_plan_get_tuning(void *plan, int *out, int n);
 /* The plan's problem signature (the cache key); returns 0 or the buffer size needed. */
 int fmm3d_lfmm3d_plan_signature(void *plan, char *buf, int n);

@@ -148,3 +148,28 @@ def test_tuner_starts_from_the_tiles_chosen_by_level(F):
     res = A.tune(plan, q, d, v, *_outs(n, m), reps=1, min_gain=1.0, cache=False)
     assert res["knobs"]["trans_kt"] == 0 and plan.get_tuning() == before
     plan.close()
+
+
+@pytest.mark.parametrize("precision,iprec,tensor_m2l,folded", [(1, 1, 3, True), (1, 1, 1, False), (0, 1, 3, True),
+                                                               (0, 2, 3, True), (0, 3, 3, False)])
+def test_knobs_of_a_kernel_that_does_not_run_are_not_reported_or_searched(F, precision, iprec, tensor_m2l, folded):
+    """The folded M2L has no tile and no staging variant: both knobs read 0, and no trial changes them."""
+    from fmmlib3d_b200 import autotune as A
+    n, m = 12000, 3000
+    src, trg, q, d, v = _problem(n, m, 57)
+    F.set_tuning_cache("")
+    F.set_precision(precision)
+    F.set_tensor_m2l(tensor_m2l)
+    try:
+        plan = F.LaplacePlan(iprec, src, 1, 1, 1, 1, trg, 1, 1)
+        t = plan.get_tuning()
+        assert t["folded"] == folded
+        res = A.tune(plan, q, d, v, *_outs(n, m), reps=1, min_gain=1.0, cache=False)
+        plan.close()
+    finally:
+        F.set_tensor_m2l(3)
+    tried = {k for knobs, _ in res["trials"] for k in knobs if knobs[k] != t[k]}
+    if folded:
+        assert t["m2l_kt"] == 0 and t["tc_variant"] == 0 and not tried & {"m2l_kt", "tc_variant"}
+    else:
+        assert t["m2l_kt"] > 0 and "m2l_kt" in tried and (t["tc_variant"] > 0) == (precision == 1)
