@@ -421,17 +421,17 @@ struct LapSetup {
     TreeView tv_quad;
 };
 
-// Problem signature of the tuning cache: the form, the flags that select
-// kernel variants, and the sizes that set the launch shapes (log2 buckets).
+// Problem signature of the tuning cache: the form and M2L kernel, the flags that
+// select kernel variants, and the sizes that set the launch shapes (log2 buckets).
 static std::string lap_signature(const LapSetup &S)
 {
     const char *form = S.tcm2l ? "mixed-tc" : S.mixed ? "mixed-cuda" : S.dense ? "fp64-dense" : "fp64-rotation";
     const char *kern = S.tri ? "laplace-triangles" : "laplace";
     char b[512];
     snprintf(b, sizeof b,
-             "%s iprec=%d form=%s charge=%d dipole=%d out=%d%d%d%d inst=2^%d ns=2^%d nt=2^%d nlev=%d "
+             "%s iprec=%d form=%s%s charge=%d dipole=%d out=%d%d%d%d inst=2^%d ns=2^%d nt=2^%d nlev=%d "
              "nboxes=2^%d dev=%s",
-             kern, S.iprec, form, S.ifcharge == 1, S.ifdipole == 1, S.ifpot == 1, S.iffld == 1,
+             kern, S.iprec, form, S.fold ? " m2l=fold" : "", S.ifcharge == 1, S.ifdipole == 1, S.ifpot == 1, S.iffld == 1,
              S.do_trg && S.ifpottarg == 1, S.do_trg && S.iffldtarg == 1, log2_bucket(S.T.ninst),
              log2_bucket(S.ns), log2_bucket(S.do_trg ? S.nt : 0), S.T.nlev, log2_bucket(S.T.nboxes),
              device_tag().c_str());

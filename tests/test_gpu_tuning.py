@@ -173,3 +173,34 @@ def test_knobs_of_a_kernel_that_does_not_run_are_not_reported_or_searched(F, pre
         assert t["m2l_kt"] == 0 and t["tc_variant"] == 0 and not tried & {"m2l_kt", "tc_variant"}
     else:
         assert t["m2l_kt"] > 0 and "m2l_kt" in tried and (t["tc_variant"] > 0) == (precision == 1)
+
+
+@pytest.mark.parametrize("precision,iprec", [(1, 1), (0, 1), (0, 2)])
+def test_settings_tuned_on_another_m2l_kernel_are_not_taken(F, precision, iprec, tmp_path):
+    """The M2L kernel is part of the cache key: a setting tuned on the split-TF32 M2L or on the
+    rotations, the same problem otherwise, is not taken by a call whose M2L is folded."""
+    from fmmlib3d_b200 import autotune as A
+    src, trg, *_ = _problem(12000, 3000, 58)
+    path = str(tmp_path / "tune.json")
+    F.set_tuning_cache(path)
+    F.set_precision(precision)
+
+    def plan():
+        return F.LaplacePlan(iprec, src, 1, 1, 1, 1, trg, 1, 1)
+
+    other = (F.set_tensor_m2l, 1, 3) if precision else (F.set_m2l_mode, 1, 0)
+    try:
+        other[0](other[1])
+        p = plan()
+        A.write_cache(path, p.signature(), {"knobs": {"trans_kt": 4, "overlap": 2}})
+        p.close()
+        F.tuning_reload()
+        p = plan()
+        assert p.get_tuning()["from_cache"]
+        p.close()
+    finally:
+        other[0](other[2])
+    p = plan()
+    t = p.get_tuning()
+    p.close()
+    assert t["folded"] and not t["from_cache"] and t["trans_kt"] == 0
