@@ -204,6 +204,7 @@ SideStreams &side_streams()
         int least = 0, greatest = 0;
         cudaDeviceGetStreamPriorityRange(&least, &greatest);
         cudaStreamCreateWithPriority(&ss.far, cudaStreamNonBlocking, greatest);
+        cudaStreamCreateWithFlags(&ss.far_even, cudaStreamNonBlocking);
         cudaStreamCreateWithFlags(&ss.copy, cudaStreamNonBlocking);
         cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ss.join, cudaEventDisableTiming);

@@ -113,10 +113,10 @@ struct Timer {
     }
 };
 
-// Per-thread high-priority stream for the far-field passes of a call, and the
-// fork / join events between it and the call's stream (made once per thread).
+// Per-thread streams for the far-field passes of a call, of high and of ordinary
+// priority, and the fork / join events between them and the call's stream (made once per thread).
 struct SideStreams {
-    cudaStream_t far = nullptr, copy = nullptr;
+    cudaStream_t far = nullptr, far_even = nullptr, copy = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, mid = nullptr, copied = nullptr;
     int dev = -1;
 };

@@ -438,17 +438,28 @@ static std::string lap_signature(const LapSetup &S)
     return b;
 }
 
-// Near field beside the far field (knob 0): unless both are long and bound by the FP64
-// pipe.  Above order 16 a leaf holds 400 or more sources, so a run of the near
-// field takes about half a millisecond, and a far-field CTA, which needs a whole
-// multiprocessor, waits for the runs on it to end: 1M + 1M cube at order 26 (4,096
-// leaves) 49.6 ms beside each other, 47.0 one after the other; 2M + 2M cube at order
-// 14 31.6 / 32.0.  Small problems (fewer leaves than 16 warps on every
-// multiprocessor) gain from it at every order.
-static bool lap_overlap(const LapSetup &S)
+// Near field beside the far field, unless a switch or the knob says otherwise.
+static bool lap_overlap(const LapSetup &S) { return sw(kSwOverlap) != 0 && S.knobs.overlap != 2; }
+
+// Whether the far field runs at the near field's priority instead of a higher one.  A CTA of the
+// folded M2L above order 15 takes a multiprocessor to itself; at high priority the multiprocessor
+// is kept free for it while the warps of the near field on it end, and these are long where a leaf
+// has many pairs (a run of 64 points meets the sources of its list 1 in turn).  The line is half a
+// million pairs a leaf (sources times points times boxes of list 1, of average leaves), with enough
+// leaves to fill the GPU (16 warps on every multiprocessor).  One call at order 26 (c: charges,
+// d: dipoles), ms: one after the other / beside at high priority / beside at the same:
+//   2.8M pairs, cube 1M + 1M, c d        46.3 / 50.4 / 44.9    0.57M, cube 450k + 450k, c d         16.6 / 16.3 / 16.4
+//   1.4M, cube 1M, d                     27.9 / 29.1 / 27.4    0.52M, Plummer 500k + 250k, d        52.5 / 49.1 / 49.6
+//   0.88M, sphere 900k + 900k, d         40.4 / 40.5 / 39.5    0.32M, Plummer 1M, c                 81.5 / 76.7 / 80.6
+//   0.60M, Plummer 900k + 900k, c d      98.5 / 99.0 / 95.8    0.23M, sphere 400k + 400k, c d       24.4 / 23.6 / 24.0
+//   0.51M, sphere 1M + 1M, c d           65.9 / 66.1 / 64.9    0.15M, cube 1.7M + 1.7M, c d        102.2 / 99.2 / 100.5
+// (Found to go the other way: cube 1.4M, c, 2.8M pairs, 37.8 / 32.1 / 36.6.)  Triangles (328k, 91.4 /
+// 89.1 / 91.3) and order 39, which is not folded (cube 1.5M + 1.5M 291 / 285 / 287), keep the high priority.
+static bool lap_even_priority(const LapSetup &S)
 {
-    if (sw(kSwOverlap) == 0 || S.knobs.overlap == 2) return false;
-    return S.knobs.overlap == 1 || S.mixed || S.p <= 16 || S.T.nleaves < 16 * 148;
+    if (!S.fold || S.plan->fold.tile != 8 || S.tri || S.T.nleaves < 16 * device_sms()) return false;
+    const double leaves = S.T.nleaves;
+    return S.ns / leaves * ((S.do_src ? S.ns : 0) + (S.do_trg ? S.nt : 0)) / leaves * (1 + S.T.l1_idx.n / leaves) >= 5e5;
 }
 
 // form code reported with the knobs: 0 FP64 rotations, 1 FP64 dense, 2 mixed CUDA-core M2L, 3 mixed tensor-core M2L.
@@ -869,7 +880,7 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     FMM_LAUNCH_CHECK(st);
     tm.mark();
     // The near field (STEP 8) runs on the call's stream while the far-field
-    // passes (STEPS 1-5) run on a high-priority side stream; they meet before
+    // passes (STEPS 1-5) run on a side stream; they meet before
     // STEPS 6-7, which add the far field to the outputs.  In the mixed form the
     // two use different units (FP32 CUDA cores, tensor cores).  With the
     // overlap switched off (fmm3d_set_overlap(0)) everything runs on the call's
@@ -877,7 +888,7 @@ static void lap_passes(LapSetup &S, const double *d_q, const double *d_dq, const
     SideStreams &ss = side_streams();
     // fmm3d_set_overlap(0) forces the passes in order (per-pass timing); else the knob decides
     const bool overlap = lap_overlap(S);
-    const cudaStream_t f = overlap ? ss.far : s;
+    const cudaStream_t f = !overlap ? s : lap_even_priority(S) ? ss.far_even : ss.far;
     if (overlap) {
         FMM_TRY(st, cudaEventRecord(ss.fork, s));
         FMM_TRY(st, cudaStreamWaitEvent(f, ss.fork, 0));

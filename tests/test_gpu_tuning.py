@@ -204,3 +204,26 @@ def test_settings_tuned_on_another_m2l_kernel_are_not_taken(F, precision, iprec,
     t = p.get_tuning()
     p.close()
     assert t["folded"] and not t["from_cache"] and t["trans_kt"] == 0
+
+
+@pytest.mark.parametrize("n,m,geom", [(500000, 500000, "cube"), (300000, 0, "sphere")])
+def test_near_and_far_field_run_beside_each_other_above_order_16(F, n, m, geom):
+    """Long calls at order 26, on both sides of the rule that picks the far field's priority: the
+    near field runs beside the far field unless it is told otherwise, with the same bits."""
+    import torch
+    src, trg, q, d, v = _problem(n, max(m, 1), 59, geom)
+    F.set_tuning_cache("")
+    outs = []
+    for on in (1, 0):
+        out = _outs(n, max(m, 1))
+        F.set_overlap(on)
+        try:
+            args = (trg, out[2], out[3]) if m else ()
+            assert F.lfmm3dparttarg_device(2, src, q, d, v, out[0], out[1], *args) == 0, F.last_error()
+            assert F.last_tuning()[0]["overlap"] == (1 if on else 2)
+        finally:
+            F.set_overlap(1)
+        torch.cuda.synchronize()
+        outs.append(out[:4 if m else 2])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
