@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(T) k_heval(const int *leaves, TreeView tv, con
 // local expansions.  List 3 is very uneven on adaptive trees (on a sphere surface
 // most leaves have none and a few have over a hundred), so the work is cut into
 // items of one leaf, one chunk of T of its points and one group of at most
-// kHM2PGroup of its list-3 boxes, one CTA each.  An item writes its points' sums
+// `group` of its list-3 boxes, one CTA each.  An item writes its points' sums
 // over its group to its own slot of a scratch array; k_hm2p_add then adds the
 // groups' sums to the outputs in group order, so results do not depend on the
 // schedule.  The scaled Hankel functions f_n = h_n(z) scale^n of h3dall (the
@@ -1038,17 +1038,21 @@ __global__ void __launch_bounds__(T) k_heval(const int *leaves, TreeView tv, con
 // every value is the one hank_dev stores and shared memory holds only the staged
 // multipole.
 // Groups of 4: with 16 an SM had 5.5 warps on average (16.8 -> 15.5 ms with the local
-// expansions at the 1M sphere, 0.88 -> 0.55 ms at a cube of 10k + 5k).
-constexpr int kHM2PGroup = 4;
+// expansions at the 1M sphere, 0.88 -> 0.55 ms at a cube of 10k + 5k).  An item has 4 KB of
+// scratch, 85 MB in all at the 1M sphere (32 with groups of 16).  Where groups of 4 would take more
+// than 256 MB they are doubled until they do not or every leaf has one: 965 -> 256 MB at most at the 5M
+// sphere for 0.4% more time (436.7 -> 438.4 ms), at a Plummer ball of 2M 110.5 -> 110.6 ms.
+constexpr int kHM2PGroup = 4, kHM2PMaxGroup = 1 << 20;
+constexpr size_t kHM2PScratch = 256u << 20;
 
-__global__ void k_hm2p_count(const int *leaves, int nleaves, TreeView tv, int do_src, int do_trg, int *cnt)
+__global__ void k_hm2p_count(const int *leaves, int nleaves, int group, TreeView tv, int do_src, int do_trg, int *cnt)
 {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= nleaves) return;
     const int b = leaves[l];
     const int ne = (do_src ? tv.nsrc[b] : 0) + (do_trg ? tv.ntrg[b] : 0);
     const int nl3 = tv.l3_start[b + 1] - tv.l3_start[b];
-    cnt[l] = (ne > 0 && nl3 > 0) ? ((ne + kHM2PThreads - 1) / kHM2PThreads) * ((nl3 + kHM2PGroup - 1) / kHM2PGroup)
+    cnt[l] = (ne > 0 && nl3 > 0) ? ((ne + kHM2PThreads - 1) / kHM2PThreads) * ((nl3 + group - 1) / group)
                                  : 0;
 }
 
@@ -1066,7 +1070,7 @@ __device__ __forceinline__ int hm2p_leaf(const int *off, int nleaves, int item)
 }
 
 template <int T>
-__global__ void __launch_bounds__(T) k_hm2p(const int *leaves, int nleaves, const int *off, TreeView tv,
+__global__ void __launch_bounds__(T) k_hm2p(const int *leaves, int nleaves, const int *off, int group, TreeView tv,
                                              const double *sx, const double *sy, const double *sz, const double *tx,
                                              const double *ty, const double *tz, HLevels lv, int NC, double2 zk,
                                              const double2 *mpole, int do_src, int do_trg, double *part)
@@ -1076,14 +1080,14 @@ __global__ void __launch_bounds__(T) k_hm2p(const int *leaves, int nleaves, cons
     const int l = hm2p_leaf(off, nleaves, item), b = leaves[l];
     const int ns = do_src ? tv.nsrc[b] : 0, nt = do_trg ? tv.ntrg[b] : 0, ne = ns + nt;
     const int l3a = tv.l3_start[b], nl3 = tv.l3_start[b + 1] - l3a;
-    const int ngr = (nl3 + kHM2PGroup - 1) / kHM2PGroup;
+    const int ngr = (nl3 + group - 1) / group;
     const int local = item - off[l], ck = local / ngr, grp = local - ck * ngr;
-    const int c0 = ck * T, x1 = min(nl3, (grp + 1) * kHM2PGroup);
+    const int c0 = ck * T, x1 = min(nl3, (grp + 1) * group);
     double2 *E = hsm;
     const int t = threadIdx.x;
     // this item's sums at its point: pot, then -fld (x, y, z)
     double2 spot = cmk(0, 0), sfx = cmk(0, 0), sfy = cmk(0, 0), sfz = cmk(0, 0);
-    for (int xi = grp * kHM2PGroup; xi < x1; xi++) {
+    for (int xi = grp * group; xi < x1; xi++) {
         const int eb = tv.l3_idx[l3a + xi];
         if (tv.nsrc[eb] == 0) continue;
         const int lev = tv.level[eb], p = lv.p[lev];
@@ -1171,14 +1175,14 @@ __global__ void __launch_bounds__(T) k_hm2p(const int *leaves, int nleaves, cons
 
 // Adds the list-3 groups' sums of a leaf to its outputs, group by group.
 template <int T>
-__global__ void k_hm2p_add(const int *leaves, const int *off, TreeView tv, OutSoA outs, OutSoA outt, int do_src,
-                           int do_trg, const double *part)
+__global__ void k_hm2p_add(const int *leaves, const int *off, int group, TreeView tv, OutSoA outs, OutSoA outt,
+                           int do_src, int do_trg, const double *part)
 {
     const int l = blockIdx.x, b = leaves[l];
     const int ns = do_src ? tv.nsrc[b] : 0, nt = do_trg ? tv.ntrg[b] : 0, ne = ns + nt;
     const int nl3 = tv.l3_start[b + 1] - tv.l3_start[b];
     if (ne == 0 || nl3 == 0) return;
-    const int ngr = (nl3 + kHM2PGroup - 1) / kHM2PGroup, nch = (ne + T - 1) / T;
+    const int ngr = (nl3 + group - 1) / group, nch = (ne + T - 1) / T;
     for (int ck = blockIdx.y; ck < nch; ck += gridDim.y) {
         const int e = ck * T + threadIdx.x;
         if (e >= ne) continue;
@@ -1419,10 +1423,15 @@ void hm2p_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src
     if (nleaves == 0 || !st.ok() || (!do_src && !do_trg)) return;
     DBuf<int> cnt;
     if (!cnt.alloc(nleaves, s, st) || !I.off.alloc(nleaves, s, st)) return;
-    k_hm2p_count<<<div_up(nleaves, 256), 256, 0, s>>>(leaves, nleaves, tv, do_src, do_trg, cnt.p);
-    FMM_COUNT_LAUNCH();
-    FMM_LAUNCH_CHECK(st);
-    scan_exclusive_int(cnt.p, I.off.p, nleaves, s, st, &I.n);
+    for (I.group = kHM2PGroup;; I.group *= 2) {
+        const int last = I.n;
+        k_hm2p_count<<<div_up(nleaves, 256), 256, 0, s>>>(leaves, nleaves, I.group, tv, do_src, do_trg, cnt.p);
+        FMM_COUNT_LAUNCH();
+        FMM_LAUNCH_CHECK(st);
+        scan_exclusive_int(cnt.p, I.off.p, nleaves, s, st, &I.n);
+        if (!st.ok() || (size_t)I.n * 8 * kHM2PThreads * sizeof(double) <= kHM2PScratch) break;
+        if (I.n == last || I.group >= kHM2PMaxGroup) break;   // one group for every leaf
+    }
     if (st.ok() && I.n > 0) I.part.alloc((size_t)I.n * 8 * kHM2PThreads, s, st);
 }
 
@@ -1435,8 +1444,8 @@ void launch_hm2p(const int *leaves, int nleaves, const HM2PItems &I, const TreeV
     const int pm = max_p(lv);
     const size_t sm = sizeof(double2) * (size_t)(pm + 1) * (pm + 1);
     FMM_TRY(st, smem_allow(k_hm2p<kHM2PThreads>, (int)sm));
-    k_hm2p<kHM2PThreads><<<I.n, kHM2PThreads, sm, s>>>(leaves, nleaves, I.off.p, tv, sx, sy, sz, tx, ty, tz, lv, NC, zk,
-                                                       mpole, do_src, do_trg, I.part.p);
+    k_hm2p<kHM2PThreads><<<I.n, kHM2PThreads, sm, s>>>(leaves, nleaves, I.off.p, I.group, tv, sx, sy, sz, tx, ty, tz, lv,
+                                                       NC, zk, mpole, do_src, do_trg, I.part.p);
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);
 }
@@ -1445,7 +1454,7 @@ void launch_hm2p_add(const int *leaves, int nleaves, const HM2PItems &I, const T
                      int do_src, int do_trg, cudaStream_t s, Status &st)
 {
     if (I.n == 0 || !st.ok()) return;
-    k_hm2p_add<kHM2PThreads><<<dim3(nleaves, 4), kHM2PThreads, 0, s>>>(leaves, I.off.p, tv, outs, outt, do_src, do_trg,
+    k_hm2p_add<kHM2PThreads><<<dim3(nleaves, 4), kHM2PThreads, 0, s>>>(leaves, I.off.p, I.group, tv, outs, outt, do_src, do_trg,
                                                                        I.part.p);
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);

@@ -75,7 +75,7 @@ void launch_hl2p(const int *leaves, int nleaves, const TreeView &tv, const doubl
 struct HM2PItems {
     DBuf<int> off;
     DBuf<double> part;
-    int n = 0;
+    int n = 0, group = 0;   // items, list-3 boxes of an item
 };
 void hm2p_prepare(const int *leaves, int nleaves, const TreeView &tv, int do_src, int do_trg, HM2PItems &I,
                   cudaStream_t s, Status &st);

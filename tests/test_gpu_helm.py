@@ -324,3 +324,42 @@ def test_hfmm_direct_points_entry(F):
     op, of = O.hdirect_at(zk, src, src[idx], idx, q, ds, dv)
     assert rel(pot.cpu().numpy().view(np.complex128).reshape(-1), op) < 1e-13
     assert rel(fld.cpu().numpy().view(np.complex128).reshape(k, 3), of) < 1e-13
+
+
+def test_list3_scratch_is_bounded(F):
+    """Sums of list-3 multipoles in groups of boxes: the groups grow until their scratch fits 256 MB.
+    2M clustered points would take about 0.5 GB in the smallest groups.  The memory a call takes
+    beyond the same call without outputs at the sources is that scratch and the outputs in tree
+    order (64 bytes a point), at most 1/8 more for buffers rounded up; accuracy as ever."""
+    import torch
+    from test_gpu_serving import _pool
+    rng = np.random.default_rng(77)
+    n, k = 2000000, 200
+    src = rng.normal(size=(n, 3))
+    src *= (0.1 / np.sqrt(np.maximum(rng.random(n), 1e-9) ** (-2 / 3) - 1)).clip(0, 1)[:, None] / np.linalg.norm(
+        src, axis=1)[:, None]
+    q = rng.uniform(-1, 1, (n, 2))
+    d_src, d_q = torch.from_numpy(src).cuda(), torch.from_numpy(q).cuda()
+    out = [torch.empty((m, w), dtype=torch.float64, device="cuda") for m, w in ((n, 2), (n, 6), (1, 2), (1, 6))]
+    trg = torch.full((1, 3), 0.5, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+
+    def peak(*args):
+        assert F.hfmm3dparttarg_device(1, 6.0, d_src, d_q, None, None, *args) == 0, F.last_error()
+        torch.cuda.synchronize()
+        _pool("HIGH")
+        base = _pool("HIGH")
+        assert F.hfmm3dparttarg_device(1, 6.0, d_src, d_q, None, None, *args) == 0, F.last_error()
+        torch.cuda.synchronize()
+        return _pool("HIGH") - base
+
+    more = peak(out[0], out[1], trg, out[2], out[3]) - peak(None, None, trg, out[2], out[3])
+    assert more < (256 * 2 ** 20 + 64 * n) * 9 / 8
+    si = rng.choice(n, k, replace=False)
+    want = [torch.empty((k, w), dtype=torch.float64, device="cuda") for w in (2, 6)]
+    assert F.hdirect_points_device(6.0, d_src, d_q, None, None, d_src[si].contiguous(),
+                                   torch.from_numpy(si.astype(np.int32)).cuda(), *want) == 0
+    torch.cuda.synchronize()
+    for a, b in zip(out, want):
+        a = a[torch.from_numpy(si).cuda()]
+        assert float((a - b).norm() / b.norm()) < EPS[1]
