@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(kP2PHThreads) k_p2p_hess(const int *leaves, Tr
                 __syncthreads();
                 if (!act) continue;
                 const int selfk = self - (js0 + c0);
-                // the self pair adds exact zeros (no strength, unit distance)
+                // the self pair adds exact zeros: no strength and no direction (which may be infinite),
+                // unit distance
 #pragma unroll 2
                 for (int k = 0; k < cn; k++) {
                     const bool me = k == selfk;
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(kP2PHThreads) k_p2p_hess(const int *leaves, Tr
                     if (DIP) {
                         // 3 ds [ (v.d)(5 d d^T / r^2 - I) - (v d^T + d v^T) ] / r^5
                         const double2 d = me ? cmk(0, 0) : sd[k];
-                        const double vx = svx[k], vy = svy[k], vz = svz[k];
+                        const double vx = me ? 0.0 : svx[k], vy = me ? 0.0 : svy[k], vz = me ? 0.0 : svz[k];
                         const double dot = dx * vx + dy * vy + dz * vz;
                         const double f = 5 * dot * ri2, c3 = 3 * ri5;
                         const double t[6] = {c3 * (f * dx * dx - dot - 2 * vx * dx), c3 * (f * dy * dy - dot - 2 * vy * dy),

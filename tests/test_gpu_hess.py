@@ -180,3 +180,18 @@ def test_expansion_evaluator_refuses_order_above_the_table(F):
     assert F.evalhess_device("local", 1.0, np.zeros(3), coef, p, t, pot) == 16
     assert "nterms" in F.last_error()
     assert bool((pot == 7.0).all())
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_a_source_takes_no_hessian_from_itself_whatever_its_dipole(F, bad):
+    """A source's Hessian leaves its own dipole out, also one of infinite or undefined direction: the
+    same bits as with that direction zero (one leaf: the near field alone)."""
+    src, q, ds, dv, _ = inputs("cube", 70, 1, 8)
+    out = []
+    for v in (bad, 0.0):
+        dv[41] = v
+        got = F.lfmm3dparttarghess(1, src, 1, q, 1, ds, dv, 1, 1, 1)
+        assert got[0] == 0, F.last_error()
+        out.append([a[41] for a in got[1:4]])
+    for a, b in zip(*out):
+        assert np.all(np.isfinite(b)) and np.array_equal(a, b)
