@@ -798,9 +798,15 @@ static int lap_setup(LapSetup &S, int iprec, int ns, const double *d_src, int if
     // (the folded kernel indexes the multipoles with 32 bits)
     S.fold = plan->folded && (unsigned long long)(T.nboxes + 1) * K < 0xffffffffull &&
              (S.tcm2l ? sw(kSwTensorM2L) == 3 : !S.mixed && m2l_mode != 1 && m2l_mode != 3);
-    if (S.fold && T.nlev >= 2 && !fold_prepare(plan->fold, S.fw, T.nboxes, T.nboxes - T.lev_start[2], s, st)) {
-        g_ti.err = cudaGetErrorString(st.err);
-        return 16;
+    // Where the device has no room for the folded M2L's workspace (a third set of expansions and
+    // up to 256 MB), the kernels without one take its place: rotations, or split TF32 in the mixed form.
+    Status fst;
+    if (S.fold && T.nlev >= 2 && !fold_prepare(plan->fold, S.fw, T.nboxes, T.nboxes - T.lev_start[2], s, fst)) {
+        if (fst.err != cudaErrorMemoryAllocation) { g_ti.err = cudaGetErrorString(fst.err); return 16; }
+        cudaGetLastError();
+        S.fw.mr.release();
+        S.fw.lr.release();
+        S.fold = false;
     }
     // launch shapes: the autotuner's cached setting for this problem, else automatic
     S.signature = lap_signature(S);

@@ -140,3 +140,62 @@ def test_switch_override_is_per_thread(F):
     for a, b in zip(res["plain"][1], fp64):
         assert np.array_equal(a, b)
     assert lib.fmm3d_set_switch_thread(1, 2) == 1 and lib.fmm3d_set_switch_thread(7, 0) == 1
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_call_without_room_for_the_folded_m2l_takes_the_kernels_without_workspace(F, precision):
+    """The folded M2L needs a third set of expansions.  With the device's memory taken up so that the
+    rotations' call still fits and half of the difference is left, the call runs by the other kernels
+    (FP64: 1e-12 from the folded one, the two M2L forms' rounding; mixed form: 1e-5, the split TF32
+    products), and folded again, with the same bits, once there is room."""
+    import torch
+    from cuda.bindings import driver as drv
+    from test_gpu_serving import _pool
+    rng = np.random.default_rng(6)
+    n = 6000000
+    src, q = torch.from_numpy(rng.random((n, 3))).cuda(), torch.from_numpy(rng.uniform(-1, 1, (n, 2))).cuda()
+    outs = [[torch.empty((n, w), dtype=torch.float64, device="cuda") for w in (2, 6)] for _ in range(3)]
+    torch.cuda.synchronize()
+
+    def call(out):
+        ier = F.lfmm3dparttarg_device(1, src, q, None, None, *out)
+        torch.cuda.synchronize()
+        return ier, F.last_tuning()[0]["folded"], *out
+
+    def peak(out):
+        _pool("HIGH")
+        base = _pool("HIGH")
+        r = call(out)
+        assert r[0] == 0, F.last_error()
+        return _pool("HIGH") - base, r
+
+    F.set_precision(precision)
+    F.set_tensor_m2l(3)
+    try:
+        high, folded = peak(outs[0])
+        plain = F.set_tensor_m2l if precision else F.set_m2l_mode
+        try:
+            plain(1)
+            low, other = peak(outs[1])
+        finally:
+            plain(3 if precision else 0)
+        assert folded[1] and not other[1] and high - low > 2 ** 28
+        torch.cuda.empty_cache()
+        err, pool = drv.cuDeviceGetDefaultMemPool(0)
+        assert drv.cuMemPoolTrimTo(pool, 0)[0] == drv.CUresult.CUDA_SUCCESS
+        room = low + (high - low) // 2
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+        tight = call(outs[1])
+        del hog
+        torch.cuda.empty_cache()
+        assert tight[0] == 0, F.last_error()
+        assert not tight[1]
+        tol = 1e-5 if precision else 1e-12
+        for a, b in zip(tight[2:], folded[2:]):
+            assert float((a - b).norm() / b.norm()) < tol
+        again = call(outs[2])
+        assert again[0] == 0 and again[1]
+        for a, b in zip(again[2:], folded[2:]):
+            assert torch.equal(a, b)
+    finally:
+        F.set_precision(0)
