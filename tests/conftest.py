@@ -27,3 +27,17 @@ def pytest_collection_modifyitems(config, items):
     for it in items:
         if "gpu" in it.keywords:
             it.add_marker(skip)
+
+
+@pytest.fixture(autouse=True)
+def default_switches(request):
+    """Every GPU test starts from the library's default switches, whatever an earlier one left."""
+    yield
+    if "gpu" in request.keywords:
+        import fmmlib3d_b200 as F
+        F.set_precision(0)
+        F.set_precision_thread(-1)
+        F.set_m2l_mode(0)
+        F.set_tensor_m2l(3)
+        F.set_overlap(True)
+        F.set_tuning_cache(None)

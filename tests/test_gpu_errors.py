@@ -59,8 +59,10 @@ def _call(F, kernel, iprec, src, q, ds, dv, trg, fill=np.nan):
     return ier.value, outs
 
 
-@pytest.mark.parametrize("kernel,precision", [("laplace", 0), ("laplace", 1), ("helmholtz", 0)])
-def test_injected_allocation_failures_return_reference_codes(F, kernel, precision):
+@pytest.mark.parametrize("kernel,precision,tensor_m2l", [("laplace", 0, 3), ("laplace", 1, 3), ("laplace", 1, 1),
+                                                         ("helmholtz", 0, 3)])
+def test_injected_allocation_failures_return_reference_codes(F, kernel, precision, tensor_m2l):
+    F.set_tensor_m2l(tensor_m2l)
     args = _inputs(30000, 8000, 3)
     F.set_precision(precision)
     lib = F.lib()
@@ -170,7 +172,6 @@ def test_a_call_without_room_for_the_folded_m2l_takes_the_kernels_without_worksp
         return _pool("HIGH") - base, r
 
     F.set_precision(precision)
-    F.set_tensor_m2l(3)
     try:
         high, folded = peak(outs[0])
         plain = F.set_tensor_m2l if precision else F.set_m2l_mode

@@ -78,7 +78,7 @@ def test_tensor_m2l_within_twice_reference_error(F, mode, geom, iprec):
         F.set_tensor_m2l(mode)
         ier, pot, fld, pt, ft = F.lfmm3dparttarg(iprec, src, 1, q, 1, ds, dv, 1, 1, trg, 1, 1)
     finally:
-        F.set_tensor_m2l(1)
+        F.set_tensor_m2l(3)
         F.set_precision(0)
     assert ier == 0 and ref[0] == 0
     # same far field as the FP32 CUDA-core M2L up to FP32-level differences
@@ -124,6 +124,7 @@ def test_tensor_m2l_gate_on_adaptive_batch(F):
     """Mixed form with tensor-core M2L on a batch of adaptive instances (Plummer
     spheres and ellipsoid surfaces): error vs the FP64 direct sum at most 2x the FP64
     form's error on the same points (the FP64 form equals the oracle to rounding)."""
+    F.set_tensor_m2l(1)
     import torch
     rng = np.random.default_rng(44)
     srcs = []
@@ -142,6 +143,8 @@ def test_tensor_m2l_gate_on_adaptive_batch(F):
         F.set_precision(form)
         try:
             assert F.lfmm3dparttarg_batched_device(1, off, d_src, d_q, None, None, pot, fld) == 0
+            assert F.last_tuning()[0]["form"] == ("mixed-tc" if form else "fp64-dense")
+            assert F.last_tuning()[0]["folded"] == (form == 0)
         finally:
             F.set_precision(0)
         torch.cuda.synchronize()

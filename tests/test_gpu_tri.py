@@ -138,10 +138,14 @@ def test_sampled_direct_sum_matches_oracle(F):
     assert rel(g[0][si], op[:300]) < 1e-12 and rel(g[1][si], of[:300]) < 1e-12
 
 
+@pytest.mark.parametrize("tensor_m2l", [None, 1])
 @pytest.mark.parametrize("iprec", [0, 1])
-def test_mixed_form_within_twice_the_oracle_error(F, iprec):
-    """set_precision(1): the triangle FMM's M2L on the tensor cores (split TF32); the exact near
-    field stays FP64.  Errors against the direct sum within 2x the oracle's."""
+def test_mixed_form_within_twice_the_oracle_error(F, iprec, tensor_m2l):
+    """set_precision(1): the triangle FMM's M2L on the tensor cores (FP64 by default, split TF32 where
+    that is chosen); the exact near field stays FP64.  Errors against the direct sum within 2x the
+    oracle's."""
+    if tensor_m2l is not None:
+        F.set_tensor_m2l(tensor_m2l)
     T = two_spheres(4, 5)
     nrm, cen, q, ds, trg = _inputs(T, 30 + iprec)
     F.set_precision(1)
@@ -151,7 +155,7 @@ def test_mixed_form_within_twice_the_oracle_error(F, iprec):
     finally:
         F.set_precision(0)
     assert ier == 0, F.last_error()
-    assert tuning["form"] == "mixed-tc"
+    assert tuning["form"] == "mixed-tc" and tuning["folded"] == (tensor_m2l is None)
     oier, opot, ofld, opt, oft = O.lfmm3dtriatarg(iprec, T, nrm, cen, q, ds, trg)
     d = O.l3dtriadirect(T, cen, q, ds, trg)
     for a, o, ref in ((pot, opot, d[0]), (fld, ofld, d[1]), (pt, opt, d[2]), (ft, oft, d[3])):

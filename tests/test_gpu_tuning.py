@@ -43,19 +43,23 @@ def _outs(n, m):
     return out
 
 
-@pytest.mark.parametrize("precision,iprec,m2l_mode,form", [(1, 1, 0, "mixed-tc"), (0, 1, 0, "fp64-dense"),
-                                                           (0, 1, 1, "fp64-rotation"), (0, 2, 0, "fp64-rotation")])
-def test_every_setting_gives_the_same_bits(F, precision, iprec, m2l_mode, form):
+@pytest.mark.parametrize("precision,iprec,m2l_mode,form,tensor_m2l",
+                         [(1, 1, 0, "mixed-tc", None), (1, 1, 0, "mixed-tc", 1), (0, 1, 0, "fp64-dense", None),
+                          (0, 1, 1, "fp64-rotation", None), (0, 2, 0, "fp64-rotation", None)])
+def test_every_setting_gives_the_same_bits(F, precision, iprec, m2l_mode, form, tensor_m2l):
     import torch
     from fmmlib3d_b200 import autotune as A
     n, m = 24000, 9000
     src, trg, q, d, v = _problem(n, m, 100 + 10 * precision + iprec + 3 * m2l_mode)
     F.set_precision(precision)
+    if tensor_m2l is not None:
+        F.set_tensor_m2l(tensor_m2l)
     F.set_m2l_mode(m2l_mode)
     F.set_tuning_cache("")
     plan = F.LaplacePlan(iprec, src, 1, 1, 1, 1, trg, 1, 1)
     t = plan.get_tuning()
     assert t["form"] == form and not t["from_cache"]
+    assert t["folded"] == (m2l_mode == 0 and tensor_m2l is None)
     ref = _outs(n, m)
     assert plan.execute(q, d, v, *ref, use_graph=False) == 0
     torch.cuda.synchronize()
