@@ -637,13 +637,13 @@ __device__ __forceinline__ PtGeo pt_geo(double dx, double dy, double dz)
 // (h3dformmp_add_trunc / h3dformta_add_trunc, src/helmrouts3d.f:2972, 3299;
 // dipoles h3dformmp_dp_add_trunc :3580, h3dformta_dp_add_trunc :3978).
 constexpr int kHFormThreads = 256, kHFormPer = 3;
-// Source set-up in batches of kHFormSetA x kHFormSetCH (32) sources, tables per kHFormSetCH.
+// Source set-up in batches of kHFormSetA x kHFormSetCH (32) or twice as many sources, tables per kHFormSetCH.
 constexpr int kHFormSetCH = 8, kHFormSetA = 4;
 
 template <int CH, bool DIP, int AX = 1>
 struct HFormSmem {
     // sizes in doubles for expansion order p
-    static __host__ __device__ size_t doubles(int p)
+    static constexpr __host__ __device__ size_t doubles(int p)
     {
         size_t W = p + 2, T = (size_t)(p + 1) * (p + 2) / 2;
         size_t d = AX * CH * (2 * W + 2 * (p + 1) + (p + 1) + 16) + CH * T;  // f, e^{-im phi}, diagonal, scalars; Y
@@ -855,12 +855,14 @@ void launch_hform(bool irreg, const int *boxes, int nboxes, const TreeView &tv, 
         FMM_COUNT_LAUNCH();                                                                                   \
     } while (0)
 #define FMM_HF(IR, C, D, CHV) FMM_HF2(IR, C, D, CHV, 1)
-    // chunks of 8 or 16 sources; 4, 2 or 1 at orders whose staging would not
-    // fit (above ~54, ~80, ~110).  The chunk size does not change the order of
-    // any sum.
-    // The sources' set-up (phase A) runs one thread per source, so it takes 32 sources
-    // at a time where that fits two CTAs per SM (the tables stay per 8 sources; phases
-    // B and C walk the four sub-chunks in order, so no sum changes order).
+    // The sources' set-up (phase A) runs one thread per source, so it takes 64 or 32 sources
+    // at a time where that fits two CTAs per SM: up to orders 28 and 40, with dipoles 16
+    // and 25 (the tables stay per 8 sources; phases B and C walk the sub-chunks in
+    // order).  Above, chunks of 16 sources (8 with dipoles) up to order 53 (54), of 4 up to 113
+    // (79), of 2.  Without dipoles each chunk's sums are added as four real ones, so
+    // the chunk of an order, which depends on nothing else, is part of its rounding.
+    static_assert(sizeof(double) * HFormSmem<2, true>::doubles(kHelmMaxP) <= 226 * 1024,
+                  "two sources' tables of the largest order in shared memory");
 #define FMM_HF_FIT(IR, C, D, CHV)                                                                             \
     do {                                                                                                      \
         if (sizeof(double) * HFormSmem<kHFormSetCH, D, 2 * kHFormSetA>::doubles(pm) <= 110 * 1024)           \
@@ -869,8 +871,7 @@ void launch_hform(bool irreg, const int *boxes, int nboxes, const TreeView &tv, 
             FMM_HF2(IR, C, D, kHFormSetCH, kHFormSetA);                                                       \
         else if (sizeof(double) * HFormSmem<CHV, D>::doubles(pm) <= 226 * 1024) FMM_HF(IR, C, D, CHV);      \
         else if (sizeof(double) * HFormSmem<4, D>::doubles(pm) <= 226 * 1024) FMM_HF(IR, C, D, 4);          \
-        else if (sizeof(double) * HFormSmem<2, D>::doubles(pm) <= 226 * 1024) FMM_HF(IR, C, D, 2);          \
-        else FMM_HF(IR, C, D, 1);                                                                             \
+        else FMM_HF(IR, C, D, 2);                                                                             \
     } while (0)
     if (irreg) {
         if (c && d) FMM_HF_FIT(true, true, true, 8);
@@ -887,12 +888,12 @@ void launch_hform(bool irreg, const int *boxes, int nboxes, const TreeView &tv, 
     FMM_LAUNCH_CHECK(st);
 }
 
-// L2P (h3dtaeval_trunc0, src/helmrouts3d.f:2732) at the leaf's own local
-// expansion when its level is >= 2, and M2P (h3dmpeval_trunc0, :2405) of the
-// multipoles of its list-3 boxes, at the leaf's sources and targets.  CTA per
-// leaf, one evaluation point per thread; per expansion the coefficients are
+// L2P (h3dtaeval_trunc0, src/helmrouts3d.f:2732) of the leaf's own local
+// expansion when its level is >= 2, at the leaf's sources and targets, for the
+// orders whose tables k_hl2p cannot hold.  CTA per
+// leaf, one evaluation point per thread; the coefficients are
 // staged in shared memory and read by all threads of a warp at once
-// (broadcast), each thread keeps its point's radial functions in a shared
+// (broadcast), each thread keeps its point's Bessel functions in a shared
 // column, and walks the orders m (outer) and degrees n (inner) with the
 // Legendre column recurrence in registers.
 constexpr int kHEvalThreads = 128, kHM2PThreads = 64;
@@ -903,14 +904,13 @@ template <int T>
 __global__ void __launch_bounds__(T) k_heval(const int *leaves, TreeView tv, const double *sx,
                                                         const double *sy, const double *sz, const double *tx,
                                                         const double *ty, const double *tz, HLevels lv, int NC,
-                                                        double2 zk, const double2 *mpole, const double2 *local,
-                                                        OutSoA outs, OutSoA outt, int do_src, int do_trg,
-                                                        int with_l3)
+                                                        double2 zk, const double2 *local, OutSoA outs, OutSoA outt,
+                                                        int do_src, int do_trg)
 {
     extern __shared__ double2 hsm[];
     const int b = leaves[blockIdx.x];
-    const int blev = tv.level[b];
-    if (!with_l3 && blev < 2) return;
+    const int lev = tv.level[b];
+    if (lev < 2) return;
     const int ns = do_src ? tv.nsrc[b] : 0, nt = do_trg ? tv.ntrg[b] : 0, ne = ns + nt;
     if (ne == 0) return;
     const int pm = max_p(lv);
@@ -918,108 +918,82 @@ __global__ void __launch_bounds__(T) k_heval(const int *leaves, TreeView tv, con
     double2 *E = hsm;
     double2 *Fs = hsm + KM;  // radial functions, [n][thread]
     const int t = threadIdx.x;
-    const int l3a = tv.l3_start[b], nl3 = with_l3 ? tv.l3_start[b + 1] - l3a : 0;
+    const int p = lv.p[lev], K = (p + 1) * (p + 1);
+    const double sc = lv.sc[lev];
+    const double *c = tv.center + 3L * b;
+    for (int i = t; i < K; i += T) E[i] = local[(size_t)b * NC + i];
+    __syncthreads();
     // CTA (leaf, y) serves the leaf's point chunks y, y + gridDim.y, ... of T points
-    for (int c0 = blockIdx.y * T; c0 < ne; c0 += gridDim.y * T)
-    for (int xi = -1; xi < nl3; xi++) {
-        int eb;
-        const bool isloc = xi < 0;
-        if (isloc) {
-            if (blev < 2) continue;
-            eb = b;
-        } else {
-            eb = tv.l3_idx[l3a + xi];
-            if (tv.nsrc[eb] == 0) continue;
-        }
-        const int lev = tv.level[eb], p = lv.p[lev];
-        const double sc = lv.sc[lev];
-        const int K = (p + 1) * (p + 1);
-        const double2 *ex = (isloc ? local : mpole) + (size_t)eb * NC;
-        __syncthreads();
-        for (int i = t; i < K; i += T) E[i] = ex[i];
-        __syncthreads();
-        const double *c = tv.center + 3L * eb;
-        {
-            const int e = c0 + t;
-            if (e >= ne) continue;
-            const bool is_src = e < ns;
-            const int i = is_src ? tv.src0[b] + e : tv.trg0[b] + e - ns;
-            double px = is_src ? sx[i] : tx[i], py = is_src ? sy[i] : ty[i], pz = is_src ? sz[i] : tz[i];
-            const PtGeo g = pt_geo(px - c[0], py - c[1], pz - c[2]);
-            double2 *f = Fs + t;
-            const double2 z = cscal(g.r, zk);
-            if (isloc) {
-                if (bess_dev(p > 1 ? p : 1, z, sc, f, nullptr, T)) continue;
-            } else {
-                if (cabsd(z) < 1.0e-15) continue;
-                hank_dev(p > 1 ? p : 1, z, sc, f, nullptr, T);
-            }
-            const double r = g.r, ct = g.ct, st = g.st, u = -st;
-            const double isc = 1.0 / sc, ir = 1.0 / r;
-            const double2 zi = cdiv(cmk(1, 0), z), e1 = cmk(g.cp, g.sp);
-            double2 pot = cmk(0, 0), ur = cmk(0, 0), ut = cmk(0, 0), up = cmk(0, 0);
-            double2 em = cmk(1, 0);
-            double ymm = 1.0;
-            for (int m = 0; m <= p; m++) {
-                if (m == 1) ymm = -sqrt(0.5);
-                else if (m > 1) ymm *= u * __ldg(&g_hc[m]);
-                if (m > 0) em = cmul(em, e1);
-                LegCol L;
-                L.x = ct;
-                L.m = m;
-                L.w = m == 0 ? 1.0 : u * u;
-                L.y1 = ymm;
-                L.d1 = m == 0 ? 0.0 : ymm * (-m) * ct;
-                L.y2 = 0;
-                L.d2 = 0;
-                for (int n = m; n <= p; n++) {
-                    if (n > m) L.step(n);
-                    const double sn = __ldg(&g_hs[n]);
-                    const double y = L.y1 * sn, dd = L.d1 * sn;
-                    const double2 fn = f[n * T];
-                    double2 fd, fu;
-                    if (isloc) {
-                        if (n == 0) { fd = cscal(-sc, f[T]); fu = cmk(0, 0); }
-                        else {
-                            // j_n' = [n j_{n-1} - (n+1) j_{n+1}] / (2n+1) in the scaled functions
-                            const double2 fm = f[(n - 1) * T], fp = f[(n + 1) * T];
-                            const double d1 = __ldg(&g_hq[n]), d2 = 1.0 - d1;
-                            fd = csub(cscal(d1 * isc, fm), cscal(d2 * sc, fp));
-                            fu = cscal(__ldg(&g_hr[n]), cmul(zk, cadd(cscal(sc, fp), cscal(isc, fm))));
-                        }
-                    } else {
-                        fd = n == 0 ? cscal(-isc, f[T]) : csub(cscal(sc, f[(n - 1) * T]), cmul(cscal(n + 1.0, zi), fn));
-                        fu = cscal(ir, fn);
-                    }
-                    fd = cmul(fd, zk);
-                    if (m == 0) {
-                        const double2 a = E[eidx(n, 0)];
-                        cfma(pot, fn, cscal(y, a));
-                        cfma(ur, fd, cscal(y, a));
-                        cfma(ut, fu, cscal(-dd * st, a));
-                    } else {
-                        const double2 z2 = cmul(E[eidx(n, m)], em), z3 = cmul(E[eidx(n, -m)], cconj(em));
-                        const double2 zs = cadd(z2, z3), zd = csub(z2, z3);
-                        cfma(pot, fn, cscal(y * st, zs));
-                        cfma(ur, fd, cscal(y * st, zs));
-                        cfma(ut, fu, cscal(-dd, zs));
-                        cfma(up, fu, cscal(y * m, cmk(-zd.y, zd.x)));  // i m (z2 - z3)
-                    }
+    for (int c0 = blockIdx.y * T; c0 < ne; c0 += gridDim.y * T) {
+        const int e = c0 + t;
+        if (e >= ne) continue;
+        const bool is_src = e < ns;
+        const int i = is_src ? tv.src0[b] + e : tv.trg0[b] + e - ns;
+        double px = is_src ? sx[i] : tx[i], py = is_src ? sy[i] : ty[i], pz = is_src ? sz[i] : tz[i];
+        const PtGeo g = pt_geo(px - c[0], py - c[1], pz - c[2]);
+        double2 *f = Fs + t;
+        const double2 z = cscal(g.r, zk);
+        if (bess_dev(p > 1 ? p : 1, z, sc, f, nullptr, T)) continue;
+        const double ct = g.ct, st = g.st, u = -st;
+        const double isc = 1.0 / sc;
+        const double2 e1 = cmk(g.cp, g.sp);
+        double2 pot = cmk(0, 0), ur = cmk(0, 0), ut = cmk(0, 0), up = cmk(0, 0);
+        double2 em = cmk(1, 0);
+        double ymm = 1.0;
+        for (int m = 0; m <= p; m++) {
+            if (m == 1) ymm = -sqrt(0.5);
+            else if (m > 1) ymm *= u * __ldg(&g_hc[m]);
+            if (m > 0) em = cmul(em, e1);
+            LegCol L;
+            L.x = ct;
+            L.m = m;
+            L.w = m == 0 ? 1.0 : u * u;
+            L.y1 = ymm;
+            L.d1 = m == 0 ? 0.0 : ymm * (-m) * ct;
+            L.y2 = 0;
+            L.d2 = 0;
+            for (int n = m; n <= p; n++) {
+                if (n > m) L.step(n);
+                const double sn = __ldg(&g_hs[n]);
+                const double y = L.y1 * sn, dd = L.d1 * sn;
+                const double2 fn = f[n * T];
+                double2 fd, fu;
+                if (n == 0) { fd = cscal(-sc, f[T]); fu = cmk(0, 0); }
+                else {
+                    // j_n' = [n j_{n-1} - (n+1) j_{n+1}] / (2n+1) in the scaled functions
+                    const double2 fm = f[(n - 1) * T], fp = f[(n + 1) * T];
+                    const double d1 = __ldg(&g_hq[n]), d2 = 1.0 - d1;
+                    fd = csub(cscal(d1 * isc, fm), cscal(d2 * sc, fp));
+                    fu = cscal(__ldg(&g_hr[n]), cmul(zk, cadd(cscal(sc, fp), cscal(isc, fm))));
+                }
+                fd = cmul(fd, zk);
+                if (m == 0) {
+                    const double2 a = E[eidx(n, 0)];
+                    cfma(pot, fn, cscal(y, a));
+                    cfma(ur, fd, cscal(y, a));
+                    cfma(ut, fu, cscal(-dd * st, a));
+                } else {
+                    const double2 z2 = cmul(E[eidx(n, m)], em), z3 = cmul(E[eidx(n, -m)], cconj(em));
+                    const double2 zs = cadd(z2, z3), zd = csub(z2, z3);
+                    cfma(pot, fn, cscal(y * st, zs));
+                    cfma(ur, fd, cscal(y * st, zs));
+                    cfma(ut, fu, cscal(-dd, zs));
+                    cfma(up, fu, cscal(y * m, cmk(-zd.y, zd.x)));  // i m (z2 - z3)
                 }
             }
-            // fld = -(ur r-hat + ut theta-hat + up phi-hat)
-            const double cp = g.cp, sp = g.sp;
-            const double2 fx = cadd(cadd(cscal(st * cp, ur), cscal(ct * cp, ut)), cscal(-sp, up));
-            const double2 fy = cadd(cadd(cscal(st * sp, ur), cscal(ct * sp, ut)), cscal(cp, up));
-            const double2 fz = csub(cscal(ct, ur), cscal(st, ut));
-            double2 *po = is_src ? outs.pot : outt.pot;
-            double2 *ox = is_src ? outs.fx : outt.fx, *oy = is_src ? outs.fy : outt.fy, *oz = is_src ? outs.fz : outt.fz;
-            if (po) po[i] = cadd(po[i], pot);
-            if (ox) {
-                ox[i] = csub(ox[i], fx);
-                oy[i] = csub(oy[i], fy);
-                oz[i] = csub(oz[i], fz);
-            }
+        }
+        // fld = -(ur r-hat + ut theta-hat + up phi-hat)
+        const double cp = g.cp, sp = g.sp;
+        const double2 fx = cadd(cadd(cscal(st * cp, ur), cscal(ct * cp, ut)), cscal(-sp, up));
+        const double2 fy = cadd(cadd(cscal(st * sp, ur), cscal(ct * sp, ut)), cscal(cp, up));
+        const double2 fz = csub(cscal(ct, ur), cscal(st, ut));
+        double2 *po = is_src ? outs.pot : outt.pot;
+        double2 *ox = is_src ? outs.fx : outt.fx, *oy = is_src ? outs.fy : outt.fy, *oz = is_src ? outs.fz : outt.fz;
+        if (po) po[i] = cadd(po[i], pot);
+        if (ox) {
+            ox[i] = csub(ox[i], fx);
+            oy[i] = csub(oy[i], fy);
+            oz[i] = csub(oz[i], fz);
         }
     }
 }
@@ -1403,13 +1377,12 @@ void launch_hl2p(const int *leaves, int nleaves, const TreeView &tv, const doubl
     } else if (sm <= 226 * 1024) {
         FMM_TRY(st, smem_allow(k_heval<kHEvalThreads>, (int)sm));
         k_heval<kHEvalThreads><<<dim3(nleaves, 2), kHEvalThreads, sm, s>>>(leaves, tv, sx, sy, sz, tx, ty, tz, lv,
-                                                                           NC, zk, nullptr, local, outs, outt, do_src,
-                                                                           do_trg, 0);
+                                                                           NC, zk, local, outs, outt, do_src, do_trg);
     } else {
         sm = sizeof(double2) * ((size_t)(pm + 1) * (pm + 1) + (size_t)(pm + 2) * 32);
         FMM_TRY(st, smem_allow(k_heval<32>, (int)sm));
-        k_heval<32><<<dim3(nleaves, 8), 32, sm, s>>>(leaves, tv, sx, sy, sz, tx, ty, tz, lv, NC, zk, nullptr, local,
-                                                     outs, outt, do_src, do_trg, 0);
+        k_heval<32><<<dim3(nleaves, 8), 32, sm, s>>>(leaves, tv, sx, sy, sz, tx, ty, tz, lv, NC, zk, local, outs, outt,
+                                                     do_src, do_trg);
     }
     FMM_COUNT_LAUNCH();
     FMM_LAUNCH_CHECK(st);

@@ -197,15 +197,15 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
             if (free_ >> i & 1) axis[bits++] = i;
         int most = 0;
         for (int c = 0; c < 8; c++) most = std::max(most, cnt[c][o.pt]);
-        const int kcap = bits == 1 ? 32 : kFoldCap;   // (four column classes a round: 32 tasks)
+        // (kFoldCap rows of at most four column classes a round: at most kFoldMaxTask tasks)
         open_cls = q;
         for (int r = 0; r < 1 << bits; r++)
-            for (int k0 = 0; k0 < most; k0 += kcap) {
+            for (int k0 = 0; k0 < most; k0 += kFoldCap) {
                 int rb = 0;   // the round's column classes: these bits on the free axes, any on the others
                 for (int i = 0; i < bits; i++) rb |= (r >> i & 1) << axis[i];
                 int depth = 0, ntask = 0;
                 for (int be = 0; be < 8; be++) {
-                    const int nb = (be & free_) == rb ? std::min(cnt[be][o.pt] - k0, kcap) : 0;
+                    const int nb = (be & free_) == rb ? std::min(cnt[be][o.pt] - k0, kFoldCap) : 0;
                     if (nb <= 0) continue;
                     depth = std::max(depth, 4 * div_up(nb, 4));
                     ntask += div_up(nb, 4);
@@ -223,7 +223,7 @@ bool fold_build(FoldPlan &F, int p, const FoldOffset *off, const double *rot, co
                 // staging tasks: the round's column classes, 4 coefficients each, zeros up to the depth
                 for (int be = 0; be < 8; be++) {
                     if ((be & free_) != rb) continue;
-                    const int nb = std::max(0, std::min(cnt[be][o.pt] - k0, kcap));
+                    const int nb = std::max(0, std::min(cnt[be][o.pt] - k0, kFoldCap));
                     for (int k = 0; k < nb; k += 4) {
                         FoldTask t = {};
                         t.src0 = (unsigned short)(base[be] + k0 + k);
