@@ -289,6 +289,14 @@ __global__ void k_split_c(int n, const double *c, double2 *o)
     if (i < n) o[i] = make_double2(c[2L * i], c[2L * i + 1]);
 }
 
+int device_sms()
+{
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 148;
+}
+
 cudaError_t smem_allow_fn(const void *func, size_t bytes)
 {
     int dev = 0;

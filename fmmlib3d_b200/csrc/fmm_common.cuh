@@ -149,6 +149,8 @@ struct DBuf {
     }
 };
 
+int device_sms();   // multiprocessors of the current device
+
 inline int div_up(long a, long b) { return (int)((a + b - 1) / b); }
 
 // ---------------------------------------------------------------- scan / sort utilities (scan_sort.cu)

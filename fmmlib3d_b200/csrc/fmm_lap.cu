@@ -356,14 +356,6 @@ __global__ void k_m2l_count(int b0, int nb, TreeView tv, const Slot *slots, int 
         if (h[i]) atomicAdd(&hist[i], (unsigned long long)h[i]);
 }
 
-static int device_sms()
-{
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 148;
-}
-
 // ---------------------------------------------------------------- one evaluation geometry
 // Device state of a Laplace evaluation for fixed sources and targets: tree and
 // lists, tree-ordered coordinates, expansion and output workspace, translation

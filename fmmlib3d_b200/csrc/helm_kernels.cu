@@ -519,7 +519,7 @@ void launch_htranslate(int kind, const Tile *tiles, int ntiles, const int *group
     DBuf<double2> gs;
     if (sm > kHTransSmemMax) {
         // high orders: the three buffers in global scratch, one slice per CTA of a grid-stride launch
-        grid = std::min(ntiles, 2 * 148);
+        grid = std::min(ntiles, 2 * device_sms());
         if (!gs.alloc((size_t)grid * 3 * kt * NC, s, st)) return;
         sm = (pmax + 1) * sizeof(double2);
     }
@@ -1724,7 +1724,7 @@ void launch_hdirect(int nsrc, const PointsSoA &src, int ifcharge, int ifdipole, 
     bool c = ifcharge == 1, d = ifdipole == 1;
     int gx = div_up(neval, kHDirThreads);
     // enough source chunks to fill the GPU (about 4 CTAs per SM), at least 1024 sources each
-    int nchunk = std::max(1, std::min(div_up(std::max(nsrc, 1), 1024), div_up(148 * 4, gx)));
+    int nchunk = std::max(1, std::min(div_up(std::max(nsrc, 1), 1024), div_up(4 * device_sms(), gx)));
     int chunk = div_up(std::max(nsrc, 1), nchunk);
     nchunk = div_up(std::max(nsrc, 1), chunk);
     DBuf<double2> part;

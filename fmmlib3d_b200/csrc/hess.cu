@@ -636,10 +636,7 @@ void launch_expeval_hess(bool loc, double rscale, const double *center, const do
     const size_t smem = per_phase * arr;
     FMM_TRY(st, smem_allow(k_expeval_hess, (int)smem));
     if (!st.ok()) return;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = std::max(1, std::min((npts + kExpEvalThreads - 1) / kExpEvalThreads, 4 * sms));
+    const int grid = std::max(1, std::min((npts + kExpEvalThreads - 1) / kExpEvalThreads, 4 * device_sms()));
     k_expeval_hess<<<grid, kExpEvalThreads, smem, s>>>(loc ? 1 : 0, rscale, center[0], center[1], center[2], coef,
                                                         nterms, npts, pts, pot, f ? fld : nullptr, h ? hess : nullptr,
                                                         nk, per_phase);

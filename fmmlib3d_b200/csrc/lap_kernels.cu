@@ -359,7 +359,7 @@ static void launch_p2p_t(const NearArgs &A, cudaStream_t s, Status &st)
     // warps: 2M + 2M cube (32,768 leaves) 19.5 against 20.1 ms, 1M + 1M cube (4,096)
     // 34.6 / 34.9; 100k sphere (1,489) 0.41 / 0.38, 64 leaves 0.13 / 0.08 ms.  The
     // line is the 16 warps a multiprocessor holds, on all of them.
-    if (A.nleaves >= 16 * 148)
+    if (A.nleaves >= 16 * device_sms())
         k_p2p<CHG, DIP, 2, 1, 8><<<dim3(ctas, 4), 32 * kNearWarps, 0, s>>>(A);
     else
         k_p2p<CHG, DIP, 1, 2, 1><<<dim3(ctas, 8), 32 * kNearWarps, 0, s>>>(A);
@@ -484,7 +484,7 @@ void launch_direct_split(int nsrc, const double *sx, const double *sy, const dou
 {
     if (neval == 0 || !st.ok()) return;
     int gx = div_up(neval, kP2PThreads);
-    int nchunk = std::max(1, std::min(div_up(4 * 148, gx), div_up(nsrc, 4096)));
+    int nchunk = std::max(1, std::min(div_up(4 * device_sms(), gx), div_up(nsrc, 4096)));
     int chunk = div_up(nsrc, nchunk);
     nchunk = div_up(nsrc, chunk);
     DBuf<double2> part;

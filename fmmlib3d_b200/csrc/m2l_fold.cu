@@ -51,13 +51,16 @@ constexpr int kFoldCap = 32;                    // operand rows per parity class
 // lanes of a half warp reading a fragment meet different banks.
 template <int NT>
 constexpr int kFoldLd = 2 * NT + 4;
-// Fewer tiles than this (two for each of 148 multiprocessors): one CTA per group.  M2L, one
+// Fewer tiles than two for each multiprocessor: one CTA per group.  M2L at 148, one
 // CTA per tile against one per (tile, group): 4 tiles 0.35 / 0.062 ms, 111 tiles 0.36 /
 // 0.29, 292 tiles 0.78 / 0.80, 1,390 tiles 3.42 / 3.58, 2,330 tiles 6.0 / 6.5.
-// Tiles of 8 targets (above order 14, one CTA per multiprocessor) always run per group: eight
+// Tiles of 8 targets (above order 15, one CTA per multiprocessor) always run per group: eight
 // times the CTAs even out the tiles at a domain's faces.  Order 26: 585 tiles 4.83 /
 // 4.53, 4,681 tiles 38.9 / 35.7, with the groups' sums held to 256 MB at a time.
-constexpr int kFoldSplitTiles = 296;
+static bool fold_split(const FoldPlan &F, int count)
+{
+    return F.tile == 8 || div_up(count, F.tile) < 2 * device_sms();
+}
 
 // ---------------------------------------------------------------- operators
 struct FoldBlock {
@@ -645,7 +648,7 @@ __global__ void __launch_bounds__(256 + 32 * SW, 1) k_m2l_fold(FoldView f, TreeV
 bool fold_prepare(const FoldPlan &F, FoldWork &W, int nboxes, int count, cudaStream_t s, Status &st)
 {
     if (count <= 0) return true;
-    W.slots = F.tile == 8 || div_up(count, F.tile) < kFoldSplitTiles ? kFoldGroups : 1;
+    W.slots = fold_split(F, count) ? kFoldGroups : 1;
     // at most 256 MB of sums at a time
     const long long most = std::max<long long>((1LL << 28) / (16LL * F.K * W.slots) / F.tile, 1) * F.tile;
     W.chunk = (int)std::min<long long>(count, most);
