@@ -36,7 +36,7 @@ __device__ __forceinline__ double box_side(const TreeView &tv, int b)
 }
 
 // Steps of degree <= nmax: for each t, the degrees 4 t .. nmax.
-__host__ __device__ inline int emm_steps(int nmax)
+__host__ __device__ constexpr int emm_steps(int nmax)
 {
     int s = 0;
     for (int t = 0; 4 * t <= nmax; t++) s += nmax - 4 * t + 1;
@@ -45,7 +45,7 @@ __host__ __device__ inline int emm_steps(int nmax)
 
 // Doubles of shared memory for degrees up to nmax and nc column blocks of 8:
 // columns, recurrence factors, diagonal factors and the step table.
-__host__ __device__ inline size_t emm_smem(int nmax, int nc)
+__host__ __device__ constexpr size_t emm_smem(int nmax, int nc)
 {
     const size_t s = emm_steps(nmax);
     return s * 8 * 8 * nc + s * 8 + nmax + 1 + (s + 1) / 2;

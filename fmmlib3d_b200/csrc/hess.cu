@@ -308,7 +308,7 @@ __device__ __forceinline__ void stage_phase(bool loc, int p, int first, int n, c
 }
 
 // ---------------------------------------------------------------- far field of the FMM
-// (orders above 34, whose two column blocks exceed shared memory: a CTA per leaf, one point per thread)
+// (orders above 36, whose two column blocks exceed shared memory: a CTA per leaf, one point per thread)
 constexpr int kEvalHThreads = 128;
 
 __global__ void __launch_bounds__(kEvalHThreads) k_eval_hess(const int *leaves, TreeView tv, const double *sx,
@@ -398,6 +398,9 @@ __global__ void k_emm_hess_tables(int p, int nstep, double2 *ab, double *cm, int
                 (loc ? fl : fm)[(2 * i + sg) * 5 + c] = v;
             }
 }
+
+static_assert(sizeof(double) * emm_smem(36 + 2, 2) <= kEmmSmemMax && sizeof(double) * emm_smem(37 + 2, 2) > kEmmSmemMax,
+              "largest order of k_eval_hess_mm");
 
 void build_emm_hess_tables(int p, EmmTables &E, cudaStream_t s, Status &st)
 {

@@ -1165,7 +1165,7 @@ __device__ __forceinline__ void eval_point(bool loc, int p, double ux, double uy
 // the scratch offsets (soff) come from k_eval_count and two scans, made with
 // the tree.
 //
-// k_eval_mm serves the orders whose columns fit shared memory (p <= 51).  k_eval, above
+// k_eval_mm serves the orders whose columns fit shared memory (p <= 52).  k_eval, above
 // them: the potential and z-gradient first, then the transverse gradients, each
 // point's harmonics generated once per phase, one point per thread.
 __global__ void k_eval_count(const int *leaves, int nleaves, TreeView tv, int do_src, int do_trg, int *cnt,
@@ -1222,6 +1222,9 @@ __global__ void k_emm_tables(int p, int nstep, double2 *ab, double *cm, int *ste
         }
     }
 }
+
+static_assert(sizeof(double) * emm_smem(52 + 1, 1) <= kEmmSmemMax && sizeof(double) * emm_smem(53 + 1, 1) > kEmmSmemMax,
+              "largest order of k_eval_mm");
 
 void build_emm_tables(int p, EmmTables &E, cudaStream_t s, Status &st)
 {

@@ -27,7 +27,7 @@
 // all 32 columns, with its rows.  Offset classes
 // that no target of the tile has a source in are skipped.
 // The sums of a target are formed in 8 fixed groups of batches, added in
-// order; a small problem, or one above order 14, runs one CTA per (tile, group) and
+// order; a small problem, or one above order 15, runs one CTA per (tile, group) and
 // adds the groups afterwards, with the same result bit for bit.
 //
 // Bound: latency of the fragments and source rows in L2 (DMMA pipe 30% busy, long
@@ -682,7 +682,7 @@ void launch_m2l_fold(const FoldPlan &F, const FoldWork &W, const TreeView &tv, i
     FoldView f;
     f.base = F.base.p; f.cls = F.cls.p; f.tasks = F.tasks.p; f.batches = F.batches.p; f.runs = F.runs.p;
     f.A = F.A.p; f.group = F.group.p; f.K = F.K;
-    // row blocks of the largest parity class: orders <= 6, <= 9, <= 14, above
+    // row blocks of the largest parity class: orders <= 5, <= 9, <= 15, above (up to 14 at kFoldMaxP)
     if (F.rows <= 1) launch_fold_t<1, 16, 8>(F, f, W, tv, first, count, out, prune, s, st);
     else if (F.rows <= 2) launch_fold_t<2, 16, 8>(F, f, W, tv, first, count, out, prune, s, st);
     else if (F.rows <= 5) launch_fold_t<5, 16, 8>(F, f, W, tv, first, count, out, prune, s, st);
